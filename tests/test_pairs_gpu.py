@@ -291,3 +291,19 @@ def test_band_reduction_wait_timeout_is_reported_and_the_plan_recovers():
         plan.close()
     finally:
         c.close()
+
+
+@pytest.mark.parametrize("kw,n,nel,mult", [("COV", 8, 8, 3), ("COV", 9, 2, 1), ("COV", 10, 4, 1), ("COV", 11, 11, 4),
+                                           ("COV", 12, 12, 3), ("COV", 13, 13, 4)])
+def test_wide_complements_take_the_frame_kernel(ctx, kw, n, nel, mult):
+    """Strings of k electrons with up to eight empty orbitals, more than a closed shell has (open
+    shells: 5 + 3, 7 + 4, 7 + 5, 8 + 5 electrons; one and two electrons over nine and ten
+    orbitals): well-conditioned overlaps leave (almost) nothing to the exact path, and the
+    structure matrices match the oracle."""
+    S, h, eri = workloads.active_space(n, 2 * n, 60 + n)
+    plan, ex = _plan(ctx, kw, n, nel, mult)
+    H, So = plan.execute(S, h, eri)
+    Hr, Sr, _ = O.structure_matrices(n, ex, S, h, eri)
+    assert _rel(H, Hr) < REL and _rel(So, Sr) < REL
+    st = plan.stats()
+    assert st["careful_spin_pairs"] <= st["spin_pairs"] // 100

@@ -264,10 +264,17 @@ vb_status vb_hs_plan_create(vb_context* ctx, const vb_expansion* ex, vb_hs_plan*
         DeviceBuffer& rd = beta ? p->rdesc_b : p->rdesc_a;
         DeviceBuffer& eb = beta ? p->ebound_b : p->ebound_a;
         DeviceBuffer& tb = beta ? p->tables_b : p->tables_a;
-        if ((st = rl.allocate(ctx, sizeof(int) * (size_t)std::max(1LL, N * (N + 1) / 2))) != VB_OK) return fail(st);
-        if ((st = rd.allocate(ctx, sizeof(unsigned) * (size_t)std::max(1LL, N * (N + 1) / 2))) != VB_OK) return fail(st);
-        if ((st = eb.allocate(ctx, sizeof(int) * (size_t)N * (k + 2))) != VB_OK) return fail(st);
-        if ((st = tb.allocate(ctx, sizeof(double) * frame_table_doubles(n, k, p->np) * N)) != VB_OK) return fail(st);
+        st = rl.allocate(ctx, sizeof(int) * (size_t)std::max(1LL, N * (N + 1) / 2));
+        if (st == VB_OK) st = rd.allocate(ctx, sizeof(unsigned) * (size_t)std::max(1LL, N * (N + 1) / 2));
+        if (st == VB_OK) st = eb.allocate(ctx, sizeof(int) * (size_t)N * (k + 2));
+        if (st == VB_OK) st = tb.allocate(ctx, sizeof(double) * frame_table_doubles(n, k, p->np) * N);
+        if (st == VB_ERR_BUDGET && frame_wide_complement(n, k)) {
+            // a budget without room for the tables leaves an open-shell table on the exact path,
+            // which needs none of these
+            for (DeviceBuffer* b : {&rl, &rd, &eb, &tb}) b->release();
+            continue;
+        }
+        if (st != VB_OK) return fail(st);
         const cudaError_t err = launch_sort_right_strings(k, (int)N, (beta ? p->occ_b : p->occ_a).as<uint64_t>(),
                                                          rl.as<int>(), rd.as<unsigned>(), eb.as<int>(), ctx->stream);
         if (err != cudaSuccess) return fail(cuda_error(ctx, err, "sort_right_strings"));
@@ -461,7 +468,7 @@ SpinTableArgs table_args(vb_hs_plan* p, bool beta, const double* S, const double
     a.careful_list = beta ? p->list_b.as<unsigned long long>() : p->list_a.as<unsigned long long>();
     a.items = nullptr;
     a.n_items = 0;
-    a.all_careful = 0;
+    a.all_careful = (beta ? p->tables_b : p->tables_a).ptr ? 0 : 1;
     a.r_pos = p->r_pos;
     a.rlist = beta ? p->rlist_b.as<int>() : p->rlist_a.as<int>();
     a.rdesc = beta ? p->rdesc_b.as<unsigned>() : p->rdesc_a.as<unsigned>();
@@ -799,9 +806,11 @@ vb_status vb_hs_plan_stats(const vb_hs_plan* p, vb_hs_stats* stats) {
         if (err == cudaSuccess) err = cudaStreamSynchronize(p->ctx->stream);
         if (err != cudaSuccess) return cuda_error(p->ctx, err, "stats download");
         if ((int)c[7]) return set_error(p->ctx, VB_ERR_TIMEOUT, "band_reduce: a tile wait timed out");
-        auto all_exact = [&](int k) { return !frame_spin_supported(p->n, k, p->R); };
-        const bool all_a = p->ka > 0 && all_exact(p->ka);
-        const bool all_b = p->kb > 0 && !p->shared_tables && all_exact(p->kb);
+        auto all_exact = [&](int k, const DeviceBuffer& tables) {
+            return !tables.ptr || !frame_spin_supported(p->n, k, p->R);
+        };
+        const bool all_a = p->ka > 0 && all_exact(p->ka, p->tables_a);
+        const bool all_b = p->kb > 0 && !p->shared_tables && all_exact(p->kb, p->tables_b);
         s.careful_spin_pairs = (long long)(all_a ? p->npairs_a : c[0]) + (long long)(all_b ? p->npairs_b : c[1]);
     }
     *stats = s;

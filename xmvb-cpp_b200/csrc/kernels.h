@@ -142,6 +142,9 @@ cudaError_t launch_spin_pairs_exact(const SpinTableArgs& a, cudaStream_t stream,
 // the once-per-table bucketing of right strings, and the table and pair launches.
 size_t frame_table_doubles(int n, int k, int R);
 bool frame_spin_supported(int n, int k, int R);
+// More complement orbitals than a closed shell of k electrons has: the register path is optional
+// there (without room for its tables the exact path evaluates every pair).
+bool frame_wide_complement(int n, int k);
 cudaError_t launch_sort_right_strings(int k, int N, const uint64_t* occ, int* rlist, unsigned* rdesc, int* ebound,
                                       cudaStream_t stream);
 cudaError_t launch_frame_tables(const SpinTableArgs& a, double* tables, cudaStream_t stream);

@@ -108,7 +108,9 @@ extern "C" vb_status vb_spin_pairs_noalloc(void* cuda_stream, int n_orbitals, in
     const long long N = n_strings;
     const long long n_pairs = N * (N + 1) / 2;
     const int np = n * (n + 1) / 2, gd = n * (n - 1) / 2;
-    // layout of the static scratch, sized for the largest factor rank (np columns)
+    // layout of the static scratch, sized for the largest factor rank (np columns).  The tables of
+    // the register path come last, so that a wide open-shell table without room for them takes the
+    // exact path within the size a closed shell of k electrons would need.
     size_t off = 0;
     auto take = [&](size_t bytes) {
         const size_t at = off;
@@ -127,9 +129,15 @@ extern "C" vb_status vb_spin_pairs_noalloc(void* cuda_stream, int n_orbitals, in
     const size_t o_signs = take(sizeof(int) * np);
     const size_t o_meta = take(sizeof(int) * 4);
     const size_t o_counters = take(sizeof(unsigned long long) * 8);
-    const size_t o_tables = take(sizeof(double) * frame_table_doubles(n, k, np) * N);
     const size_t o_records = take(sizeof(double) * (size_t)record_stride_for(np) * n_pairs);
     const size_t o_list = take(sizeof(unsigned long long) * n_pairs);
+    const size_t fixed = off;
+    const size_t o_tables = take(sizeof(double) * frame_table_doubles(n, k, np) * N);
+    bool tables = true;
+    if (off > kNoAllocScratchBytes && frame_wide_complement(n, k)) {
+        off = align256(fixed + sizeof(double) * frame_table_doubles(2 * k, k, np) * N);
+        tables = false;
+    }
     if (off > kNoAllocScratchBytes)
         return set_error(nullptr, VB_ERR_BUDGET,
                          "vb_spin_pairs_noalloc: this string table needs " + std::to_string(off) +
@@ -193,7 +201,7 @@ extern "C" vb_status vb_spin_pairs_noalloc(void* cuda_stream, int n_orbitals, in
 
     err = cudaMemsetAsync(counters, 0, sizeof(unsigned long long) * 8, s);
     if (err != cudaSuccess) return cuda_error(nullptr, err, "cudaMemsetAsync");
-    if (frame_spin_supported(n, k, 0)) {
+    if (tables && frame_spin_supported(n, k, 0)) {
         err = launch_sort_right_strings(k, n_strings, rows, rlist, rdesc, ebound, s);
         if (err != cudaSuccess) return cuda_error(nullptr, err, "sort_right_strings");
     }
@@ -217,7 +225,7 @@ extern "C" vb_status vb_spin_pairs_noalloc(void* cuda_stream, int n_orbitals, in
     a.careful_list = reinterpret_cast<unsigned long long*>(b + o_list);
     a.items = nullptr;
     a.n_items = 0;
-    a.all_careful = 0;
+    a.all_careful = tables ? 0 : 1;
     a.r_pos = meta[0];
     a.rlist = rlist;
     a.rdesc = rdesc;

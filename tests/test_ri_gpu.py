@@ -151,3 +151,16 @@ def test_pair_factors_in_a_new_frame(ctx, n, n_aux):
 def test_pair_factors_frame_rejects_bad_input(ctx):
     with pytest.raises(vbcore.VbError):
         vbcore.ri_pair_factors_frame(ctx, np.zeros((2, 3)), np.eye(2), mode=1)
+
+
+@pytest.mark.parametrize("n_aux,n_bf,n_act", [(1, 1, 1), (15, 3, 2), (16, 33, 8), (17, 31, 9), (34, 257, 16), (66, 65, 13)])
+def test_second_index_packing_and_adjoint_tile_edges(ctx, n_aux, n_bf, n_act):
+    """Remainders of the 16-row, 256-column and 32-row tiles of the second index, the packing and
+    the adjoint, with rows that start 16-byte aligned (even n_aux) and not.  The bound is the
+    rounding of sums of at most n_act n_aux products of order-one terms."""
+    B, C = _inputs(n_aux, n_bf, n_act, 3 * n_aux + n_bf)
+    L, K, T = vbcore.active_transform_ri(ctx, B, C, one_index=True)
+    Lr, Kr = O.ri_transform(B, C)
+    assert _rel(L, Lr) < 1e-13 and _rel(K, Kr) < 1e-13
+    G = np.random.default_rng(n_aux).standard_normal(L.shape)
+    assert _rel(vbcore.active_transform_ri_adjoint(ctx, T, G, n_bf), O.ri_adjoint(T, G, n_act)) < 1e-13

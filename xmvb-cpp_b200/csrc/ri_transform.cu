@@ -226,12 +226,15 @@ __global__ void __launch_bounds__(32 * kPipeWarps, 2) one_index_pipelined_kernel
 // once ([nu][20], padded so the B-fragment loads are conflict-free) and loop over (8 AO indices,
 // 64 auxiliary rows) items; each warp streams its mu's columns through a private 3-stage
 // cp.async ring of 8 columns x 64 rows (row stride 68: conflict-free A-fragment loads) and keeps
-// 8 x 2 accumulator tiles in registers.  Items run with the auxiliary tile fastest, so the
-// CTAs resident together read whole packed columns.  The sum over nu runs in a fixed order.
+// 8 x 2 accumulator tiles in registers.  Items run with the AO block fastest, so that the packed
+// columns of the few auxiliary tiles in flight are read a second time (for the other index) while
+// they may still be in L2: the transform and its adjoint at n_bf 400, n_aux 1600, n_act 16 take
+// 457 us this way, 471 us with the auxiliary tile fastest (whole columns read at once), and 515 to
+// 630 us with 32 or 16 rows per item in either order.  The sum over nu runs in a fixed order.
 constexpr int kDmmaWarps = 8;
-constexpr int kDmmaRows = 64;      // auxiliary rows per item (8 M tiles)
 constexpr int kDmmaNu = 8;         // columns per ring stage (two k-steps)
 constexpr int kDmmaStages = 3;
+constexpr int kDmmaRows = 64;      // auxiliary rows per item (8 M tiles)
 constexpr int kDmmaRing = 68;      // ring row stride (doubles; = 4 mod 16)
 constexpr int kDmmaCt = 20;        // staged C stride (doubles; = 4 mod 16)
 constexpr int kDmmaMaxBf = 768;   // shared memory: C staging plus the rings
@@ -265,8 +268,8 @@ __global__ void __launch_bounds__(32 * kDmmaWarps, 1) one_index_dmma_kernel(cons
     const int n_steps = (n_bf + kDmmaNu - 1) / kDmmaNu;
     const long long ld = (long long)n_act * n_aux;
     for (long long item = blockIdx.x; item < (long long)mu_blocks * aux_tiles; item += gridDim.x) {
-        const int mu = (int)(item / aux_tiles) * kDmmaWarps + warp;
-        const int aux0 = (int)(item % aux_tiles) * kDmmaRows;
+        const int mu = (int)(item % mu_blocks) * kDmmaWarps + warp;
+        const int aux0 = (int)(item / mu_blocks) * kDmmaRows;
         if (mu >= n_bf) continue;  // warp-private work below: no CTA-wide barrier
         auto issue = [&](int step) {
             if (step < n_steps) {
@@ -579,123 +582,230 @@ __global__ void __launch_bounds__(32 * kSplitWarps, 2) one_index_split_pipelined
         }
 }
 
-// L[P, pair(a, b)] = sum_mu T[a, P, mu] C(mu, b) for b <= a.  CTA = (32 auxiliary rows, one
-// orbital a); its four warps split the mu range (lane = auxiliary row, 16 accumulators for b)
-// and reduce through shared memory.
-__global__ void __launch_bounds__(128) second_index_kernel(const double* __restrict__ T, int n_aux, int n_bf,
-                                                           const double* __restrict__ C, int n_act,
-                                                           double* __restrict__ L) {
-    __shared__ double red[4][kMaxActive][33];
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int P = blockIdx.x * 32 + lane;
+// Two consecutive doubles at p (the second one only when `second`), as one 16-byte load when VEC
+// (p 16-byte aligned and both present).
+template <bool VEC>
+__device__ __forceinline__ double2 load_two(const double* p, bool first, bool second) {
+    if (VEC) return first ? __ldg(reinterpret_cast<const double2*>(p)) : make_double2(0.0, 0.0);
+    return make_double2(first ? __ldg(p) : 0.0, second ? __ldg(p + 1) : 0.0);
+}
+
+// L[P, pair(a, b)] = sum_mu T[a, P, mu] C(mu, b) for b <= a: per orbital a, an n_aux x (a + 1) x n_bf
+// product on the FP64 tensor cores.  A warp owns 16 auxiliary rows as two M tiles (row 2 g + i of
+// the warp's rows is row g of tile i, so a lane's two A elements are one 16-byte load and a k-step
+// reads four 128-byte pieces of T) and both N tiles (one when a < 8); C is staged in shared memory,
+// orbital-major with a stride of 4 mod 16 doubles (conflict-free B fragments).  The grid's blocks
+// take kSecondWarps row groups of one orbital; the sum over mu runs in a fixed order.  Bound by the
+// read of T (82 MB at n_bf 400, n_aux 1600, n_act 16, mostly from L2): the earlier form, one lane
+// per row with 16 broadcast loads of C per element, took 52 us there.
+constexpr int kSecondWarps = 4;
+constexpr int kSecondUnroll = 8;   // k-steps (four AO indices each) whose loads are in flight
+constexpr int kSecondChunk = 256;  // AO indices of C staged at a time
+constexpr int kSecondStride = kSecondChunk + 4;
+
+template <bool VEC>
+__global__ void __launch_bounds__(32 * kSecondWarps) second_index_kernel(const double* __restrict__ T, int n_aux,
+                                                                         int n_bf, const double* __restrict__ C,
+                                                                         int n_act, double* __restrict__ L) {
+    __shared__ double sCo[kMaxActive * kSecondStride];  // [b][AO index of the chunk], zero past the end
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, gr = lane >> 2, gc = lane & 3;
     const int a = blockIdx.y;
+    const int nt = a < 8 ? 1 : 2;
+    const int P = (blockIdx.x * kSecondWarps + warp) * 16 + 2 * gr;
+    const bool ok0 = P < n_aux, ok1 = P + 1 < n_aux;
     const long long ld = (long long)n_act * n_aux;
-    double acc[kMaxActive];
+    const double* t = T + (long long)a * n_aux + (ok0 ? P : 0);
+    double acc[2][2][2] = {};
+    for (int c0 = 0; c0 < n_bf; c0 += kSecondChunk) {
+        __syncthreads();
+        for (int e = threadIdx.x; e < 8 * nt * kSecondChunk; e += blockDim.x) {
+            const int b = e / kSecondChunk, m = e % kSecondChunk;
+            sCo[b * kSecondStride + m] = (b <= a && c0 + m < n_bf) ? __ldg(C + c0 + m + (long long)b * n_bf) : 0.0;
+        }
+        __syncthreads();
+        const int cnt = min(kSecondChunk, n_bf - c0);
+        for (int m0 = 0; m0 < cnt; m0 += 4 * kSecondUnroll) {
+            double2 v[kSecondUnroll];
 #pragma unroll
-    for (int b = 0; b < kMaxActive; ++b) acc[b] = 0.0;
-    const int chunk = (n_bf + 3) / 4;
-    const int m0 = warp * chunk, m1 = min(n_bf, m0 + chunk);
-    if (P < n_aux) {
-        const double* t = T + (long long)a * n_aux + P;
-#pragma unroll 4
-        for (int m = m0; m < m1; ++m) {
-            const double tv = __ldg(t + (long long)m * ld);
+            for (int u = 0; u < kSecondUnroll; ++u) {
+                const int m = m0 + 4 * u + gc;
+                v[u] = load_two<VEC>(t + (long long)(c0 + (m < cnt ? m : 0)) * ld, ok0 && m < cnt, ok1 && m < cnt);
+            }
 #pragma unroll
-            for (int b = 0; b < kMaxActive; ++b)
-                if (b <= a) acc[b] = fma(tv, __ldg(C + m + (long long)b * n_bf), acc[b]);
+            for (int u = 0; u < kSecondUnroll; ++u) {
+                const int m = m0 + 4 * u + gc;
+                const double b0 = sCo[gr * kSecondStride + m];
+                dmma_f64(acc[0][0], v[u].x, b0);
+                dmma_f64(acc[1][0], v[u].y, b0);
+                if (nt == 2) {
+                    const double b1 = sCo[(8 + gr) * kSecondStride + m];
+                    dmma_f64(acc[0][1], v[u].x, b1);
+                    dmma_f64(acc[1][1], v[u].y, b1);
+                }
+            }
         }
     }
 #pragma unroll
-    for (int b = 0; b < kMaxActive; ++b) red[warp][b][lane] = acc[b];
-    __syncthreads();
-    for (int e = threadIdx.x; e < 32 * kMaxActive; e += blockDim.x) {
-        const int l = e % 32, b = e / 32;
-        const int PP = blockIdx.x * 32 + l;
-        if (b > a || PP >= n_aux) continue;
-        L[PP + ao_pair(a, b) * n_aux] = red[0][b][l] + red[1][b][l] + red[2][b][l] + red[3][b][l];
-    }
+    for (int i = 0; i < 2; ++i)
+#pragma unroll
+        for (int j = 0; j < 2; ++j)
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const int b = 8 * j + 2 * gc + h;
+                if (b <= a && P + i < n_aux) L[P + i + ao_pair(a, b) * n_aux] = acc[i][j][h];
+            }
 }
 
-// K[pair(p, q)] = sum_P L[P, p] L[P, q] (q <= p): one warp per packed element.
-__global__ void __launch_bounds__(256) pack_kernel(const double* __restrict__ L, int n_aux, int npair,
-                                                   double* __restrict__ K) {
-    const long long w = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const int lane = threadIdx.x & 31;
-    const long long total = (long long)npair * (npair + 1) / 2;
-    if (w >= total) return;
-    int p = (int)((sqrt(8.0 * (double)w + 1.0) - 1.0) / 2.0);
-    while ((long long)p * (p + 1) / 2 > w) --p;
-    while ((long long)(p + 1) * (p + 2) / 2 <= w) ++p;
-    const int q = (int)(w - (long long)p * (p + 1) / 2);
-    const double* lp = L + (long long)p * n_aux;
-    const double* lq = L + (long long)q * n_aux;
-    double acc = 0.0;
-    for (int P = lane; P < n_aux; P += 32) acc = fma(__ldg(lp + P), __ldg(lq + P), acc);
+// Four consecutive k of one operand row (k0 + 4 gc .. + 3) for the tiles below: an m8n8k4 step sums
+// over any four k, so step s takes element s of every lane's four and the loads are 16-byte (VEC)
+// pieces of the k-contiguous rows.
+template <bool VEC>
+__device__ __forceinline__ void load_four(const double* p, int left, double (&v)[4]) {
+    const double2 x = load_two<VEC>(p, left > 0, left > 1), y = load_two<VEC>(p + 2, left > 2, left > 3);
+    v[0] = x.x;
+    v[1] = x.y;
+    v[2] = y.x;
+    v[3] = y.y;
+}
+
+// K[pair(p, q)] = sum_P L[P, p] L[P, q] (q <= p) on the FP64 tensor cores: a CTA per 16 x 16 tile of
+// the lower triangle, its eight warps taking every eighth 16-row block of P, their accumulators
+// summed through shared memory in warp order.  Bound by latency (1600 rows of 136 columns: 100
+// blocks over eight warps); a warp per element took 14.8 us there.
+constexpr int kPackWarps = 8;
+
+template <bool VEC>
+__global__ void __launch_bounds__(32 * kPackWarps) pack_kernel(const double* __restrict__ L, int n_aux, int npair,
+                                                               double* __restrict__ K) {
+    __shared__ double red[kPackWarps][256];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, gr = lane >> 2, gc = lane & 3;
+    int tp = (int)((sqrt(8.0 * (double)blockIdx.x + 1.0) - 1.0) / 2.0);
+    while (tp * (tp + 1) / 2 > (int)blockIdx.x) --tp;
+    while ((tp + 1) * (tp + 2) / 2 <= (int)blockIdx.x) ++tp;
+    const int tq = (int)blockIdx.x - tp * (tp + 1) / 2;
+    double acc[2][2][2] = {};
+    const double* rows[4];
+    bool ok[4];
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-    if (lane == 0) K[w] = acc;
+    for (int i = 0; i < 4; ++i) {
+        const int r = 16 * (i < 2 ? tp : tq) + 8 * (i & 1) + gr;
+        ok[i] = r < npair;
+        rows[i] = L + (long long)(ok[i] ? r : 0) * n_aux + 4 * gc;
+    }
+    for (int k0 = 16 * warp; k0 < n_aux; k0 += 16 * kPackWarps) {
+        double v[4][4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) load_four<VEC>(rows[i] + k0, ok[i] ? n_aux - k0 - 4 * gc : 0, v[i]);
+#pragma unroll
+        for (int s = 0; s < 4; ++s)
+#pragma unroll
+            for (int i = 0; i < 2; ++i)
+#pragma unroll
+                for (int j = 0; j < 2; ++j) dmma_f64(acc[i][j], v[i][s], v[2 + j][s]);
+    }
+#pragma unroll
+    for (int i = 0; i < 2; ++i)
+#pragma unroll
+        for (int j = 0; j < 2; ++j)
+#pragma unroll
+            for (int h = 0; h < 2; ++h) red[warp][(8 * i + gr) * 16 + 8 * j + 2 * gc + h] = acc[i][j][h];
+    __syncthreads();
+    const int e = threadIdx.x, p = 16 * tp + e / 16, q = 16 * tq + e % 16;
+    double sum = 0.0;
+#pragma unroll
+    for (int w = 0; w < kPackWarps; ++w) sum += red[w][e];
+    if (p < npair && q <= p) K[(long long)p * (p + 1) / 2 + q] = sum;
 }
 
 // Adjoint.  With G = dE/dL and Gs[P, c, b] = G[P, pair(c, b)] (1 + delta_cb):
-//   dE/dC(kappa, c) = sum_{P, b} Gs[P, c, b] T[b, P, kappa].
-// adjoint_kernel: one CTA per (AO tile of 32, slice of the (b, P) range); partial sums go to
-// a [slices x n_bf x n_act] buffer reduced in a fixed order by adjoint_reduce_kernel.
-constexpr int kAdjSlices = 16;
+//   dE/dC(kappa, c) = sum_{P, b} Gs[P, c, b] T[b, P, kappa],
+// an n_bf x n_act x (n_act n_aux) product on the FP64 tensor cores: a CTA per (kAdjRows AO indices,
+// slice of the (b, 16 auxiliary rows) blocks), its eight warps taking every eighth block of the
+// slice.  Both operands are read k-contiguously straight into fragments (load_four); a warp keeps
+// 4 M tiles x 2 N tiles so that a block of G serves 32 AO indices.  Warp sums go through shared
+// memory, slice sums to a [slices x n_bf x 16] buffer that adjoint_reduce_kernel adds up, both in a
+// fixed order.  Bound by the read of T (82 MB at n_bf 400, n_aux 1600, n_act 16); staging 32 x 32
+// tiles through shared memory for two FMAs per element took 176 us there.
+constexpr int kAdjSlices = 24;   // most slices: 13 x 24 CTAs fill the GPU at n_bf = 400
+constexpr int kAdjRows = 32;
+constexpr int kAdjWarps = 8;
 
-__global__ void __launch_bounds__(256) adjoint_kernel(const double* __restrict__ T, const double* __restrict__ G,
-                                                      int n_aux, int n_bf, int n_act, double* __restrict__ partial) {
-    __shared__ double sT[32][33];   // [kappa local][k local]
-    __shared__ double sG[32][kMaxActive + 1];  // [k local][c]
-    const int k0_tile = blockIdx.x * 32;
-    const int slice = blockIdx.y;
-    const long long Ktot = (long long)n_act * n_aux;
-    const long long per = (Ktot + kAdjSlices - 1) / kAdjSlices;
-    const long long kb = slice * per, ke = min(Ktot, kb + per);
-    const int tid = threadIdx.x;
-    const int kl = tid & 31, cg = tid >> 5;  // thread: kappa local kl, c in {cg, cg + 8}
-    double acc0 = 0.0, acc1 = 0.0;
-    for (long long k0 = kb; k0 < ke; k0 += 32) {
-        __syncthreads();
-        for (int e = tid; e < 32 * 32; e += blockDim.x) {
-            const int kk = e % 32, r = e / 32;
-            const long long k = k0 + kk;
-            const int kappa = k0_tile + r;
-            sT[r][kk] = (k < ke && kappa < n_bf) ? __ldg(T + k + (long long)kappa * Ktot) : 0.0;
-        }
-        for (int e = tid; e < 32 * kMaxActive; e += blockDim.x) {
-            const int kk = e % 32, c = e / 32;
-            const long long k = k0 + kk;
-            double g = 0.0;
-            if (k < ke && c < n_act) {
-                const int b = (int)(k / n_aux), P = (int)(k % n_aux);
-                g = __ldg(G + P + ao_pair(c, b) * n_aux) * (c == b ? 2.0 : 1.0);
-            }
-            sG[kk][c] = g;
-        }
-        __syncthreads();
-#pragma unroll 8
-        for (int kk = 0; kk < 32; ++kk) {
-            const double t = sT[kl][kk];
-            acc0 = fma(t, sG[kk][cg], acc0);
-            acc1 = fma(t, sG[kk][cg + 8], acc1);
-        }
+// slices used for n_blocks (b, 16 auxiliary rows) blocks: at least two blocks per warp
+__host__ inline int adjoint_slices(long long n_blocks) {
+    const long long s = (n_blocks + 2 * kAdjWarps - 1) / (2 * kAdjWarps);
+    return (int)(s < 1 ? 1 : (s > kAdjSlices ? kAdjSlices : s));
+}
+
+template <bool VEC>
+__global__ void __launch_bounds__(32 * kAdjWarps, 2) adjoint_kernel(const double* __restrict__ T,
+                                                                    const double* __restrict__ G, int n_aux, int n_bf,
+                                                                    int n_act, double* __restrict__ partial) {
+    __shared__ double red[kAdjWarps][kAdjRows * kMaxActive];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, gr = lane >> 2, gc = lane & 3;
+    const int kappa0 = blockIdx.x * kAdjRows;
+    const int per_b = (n_aux + 15) / 16;
+    const long long n_blocks = (long long)per_b * n_act;
+    const long long b0 = n_blocks * blockIdx.y / gridDim.y, b1 = n_blocks * (blockIdx.y + 1) / gridDim.y;
+    const long long ld = (long long)n_act * n_aux;
+    double acc[4][2][2] = {};
+    const double* rows[4];
+    bool ok[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const int kappa = kappa0 + 8 * i + gr;
+        ok[i] = kappa < n_bf;
+        rows[i] = T + (long long)(ok[i] ? kappa : 0) * ld + 4 * gc;
     }
-    const int kappa = k0_tile + kl;
-    if (kappa < n_bf) {
-        double* out = partial + (long long)slice * n_bf * kMaxActive;
-        out[(long long)kappa * kMaxActive + cg] = acc0;
-        out[(long long)kappa * kMaxActive + cg + 8] = acc1;
+    for (long long q = b0 + warp; q < b1; q += kAdjWarps) {
+        const int b = (int)(q / per_b), P = (int)(q % per_b) * 16;
+        const int left = n_aux - P - 4 * gc;
+        double va[4][4], vb[2][4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) load_four<VEC>(rows[i] + (long long)b * n_aux + P, ok[i] ? left : 0, va[i]);
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+            const int c = 8 * j + gr;
+            load_four<VEC>(G + ao_pair(c < n_act ? c : 0, b) * n_aux + P + 4 * gc, c < n_act ? left : 0, vb[j]);
+            if (c == b)
+#pragma unroll
+                for (int s = 0; s < 4; ++s) vb[j][s] *= 2.0;
+        }
+#pragma unroll
+        for (int s = 0; s < 4; ++s)
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+#pragma unroll
+                for (int j = 0; j < 2; ++j) dmma_f64(acc[i][j], va[i][s], vb[j][s]);
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int j = 0; j < 2; ++j)
+#pragma unroll
+            for (int h = 0; h < 2; ++h) red[warp][(8 * i + gr) * kMaxActive + 8 * j + 2 * gc + h] = acc[i][j][h];
+    __syncthreads();
+    double* out = partial + ((long long)blockIdx.y * n_bf + kappa0) * kMaxActive;
+    for (int e = threadIdx.x; e < kAdjRows * kMaxActive; e += blockDim.x) {
+        double sum = 0.0;
+#pragma unroll
+        for (int w = 0; w < kAdjWarps; ++w) sum += red[w][e];
+        if (kappa0 + e / kMaxActive < n_bf) out[e] = sum;
     }
 }
 
-__global__ void adjoint_reduce_kernel(const double* __restrict__ partial, int n_bf, int n_act, double* __restrict__ dC) {
+__global__ void adjoint_reduce_kernel(const double* __restrict__ partial, int slices, int n_bf, int n_act,
+                                      double* __restrict__ dC) {
     const int e = blockIdx.x * blockDim.x + threadIdx.x;
     if (e >= n_bf * n_act) return;
-    const int kappa = e % n_bf, c = e / n_bf;
+    const int c = e % n_act, kappa = e / n_act;
     double s = 0.0;
-    for (int sl = 0; sl < kAdjSlices; ++sl) s += partial[(long long)sl * n_bf * kMaxActive + (long long)kappa * kMaxActive + c];
+#pragma unroll 8
+    for (int sl = 0; sl < slices; ++sl) s += __ldg(partial + ((long long)sl * n_bf + kappa) * kMaxActive + c);
     dC[kappa + (long long)c * n_bf] = s;
 }
+
+// 16-byte loads of consecutive auxiliary rows: every row of the array starts 16-byte aligned
+bool rows_aligned(const void* p, int n_aux) { return n_aux % 2 == 0 && reinterpret_cast<uintptr_t>(p) % 16 == 0; }
 
 size_t align_up(size_t x) { return (x + 255) / 256 * 256; }
 
@@ -821,12 +931,15 @@ vb_status vb_active_transform_ri_precision(vb_context* ctx, const double* B_pack
         }
     }
     if (err == cudaSuccess) {
-        second_index_kernel<<<dim3((n_aux + 31) / 32, n_act), 128, 0, s>>>(dT, n_aux, n_bf, dC, n_act, dL);
+        const auto kernel = rows_aligned(dT, n_aux) ? second_index_kernel<true> : second_index_kernel<false>;
+        const int rows = 16 * kSecondWarps;
+        kernel<<<dim3((n_aux + rows - 1) / rows, n_act), 32 * kSecondWarps, 0, s>>>(dT, n_aux, n_bf, dC, n_act, dL);
         err = cudaGetLastError();
     }
     if (err == cudaSuccess && K_packed) {
-        const long long warps = (long long)npair * (npair + 1) / 2;
-        pack_kernel<<<(unsigned)((warps * 32 + 255) / 256), 256, 0, s>>>(dL, n_aux, npair, dK);
+        const int tiles = (npair + 15) / 16;
+        const auto kernel = rows_aligned(dL, n_aux) ? pack_kernel<true> : pack_kernel<false>;
+        kernel<<<tiles * (tiles + 1) / 2, 32 * kPackWarps, 0, s>>>(dL, n_aux, npair, dK);
         err = cudaGetLastError();
     }
     if (err == cudaSuccess && host) {
@@ -854,7 +967,8 @@ vb_status vb_active_transform_ri_adjoint(vb_context* ctx, const double* one_inde
     const int npair = n_act * (n_act + 1) / 2;
     const size_t bT = sizeof(double) * (size_t)n_act * n_aux * n_bf, bG = sizeof(double) * (size_t)n_aux * npair;
     const size_t bD = sizeof(double) * (size_t)n_bf * n_act;
-    const size_t bP = sizeof(double) * (size_t)kAdjSlices * n_bf * kMaxActive;
+    const int slices = adjoint_slices((long long)((n_aux + 15) / 16) * n_act);
+    const size_t bP = sizeof(double) * (size_t)slices * n_bf * kMaxActive;
     size_t off = 0;
     auto take = [&](size_t bytes, bool need) {
         const size_t at = off;
@@ -876,11 +990,13 @@ vb_status vb_active_transform_ri_adjoint(vb_context* ctx, const double* one_inde
         if (err == cudaSuccess) err = cudaMemcpyAsync(const_cast<double*>(dG), dL, bG, cudaMemcpyHostToDevice, s);
     }
     if (err == cudaSuccess) {
-        adjoint_kernel<<<dim3((n_bf + 31) / 32, kAdjSlices), 256, 0, s>>>(dT, dG, n_aux, n_bf, n_act, partial);
+        const bool vec = rows_aligned(dT, n_aux) && rows_aligned(dG, n_aux);
+        const auto kernel = vec ? adjoint_kernel<true> : adjoint_kernel<false>;
+        kernel<<<dim3((n_bf + kAdjRows - 1) / kAdjRows, slices), 32 * kAdjWarps, 0, s>>>(dT, dG, n_aux, n_bf, n_act, partial);
         err = cudaGetLastError();
     }
     if (err == cudaSuccess) {
-        adjoint_reduce_kernel<<<(n_bf * n_act + 255) / 256, 256, 0, s>>>(partial, n_bf, n_act, dOut);
+        adjoint_reduce_kernel<<<(n_bf * n_act + 63) / 64, 64, 0, s>>>(partial, slices, n_bf, n_act, dOut);
         err = cudaGetLastError();
     }
     if (err == cudaSuccess && host) err = cudaMemcpyAsync(dC, dOut, bD, cudaMemcpyDeviceToHost, s);

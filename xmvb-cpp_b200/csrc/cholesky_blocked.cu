@@ -5,13 +5,16 @@
 // Factorization M = U^T U (upper triangle of M read; Eigen::LLT / LAPACK dpotrf semantics: the
 // first non-positive or non-finite pivot stops it with info = its order), right-looking over
 // 64-column panels:
-//   1. bc_panel_kernel (one CTA): Cholesky of the updated diagonal block in shared memory and the
-//      inverse of the resulting triangular block;
-//   2. bc_panel_row_kernel: U_12 = U_11^-T A_12;
-//   3. bc_trailing_kernel: A_22 -= U_12^T U_12 over the upper 64 x 64 tiles.
-// Look-ahead: the trailing update's first tile (the next panel's diagonal block) runs first, then
-// the next panel's factorization on a high-priority auxiliary stream while the remaining tiles run
-// on the caller's stream.
+//   1. bc_panel_kernel (one CTA): the previous panel's update of the diagonal block, its Cholesky
+//      factor and the inverse of that triangular block, in shared memory;
+//   2. bc_panel_row_kernel: the previous panel's update of the row block A_12, then
+//      U_12 = U_11^-T A_12;
+//   3. bc_trailing_kernel: A_22 -= U_12^T U_12 over the upper 64 x 64 tiles from the row block after
+//      the next one on.
+// The chain of 1 and 2 bounds the factorization (n = 2048: 32 panels, 1.88 ms before the panel's
+// pivots moved into one warp and the next panel's updates into these two kernels, 1.31 ms now); it
+// runs on a high-priority auxiliary stream while the trailing updates run one panel behind it on
+// the caller's stream.
 // Inverse U^-1 (optional): the panel kernels leave U_JJ^-1 on the diagonal blocks; then for block
 // sizes b = 64, 128, ... consecutive diagonal blocks are paired,
 //   [[A, B], [0, C]]^-1 = [[A^-1, -A^-1 B C^-1], [0, C^-1]],
@@ -163,139 +166,275 @@ __global__ void bc_init_kernel(const double* __restrict__ M, double* __restrict_
     }
 }
 
-// Panel j0: Cholesky of the (updated) diagonal block, rows beyond the matrix padded with the
-// identity.  Thread (g, c) keeps rows 16 g .. 16 g + 15 of column c in registers.  Pivot k is
-// published through a double-buffered row in shared memory (one barrier per pivot): entries
-// a[k][c] for c > k (zeros elsewhere), 1 / p_k and p_k, so the update a[r][c] -= a[k][r] a[k][c] / p_k
-// needs no row or column test (rows r <= k and columns c <= k see zeros; the lower triangle takes
-// values that are never read and is cleared at the end).  Row r is divided by sqrt(p_r) at the
-// end.  The inverse of the triangular block follows the same way, pivots from the last up
-// (X = I; X[k, :] /= u_kk; X[r, :] -= u_rk X[k, :] for r < k), with u held transposed in shared
-// memory so that a thread's 16 entries of column k are 8 vector loads.  Writes U_JJ into U, its
-// inverse into Ub (64 x 64, column-major) and, when Ui is given, onto Ui's diagonal block.
-constexpr int kPanelRows = kNB / (kThreadsB / kNB);  // rows per thread (16)
-constexpr int kUtStride = kNB + 2;                   // even: rows of the transposed factor stay 16-byte aligned
-constexpr int kPrStride = kNB + 2;                   // published row: kNB entries, 1 / p, p
-constexpr size_t kPanelSmem = sizeof(double) * (kNB * kUtStride + 2 * kPrStride + kNB);
+// Panel j0: Cholesky of the (updated) 64 x 64 diagonal block and the inverse of its factor, one CTA;
+// rows beyond the matrix are padded with the identity.  The serial chain of 64 pivots bounds it, so
+// the chain runs inside one warp without barriers: 16 x 16 blocks, each factored and inverted by
+// warp 0 in registers (panel_factor16: lane (h, c) holds rows 8 h .. 8 h + 7 of column c, the pivot
+// row travels by shuffles), while the other warps still apply the previous block's rank-16 update;
+// then U_12 = U_11^-T A_12 on the tensor cores.  Two barriers per 16 pivots.  The 64 x 64 inverse
+// pairs the 16 x 16 ones (and then the 32 x 32 ones) as bc_level_kernel does.  n = 2048: 41 us a
+// panel when every pivot was published through shared memory to 256 threads (64 + 64 barriers).
+// Shared layout: column-major, stride 68 = 4 mod 16 doubles, so that the fragments of both operand
+// orders load without bank conflicts.  Writes U_JJ into U, its inverse into Ub (64 x 64,
+// column-major) and, when Ui is given, onto Ui's diagonal block.
+constexpr int kPL = kNB + 4;  // column stride of the panel's shared blocks
+constexpr int kPT = 36;       // column stride of the 32 x 32 scratch of the inverse
+constexpr int kPW = kThreadsB / 32;
+constexpr size_t kPanelSmem = sizeof(double) * (2 * kNB * kPL + 32 * kPT);
 
-// v[kk] by a tree of selects on the bits of kk (depth 4, no dynamic register index)
-__device__ __forceinline__ double pick(const double (&v)[kPanelRows], int kk) {
-    static_assert(kPanelRows == 16, "four select levels");
-    double l1[8], l2[4], l3[2];
+// Warp 0: the 16 x 16 block at sA (column-major, stride kPL; upper triangle) becomes its Cholesky
+// factor (zeros below), sX its inverse.  Returns the order of the first failing pivot, 0 when there
+// is none.  Entries below the diagonal carry values that no later step reads.
+__device__ __forceinline__ int panel_factor16(double* sA, double* sX) {
+    const unsigned full = 0xffffffffu;
+    const int lane = threadIdx.x & 31, h = lane >> 4, c = lane & 15;
+    double v[8], mine = 1.0;
 #pragma unroll
-    for (int i = 0; i < 8; ++i) l1[i] = (kk & 1) ? v[2 * i + 1] : v[2 * i];
+    for (int i = 0; i < 8; ++i) v[i] = sA[c * kPL + 8 * h + i];
+    int bad = 0;
 #pragma unroll
-    for (int i = 0; i < 4; ++i) l2[i] = (kk & 2) ? l1[2 * i + 1] : l1[2 * i];
+    for (int k = 0; k < 16; ++k) {
+        const int src = (k >> 3) * 16, kk = k & 7;  // the lanes and register that hold row k
+        const double p = __shfl_sync(full, v[kk], src + k);
+        if (bad == 0 && (!(p > 0.0) || !isfinite(p))) bad = k + 1;  // the same decision in every lane
+        if (c == k) mine = p;
+        const double inv = 1.0 / p;
+        const double x = __shfl_sync(full, v[kk], src + c);
+        const double f = c > k ? x * inv : 0.0;
 #pragma unroll
-    for (int i = 0; i < 2; ++i) l3[i] = (kk & 4) ? l2[2 * i + 1] : l2[2 * i];
-    return (kk & 8) ? l3[1] : l3[0];
+        for (int i = 0; i < 8; ++i) {
+            if (8 + i <= k) continue;  // no row left in either half
+            const double q = __shfl_sync(full, v[kk], src + 8 * h + i);
+            v[i] = fma(8 * h + i > k ? -q : 0.0, f, v[i]);
+        }
+    }
+    if (bad) return bad;
+    // rows scaled by 1 / sqrt(pivot); lane c holds pivot c
+    const double d = sqrt(mine), di = 1.0 / d;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        const int r = 8 * h + i;
+        const double dr = __shfl_sync(full, di, r);
+        v[i] = r < c ? v[i] * dr : (r == c ? d : 0.0);
+        sA[c * kPL + r] = v[i];
+    }
+    __syncwarp();
+    // inverse, rows from the last up: X[k, :] = w[k, :] / u_kk, w[r, :] -= u_rk X[k, :] (r < k)
+    double w[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) w[i] = 8 * h + i == c ? 1.0 : 0.0;
+#pragma unroll
+    for (int k = 15; k >= 0; --k) {
+        const int src = (k >> 3) * 16, kk = k & 7;
+        const double dk = __shfl_sync(full, di, k);
+        const double xk = __shfl_sync(full, w[kk], src + c) * dk;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            if (i > k) continue;
+            const int r = 8 * h + i;
+            const double u = sA[k * kPL + r];  // zero below the diagonal
+            w[i] = r < k ? fma(-u, xk, w[i]) : (r == k ? xk : w[i]);
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < 8; ++i) sX[c * kPL + 8 * h + i] = w[i];
+    __syncwarp();
+    return 0;
+}
+
+// One 8 x 8 tile of A - U_12^T U_12 over the 16 rows k0 .. k0 + 15 at (r0, c0), in place.
+__device__ __forceinline__ void panel_update_tile(double* sA, int k0, int r0, int c0) {
+    const int lane = threadIdx.x & 31, gr = lane >> 2, gc = lane & 3;
+    double acc[2] = {0.0, 0.0};
+#pragma unroll
+    for (int ks = 0; ks < 4; ++ks)
+        dmma(acc, sA[(r0 + gr) * kPL + k0 + 4 * ks + gc], sA[(c0 + gr) * kPL + k0 + 4 * ks + gc]);
+#pragma unroll
+    for (int i = 0; i < 2; ++i) sA[(c0 + 2 * gc + i) * kPL + r0 + gr] -= acc[i];
+}
+
+// One 8 x 8 tile (row r0, column c0) of s A B, A(i, k) at a[k la + i], B(k, j) at b[j lb + k], over
+// k in [kb, ke).
+__device__ __forceinline__ void panel_product_tile(const double* a, int la, const double* b, int lb, int r0, int c0,
+                                                   int kb, int ke, double s, double* out, int lo) {
+    const int lane = threadIdx.x & 31, gr = lane >> 2, gc = lane & 3;
+    double acc[2] = {0.0, 0.0};
+    for (int k = kb; k < ke; k += 4) dmma(acc, a[(k + gc) * la + r0 + gr], b[(c0 + gr) * lb + k + gc]);
+#pragma unroll
+    for (int i = 0; i < 2; ++i) out[(c0 + 2 * gc + i) * lo + r0 + gr] = s * acc[i];
 }
 
 __global__ void __launch_bounds__(kThreadsB) bc_panel_kernel(double* __restrict__ U, double* __restrict__ Ub,
                                                              double* __restrict__ Ui, int n, int j0, int* status) {
     extern __shared__ __align__(16) double psm[];
-    double* ut = psm;                          // ut[c * kUtStride + r] = u[r][c]
-    double* prow = psm + kNB * kUtStride;      // 2 x kPrStride
-    double* piv = prow + 2 * kPrStride;        // pivots p_k
+    double* sA = psm;               // the block, then its factor
+    double* sX = psm + kNB * kPL;   // the inverse
+    double* sT = sX + kNB * kPL;    // scratch of the inverse
+    __shared__ int s_bad;
     if (failed(status)) return;
-    const int t = threadIdx.x, c = t & (kNB - 1), g = t / kNB;
+    const int t = threadIdx.x, warp = t >> 5, lane = t & 31, gr = lane >> 2, gc = lane & 3;
     const int jb = min(kNB, n - j0);
-    double v[kPanelRows];
+    if (t == 0) s_bad = 0;
+    {
+        // the previous panel's update of this block, A_JJ -= U_IJ^T U_IJ (I the 64 rows above), whose
+        // shared tiles overlap sA and sX
+        double cur[2][4][2], acc[2][4][2] = {};
 #pragma unroll
-    for (int i = 0; i < kPanelRows; ++i) {
-        const int r = kPanelRows * g + i;
-        double x = 0.0;
-        if (r < jb && c < jb) {
-            if (r <= c) x = U[(j0 + r) + (long long)(j0 + c) * n];
-        } else if (r == c) {
-            x = 1.0;
+        for (int i = 0; i < 2; ++i)
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+#pragma unroll
+                for (int x = 0; x < 2; ++x) {
+                    const int r = out_row(i), c = out_col(j, x);
+                    cur[i][j][x] = r == c ? 1.0 : 0.0;
+                    if (r < jb && c < jb) cur[i][j][x] = r <= c ? U[(j0 + r) + (long long)(j0 + c) * n] : 0.0;
+                }
+        if (j0 > 0) {
+            const Opnd P{U + j0 - kNB, n, n, kNB};
+            tile_product<true, true>(P, P, j0, j0, 0, kNB, psm, acc);
         }
-        v[i] = x;
+#pragma unroll
+        for (int i = 0; i < 2; ++i)
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+#pragma unroll
+                for (int x = 0; x < 2; ++x) {
+                    const int r = out_row(i), c = out_col(j, x);
+                    // padded rows and columns of the product are zero
+                    sA[c * kPL + r] = r <= c ? cur[i][j][x] - acc[i][j][x] : 0.0;
+                    sX[c * kPL + r] = 0.0;
+                }
     }
-    // the pivot loops stay rolled (a short body that stays in the instruction cache); a thread's
-    // row k % kPanelRows is picked from its registers by selects, not by a dynamic index
-#pragma unroll 1
-    for (int k = 0; k < kNB; ++k) {
-        double* pr = prow + (k & 1) * kPrStride;
-        if (g == k / kPanelRows) {
-            const double x = pick(v, k % kPanelRows);  // a[k][c]
-            pr[c] = c > k ? x : 0.0;
-            if (c == k) {
-                pr[kNB] = 1.0 / x;
-                pr[kNB + 1] = x;
+    __syncthreads();
+    for (int kb = 0; kb < kNB; kb += 16) {
+        const int tiles = (kNB - kb) / 8;  // 8-wide tiles from kb on
+        if (warp == 0) {
+            if (kb > 0) {
+                panel_update_tile(sA, kb - 16, kb, kb);
+                panel_update_tile(sA, kb - 16, kb, kb + 8);
+                panel_update_tile(sA, kb - 16, kb + 8, kb + 8);
+                __syncwarp();
             }
+            const int bad = panel_factor16(sA + kb * kPL + kb, sX + kb * kPL + kb);
+            if (bad && lane == 0) s_bad = kb + bad;
+        } else if (kb > 0) {
+            // the rest of the previous block's update: upper tiles (ti <= tj) but the three above
+            int q = 0;
+            for (int tj = 2; tj < tiles; ++tj)
+                for (int ti = 0; ti <= tj; ++ti, ++q)
+                    if (q % (kPW - 1) == warp - 1) panel_update_tile(sA, kb - 16, kb + 8 * ti, kb + 8 * tj);
         }
         __syncthreads();
-        const double p = pr[kNB + 1];
-        if (k < jb && (!(p > 0.0) || !isfinite(p))) {  // the same decision in every thread
-            if (t == 0) atomicCAS(status, 0, j0 + k + 1);
+        if (s_bad) {
+            if (t == 0) atomicCAS(status, 0, j0 + s_bad);
             return;
         }
-        if (t == 0) piv[k] = p;
-        const double f = pr[c] * pr[kNB];
-        const double2* q2 = reinterpret_cast<const double2*>(pr + kPanelRows * g);
+        // U_12 = U_11^-T A_12 in place: a warp per 8 columns, both row tiles
+        const int c0 = kb + 16 + 8 * warp;
+        if (c0 < kNB) {
+            double acc[2][2] = {};
 #pragma unroll
-        for (int i = 0; i < kPanelRows / 2; ++i) {
-            const double2 q = q2[i];
-            v[2 * i] = fma(-q.x, f, v[2 * i]);
-            v[2 * i + 1] = fma(-q.y, f, v[2 * i + 1]);
-        }
-    }
-    __syncthreads();
+            for (int ks = 0; ks < 4; ++ks) {
+                const double bf = sA[(c0 + gr) * kPL + kb + 4 * ks + gc];
 #pragma unroll
-    for (int i = 0; i < kPanelRows; ++i) {
-        const int r = kPanelRows * g + i;
-        const double d = sqrt(piv[r]);
-        v[i] = r < c ? v[i] / d : (r == c ? d : 0.0);
-        ut[c * kUtStride + r] = v[i];
-        if (r <= c && c < jb) U[(j0 + r) + (long long)(j0 + c) * n] = v[i];
-    }
-    __syncthreads();
-    if (t < kNB) piv[t] = 1.0 / ut[t * kUtStride + t];  // 1 / u_kk, off the pivot chain
-    __syncthreads();
+                for (int i = 0; i < 2; ++i)  // A(i, k) = X(k, i)
+                    dmma(acc[i], sX[(kb + 8 * i + gr) * kPL + kb + 4 * ks + gc], bf);
+            }
+            __syncwarp();
 #pragma unroll
-    for (int i = 0; i < kPanelRows; ++i) v[i] = (kPanelRows * g + i == c) ? 1.0 : 0.0;
-#pragma unroll 1
-    for (int k = kNB - 1; k >= 0; --k) {
-        double* pr = prow + (k & 1) * kPrStride;
-        const bool owner = g == k / kPanelRows;
-        const int kk = k % kPanelRows;
-        double own = 0.0;
-        if (owner) {
-            own = pick(v, kk) * piv[k];
-            pr[c] = own;
+            for (int i = 0; i < 2; ++i)
+#pragma unroll
+                for (int x = 0; x < 2; ++x) sA[(c0 + 2 * gc + x) * kPL + kb + 8 * i + gr] = acc[i][x];
         }
         __syncthreads();
-        const double xk = pr[c];
-        const double2* u2 = reinterpret_cast<const double2*>(ut + k * kUtStride + kPanelRows * g);  // u[r][k]
-#pragma unroll
-        for (int i = 0; i < kPanelRows / 2; ++i) {
-            const double2 q = u2[i];
-            v[2 * i] = fma(-q.x, xk, v[2 * i]);
-            v[2 * i + 1] = fma(-q.y, xk, v[2 * i + 1]);
-        }
-        if (owner) {
-#pragma unroll
-            for (int i = 0; i < kPanelRows; ++i) v[i] = i == kk ? own : v[i];
-        }
     }
-#pragma unroll
-    for (int i = 0; i < kPanelRows; ++i) {
-        const int r = kPanelRows * g + i;
-        Ub[r + kNB * c] = v[i];
-        if (Ui && r <= c && c < jb) Ui[(j0 + r) + (long long)(j0 + c) * n] = v[i];
+    // inverse: pairs of 16, then of 32: X_01 = -X_00 (U_01 X_11)
+    {
+        const int o = 32 * (warp >> 2), r0 = 8 * ((warp >> 1) & 1), c0 = 8 * (warp & 1);
+        panel_product_tile(sA + (o + 16) * kPL + o, kPL, sX + (o + 16) * kPL + o + 16, kPL, r0, c0, 0, 16, 1.0,
+                           sT + (warp >> 2) * 16 * kPT, kPT);
+        __syncthreads();
+        panel_product_tile(sX + o * kPL + o, kPL, sT + (warp >> 2) * 16 * kPT, kPT, r0, c0, 0, 16, -1.0,
+                           sX + (o + 16) * kPL + o, kPL);
+        __syncthreads();
+        for (int q = warp; q < 16; q += kPW)
+            panel_product_tile(sA + 32 * kPL, kPL, sX + 32 * kPL + 32, kPL, 8 * (q & 3), 8 * (q >> 2), 0,
+                               8 * (q >> 2) + 8, 1.0, sT, kPT);
+        __syncthreads();
+        for (int q = warp; q < 16; q += kPW)
+            panel_product_tile(sX, kPL, sT, kPT, 8 * (q & 3), 8 * (q >> 2), 8 * (q & 3), 32, -1.0, sX + 32 * kPL, kPL);
+        __syncthreads();
+    }
+    for (int e = t; e < kNB * kNB; e += kThreadsB) {
+        const int r = e % kNB, c = e / kNB;
+        const double x = sX[c * kPL + r];
+        Ub[e] = x;
+        if (r <= c && c < jb) {
+            U[(j0 + r) + (long long)(j0 + c) * n] = sA[c * kPL + r];
+            if (Ui) Ui[(j0 + r) + (long long)(j0 + c) * n] = x;
+        }
     }
 }
 
-// U_12 = U_11^-T A_12 in place, 64 columns per CTA: A(i, k) = Ub[k + 64 i], B(k, c) = U[j0 + k + c n].
+// Row block of panel j0, 64 columns per CTA: A_12 -= U_I1^T U_I2 (I the previous panel's 64 rows, its
+// update of this row block), then U_12 = U_11^-T A_12 in place.  Doing the update here (and that of
+// the diagonal block in the panel kernel) takes the trailing kernel of panel j0 - 64 off the chain of
+// panels, which needs the trailing update of panel j0 - 128 only.
 __global__ void __launch_bounds__(kThreadsB) bc_panel_row_kernel(double* __restrict__ U, const double* __restrict__ Ub,
                                                                  int n, int j0, const int* status) {
     extern __shared__ double smem[];
-    if (failed(status)) return;
     const int jb = min(kNB, n - j0), j1 = j0 + jb;
     const int c0 = j1 + blockIdx.x * kNB;
-    double acc[2][4][2] = {};
-    tile_product<true, true>(Opnd{Ub, kNB, jb, jb}, Opnd{U + j0, n, n, jb}, 0, c0, 0, jb, smem, acc);
+    double cur[2][4][2], acc[2][4][2] = {};
+#pragma unroll
+    for (int i = 0; i < 2; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const int r = out_row(i), c = c0 + out_col(j, h);
+                cur[i][j][h] = (r < jb && c < n) ? U[(j0 + r) + (long long)c * n] : 0.0;
+            }
+    if (j0 > 0) {
+        const Opnd P{U + j0 - kNB, n, n, kNB};
+        tile_product<true, true>(P, P, j0, c0, 0, kNB, smem, acc);
+    }
+    if (failed(status)) return;
+    // the updated tile as the k-contiguous B operand and U_11^-T as the A operand, two 32-deep halves each
+#pragma unroll
+    for (int i = 0; i < 2; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const int r = out_row(i), c = out_col(j, h);
+                smem[(2 + (r >> 5)) * kTileDoubles + c * kStrideKC + (r & 31)] = cur[i][j][h] - acc[i][j][h];
+                acc[i][j][h] = 0.0;
+            }
+    for (int e = threadIdx.x; e < kNB * kNB; e += kThreadsB) {
+        const int k = e % kNB, i = e / kNB;
+        smem[(k >> 5) * kTileDoubles + i * kStrideKC + (k & 31)] = Ub[e];
+    }
+    __syncthreads();
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, gr = lane >> 2, gc = lane & 3;
+    const int wm = (warp & 3) * 16, wn = (warp >> 2) * 32;
+#pragma unroll
+    for (int half = 0; half < 2; ++half) {
+        const double* a = smem + half * kTileDoubles;
+        const double* b = smem + (2 + half) * kTileDoubles;
+#pragma unroll
+        for (int kk = 0; kk < kKS; kk += 4) {
+            double af[2], bf[4];
+#pragma unroll
+            for (int i = 0; i < 2; ++i) af[i] = frag<true>(a, wm + 8 * i + gr, kk + gc);
+#pragma unroll
+            for (int j = 0; j < 4; ++j) bf[j] = frag<true>(b, wn + 8 * j + gr, kk + gc);
+#pragma unroll
+            for (int i = 0; i < 2; ++i)
+#pragma unroll
+                for (int j = 0; j < 4; ++j) dmma(acc[i][j], af[i], bf[j]);
+        }
+    }
 #pragma unroll
     for (int i = 0; i < 2; ++i)
 #pragma unroll
@@ -307,21 +446,22 @@ __global__ void __launch_bounds__(kThreadsB) bc_panel_row_kernel(double* __restr
             }
 }
 
-// A_22 -= U_12^T U_12 on the upper 64 x 64 tiles (ti <= tj) of the trailing matrix.
-// Tiles first .. first + gridDim.x - 1 of the upper-tile enumeration (t = tj (tj + 1) / 2 + ti).
+// A_22 -= U_12^T U_12 over the row blocks that the next panel and row kernels do not update
+// themselves: the upper 64 x 64 tiles (ti <= tj) of the matrix from row j0 + 128 on, enumerated as
+// t = tj (tj + 1) / 2 + ti.  Each tile's current entries are loaded first, so that their latency
+// overlaps the product.
 __global__ void __launch_bounds__(kThreadsB, 2) bc_trailing_kernel(double* __restrict__ U, int n, int j0,
-                                                                   const int* status, int first) {
+                                                                   const int* status) {
     extern __shared__ double smem[];
     if (failed(status)) return;
-    const int jb = min(kNB, n - j0), j1 = j0 + jb;
-    const long long b = (long long)blockIdx.x + first;
+    const int j2 = j0 + 2 * kNB;
+    const long long b = blockIdx.x;
     int tj = (int)((sqrt(8.0 * (double)b + 1.0) - 1.0) * 0.5);
     while ((long long)tj * (tj + 1) / 2 > b) --tj;
     while ((long long)(tj + 1) * (tj + 2) / 2 <= b) ++tj;
     const int ti = (int)(b - (long long)tj * (tj + 1) / 2);
-    const int r0 = j1 + kNB * ti, c0 = j1 + kNB * tj;
-    const Opnd P{U + j0, n, n, jb};
-    // the tile's current entries are loaded first, so that their latency overlaps the product
+    const int r0 = j2 + kNB * ti, c0 = j2 + kNB * tj;
+    const Opnd P{U + j0, n, n, kNB};
     double cur[2][4][2];
 #pragma unroll
     for (int i = 0; i < 2; ++i)
@@ -333,7 +473,7 @@ __global__ void __launch_bounds__(kThreadsB, 2) bc_trailing_kernel(double* __res
                 cur[i][j][h] = (r <= c && c < n) ? U[r + (long long)c * n] : 0.0;
             }
     double acc[2][4][2] = {};
-    tile_product<true, true>(P, P, r0, c0, 0, jb, smem, acc);
+    tile_product<true, true>(P, P, r0, c0, 0, kNB, smem, acc);
 #pragma unroll
     for (int i = 0; i < 2; ++i)
 #pragma unroll
@@ -404,7 +544,7 @@ namespace {
 struct AuxStream {
     int device = -1;
     cudaStream_t stream = nullptr;
-    cudaEvent_t block_ready = nullptr, panel_done = nullptr;
+    cudaEvent_t row_done = nullptr, trailing_done[2] = {nullptr, nullptr};
 };
 std::mutex g_aux_mutex;
 std::vector<AuxStream> g_aux_free;
@@ -427,10 +567,10 @@ cudaError_t acquire_aux(AuxStream* out) {
     int least = 0, greatest = 0;
     err = cudaDeviceGetStreamPriorityRange(&least, &greatest);
     if (err == cudaSuccess) err = cudaStreamCreateWithPriority(&a.stream, cudaStreamNonBlocking, greatest);
-    if (err == cudaSuccess) err = cudaEventCreateWithFlags(&a.block_ready, cudaEventDisableTiming);
-    if (err == cudaSuccess) err = cudaEventCreateWithFlags(&a.panel_done, cudaEventDisableTiming);
+    if (err == cudaSuccess) err = cudaEventCreateWithFlags(&a.row_done, cudaEventDisableTiming);
+    for (cudaEvent_t& e : a.trailing_done)
+        if (err == cudaSuccess) err = cudaEventCreateWithFlags(&e, cudaEventDisableTiming);
     if (err != cudaSuccess) return err;
-    // a fresh event counts as complete, so the first waits on it return at once
     *out = a;
     return cudaSuccess;
 }
@@ -459,31 +599,33 @@ cudaError_t blocked_cholesky(const double* M, int n, double* U, double* Ui, void
     if (err != cudaSuccess) return err;
     const long long total = (long long)n * n;
     bc_init_kernel<<<(unsigned)std::min<long long>(4096, (total + 255) / 256), 256, 0, s>>>(M, U, n);
-    // Look-ahead: after the panel row, the trailing update's first tile (the next panel's
-    // diagonal block) runs alone, then the next panel's factorization goes to a high-priority
-    // auxiliary stream while the other tiles run on s, so that the one-CTA panel takes an SM as
-    // soon as a trailing CTA retires; the next panel row waits for it.
+    // Look-ahead: the chain panel J, row J, panel J + 1, row J + 1, ... runs on a high-priority
+    // auxiliary stream, each kernel applying the previous panel's update to its own blocks; the
+    // trailing update of panel J (row blocks J + 2 on) runs on s and has until panel J + 2.
     AuxStream aux;
     if ((err = acquire_aux(&aux)) != cudaSuccess) return err;
-    bc_panel_kernel<<<1, kThreadsB, kPanelSmem, s>>>(U, Ub, Ui, n, 0, status);
+    err = cudaEventRecord(aux.row_done, s);
+    if (err == cudaSuccess) err = cudaStreamWaitEvent(aux.stream, aux.row_done, 0);
     for (int j0 = 0; j0 < n && err == cudaSuccess; j0 += kNB) {
-        const int j1 = std::min(n, j0 + kNB);
+        const cudaEvent_t trailing = aux.trailing_done[(j0 / kNB) & 1];
+        if (j0 >= 2 * kNB && (err = cudaStreamWaitEvent(aux.stream, trailing, 0)) != cudaSuccess) break;
+        bc_panel_kernel<<<1, kThreadsB, kPanelSmem, aux.stream>>>(U, Ub, Ui, n, j0, status);
+        const int j1 = j0 + kNB;
         if (j1 >= n) break;
-        const int m = n - j1, nt = (m + kNB - 1) / kNB;
-        const long long tiles = (long long)nt * (nt + 1) / 2;
-        if (j0 > 0 && (err = cudaStreamWaitEvent(s, aux.panel_done, 0)) != cudaSuccess) break;
-        bc_panel_row_kernel<<<nt, kThreadsB, kProductSmem, s>>>(U, Ub, n, j0, status);
-        bc_trailing_kernel<<<1, kThreadsB, kProductSmem, s>>>(U, n, j0, status, 0);
-        if ((err = cudaEventRecord(aux.block_ready, s)) != cudaSuccess) break;
-        if ((err = cudaStreamWaitEvent(aux.stream, aux.block_ready, 0)) != cudaSuccess) break;
-        bc_panel_kernel<<<1, kThreadsB, kPanelSmem, aux.stream>>>(U, Ub, Ui, n, j1, status);
-        if ((err = cudaEventRecord(aux.panel_done, aux.stream)) != cudaSuccess) break;
-        if (tiles > 1)
-            bc_trailing_kernel<<<(unsigned)(tiles - 1), kThreadsB, kProductSmem, s>>>(U, n, j0, status, 1);
+        bc_panel_row_kernel<<<(n - j1 + kNB - 1) / kNB, kThreadsB, kProductSmem, aux.stream>>>(U, Ub, n, j0, status);
+        const int m = n - j1 - kNB;
+        if (m > 0) {
+            if ((err = cudaEventRecord(aux.row_done, aux.stream)) != cudaSuccess) break;
+            if ((err = cudaStreamWaitEvent(s, aux.row_done, 0)) != cudaSuccess) break;
+            const long long nt = (m + kNB - 1) / kNB;
+            bc_trailing_kernel<<<(unsigned)(nt * (nt + 1) / 2), kThreadsB, kProductSmem, s>>>(U, n, j0, status);
+            if ((err = cudaEventRecord(trailing, s)) != cudaSuccess) break;
+        }
         err = cudaGetLastError();
     }
-    // join: the last panel on the auxiliary stream precedes the rest of s
-    const cudaError_t join = cudaStreamWaitEvent(s, aux.panel_done, 0);
+    // join: the chain precedes the rest of s
+    cudaError_t join = cudaEventRecord(aux.row_done, aux.stream);
+    if (join == cudaSuccess) join = cudaStreamWaitEvent(s, aux.row_done, 0);
     if (err == cudaSuccess) err = join;
     release_aux(aux);
     if (Ui) {

@@ -181,3 +181,38 @@ def test_grid_barrier_timeout_is_reported_and_the_context_stays_usable():
             c.set_barrier_spin_limit(-1)
     finally:
         c.close()
+
+
+@pytest.mark.parametrize("n", [98, 112, 127, 128, 129, 144, 191, 192, 193, 257, 320, 705])
+def test_blocked_cholesky_panel_edges(ctx, n):
+    """Sizes at and around the 64-column panels and the 16-column blocks inside them (one, two,
+    three and more panels: the look-ahead chain's first links)."""
+    S = O.conditioned_metric(n, 1e4, seed=n)
+    U = vbcore.metric_cholesky(ctx, S)
+    assert np.array_equal(U, np.triu(U))
+    assert np.linalg.norm(U.T @ U - S) / np.linalg.norm(S) < 4e-15 * n ** 0.5
+
+
+@pytest.mark.parametrize("bad", [1, 16, 17, 33, 64, 65, 80, 128, 129, 200])
+def test_blocked_cholesky_failing_minor_at_block_edges(ctx, bad):
+    n = 200
+    S = O.conditioned_metric(n, 1e2, seed=bad)
+    S[bad - 1, bad - 1] = -1.0
+    with pytest.raises(vbcore.VbError) as e:
+        vbcore.metric_cholesky(ctx, S)
+    assert e.value.status == 4 and e.value.info == bad
+
+
+@pytest.mark.parametrize("n", [1, 2, 3, 7, 47, 48, 49, 63, 64, 65, 130, 300, 700])
+def test_lowest_root_sizes(ctx, n):
+    """Davidson at the edges of its 64-row tiles and of the 48-vector subspace: full subspaces
+    (n <= 48), the thick restart and the shift-invert phase.  The eigenvalue of a vector with
+    relative residual 1e-11 is off by less than 1e-11 cond(S) of the spectrum's scale."""
+    H = _random_symmetric(n, 300 + n) + np.diag(np.linspace(-3.0, 8.0, n))
+    S = O.conditioned_metric(n, 1e3, seed=400 + n)
+    e, c, its = vbcore.lowest_root(ctx, H, S, tolerance=1e-11)
+    wr, _ = O.generalized_eigh(H, S)
+    assert abs(e - wr[0]) < 1e-8 * np.abs(wr).max()
+    assert abs(c @ S @ c - 1.0) < 1e-9
+    r = H @ c - e * (S @ c)
+    assert np.linalg.norm(r) < 1e-10 * (np.linalg.norm(H @ c) + abs(e) * np.linalg.norm(S @ c))

@@ -105,6 +105,18 @@ void* context_scratch(vb_context* ctx, int slot, size_t bytes, vb_status* status
     return p;
 }
 
+void* context_pinned(vb_context* ctx, vb_status* status) {
+    *status = VB_OK;
+    if (!ctx->pinned) {
+        const cudaError_t err = cudaMallocHost(&ctx->pinned, kContextPinnedBytes);
+        if (err != cudaSuccess) {
+            ctx->pinned = nullptr;
+            *status = cuda_error(ctx, err, "cudaMallocHost");
+        }
+    }
+    return ctx->pinned;
+}
+
 }  // namespace vbcore
 
 using namespace vbcore;
@@ -173,6 +185,7 @@ vb_status vb_context_destroy(vb_context* ctx) {
         cudaDeviceSynchronize();
         cudaMemPoolDestroy(ctx->pool);
     }
+    if (ctx->pinned) cudaFreeHost(ctx->pinned);
     delete ctx;
     return VB_OK;
 }

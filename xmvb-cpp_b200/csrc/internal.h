@@ -18,6 +18,7 @@ struct vb_context {
     // in order on its stream): the determinant-pair bands and the structure-reduce buffers
     void* scratch[6] = {nullptr, nullptr, nullptr, nullptr, nullptr, nullptr};
     size_t scratch_bytes[6] = {0, 0, 0, 0, 0, 0};
+    void* pinned = nullptr;  // kContextPinnedBytes of page-locked host memory for small read-backs
     size_t budget = 0;
     long long barrier_spin_limit = 0;  // grid-barrier polls before a timeout (0: the built-in default)
     size_t current = 0;
@@ -82,6 +83,11 @@ cudaError_t allow_dynamic_smem(const void* kernel, size_t bytes);
 // Slot `slot` (< 6) of the context's execute scratch, grown to at least `bytes` (contents are
 // not kept across growth); nullptr with *status set on failure.
 void* context_scratch(vb_context* ctx, int slot, size_t bytes, vb_status* status);
+
+// The context's page-locked buffer for small read-backs (allocated at the first use, freed with the
+// context); nullptr with *status set on failure.
+constexpr size_t kContextPinnedBytes = 4096;
+void* context_pinned(vb_context* ctx, vb_status* status);
 
 // Budgeted device allocation; returns nullptr (and records VB_ERR_BUDGET / VB_ERR_CUDA) on failure.
 void* device_alloc(vb_context* ctx, size_t bytes, vb_status* status);

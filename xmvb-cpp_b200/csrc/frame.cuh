@@ -1,0 +1,116 @@
+// Layout and per-pair algebra of the left-string frame, shared by the forward kernels
+// (spin_frame.cu) and the gradient's (gradient_frame.cu).
+#pragma once
+
+#include <cuda_runtime.h>
+#include <math.h>
+#include <stdint.h>
+
+#include "kernels.h"
+
+namespace vbcore {
+
+// The (hole position x particle) grid and the 8-bit particle masks hold up to eight complement
+// orbitals.  A block is laid out for fr_nbmin(K) of them (a closed shell's n - K = K fits) or, for
+// more, for all eight: an open shell's minority spin has n - K > K.  On the exact path the 5
+// beta electrons of a 12-orbital triplet took 1895 us of the evaluation's 2290 us; here the
+// whole evaluation takes 528 us.
+constexpr int kFrameMaxComplement = 8;
+__host__ __device__ constexpr int fr_nbmin(int K) { return K <= 4 ? K + 4 : K; }
+__host__ __device__ constexpr bool fr_wide(int n, int K) { return n - K > fr_nbmin(K); }
+__host__ __device__ constexpr int fr_nb(bool wide, int K) { return wide ? kFrameMaxComplement : fr_nbmin(K); }
+__host__ __device__ constexpr int fr_kfs(int K) { return 8 * K + 4; }  // 8 columns per hole position + trace block
+__host__ __device__ constexpr int fr_cp(int K) { return K * (K - 1) / 2; }
+__host__ __device__ constexpr int fr_bp(bool wide, int K) { return fr_nb(wide, K) * (fr_nb(wide, K) - 1) / 2; }
+
+// Layout of one left string's block (doubles; every part starts on a 2-double boundary).
+struct FrameLayout {
+    int rows;    // table rows: 0 = h, 1 = two-electron linear part, 2 + m = factor column m; padded to 8
+    int kfs;     // table row stride
+    int o_q;     // Q[bp * CP + cp]
+    int o_p;     // P[b * K + c]
+    int o_rowsq; // sum_c S(o, L_c)^2 for o = L_0 .. L_{K-1}, then o = Lbar_0 .. Lbar_{NB-1}
+    int o_prow2; // sum_c P(b, c)^2
+    int o_scal;  // det S_LL, ||Sinv||_F^2, sum_c rowsq(L_c)
+    int total;
+};
+
+__host__ __device__ inline int even_up(int x) { return (x + 1) / 2 * 2; }
+
+__host__ __device__ inline FrameLayout frame_layout(int n, int K, int R) {
+    const bool wide = fr_wide(n, K);
+    FrameLayout f{};
+    f.rows = (R + 2 + 7) / 8 * 8;
+    f.kfs = fr_kfs(K);
+    int o = f.rows * f.kfs;
+    f.o_q = o;
+    o += even_up(fr_bp(wide, K) * fr_cp(K));
+    f.o_p = o;
+    o += even_up(fr_nb(wide, K) * K);
+    f.o_rowsq = o;
+    o += even_up(K + fr_nb(wide, K));
+    f.o_prow2 = o;
+    o += even_up(fr_nb(wide, K));
+    f.o_scal = o;
+    o += 4;
+    f.total = o;
+    return f;
+}
+
+__device__ __forceinline__ void mma_f64(double (&c)[2], double a, double b) {
+    asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};"
+                 : "+d"(c[0]), "+d"(c[1])
+                 : "d"(a), "d"(b));
+}
+
+__device__ __forceinline__ uint64_t occ_mask(uint64_t w, int k) {
+    uint64_t m = 0;
+    for (int c = 0; c < k; ++c) m |= 1ull << ((w >> (8 * c)) & 0xFFu);
+    return m;
+}
+
+// The certificate of kernels.h for X = P[R, :] S_LL with B^-1 = A / detb, without the division:
+// ||X||_F^2 from the row norms, ||X^-1||_F <= ||S_LL^-1||_F ||P[R, :]^-1||_F and
+// ||P[R, :]^-1||_F^2 <= (K - E) + ||B^-1||_F^2 (1 + sum_i ||P[p_i, :]||^2).
+template <int K, int E>
+__device__ __forceinline__ bool frame_certificate(const double* __restrict__ blk, const FrameLayout& F,
+                                                  const int (&hc)[E > 0 ? E : 1], const int (&pb)[E > 0 ? E : 1],
+                                                  double na2, double detb) {
+    const double* scal = blk + F.o_scal;
+    const double* rowsq = blk + F.o_rowsq;
+    const double* prow2 = blk + F.o_prow2;
+    double nx2 = scal[2], pr = 0.0;
+#pragma unroll
+    for (int j = 0; j < E; ++j) {
+        nx2 += rowsq[K + pb[j]] - rowsq[hc[j]];
+        pr += prow2[pb[j]];
+    }
+    const double det2 = detb * detb;
+    const double lhs = nx2 * scal[1] * ((double)(K - E) * det2 + na2 * (1.0 + pr));
+    return isfinite(lhs) && det2 > 0.0 && lhs < kCertificate2 * det2;
+}
+
+// An uncertified pair is still evaluated here, by polynomials in the entries of B, when the frame is
+// sound: kappa_F(S_LL)^2 below this bound leaves P = S[:, L] S_LL^-1 with an error near 1e4 eps at
+// worst (of order eps for the near-orthogonal orbitals of a stretched geometry).
+constexpr double kFrameCondition2 = 1.0e8;
+
+__host__ __device__ constexpr int pair_slot(int x, int y) { return x < y ? y * (y - 1) / 2 + x : x * (x - 1) / 2 + y; }
+// n-th element of {0, 1, ...} without i1 < i2
+__host__ __device__ constexpr int nth_other(int i1, int i2, int n) {
+    int r = n;
+    if (r >= i1) ++r;
+    if (r >= i2) ++r;
+    return r;
+}
+
+// Slots of adj B: an E <= 5 pair's 25 doubles (stride 26 spreads a tile's pairs over banks).  Higher
+// levels use fewer pairs per chunk with E^2 + 1 doubles per slot in the same 32 x 26 doubles of the
+// warp: 16 pairs for E = 6, 7, 8 pairs for E = 8.
+constexpr int kMinorsEMax = 5;
+constexpr int kCompactSlot = 26;
+
+__host__ __device__ constexpr int compact_chunk_pairs(int e) { return e <= kMinorsEMax ? 32 : (e <= 7 ? 16 : 8); }
+__host__ __device__ constexpr int compact_slot(int e) { return e <= kMinorsEMax ? kCompactSlot : e * e + 1; }
+
+}  // namespace vbcore

@@ -40,6 +40,7 @@
 #include <vector>
 
 #include "device_algebra.cuh"
+#include "frame_adjoint.h"
 #include "internal.h"
 #include "kernels.h"
 #include "pair_value.cuh"
@@ -81,7 +82,7 @@ struct AdjArgs {
     double lambda;
     double* adj_a;
     double* adj_b;
-    int adj_stride;  // R + 2: [u adjoint (R)], adj(det), adj(H)
+    int adj_stride;  // R + 2, rounded up to even: [u adjoint (R)], adj(det), adj(H)
 };
 
 // With shared alpha/beta string tables and a spin-flip symmetric determinant list (the flipped
@@ -955,7 +956,7 @@ extern "C" vb_status vb_hs_plan_gradient(vb_hs_plan* p, const double* S, const d
         return st;
     }
     const int n = p->n, np = p->np, gd = p->gd, R = p->R;
-    const int adj_stride = R + 2;
+    const int adj_stride = (R + 2 + 1) / 2 * 2;  // even: 16-byte rows
     // scratch: w, coefficients, adjoint records, gradient accumulators
     const size_t n_gS = (size_t)n * n, n_gG = (size_t)std::max(gd, 1) * std::max(gd, 1), n_gL = (size_t)np * np;
     const size_t acc_doubles = 2 * n_gS + n_gG + n_gL;
@@ -1048,7 +1049,59 @@ extern "C" vb_status vb_hs_plan_gradient(vb_hs_plan* p, const double* S, const d
         err = cudaMemsetAsync(b.careful_count, 0, sizeof(unsigned long long), s);
         if (err != cudaSuccess) break;
         const bool fast = k <= 8 && frame_spin_supported(n, k, R);
-        if (fast) {
+        const DeviceBuffer& tables = beta ? p->tables_b : p->tables_a;
+        // the frame form (gradient_frame.cu) folds the same-spin two-electron energy into the factor
+        // columns; a gradient per packed integral keeps its table separate (the map from factor
+        // columns to integrals loses accuracy with the kernel's condition)
+        DeviceBuffer blocks, sums;
+        bool frame = !deri_out && tables.ptr && frame_adjoint_supported(n, k, R);
+        if (frame) {
+            st = blocks.allocate(ctx, sizeof(double) * frame_adjoint_block_doubles(n, k, R) * b.N);
+            if (st == VB_OK)
+                st = sums.allocate(ctx, sizeof(double) * kAdjointMaxParts * ((size_t)np * R + 2 * (size_t)n * n));
+            if (st != VB_OK && st != VB_ERR_BUDGET) return st;
+            if (st == VB_ERR_BUDGET) {  // no room for the blocks: the pair-by-pair form works in chunks
+                blocks.release();
+                frame = false;
+            }
+        }
+        auto listed_pairs = [&](unsigned long long* listed) {
+            cudaError_t e = cudaMemcpyAsync(listed, b.careful_count, sizeof(*listed), cudaMemcpyDeviceToHost, s);
+            return e == cudaSuccess ? cudaStreamSynchronize(s) : e;
+        };
+        if (frame) {
+            FrameAdjointArgs f{};
+            f.n = n;
+            f.k = k;
+            f.n_strings = b.N;
+            f.R = R;
+            f.r_pos = p->r_pos;
+            f.occ = b.occ;
+            f.S = dS;
+            f.h = dh;
+            f.lf = b.lf;
+            f.ld = np;
+            f.tables = tables.as<double>();
+            f.rlist = (beta ? p->rlist_b : p->rlist_a).as<int>();
+            f.rdesc = (beta ? p->rdesc_b : p->rdesc_a).as<unsigned>();
+            f.ebound = (beta ? p->ebound_b : p->ebound_a).as<int>();
+            f.adj = b.adj;
+            f.adj_stride = adj_stride;
+            f.task_counter = p->counters.as<unsigned long long>() + 4 + beta;
+            f.careful_count = b.careful_count;
+            f.careful_list = b.careful_list;
+            f.out = blocks.as<double>();
+            f.partial = sums.as<double>();
+            f.gL = gL;
+            f.gS = gS;
+            f.gh = gh;
+            err = cudaMemsetAsync(f.task_counter, 0, sizeof(unsigned long long), s);
+            if (err == cudaSuccess) err = launch_frame_adjoint(f, s);
+            unsigned long long listed = 0;
+            if (err == cudaSuccess) err = listed_pairs(&listed);
+            if (err != cudaSuccess) break;
+            if ((st = careful_chunks(ctx, b, (long long)listed, 0, partial.as<double>())) != VB_OK) return st;
+        } else if (fast) {
             // chunks of whole work items (left string u, right strings v0 .. v0 + 127): per chunk
             // Q = L_f^T adj_U (the u-adjoint contracted with every factor column at every packed
             // pair), the backward kernel (writes P = A scattered onto packed pairs), then
@@ -1104,8 +1157,7 @@ extern "C" vb_status vb_hs_plan_gradient(vb_hs_plan* p, const double* S, const d
             }
             if (err != cudaSuccess) break;
             unsigned long long listed = 0;
-            err = cudaMemcpyAsync(&listed, b.careful_count, sizeof(listed), cudaMemcpyDeviceToHost, s);
-            if (err == cudaSuccess) err = cudaStreamSynchronize(s);
+            err = listed_pairs(&listed);
             if (err != cudaSuccess) break;
             if ((st = careful_chunks(ctx, b, (long long)listed, 0, partial.as<double>())) != VB_OK) return st;
         } else {

@@ -253,7 +253,7 @@ vb_status vb_hs_plan_create(vb_context* ctx, const vb_expansion* ex, vb_hs_plan*
     if (!p->shared_tables &&
         (st = p->list_b.allocate(ctx, sizeof(unsigned long long) * std::max(1LL, p->npairs_b))) != VB_OK)
         return fail(st);
-    if ((st = p->counters.allocate(ctx, 8 * sizeof(unsigned long long))) != VB_OK) return fail(st);
+    if ((st = p->counters.allocate(ctx, kPlanCounters * sizeof(unsigned long long))) != VB_OK) return fail(st);
     // right strings of every left string bucketed by hole set (depends on the strings only), and
     // the per-left-string frame tables, sized for the largest factor rank
     for (int beta = 0; beta < 2; ++beta) {
@@ -466,6 +466,7 @@ SpinTableArgs table_args(vb_hs_plan* p, bool beta, const double* S, const double
     a.rec_stride = record_stride(p->R);
     a.careful_count = p->counters.as<unsigned long long>() + (beta ? 1 : 0);
     a.careful_list = beta ? p->list_b.as<unsigned long long>() : p->list_a.as<unsigned long long>();
+    a.uncertified = p->counters.as<unsigned long long>() + 8 + (beta ? 1 : 0);
     a.items = nullptr;
     a.n_items = 0;
     a.all_careful = (beta ? p->tables_b : p->tables_a).ptr ? 0 : 1;
@@ -575,7 +576,7 @@ vb_status prepare_spin_records(vb_hs_plan* p, const double* S, const double* h, 
         }
     }
     PhaseMark spin(p, VB_PHASE_SPIN_PAIRS);
-    err = cudaMemsetAsync(p->counters.ptr, 0, 8 * sizeof(unsigned long long), s);
+    err = cudaMemsetAsync(p->counters.ptr, 0, kPlanCounters * sizeof(unsigned long long), s);
     if (err != cudaSuccess) return cuda_error(ctx, err, "cudaMemsetAsync");
     if (p->ka > 0) {
         err = launch_spin_pairs(table_args(p, false, *dS, *dh, *deri), p->tables_a.as<double>(), s, launches);
@@ -801,7 +802,7 @@ vb_status vb_hs_plan_stats(const vb_hs_plan* p, vb_hs_stats* stats) {
     if (!p || !stats) return VB_ERR_INVALID;
     vb_hs_stats s = p->stats;
     if (p->evaluated) {
-        unsigned long long c[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+        unsigned long long c[kPlanCounters] = {};
         cudaError_t err = cudaMemcpyAsync(c, p->counters.ptr, sizeof(c), cudaMemcpyDeviceToHost, p->ctx->stream);
         if (err == cudaSuccess) err = cudaStreamSynchronize(p->ctx->stream);
         if (err != cudaSuccess) return cuda_error(p->ctx, err, "stats download");
@@ -811,7 +812,7 @@ vb_status vb_hs_plan_stats(const vb_hs_plan* p, vb_hs_stats* stats) {
         };
         const bool all_a = p->ka > 0 && all_exact(p->ka, p->tables_a);
         const bool all_b = p->kb > 0 && !p->shared_tables && all_exact(p->kb, p->tables_b);
-        s.careful_spin_pairs = (long long)(all_a ? p->npairs_a : c[0]) + (long long)(all_b ? p->npairs_b : c[1]);
+        s.careful_spin_pairs = (long long)(all_a ? p->npairs_a : c[0]) + (long long)(all_b ? p->npairs_b : c[1]) + (long long)(c[8] + c[9]);
     }
     *stats = s;
     return VB_OK;

@@ -35,6 +35,8 @@ struct SpinTableArgs {
     int rec_stride;
     unsigned long long* careful_count;
     unsigned long long* careful_list;  // (u << 32) | v
+    // pairs evaluated outside the certificate by the frame kernel; null: it lists those instead
+    unsigned long long* uncertified;
     const int2* items;                 // fast-kernel work items: (left string u, first right string v0)
     int n_items;
     int all_careful;  // 1: every pair takes the exact path

@@ -669,8 +669,10 @@ cudaError_t launch_spin_pairs(const SpinTableArgs& a, double* tables, cudaStream
         const int tuned = autotune_run(
             key, frame_pair_variants(a.n, a.k, a.R), stream, [&](int v) { return launch_frame_pairs(a, tables, stream, v); },
             [&]() {
-                // the listed-pair counter and the task counter
+                // the counters of listed and uncertified pairs and the task counter
                 cudaError_t e = cudaMemsetAsync(a.careful_count, 0, sizeof(unsigned long long), stream);
+                if (e == cudaSuccess && a.uncertified)
+                    e = cudaMemsetAsync(a.uncertified, 0, sizeof(unsigned long long), stream);
                 if (e == cudaSuccess) e = cudaMemsetAsync(a.task_counter, 0, sizeof(unsigned long long), stream);
                 return e;
             },

@@ -19,6 +19,8 @@ struct BandSegments {
     DeviceBuffer tiles, tile_off;
 };
 
+constexpr int kPlanCounters = 10;
+
 struct vb_hs_plan {
     vb_context* ctx = nullptr;
     int n = 0, ka = 0, kb = 0, np = 0, gd = 0;
@@ -32,7 +34,7 @@ struct vb_hs_plan {
     long long npairs_a = 0, npairs_b = 0;
     // counters: [0, 1] listed (exact-path) spin pairs alpha/beta, [2, 3] the gradient's listed
     // pairs, [4, 5] the frame kernel's task counters alpha/beta, [7] the band reduction's
-    // timeout flag
+    // timeout flag, [8, 9] pairs the frame kernel evaluated outside the certificate alpha/beta
     DeviceBuffer counters, list_a, list_b;
     // right strings of each left string bucketed by hole set (see SpinTableArgs::rlist)
     DeviceBuffer rlist_a, rlist_b, rdesc_a, rdesc_b, ebound_a, ebound_b;

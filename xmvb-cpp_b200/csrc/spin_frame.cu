@@ -31,18 +31,21 @@
 //    Q, and the norms of the conditioning certificate;
 //  * spin_pairs_frame<K> (persistent): a CTA takes left strings from a counter, stages the
 //    string's block in shared memory, and its warps take chunks of 32 pairs of one excitation
-//    level E (so every lane runs the same compile-time-E code).  Phase A, a lane per pair: B,
-//    Gauss-Jordan with partial pivoting, sign, certificate, quadratic two-electron term, and the
-//    pair's row Y' (W scattered onto the grid, 1 in the trace slot) to shared memory.  Phase B,
-//    per 8-pair tile: [h | 2e-linear | u] / det X = Y' Table^T on the FP64 tensor cores
-//    (mma.sync m8n8k4), k-steps only over the hole positions present in the tile (pairs are
-//    sorted by hole set, so a tile's union is usually its own hole set).
-// Blocks failing the certificate go to the exact path (spin_pairs_exact) through the list.
+//    level E (so every lane runs the same compile-time-E code).  Phase A, a lane per pair: adj B,
+//    det B and the quadratic two-electron term by minors (E <= 5; a pivoted inverse above), sign and
+//    certificate; adj B goes to shared memory.  Phase B, per 8-pair tile: [h | 2e-linear | u] =
+//    D [adj B | det B] Table^T on the FP64 tensor cores (mma.sync m8n8k4), k-steps only over the
+//    hole positions present in the tile (pairs are sorted by hole set, so a tile's union is usually
+//    its own hole set).
+// Pairs failing the certificate are evaluated all the same by their polynomials at E <= 5 (every
+// quantity above times det B is a polynomial in B) unless S_LL itself is ill conditioned; the rest go
+// to the exact path (spin_pairs_exact) through the list.
 #include <cuda_runtime.h>
 #include <math.h>
 #include <stdint.h>
 
 #include "device_algebra.cuh"
+#include "frame.cuh"
 #include "internal.h"
 #include "kernels.h"
 #include "pair_value.cuh"
@@ -53,65 +56,6 @@ namespace {
 constexpr int kFrameWarps = 4;  // warps per CTA of the bucketing kernel
 constexpr int kFrameThreads = 32 * kFrameWarps;
 constexpr int kFrameMaxWarps = 8;  // warps per CTA of the pair kernel: a launch variant (2, 4 or 8)
-
-// The (hole position x particle) grid and the 8-bit particle masks hold up to eight complement
-// orbitals.  A block is laid out for fr_nbmin(K) of them (a closed shell's n - K = K fits) or, for
-// more, for all eight: an open shell's minority spin has n - K > K.  On the exact path the 5
-// beta electrons of a 12-orbital triplet took 1895 us of the evaluation's 2290 us; here the
-// whole evaluation takes 528 us.
-constexpr int kFrameMaxComplement = 8;
-__host__ __device__ constexpr int fr_nbmin(int K) { return K <= 4 ? K + 4 : K; }
-__host__ __device__ constexpr bool fr_wide(int n, int K) { return n - K > fr_nbmin(K); }
-__host__ __device__ constexpr int fr_nb(bool wide, int K) { return wide ? kFrameMaxComplement : fr_nbmin(K); }
-__host__ __device__ constexpr int fr_kfs(int K) { return 8 * K + 4; }  // 8 columns per hole position + trace block
-__host__ __device__ constexpr int fr_cp(int K) { return K * (K - 1) / 2; }
-__host__ __device__ constexpr int fr_bp(bool wide, int K) { return fr_nb(wide, K) * (fr_nb(wide, K) - 1) / 2; }
-
-// Layout of one left string's block (doubles; every part starts on a 2-double boundary).
-struct FrameLayout {
-    int rows;    // table rows: 0 = h, 1 = two-electron linear part, 2 + m = factor column m; padded to 8
-    int kfs;     // table row stride
-    int o_q;     // Q[bp * CP + cp]
-    int o_p;     // P[b * K + c]
-    int o_rowsq; // sum_c S(o, L_c)^2 for o = L_0 .. L_{K-1}, then o = Lbar_0 .. Lbar_{NB-1}
-    int o_prow2; // sum_c P(b, c)^2
-    int o_scal;  // det S_LL, ||Sinv||_F^2, sum_c rowsq(L_c)
-    int total;
-};
-
-__host__ __device__ inline int even_up(int x) { return (x + 1) / 2 * 2; }
-
-__host__ __device__ inline FrameLayout frame_layout(int n, int K, int R) {
-    const bool wide = fr_wide(n, K);
-    FrameLayout f{};
-    f.rows = (R + 2 + 7) / 8 * 8;
-    f.kfs = fr_kfs(K);
-    int o = f.rows * f.kfs;
-    f.o_q = o;
-    o += even_up(fr_bp(wide, K) * fr_cp(K));
-    f.o_p = o;
-    o += even_up(fr_nb(wide, K) * K);
-    f.o_rowsq = o;
-    o += even_up(K + fr_nb(wide, K));
-    f.o_prow2 = o;
-    o += even_up(fr_nb(wide, K));
-    f.o_scal = o;
-    o += 4;
-    f.total = o;
-    return f;
-}
-
-__device__ __forceinline__ void mma_f64(double (&c)[2], double a, double b) {
-    asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};"
-                 : "+d"(c[0]), "+d"(c[1])
-                 : "d"(a), "d"(b));
-}
-
-__device__ __forceinline__ uint64_t occ_mask(uint64_t w, int k) {
-    uint64_t m = 0;
-    for (int c = 0; c < k; ++c) m |= 1ull << ((w >> (8 * c)) & 0xFFu);
-    return m;
-}
 
 // Hole mask of (L, R): bit c set when L's c-th orbital is not in R.
 template <int K>
@@ -543,23 +487,39 @@ size_t frame_tables_smem(int n, int R) {
     return sizeof(double) * ((sc * kZS > 4096 ? sc * kZS : 4096) + 64 * kXS + 3 * (size_t)kTableWarps * 64);
 }
 
-// Phase A of one pair at excitation level E (compile time).  Writes the pair's Y' row and
-// returns the certificate, det X, the quadratic two-electron term / det X and the hole mask.
-// COMPACT: W is stored in canonical order (hole slot j, particle slot i) at yrow[j E + i] and the
-// slot maps are returned (*hmap: nibble c = hole slot of position c, *pmap: nibble b = particle
-// slot of complement index b, 0xF elsewhere); otherwise W is scattered on the pair's dense row
-// (zeroed beforehand) with 1 in the trace slot.
-template <int K, int E, bool COMPACT>
-__device__ __forceinline__ void frame_pair(const double* __restrict__ blk, const FrameLayout& F, unsigned desc,
-                                           double* __restrict__ yrow, bool* ok_out, double* det_out,
-                                           double* quad_out, unsigned* hm_out, unsigned* hmap_out,
-                                           unsigned* pmap_out) {
+// What phase A leaves of one pair: d = sign det S_LL, detb = det B, quad = the quadratic two-electron
+// term times det B, the hole mask and the slot maps (hmap: nibble c = hole slot of position c, pmap:
+// nibble b = particle slot of complement index b, 0xF elsewhere).  adj B = det B B^-1 goes to
+// yrow[j E + i] (hole slot j, particle slot i).
+struct FramePair {
+    double d, detb, quad;
+    unsigned hm, hmap, pmap;
+    bool ok;         // evaluated here (else listed for the exact path)
+    bool certified;  // well conditioned under the certificate
+};
+
+// Phase A at excitation level E <= 5, by minors: every quantity is a polynomial in the E x E entries
+// of B = P[p, h], so nothing is divided by det B and blocks of any rank come out right (in the
+// reference's terms: singular values below its 1e-12 are not truncated, a difference of that order).
+// For each particle pair I (ascending) the minors m(J^c) of the other E - 2 rows over the columns
+// outside the hole pair J give the quadratic term, as the 2 x 2 minors of B^-1 are
+// (-1)^(I + J) m / det B (Jacobi); one more row of the Laplace expansion gives adj B, the last one
+// det B.  700 multiply-adds at E = 5 and 160 at E = 4 (36 % of the pairs at K = 7), no division and
+// no pivoting: the Gauss-Jordan inverse with row selects before it needed both (n = 14, 5.9 M
+// certified pairs: 1378 -> 1280 us for the kernel).  Uncertified pairs no longer go to the
+// one-thread-per-block exact path: 14 stretched hydrogen atoms, 268 ms -> 1.3 ms here and 3.0 ms for
+// the levels E >= 6.
+template <int K, int E>
+__device__ __forceinline__ FramePair frame_pair_minors(const double* __restrict__ blk, const FrameLayout& F,
+                                                       unsigned desc, double* __restrict__ yrow) {
     constexpr int CP = fr_cp(K);
-    const unsigned hm = desc & 0xFFu;
-    // holes (positions in L, ascending) and particles (Lbar indices, ascending)
-    int hc[E > 0 ? E : 1], pb[E > 0 ? E : 1];
+    constexpr int EE = E > 0 ? E : 1;
+    constexpr int NP = E > 1 ? E * (E - 1) / 2 : 1;
+    FramePair o;
+    o.hm = desc & 0xFFu;
+    int hc[EE], pb[EE];  // holes (positions in L) and particles (Lbar indices), ascending
     {
-        unsigned h = hm, pm = (desc >> 8) & 0xFFu;
+        unsigned h = o.hm, pm = (desc >> 8) & 0xFFu;
 #pragma unroll
         for (int j = 0; j < E; ++j) {
             hc[j] = __ffs(h) - 1;
@@ -569,12 +529,137 @@ __device__ __forceinline__ void frame_pair(const double* __restrict__ blk, const
         }
     }
     const double* P = blk + F.o_p;
-    double x[E > 0 ? E : 1][E > 0 ? E : 1];
+    double b[EE][EE];
+#pragma unroll
+    for (int i = 0; i < E; ++i)
+#pragma unroll
+        for (int j = 0; j < E; ++j) b[i][j] = P[pb[i] * K + hc[j]];
+    double detb = 1.0, quad = 0.0, na2 = 0.0;
+    if constexpr (E == 1) {
+        detb = b[0][0];
+        na2 = 1.0;
+        yrow[0] = 1.0;
+    }
+    if constexpr (E >= 2) {
+        const double* Q = blk + F.o_q;
+        int cp[NP];
+#pragma unroll
+        for (int j2 = 1; j2 < E; ++j2)
+#pragma unroll
+            for (int j1 = 0; j1 < j2; ++j1) cp[pair_slot(j1, j2)] = hc[j2] * (hc[j2] - 1) / 2 + hc[j1];
+        // row i of the cofactors from the minors m of rows (all but i and r) by expansion along row r
+        auto cofactor_row = [&](const double (&m)[NP], int i, int r, bool last) {
+#pragma unroll
+            for (int j = 0; j < E; ++j) {
+                double acc = 0.0;
+#pragma unroll
+                for (int t = 0; t < E - 1; ++t) {
+                    const int c = t < j ? t : t + 1;
+                    const double v = b[r][c] * m[pair_slot(j, c)];
+                    acc = ((E - 2 + t) & 1) ? acc - v : acc + v;
+                }
+                if ((i + j) & 1) acc = -acc;
+                yrow[j * E + i] = acc;
+                na2 = fma(acc, acc, na2);
+                if (last) detb = j == 0 ? b[i][j] * acc : fma(b[i][j], acc, detb);
+            }
+        };
+#pragma unroll
+        for (int i2 = 1; i2 < E; ++i2)
+#pragma unroll
+            for (int i1 = 0; i1 < i2; ++i1) {
+                double m[NP];
+                if constexpr (E == 2) {
+                    m[0] = 1.0;
+                } else if constexpr (E == 3) {
+                    const int ra = nth_other(i1, i2, 0);
+#pragma unroll
+                    for (int j2 = 1; j2 < E; ++j2)
+#pragma unroll
+                        for (int j1 = 0; j1 < j2; ++j1) m[pair_slot(j1, j2)] = b[ra][nth_other(j1, j2, 0)];
+                } else if constexpr (E == 4) {
+                    const int ra = nth_other(i1, i2, 0), rb = nth_other(i1, i2, 1);
+#pragma unroll
+                    for (int j2 = 1; j2 < E; ++j2)
+#pragma unroll
+                        for (int j1 = 0; j1 < j2; ++j1) {
+                            const int x = nth_other(j1, j2, 0), y = nth_other(j1, j2, 1);
+                            m[pair_slot(j1, j2)] = fma(b[ra][x], b[rb][y], -b[ra][y] * b[rb][x]);
+                        }
+                } else {
+                    const int ra = nth_other(i1, i2, 0), rb = nth_other(i1, i2, 1), rc = nth_other(i1, i2, 2);
+                    double m2[NP];
+#pragma unroll
+                    for (int y = 1; y < E; ++y)
+#pragma unroll
+                        for (int x = 0; x < y; ++x) m2[pair_slot(x, y)] = fma(b[ra][x], b[rb][y], -b[ra][y] * b[rb][x]);
+#pragma unroll
+                    for (int j2 = 1; j2 < E; ++j2)
+#pragma unroll
+                        for (int j1 = 0; j1 < j2; ++j1) {
+                            const int x = nth_other(j1, j2, 0), y = nth_other(j1, j2, 1), z = nth_other(j1, j2, 2);
+                            m[pair_slot(j1, j2)] =
+                                fma(b[rc][x], m2[pair_slot(y, z)],
+                                    fma(-b[rc][y], m2[pair_slot(x, z)], b[rc][z] * m2[pair_slot(x, y)]));
+                        }
+                }
+                const double* q = Q + (pb[i2] * (pb[i2] - 1) / 2 + pb[i1]) * CP;
+                double part = 0.0;
+#pragma unroll
+                for (int j2 = 1; j2 < E; ++j2)
+#pragma unroll
+                    for (int j1 = 0; j1 < j2; ++j1) {
+                        const double v = m[pair_slot(j1, j2)];
+                        part = fma(((i1 + i2 + j1 + j2) & 1) ? -v : v, q[cp[pair_slot(j1, j2)]], part);
+                    }
+                quad += part;
+                if (i2 == E - 1) {
+                    cofactor_row(m, i1, E - 1, false);
+                    if (i1 == E - 2) cofactor_row(m, E - 1, E - 2, true);
+                }
+            }
+    }
+    const double* scal = blk + F.o_scal;
+    o.d = ((desc >> 16) & 1u ? -1.0 : 1.0) * scal[0];
+    o.detb = detb;
+    o.quad = quad;
+    o.certified = frame_certificate<K, E>(blk, F, hc, pb, na2, detb);
+    o.ok = o.certified || (scal[1] * scal[2] < kFrameCondition2 && isfinite(detb) && isfinite(na2) && isfinite(quad));
+    o.hmap = o.pmap = 0xFFFFFFFFu;
+#pragma unroll
+    for (int j = 0; j < E; ++j) {
+        o.hmap &= ~((0xFu ^ (unsigned)j) << (4 * hc[j]));
+        o.pmap &= ~((0xFu ^ (unsigned)j) << (4 * pb[j]));
+    }
+    return o;
+}
+
+// Phase A at the levels E >= 6 (about 1.5 % of the pairs at K = 7): Gauss-Jordan inverse of B with
+// partial pivoting; uncertified blocks are listed.
+template <int K, int E>
+__device__ __forceinline__ FramePair frame_pair_inverse(const double* __restrict__ blk, const FrameLayout& F,
+                                                        unsigned desc, double* __restrict__ yrow) {
+    constexpr int CP = fr_cp(K);
+    FramePair o;
+    o.hm = desc & 0xFFu;
+    int hc[E], pb[E];
+    {
+        unsigned h = o.hm, pm = (desc >> 8) & 0xFFu;
+#pragma unroll
+        for (int j = 0; j < E; ++j) {
+            hc[j] = __ffs(h) - 1;
+            h &= h - 1;
+            pb[j] = __ffs(pm) - 1;
+            pm &= pm - 1;
+        }
+    }
+    const double* P = blk + F.o_p;
+    double x[E][E];
 #pragma unroll
     for (int i = 0; i < E; ++i)
 #pragma unroll
         for (int j = 0; j < E; ++j) x[i][j] = P[pb[i] * K + hc[j]];
-    int lab[E > 0 ? E : 1];
+    int lab[E];
 #pragma unroll
     for (int i = 0; i < E; ++i) lab[i] = i;
     double detb = 1.0;
@@ -619,128 +704,81 @@ __device__ __forceinline__ void frame_pair(const double* __restrict__ blk, const
             for (int j = 0; j < E; ++j) x[i][j] = fma(-f, x[s][j], x[i][j]);
         }
     }
-    // x[j][jj] = W(j, lab[jj]): hole slot j, particle slot lab[jj]
-    const double* scal = blk + F.o_scal;
-    const double det = ((desc >> 16) & 1u ? -1.0 : 1.0) * scal[0] * detb;
-    double nw2 = 0.0;
+    // x[j][jj] = B^-1(j, lab[jj]): hole slot j, particle slot lab[jj]
+    double na2 = 0.0;
 #pragma unroll
     for (int i = 0; i < E; ++i)
 #pragma unroll
-        for (int j = 0; j < E; ++j) nw2 = fma(x[i][j], x[i][j], nw2);
-    const double* rowsq = blk + F.o_rowsq;
-    const double* prow2 = blk + F.o_prow2;
-    double nx2 = scal[2], pr = 0.0;
-#pragma unroll
-    for (int j = 0; j < E; ++j) {
-        nx2 += rowsq[K + pb[j]] - rowsq[hc[j]];
-        pr += prow2[pb[j]];
-    }
-    const double bnd = scal[1] * ((double)(K - E) + nw2 * (1.0 + pr));
-    const bool ok = isfinite(det) && det != 0.0 && (nx2 * bnd < kCertificate2);
+        for (int j = 0; j < E; ++j) {
+            const double v = detb * x[i][j];
+            na2 = fma(v, v, na2);
+        }
     // packed particle Lbar indices by slot, to read the particle of a permuted column
     uint64_t bword = 0;
 #pragma unroll
     for (int i = 0; i < E; ++i) bword |= (uint64_t)pb[i] << (8 * i);
-    int bj[E > 0 ? E : 1];
+    int bj[E];
 #pragma unroll
     for (int jj = 0; jj < E; ++jj) bj[jj] = (int)((bword >> (8 * lab[jj])) & 0xFFu);
     double quad = 0.0;
-    if (E >= 2) {
-        const double* Q = blk + F.o_q;
+    const double* Q = blk + F.o_q;
 #pragma unroll
-        for (int j1 = 0; j1 < E; ++j1)
+    for (int j1 = 0; j1 < E; ++j1)
 #pragma unroll
-            for (int j2 = j1 + 1; j2 < E; ++j2) {
-                const int cp = hc[j2] * (hc[j2] - 1) / 2 + hc[j1];
-                double part = 0.0;
+        for (int j2 = j1 + 1; j2 < E; ++j2) {
+            const int cp = hc[j2] * (hc[j2] - 1) / 2 + hc[j1];
+            double part = 0.0;
 #pragma unroll
-                for (int jj1 = 0; jj1 < E; ++jj1)
+            for (int jj1 = 0; jj1 < E; ++jj1)
 #pragma unroll
-                    for (int jj2 = jj1 + 1; jj2 < E; ++jj2) {
-                        const int ba = bj[jj1], bb = bj[jj2];
-                        const bool ordered = ba < bb;
-                        const int lo = ordered ? ba : bb, hi = ordered ? bb : ba;
-                        const double m2 = fma(x[j1][jj1], x[j2][jj2], -x[j1][jj2] * x[j2][jj1]);
-                        const double qv = Q[(hi * (hi - 1) / 2 + lo) * CP + cp];
-                        part = fma(ordered ? qv : -qv, m2, part);
-                    }
-                quad += part;
-            }
-    }
-    unsigned hmap = 0xFFFFFFFFu, pmap = 0xFFFFFFFFu;
-    if (COMPACT) {
-        if (ok) {
-#pragma unroll
-            for (int j = 0; j < E; ++j) {
-                hmap &= ~(0xFu << (4 * hc[j]));
-                hmap |= (unsigned)j << (4 * hc[j]);
-                pmap &= ~(0xFu << (4 * pb[j]));
-                pmap |= (unsigned)j << (4 * pb[j]);
-#pragma unroll
-                for (int jj = 0; jj < E; ++jj) yrow[j * E + lab[jj]] = x[j][jj];
-            }
+                for (int jj2 = jj1 + 1; jj2 < E; ++jj2) {
+                    const int ba = bj[jj1], bb = bj[jj2];
+                    const bool ordered = ba < bb;
+                    const int lo = ordered ? ba : bb, hi = ordered ? bb : ba;
+                    const double m2 = fma(x[j1][jj1], x[j2][jj2], -x[j1][jj2] * x[j2][jj1]);
+                    const double qv = Q[(hi * (hi - 1) / 2 + lo) * CP + cp];
+                    part = fma(ordered ? qv : -qv, m2, part);
+                }
+            quad += part;
         }
-    } else if (ok) {
-        // the pair's row (zeroed by the warp beforehand): W on the (hole position, particle)
-        // grid, 1 in the trace slot
+    o.d = ((desc >> 16) & 1u ? -1.0 : 1.0) * blk[F.o_scal];
+    o.detb = detb;
+    o.quad = detb * quad;
+    o.certified = frame_certificate<K, E>(blk, F, hc, pb, na2, detb);
+    o.ok = o.certified;
+    o.hmap = o.pmap = 0xFFFFFFFFu;
+    if (o.ok) {
 #pragma unroll
-        for (int j = 0; j < E; ++j)
+        for (int j = 0; j < E; ++j) {
+            o.hmap &= ~((0xFu ^ (unsigned)j) << (4 * hc[j]));
+            o.pmap &= ~((0xFu ^ (unsigned)j) << (4 * pb[j]));
 #pragma unroll
-            for (int jj = 0; jj < E; ++jj) yrow[hc[j] * 8 + bj[jj]] = x[j][jj];
-        yrow[8 * K] = 1.0;
+            for (int jj = 0; jj < E; ++jj) yrow[j * E + lab[jj]] = detb * x[j][jj];
+        }
     }
-    *hmap_out = hmap;
-    *pmap_out = pmap;
-    *ok_out = ok;
-    *det_out = det;
-    *quad_out = quad;
-    *hm_out = hm;
-}
-
-// Compact slots: W of an E <= 5 pair (25 doubles; stride 26 spreads a tile's pairs over banks).
-// Higher levels use fewer pairs per chunk with E^2 + 1 doubles per slot in the same 32 x 26
-// doubles of the warp: 16 pairs for E = 6, 7, 8 pairs for E = 8.
-constexpr int kCompactEMax = 5;
-constexpr int kCompactSlot = 26;
-
-__host__ __device__ constexpr int compact_chunk_pairs(int e) { return e <= kCompactEMax ? 32 : (e <= 7 ? 16 : 8); }
-__host__ __device__ constexpr int compact_slot(int e) { return e <= kCompactEMax ? kCompactSlot : e * e + 1; }
-
-// The high excitation levels (E > kCompactEMax, about 1.5 % of the pairs at K = 7) out of line:
-// their E x E registers do not count against the register budget of the common levels.
-struct PairOut {
-    double det, quad;
-    unsigned hm, hmap, pmap;
-    bool ok;
-};
-
-template <int K, int E>
-__device__ __noinline__ PairOut frame_pair_out_of_line(const double* __restrict__ blk, const FrameLayout* F,
-                                                       unsigned desc, double* __restrict__ yrow) {
-    PairOut o;
-    frame_pair<K, E, true>(blk, *F, desc, yrow, &o.ok, &o.det, &o.quad, &o.hm, &o.hmap, &o.pmap);
     return o;
 }
 
-template <int K, int ELO, int EHI, bool COMPACT>
-__device__ __forceinline__ void frame_pair_dispatch(int e, const double* blk, const FrameLayout& F, unsigned desc,
-                                                    double* yrow, bool* ok, double* det, double* quad, unsigned* hm,
-                                                    unsigned* hmap, unsigned* pmap) {
-#define VB_FRAME_CASE(E_)                                                                             \
-    case E_:                                                                                          \
-        if constexpr (E_ >= ELO && E_ <= EHI && E_ <= K) {                                            \
-            if constexpr (COMPACT && E_ > kCompactEMax) {                                             \
-                const PairOut o = frame_pair_out_of_line<K, E_>(blk, &F, desc, yrow);                 \
-                *ok = o.ok;                                                                           \
-                *det = o.det;                                                                         \
-                *quad = o.quad;                                                                       \
-                *hm = o.hm;                                                                           \
-                *hmap = o.hmap;                                                                       \
-                *pmap = o.pmap;                                                                       \
-            } else {                                                                                  \
-                frame_pair<K, E_, COMPACT>(blk, F, desc, yrow, ok, det, quad, hm, hmap, pmap);         \
-            }                                                                                         \
-        }                                                                                             \
+// The high excitation levels out of line: their E x E registers do not count against the register
+// budget of the common levels.
+template <int K, int E>
+__device__ __noinline__ FramePair frame_pair_out_of_line(const double* __restrict__ blk, const FrameLayout* F,
+                                                         unsigned desc, double* __restrict__ yrow) {
+    return frame_pair_inverse<K, E>(blk, *F, desc, yrow);
+}
+
+template <int K>
+__device__ __forceinline__ FramePair frame_pair_dispatch(int e, const double* blk, const FrameLayout& F, unsigned desc,
+                                                         double* yrow) {
+    FramePair o{};
+#define VB_FRAME_CASE(E_)                                                      \
+    case E_:                                                                   \
+        if constexpr (E_ <= K) {                                               \
+            if constexpr (E_ > kMinorsEMax)                                    \
+                o = frame_pair_out_of_line<K, E_>(blk, &F, desc, yrow);        \
+            else                                                               \
+                o = frame_pair_minors<K, E_>(blk, F, desc, yrow);              \
+        }                                                                      \
         break;
     switch (e) {
         VB_FRAME_CASE(0)
@@ -755,21 +793,19 @@ __device__ __forceinline__ void frame_pair_dispatch(int e, const double* blk, co
         default: break;
     }
 #undef VB_FRAME_CASE
+    return o;
 }
 
-
-__host__ __device__ constexpr int frame_row_doubles(int K, bool compact) { return compact ? kCompactSlot : fr_kfs(K); }
-
-// The pairs of excitation levels ELO .. EHI of every left string.  COMPACT (EHI <= 4): each pair's
-// W is kept as an E x E slot and the tensor-core A fragments are read through the pair's slot
-// maps (a few registers and 4.3 KB of shared memory per warp); otherwise each pair has a dense row
-// on the (hole position x particle) grid.  Task counter: a.task_counter (+2 for the dense kernel).
-template <int K, int ELO, int EHI, bool COMPACT>
-__global__ void __launch_bounds__(32 * kFrameMaxWarps, COMPACT ? 2 : 1)
-    spin_pairs_frame(SpinTableArgs a, const double* __restrict__ tables) {
+// The pairs of every left string.  Each pair's adj B is kept as an E x E slot and the tensor-core A
+// fragments are read through the pair's slot maps (a few registers and 6.6 KB of shared memory per
+// warp).  Uncertified pairs are counted in a.uncertified and evaluated by their polynomials when the
+// frame is sound; when a.uncertified is null they are listed for the exact path instead (whose
+// records carry the reference's nullity).
+template <int K>
+__global__ void __launch_bounds__(32 * kFrameMaxWarps, 2) spin_pairs_frame(SpinTableArgs a,
+                                                                           const double* __restrict__ tables) {
     extern __shared__ double smem[];
     constexpr int KFS = fr_kfs(K);
-    constexpr int ROW = frame_row_doubles(K, COMPACT);
     const int R = a.R;
     const FrameLayout F = frame_layout(a.n, K, R);
     const int NT = F.rows / 8;
@@ -779,11 +815,10 @@ __global__ void __launch_bounds__(32 * kFrameMaxWarps, COMPACT ? 2 : 1)
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int g = lane >> 2, tq = lane & 3;
     const long long N = a.n_strings;
-    double* yw = sY + (size_t)warp * 32 * ROW;
-    unsigned long long* task_counter = a.task_counter + (COMPACT ? 0 : 2);
+    double* yw = sY + (size_t)warp * 32 * kCompactSlot;
     for (;;) {
         if (threadIdx.x == 0) {
-            s_task = (int)atomicAdd(task_counter, 1ull);
+            s_task = (int)atomicAdd(a.task_counter, 1ull);
             s_chunk = 0;
         }
         __syncthreads();
@@ -793,16 +828,6 @@ __global__ void __launch_bounds__(32 * kFrameMaxWarps, COMPACT ? 2 : 1)
         int bound[K + 2];
 #pragma unroll
         for (int e = 0; e < K + 2; ++e) bound[e] = __ldg(eb + e);
-        int nchunks = 0;
-#pragma unroll
-        for (int e = ELO; e <= EHI && e <= K; ++e) {
-            const int cs = COMPACT ? compact_chunk_pairs(e) : 32;
-            nchunks += (bound[e + 1] - bound[e] + cs - 1) / cs;
-        }
-        if (nchunks == 0) {
-            __syncthreads();
-            continue;
-        }
         {
             const double2* src = reinterpret_cast<const double2*>(tables + (long long)u * F.total);
             double2* dst = reinterpret_cast<double2*>(sBlk);
@@ -819,8 +844,8 @@ __global__ void __launch_bounds__(32 * kFrameMaxWarps, COMPACT ? 2 : 1)
             ch = __shfl_sync(0xffffffffu, ch, 0);
             int e = -1, start = 0, cnt = 0, left = ch;
 #pragma unroll
-            for (int ee = (EHI < K ? EHI : K); ee >= ELO; --ee) {
-                const int cs = COMPACT ? compact_chunk_pairs(ee) : 32;
+            for (int ee = K; ee >= 0; --ee) {
+                const int cs = compact_chunk_pairs(ee);
                 const int c = (bound[ee + 1] - bound[ee] + cs - 1) / cs;
                 if (left >= 0 && left < c) {
                     e = ee;
@@ -844,56 +869,50 @@ __global__ void __launch_bounds__(32 * kFrameMaxWarps, COMPACT ? 2 : 1)
             if (e < 0) break;
             claim(&e_next, &cnt_next, &v_next, &d_next);
             const bool valid = lane < cnt;
-            if (!COMPACT) {
-                // zero the warp's 32 rows, consecutive lanes on consecutive 16-byte words
-                double2* z = reinterpret_cast<double2*>(yw);
-#pragma unroll
-                for (int f = lane; f < 16 * KFS; f += 32) z[f] = make_double2(0.0, 0.0);
-                __syncwarp();
-            }
-            const int slot = COMPACT ? compact_slot(e) : ROW;
-            double* yrow = yw + lane * slot;
-            bool ok = false;
-            double det = 0.0, quad = 0.0;
-            unsigned hm = 0, hmap = 0xFFFFFFFFu, pmap = 0xFFFFFFFFu;
+            const int slot = compact_slot(e);
+            FramePair o{};
+            o.hmap = o.pmap = 0xFFFFFFFFu;
             if (valid) {
-                frame_pair_dispatch<K, ELO, EHI, COMPACT>(e, sBlk, F, desc, yrow, &ok, &det, &quad, &hm, &hmap,
-                                                          &pmap);
-                if (!ok) {
-                    const unsigned long long slot = atomicAdd(a.careful_count, 1ull);
-                    a.careful_list[slot] = ((unsigned long long)u << 32) | (unsigned long long)v;
+                o = frame_pair_dispatch<K>(e, sBlk, F, desc, yw + lane * slot);
+                if (!o.certified && !a.uncertified) o.ok = false;
+                if (!o.ok) {
+                    const unsigned long long at = atomicAdd(a.careful_count, 1ull);
+                    a.careful_list[at] = ((unsigned long long)u << 32) | (unsigned long long)v;
                 }
             }
+            const unsigned okbits = __ballot_sync(0xffffffffu, o.ok);
+            const unsigned poly = __ballot_sync(0xffffffffu, o.ok && !o.certified);
+            if (poly && lane == 0) atomicAdd(a.uncertified, (unsigned long long)__popc(poly));
             const long long t = record_index(u, v, N);
-            const unsigned okbits = __ballot_sync(0xffffffffu, ok);
             __syncwarp();
             // phase B, one 8-pair tile at a time
-            const int tiles = COMPACT ? compact_chunk_pairs(e) / 8 : 4;
+            const int tiles = compact_chunk_pairs(e) / 8;
 #pragma unroll 1
             for (int mt = 0; mt < tiles; ++mt) {
-                const unsigned uh = __reduce_or_sync(0xffffffffu, ((lane >> 3) == mt && ok) ? hm : 0u);
+                const unsigned uh = __reduce_or_sync(0xffffffffu, ((lane >> 3) == mt && o.ok) ? o.hm : 0u);
                 if (((okbits >> (8 * mt)) & 0xFFu) == 0) continue;
                 const int owner = 8 * mt + g;
-                const double det_g = __shfl_sync(0xffffffffu, det, owner);
-                const double quad_g = __shfl_sync(0xffffffffu, quad, owner);
+                const double d_g = __shfl_sync(0xffffffffu, o.d, owner);
+                const double detb_g = __shfl_sync(0xffffffffu, o.detb, owner);
+                const double quad_g = __shfl_sync(0xffffffffu, o.quad, owner);
                 const long long t_g = __shfl_sync(0xffffffffu, t, owner);
-                const unsigned hmap_g = __shfl_sync(0xffffffffu, hmap, owner);
-                const unsigned pmap_g = __shfl_sync(0xffffffffu, pmap, owner);
+                const unsigned hmap_g = __shfl_sync(0xffffffffu, o.hmap, owner);
+                const unsigned pmap_g = __shfl_sync(0xffffffffu, o.pmap, owner);
                 const bool ok_g = (okbits >> owner) & 1u;
                 const double* yr = yw + owner * slot;
                 double* rec = a.records + t_g * (long long)a.rec_stride;
                 // this lane's particle slots for the two k-steps of a hole block (b = tq, tq + 4)
                 const unsigned i0 = (pmap_g >> (4 * tq)) & 0xFu, i1 = (pmap_g >> (4 * (tq + 4))) & 0xFu;
-                // the trace from column 7 of each pair's first hole block (compact, level >= 1,
+                // the trace (times det B) from column 7 of each pair's first hole block (level >= 1,
                 // at most 7 complement orbitals) instead of a separate k-step
-                const bool pad_trace = COMPACT && e >= 1 && a.n - K <= 7;
+                const bool pad_trace = e >= 1 && a.n - K <= 7;
 #pragma unroll 1
                 for (int nt0 = 0; nt0 < NT; nt0 += 6) {
                     double acc[6][2];
 #pragma unroll
                     for (int j = 0; j < 6; ++j) acc[j][0] = acc[j][1] = 0.0;
                     if (!pad_trace) {
-                        const double af = COMPACT ? ((tq == 0 && ok_g) ? 1.0 : 0.0) : yr[8 * K + tq];
+                        const double af = (tq == 0 && ok_g) ? detb_g : 0.0;
 #pragma unroll
                         for (int j = 0; j < 6; ++j) {
                             const double bf = (nt0 + j < NT) ? sBlk[(8 * (nt0 + j) + g) * KFS + 8 * K + tq] : 0.0;
@@ -908,14 +927,9 @@ __global__ void __launch_bounds__(32 * kFrameMaxWarps, COMPACT ? 2 : 1)
 #pragma unroll
                         for (int ks = 0; ks < 2; ++ks) {
                             const int col = 8 * c + 4 * ks + tq;
-                            double af;
-                            if (COMPACT) {
-                                const unsigned ip = ks ? i1 : i0;
-                                af = (jh < (unsigned)e && ip < (unsigned)e) ? yr[jh * e + ip] : 0.0;
-                                if (pad_trace && ks == 1 && tq == 3) af = jh == 0 ? 1.0 : 0.0;
-                            } else {
-                                af = yr[col];
-                            }
+                            const unsigned ip = ks ? i1 : i0;
+                            double af = (jh < (unsigned)e && ip < (unsigned)e) ? yr[jh * e + ip] : 0.0;
+                            if (pad_trace && ks == 1 && tq == 3) af = jh == 0 ? detb_g : 0.0;
 #pragma unroll
                             for (int j = 0; j < 6; ++j) {
                                 const double bf = (nt0 + j < NT) ? sBlk[(8 * (nt0 + j) + g) * KFS + col] : 0.0;
@@ -929,13 +943,13 @@ __global__ void __launch_bounds__(32 * kFrameMaxWarps, COMPACT ? 2 : 1)
 #pragma unroll
                             for (int i = 0; i < 2; ++i) {
                                 const int row = 8 * (nt0 + j) + 2 * tq + i;
-                                if (row >= 2 && row < R + 2) rec[row - 2] = det_g * acc[j][i];
+                                if (row >= 2 && row < R + 2) rec[row - 2] = d_g * acc[j][i];
                             }
                         if (nt0 == 0 && tq == 0) {
                             const double h1 = acc[0][0], e2 = acc[0][1];
-                            rec[R + 0] = det_g;
-                            rec[R + 1] = det_g * (h1 + e2 + quad_g);
-                            rec[R + 2] = det_g * h1;
+                            rec[R + 0] = d_g * detb_g;
+                            rec[R + 1] = d_g * (h1 + e2 + quad_g);
+                            rec[R + 2] = d_g * h1;
                             rec[R + 3] = 0.0;
                         }
                     }
@@ -948,14 +962,14 @@ __global__ void __launch_bounds__(32 * kFrameMaxWarps, COMPACT ? 2 : 1)
 }
 
 template <int K>
-size_t frame_spin_smem(int n, int R, int warps = 4, bool compact = false) {
-    return sizeof(double) * ((size_t)frame_layout(n, K, R).total + (size_t)warps * 32 * frame_row_doubles(K, compact));
+size_t frame_spin_smem(int n, int R, int warps) {
+    return sizeof(double) * ((size_t)frame_layout(n, K, R).total + (size_t)warps * 32 * kCompactSlot);
 }
 
 // Shared memory of the largest launch variant (8 warps per CTA).
 template <int K>
 size_t frame_spin_smem_max(int n, int R) {
-    return frame_spin_smem<K>(n, R, 8, true);
+    return frame_spin_smem<K>(n, R, 8);
 }
 
 size_t frame_spin_smem_rt(int n, int k, int R) {
@@ -987,10 +1001,10 @@ cudaError_t launch_tables(const SpinTableArgs& a, double* tables, cudaStream_t s
 constexpr int kFrameVariants = 3;
 constexpr int kFrameVariantWarps[kFrameVariants] = {8, 4, 2};
 
-template <int K, int ELO, int EHI, bool COMPACT>
+template <int K>
 cudaError_t launch_frame_part(const SpinTableArgs& a, const double* tables, cudaStream_t stream, int warps) {
-    const size_t smem = frame_spin_smem<K>(a.n, a.R, warps, COMPACT);
-    auto kernel = spin_pairs_frame<K, ELO, EHI, COMPACT>;
+    const size_t smem = frame_spin_smem<K>(a.n, a.R, warps);
+    auto kernel = spin_pairs_frame<K>;
     cudaError_t err = allow_dynamic_smem((const void*)kernel, smem);
     if (err != cudaSuccess) return err;
     int per_sm = 1, dev = 0, sms = 148;
@@ -1006,7 +1020,7 @@ cudaError_t launch_frame_part(const SpinTableArgs& a, const double* tables, cuda
 
 template <int K>
 cudaError_t launch_frame(const SpinTableArgs& a, const double* tables, cudaStream_t stream, int variant) {
-    return launch_frame_part<K, 0, K, true>(a, tables, stream, kFrameVariantWarps[variant]);
+    return launch_frame_part<K>(a, tables, stream, kFrameVariantWarps[variant]);
 }
 
 template <int K>
@@ -1084,7 +1098,7 @@ cudaError_t preload_k() {
     cudaError_t err = cudaFuncGetAttributes(&fa, (const void*)sort_right_strings<K>);
     if (err == cudaSuccess) err = cudaFuncGetAttributes(&fa, (const void*)frame_tables<K, false>);
     if (err == cudaSuccess) err = cudaFuncGetAttributes(&fa, (const void*)frame_tables<K, true>);
-    if (err == cudaSuccess) err = cudaFuncGetAttributes(&fa, (const void*)spin_pairs_frame<K, 0, K, true>);
+    if (err == cudaSuccess) err = cudaFuncGetAttributes(&fa, (const void*)spin_pairs_frame<K>);
     return err;
 }
 

@@ -216,3 +216,34 @@ def test_lowest_root_sizes(ctx, n):
     assert abs(c @ S @ c - 1.0) < 1e-9
     r = H @ c - e * (S @ c)
     assert np.linalg.norm(r) < 1e-10 * (np.linalg.norm(H @ c) + abs(e) * np.linalg.norm(S @ c))
+
+
+@pytest.mark.parametrize("n", [33, 34, 47, 64, 95, 96, 127, 128, 129, 159, 160])
+@pytest.mark.parametrize("spectrum", ["random", "close", "degenerate", "diagonal", "zero"])
+def test_tridiagonal_eigh_sizes_and_clusters(ctx, n, spectrum):
+    """The tridiagonal path (33 <= n <= 160) at the edges of its tiles, for spread, nearly equal
+    (1e-9 apart) and equal roots, a matrix that is already diagonal, and H = 0.  Backward-stable
+    bounds: residual and S-orthonormality of order n eps cond(S)^(1/2), below 1e-10 here."""
+    rng = np.random.default_rng(n)
+    S = O.conditioned_metric(n, 1e3, seed=n)
+    if spectrum == "random":
+        H = _random_symmetric(n, n + 1)
+    elif spectrum == "diagonal":
+        S, H = np.eye(n), np.diag(rng.permutation(np.arange(n, dtype=np.float64)))
+    elif spectrum == "zero":
+        H = np.zeros((n, n))
+    else:
+        q, _ = np.linalg.qr(rng.standard_normal((n, n)))
+        d = np.repeat(np.arange((n + 4) // 5, dtype=np.float64), 5)[:n]
+        if spectrum == "close":
+            d = d + 1e-9 * np.arange(n)
+        L = np.linalg.cholesky(S)
+        H = L @ ((q * d) @ q.T) @ L.T
+        H = 0.5 * (H + H.T)
+    w, C = vbcore.generalized_eigh(ctx, H, S)
+    wr, _ = O.generalized_eigh(H, S)
+    scale = max(np.abs(wr).max(), 1e-3)
+    assert np.abs(w - wr).max() < 1e-11 * scale
+    assert np.all(np.diff(w) >= 0)
+    assert np.abs(C.T @ S @ C - np.eye(n)).max() < 1e-10
+    assert np.abs(H @ C - S @ C * w).max() < 1e-10 * scale * max(1.0, np.abs(C).max())

@@ -29,6 +29,7 @@
 #include <string>
 #include <vector>
 
+#include "eigh_tridiagonal.h"
 #include "internal.h"
 
 namespace vbcore {
@@ -978,6 +979,35 @@ vb_status run_blocked_cholesky(vb_context* ctx, const double* S, int n, bool hos
     return VB_OK;
 }
 
+// The dense problem through a tridiagonal form; *settled = false when it has to be solved otherwise.
+// Device pointers.
+vb_status run_tridiagonal(vb_context* ctx, const double* H, const double* S, int n, double* values, double* vectors,
+                          int* info, bool* settled, const char* name) {
+    *settled = false;
+    cudaStream_t s = ctx->stream;
+    DeviceBuffer ws;
+    const size_t m2 = sizeof(double) * (size_t)n * n;
+    const size_t chol = align_up(blocked_cholesky_workspace(n, true));
+    vb_status st = ws.allocate(ctx, chol + 2 * m2 + sizeof(double) * tridiagonal_workspace_doubles(n));
+    if (st != VB_OK) return st;
+    unsigned char* base = static_cast<unsigned char*>(ws.ptr);
+    double* U = reinterpret_cast<double*>(base + chol);
+    double* Ui = U + (size_t)n * n;
+    int bad = 0, status = 0;
+    cudaError_t err = blocked_cholesky(S, n, U, Ui, base, &bad, s);
+    if (err != cudaSuccess) return cuda_error(ctx, err, name);
+    if (bad) {
+        if (info) *info = n + bad;
+        return set_error(ctx, VB_ERR_NUMERIC,
+                         std::string(name) + ": overlap_matrix is not positive definite (info=" +
+                             std::to_string(n + bad) + ")");
+    }
+    err = tridiagonal_eigh(H, Ui, n, values, vectors, Ui + (size_t)n * n, &status, s);
+    if (err != cudaSuccess) return cuda_error(ctx, err, name);
+    *settled = status == 0;
+    return VB_OK;
+}
+
 vb_status run_single(vb_context* ctx, int mode, const double* H, const double* S, int n, int mem, double* evals,
                      double* evecs, double* U_out, int* info, const char* name) {
     if (!ctx) return VB_ERR_INVALID;
@@ -1012,7 +1042,21 @@ vb_status run_single(vb_context* ctx, int mode, const double* H, const double* S
         }
         dU = nullptr;
     }
-    if (err == cudaSuccess) err = clear_workspace(base, L, n, mode, s);
+    if (err != cudaSuccess) return cuda_error(ctx, err, name);
+    // the reduction's registers hold the matrix up to kTridiagonalMax (n = 132: 3.3 ms by block Jacobi);
+    // clusters that do not separate there go to Jacobi
+    if (mode == 1 && n >= kTridiagonalMin && n <= kTridiagonalMax) {
+        bool settled = false;
+        if ((st = run_tridiagonal(ctx, dH, dS, n, dvals, dvecs, info, &settled, name)) != VB_OK) return st;
+        if (settled && host) {
+            err = cudaMemcpyAsync(evals, dvals, sizeof(double) * n, cudaMemcpyDeviceToHost, s);
+            if (err == cudaSuccess) err = cudaMemcpyAsync(evecs, dvecs, m2, cudaMemcpyDeviceToHost, s);
+            if (err == cudaSuccess) err = cudaStreamSynchronize(s);
+            if (err != cudaSuccess) return cuda_error(ctx, err, name);
+        }
+        if (settled) return VB_OK;
+    }
+    err = clear_workspace(base, L, n, mode, s);
     if (err != cudaSuccess) return cuda_error(ctx, err, name);
     EighArgs a = args_for(base, L, n, mode, dH, dS, dvals, dvecs, mode == 0 ? dU : nullptr);
     if (ctx->barrier_spin_limit > 0) a.spin_limit = ctx->barrier_spin_limit;

@@ -137,8 +137,9 @@ vb_status vb_hs_plan_execute(vb_hs_plan* plan, const double* ovlp_act, const dou
                              double* overlap_out);
 
 /* Diagnostics of the last execute: spin pairs evaluated, pairs routed to the exact
- * full-pivot/SVD path, unordered determinant pairs evaluated (with alpha/beta-exchange
- * symmetry one pair per orbit {(d, e), (flip d, flip e)}), kernel launches, and the number of
+ * full-pivot/SVD path or evaluated outside the conditioning certificate, distinct unordered
+ * determinant pairs (with alpha/beta-exchange symmetry one pair per orbit {(d, e),
+ * (flip d, flip e)}), kernel launches, and the number of
  * columns of the pivoted LDL^T factorization of the pair kernel (ij|kl) (its numerical rank). */
 typedef struct {
     int64_t spin_pairs;

@@ -164,3 +164,63 @@ def test_root_gradient_matches_separate_steps(ctx, kw, n, seed):
     for key in ("S", "h", "ri"):
         assert np.abs(g[key] - gr[key]).max() < 1e-8 * max(1.0, np.abs(gr[key]).max()), key
     plan.close()
+
+
+def _graded_overlap(n, rate, power, seed):
+    dist = np.abs(np.subtract.outer(np.arange(n), np.arange(n))).astype(float)
+    sign = np.sign(_sym(np.random.default_rng(seed), n))
+    return np.exp(-rate * dist ** power) * (np.triu(sign, 1) + np.triu(sign, 1).T + np.eye(n))
+
+
+@pytest.mark.parametrize("kw,n,nel,mult", [("COV", 4, 2, 1), ("COV ION(1)", 5, 4, 1), ("COV", 7, 7, 2), ("COV", 8, 8, 3),
+                                           ("COV ION(1)", 8, 8, 1), ("COV", 10, 10, 1), ("COV", 11, 11, 4),
+                                           ("COV", 12, 12, 1), ("COV", 13, 13, 2)])
+@pytest.mark.parametrize("overlap", ["random", "chain", "orthogonal"])
+def test_frame_gradient_matches_pair_by_pair(ctx, kw, n, nel, mult, overlap):
+    """The gradient in the left strings' frames (the path without packed integrals) against the
+    pair-by-pair kernels (the path with them) for 1 .. 7 electrons per string, equal and unequal
+    string tables, all excitation levels, well conditioned and exactly singular blocks.  Both are
+    exact derivatives; the pair-by-pair form subtracts terms of size G / |X| (inverse of a block of
+    norm |X|), which leaves eps G / |X|: below 1e-11 for these overlaps (|X| > 1e-4 or X = 0), but
+    up to 1e-4 for graded ones, which the next test takes against differences."""
+    rng = np.random.default_rng(100 * n + nel)
+    S = {"random": lambda: workloads.active_space(n, 3 * n, 70 + n)[0],
+         "chain": lambda: np.exp(-0.8 * np.abs(np.subtract.outer(np.arange(n), np.arange(n)))),
+         "orthogonal": lambda: np.eye(n)}[overlap]()
+    h = _sym(rng, n)
+    P = n * (n + 1) // 2
+    F = 0.05 * rng.standard_normal((P, P)) + 0.1 * np.eye(P)
+    eri = workloads.pack_pair_kernel(F @ F.T)
+    rows = vbcore.generate_structures(kw, n, nel, mult)
+    plan = vbcore.HsPlan(ctx, vbcore.expand_structures(rows, nel, mult), n)
+    c = rng.standard_normal(plan.n_structures)
+    c /= np.linalg.norm(c)
+    a = plan.gradient(S, h, eri, c, -1.3, packed_eri=False, ri_factors=F)
+    b = plan.gradient(S, h, eri, c, -1.3, packed_eri=True, ri_factors=F)
+    for key in ("S", "h", "ri"):
+        assert np.abs(a[key] - b[key]).max() < 1e-8 * max(1e-3, np.abs(b[key]).max()), key
+    plan.close()
+
+
+@pytest.mark.parametrize("kw,n,nel,mult", [("COV", 4, 2, 1), ("COV", 8, 8, 1), ("COV", 7, 7, 2), ("COV ION(1)", 6, 6, 1)])
+def test_frame_gradient_graded_overlaps(ctx, kw, n, nel, mult):
+    """Overlaps S_ij = +-exp(-3 |i - j|^2) (0.05, 6e-6, 2e-12, ...): most blocks are outside the
+    conditioning certificate or rank deficient under the reference semantics.  Against Richardson
+    differences of the oracle's energy (step 1e-4, error of order 1e-9)."""
+    S = _graded_overlap(n, 3.0, 2, n)
+    rng = np.random.default_rng(31 * n)
+    h = _sym(rng, n)
+    P = n * (n + 1) // 2
+    F = 0.05 * rng.standard_normal((P, P)) + 0.1 * np.eye(P)
+    eri = workloads.pack_pair_kernel(F @ F.T)
+    plan, ex_o, lam, c = _setup(ctx, kw, n, nel, mult, S, h, eri)
+    g = plan.gradient(S, h, eri, c, lam, packed_eri=False, ri_factors=F)
+    for (i, j) in ((0, 1), (2, 2), (1, 3), (0, n - 1)):
+        E = np.zeros((n, n))
+        E[i, j] = E[j, i] = 1.0
+        fd = _richardson(lambda t: _energy(n, ex_o, S + t * E, h, eri), 1e-4)
+        assert abs(fd - np.sum(g["S"] * E)) < 1e-7 * max(1.0, abs(fd)), (i, j, fd, np.sum(g["S"] * E))
+    dF = rng.standard_normal(F.shape)
+    fd = _richardson(lambda t: _energy(n, ex_o, S, h, workloads.pack_pair_kernel((F + t * dF) @ (F + t * dF).T)), 1e-4)
+    assert abs(fd - np.sum(g["ri"] * dF)) < 1e-7 * max(1.0, abs(fd))
+    plan.close()

@@ -307,3 +307,28 @@ def test_wide_complements_take_the_frame_kernel(ctx, kw, n, nel, mult):
     assert _rel(H, Hr) < REL and _rel(So, Sr) < REL
     st = plan.stats()
     assert st["careful_spin_pairs"] <= st["spin_pairs"] // 100
+
+
+@pytest.mark.parametrize("kw,n,nel,mult", [("COV ION(1)", 8, 8, 1), ("COV ION(1)", 9, 9, 2), ("COV ION(1)", 8, 8, 3),
+                                           ("COV ION(1)", 10, 10, 1), ("COV ION(1-2)", 8, 8, 1), ("FULL", 6, 6, 1),
+                                           ("COV ION(1)", 9, 8, 1)])
+def test_block_ordered_determinants_match_oracle(ctx, kw, n, nel, mult):
+    """Determinant lists that fill blocks of alpha x beta strings (5 x 5 to 8 x 8, with and without
+    empty cells, equal and unequal string tables, sets cut into several blocks): structure matrices
+    against the oracle, through host and device pointers, and determinant pairs in the caller's order."""
+    S, h, eri = workloads.active_space(n, 2 * n, 80 + n)
+    plan, ex = _plan(ctx, kw, n, nel, mult)
+    H, So = plan.execute(S, h, eri)
+    Hr, Sr, _ = O.structure_matrices(n, ex, S, h, eri, threads=8)
+    assert _rel(H, Hr) < REL and _rel(So, Sr) < REL
+    H2, S2 = plan.execute(S, h, eri)
+    assert np.array_equal(H, H2) and np.array_equal(So, S2)
+    rng = np.random.default_rng(n)
+    pairs = rng.integers(0, plan.expansion.n_determinants, size=(500, 2))
+    ho, so = plan.determinant_pairs(S, h, eri, pairs)
+    a, b = plan.expansion.occupations(), plan.expansion.occupations(beta=True)
+    for q, (d, e) in enumerate(pairs[:100]):
+        x = S[np.ix_(a[e], a[d])]
+        y = S[np.ix_(b[e], b[d])]
+        ref = np.linalg.det(x) * np.linalg.det(y)
+        assert abs(so[q] - ref) < 1e-11 * max(1.0, abs(ref))

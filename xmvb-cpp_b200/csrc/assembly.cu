@@ -27,8 +27,12 @@ constexpr int kZPad = kBandColumns + 1;
 
 __device__ __forceinline__ unsigned smem_addr(const void* p) { return (unsigned)__cvta_generic_to_shared(p); }
 
-__device__ __forceinline__ void mbar_init(unsigned long long* bar) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_addr(bar)) : "memory");
+__device__ __forceinline__ void mbar_init(unsigned long long* bar, unsigned arrivals) {
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_addr(bar)), "r"(arrivals) : "memory");
+}
+
+__device__ __forceinline__ void copy_async16(void* dst, const void* src) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_addr(dst)), "l"(src) : "memory");
 }
 
 __device__ __forceinline__ void mbar_expect_tx(unsigned long long* bar, unsigned bytes) {
@@ -83,6 +87,13 @@ __device__ __forceinline__ void bulk_load(void* dst, const void* src, unsigned b
 // Tiles that reach below the diagonal have their entries d > e zeroed in shared memory first,
 // so the term loop carries no mask.  The accumulators then pass through shared memory so that
 // Z is written in coalesced runs of structures.
+//
+// GATHER (block-ordered determinant lists): a structure group's rows lie anywhere, so a tile is a list
+// of 64 of them, copied by cp.async (16 bytes per thread and copy; completion through the stage's
+// mbarrier, one arrival per thread).  The n = 12 covalent + ionic groups have 252 to 504 rows each, 4 to
+// 8 full tiles; with rows only grouped by structure a group met 30 partly used ones.  Both forms take
+// 10.1 to 10.4 ms there; a bulk copy per 256-byte row ran at 110 cycles a copy (16.7 ms).
+template <bool GATHER>
 __global__ void __launch_bounds__(kBandWarps * 32, 3)
     band_reduce_kernel(const __grid_constant__ CUtensorMap map_h, const __grid_constant__ CUtensorMap map_s,
                        BandReduceArgs a, int stage_bytes) {
@@ -96,18 +107,16 @@ __global__ void __launch_bounds__(kBandWarps * 32, 3)
     const long long b = nb - 1 - (long long)blockIdx.x / G;
     const int g = (int)(blockIdx.x % G);
     const long long col0 = b * kBandColumns;
-    long long rows = a.e0 + col0 + kBandColumns;
-    if (rows > a.n_det) rows = a.n_det;
-    const int ntiles = (int)((rows + kBandTileRows - 1) / kBandTileRows);
     const int seg_max = a.seg_max;
-    // the group's row tiles with terms (ascending), up to the last one this column block reaches
-    const int* tl = a.seg_tiles + a.seg_tile_off[g];
-    int nt = a.seg_tile_off[g + 1] - a.seg_tile_off[g];
+    // the group's row tiles (ascending), up to the last one this column block reaches
+    const int t_begin = a.seg_tile_off[g];
+    int nt = a.seg_tile_off[g + 1] - t_begin;
     {
+        const long long last = a.e0 + col0 + kBandColumns - 1;  // largest column of the block
         int lo = 0, hi = nt;
         while (lo < hi) {
             const int mid = (lo + hi) >> 1;
-            if (tl[mid] < ntiles)
+            if (a.seg_first[t_begin + mid] <= last)
                 lo = mid + 1;
             else
                 hi = mid;
@@ -115,31 +124,46 @@ __global__ void __launch_bounds__(kBandWarps * 32, 3)
         nt = lo;
     }
 
-    // stage st <- the i-th listed tile
+    // stage st <- the i-th tile: thread 0 by TMA, or (GATHER) every thread its share of the rows
+    constexpr int kRowChunks = kBandColumns * 8 / 16;  // 16-byte pieces of a row
     auto issue = [&](int i, int st) {
-        const int t = tl[i];
+        const int t = t_begin + i;
         unsigned char* base = bsm + (size_t)st * stage_bytes;
-        const long long seg = (long long)g * a.n_tiles + t;
-        const long long o0 = a.seg_off[seg];
-        const unsigned len = (unsigned)(a.seg_off[seg + 1] - o0);
-        mbar_expect_tx(&full[st], 2u * kTileBytes + 9u * len + kBandMetaBytes);
-        tma_band_tile(base, &map_h, (int)col0, t * kBandTileRows, &full[st]);
-        tma_band_tile(base + kTileBytes, &map_s, (int)col0, t * kBandTileRows, &full[st]);
+        if (GATHER) {
+            for (int q = tid; q < kBandTileRows * kRowChunks; q += kBandWarps * 32) {
+                const int row = a.seg_rows[(long long)t * kBandTileRows + q / kRowChunks], piece = q % kRowChunks;
+                if (row < 0) continue;
+                const long long at = row * a.ldb + col0 + 2 * piece;
+                copy_async16(base + 16 * q, a.Hb + at);
+                copy_async16(base + kTileBytes + 16 * q, a.Sb + at);
+            }
+            asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(smem_addr(&full[st])) : "memory");
+            if (tid != 0) return;
+        }
+        const long long o0 = a.seg_off[t];
+        const unsigned len = (unsigned)(a.seg_off[t + 1] - o0);
+        mbar_expect_tx(&full[st], (GATHER ? 0u : 2u * kTileBytes) + 9u * len + kBandMetaBytes);
+        if (!GATHER) {
+            tma_band_tile(base, &map_h, (int)col0, a.seg_first[t], &full[st]);
+            tma_band_tile(base + kTileBytes, &map_s, (int)col0, a.seg_first[t], &full[st]);
+        }
         if (len) {
             bulk_load(base + 2 * kTileBytes, a.term_c + o0, 8u * len, &full[st]);
             bulk_load(base + 2 * kTileBytes + 8 * seg_max, a.term_d + o0, len, &full[st]);
         }
-        bulk_load(base + 2 * kTileBytes + 9 * seg_max, a.seg_meta + seg * kBandMetaBytes, kBandMetaBytes, &full[st]);
+        bulk_load(base + 2 * kTileBytes + 9 * seg_max, a.seg_meta + (long long)t * kBandMetaBytes, kBandMetaBytes, &full[st]);
     };
+    const bool issuer = GATHER || tid == 0;
 
     if (tid == 0) {
-        mbar_init(&full[0]);
-        mbar_init(&full[1]);
+        // thread 0 arrives with the expected bytes, and (GATHER) every thread when its copies landed
+        mbar_init(&full[0], GATHER ? 1 + kBandWarps * 32 : 1);
+        mbar_init(&full[1], GATHER ? 1 + kBandWarps * 32 : 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     __syncthreads();
-    int issued = 0;  // tiles issued so far (thread 0)
-    if (tid == 0 && nt > 0) {
+    int issued = 0;  // tiles issued so far (the issuing threads)
+    if (issuer && nt > 0) {
         issue(0, 0);
         if (nt > 1) issue(1, 1);
         issued = nt > 1 ? 2 : 1;
@@ -158,16 +182,17 @@ __global__ void __launch_bounds__(kBandWarps * 32, 3)
     for (; ok && i < nt; ++i) {
         const int st = i & 1;
         unsigned char* base = bsm + (size_t)st * stage_bytes;
-        const long long r0 = (long long)tl[i] * kBandTileRows;
-        if (r0 + kBandTileRows - 1 > a.e0 + col0) {
+        const int r0 = a.seg_first[t_begin + i];
+        if (a.seg_last[t_begin + i] > a.e0 + col0) {
             // rows below the diagonal of this column block hold no data: zero them
             double* zH = reinterpret_cast<double*>(base);
             double* zS = zH + kBandTileRows * kBandColumns;
-            for (int i = tid; i < kBandTileRows * kBandColumns; i += blockDim.x) {
-                const int dl = i / kBandColumns, l = i % kBandColumns;
-                if (r0 + dl > a.e0 + col0 + l) {
-                    zH[i] = 0.0;
-                    zS[i] = 0.0;
+            const int* listed = GATHER ? a.seg_rows + (long long)(t_begin + i) * kBandTileRows : nullptr;
+            for (int q = tid; q < kBandTileRows * kBandColumns; q += blockDim.x) {
+                const int dl = q / kBandColumns, l = q % kBandColumns;
+                if ((GATHER ? listed[dl] : r0 + dl) > a.e0 + col0 + l) {
+                    zH[q] = 0.0;
+                    zS[q] = 0.0;
                 }
             }
             // these generic-proxy writes precede the stage's next TMA fill
@@ -196,7 +221,7 @@ __global__ void __launch_bounds__(kBandWarps * 32, 3)
         }
         const bool next = i + 1 >= nt || mbar_wait(&full[st ^ 1], (unsigned)((i + 1) >> 1) & 1u, limit);
         ok = __syncthreads_and(next) != 0;
-        if (ok && tid == 0 && i + 2 < nt) {
+        if (ok && issuer && i + 2 < nt) {
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
             issue(i + 2, st);
             ++issued;
@@ -205,6 +230,7 @@ __global__ void __launch_bounds__(kBandWarps * 32, 3)
     if (!ok) {
         // a tile never landed: flag it, let the copies still in flight land (a generous bound of
         // its own: no copy may outlive the CTA), and leave
+        if (GATHER) asm volatile("cp.async.wait_all;" ::: "memory");
         if (tid == 0) {
             atomicExch(a.error, 1);
             for (int u = i; u < issued; ++u) mbar_wait(&full[u & 1], (unsigned)(u >> 1) & 1u, kDrainPolls);
@@ -340,10 +366,11 @@ cudaError_t launch_band_reduce(const BandReduceArgs& a, cudaStream_t stream, int
     if (!band_tensor_map(&mh, a.Hb, a.width, a.n_det, a.ldb) || !band_tensor_map(&ms, a.Sb, a.width, a.n_det, a.ldb))
         return cudaErrorInvalidValue;
     const size_t smem = band_reduce_smem_bytes(a.seg_max);
-    cudaError_t err = allow_dynamic_smem((const void*)band_reduce_kernel, smem);
+    const auto kernel = a.seg_rows ? band_reduce_kernel<true> : band_reduce_kernel<false>;
+    cudaError_t err = allow_dynamic_smem((const void*)kernel, smem);
     if (err != cudaSuccess) return err;
     const long long blocks = (a.width + kBandColumns - 1) / kBandColumns * a.n_groups;
-    band_reduce_kernel<<<(unsigned)blocks, kBandWarps * 32, smem, stream>>>(mh, ms, a, band_stage_bytes(a.seg_max));
+    kernel<<<(unsigned)blocks, kBandWarps * 32, smem, stream>>>(mh, ms, a, band_stage_bytes(a.seg_max));
     ++*launches;
     return cudaGetLastError();
 }

@@ -10,7 +10,9 @@
 // (src/vbscf/structures/assembly/hamiltonian_overlap.hpp:70-107 in the reference).
 #include <algorithm>
 #include <cstring>
+#include <map>
 #include <new>
+#include <set>
 #include <string>
 #include <vector>
 
@@ -96,6 +98,138 @@ struct PhaseMark {
     ~PhaseMark() { close(); }
 };
 
+// Blocks of (at most 8 alpha strings) x (at most 8 beta strings) that the determinant list fills (see
+// BlockPairArgs); block h holds determinants first[h] .. first[h + 1] - 1 of the new order.
+struct DeterminantBlocks {
+    int n = 0, max_a = 0, max_b = 0, max_dets = 0;
+    std::vector<int> first;
+    std::vector<BlockStrings> strings;
+};
+
+// Determinants with the same alpha-only orbitals (alpha minus beta) pair a set of alpha strings with a
+// set of beta strings: for singly ionic structures X + {d} with the complement of X minus {e}, every
+// d != e, n - |X| strings of each spin.  Determinants alone in their set (the covalent ones, d = e)
+// join a set that holds both their strings.  Sets are cut into blocks; the blocks are taken when they
+// are dense enough that the padding of their pair products stays below the gathers they replace (40 %
+// filled, ten determinants per block on average) and the list is not tiny.
+bool determinant_blocks(const vb_expansion& ex, DeterminantBlocks* out, std::vector<long long>* order) {
+    const long long nd = ex.n_determinants;
+    if (nd < 512 || ex.n_alpha_strings >= 0xFFFF || ex.n_beta_strings >= 0xFFFF) return false;
+    std::map<uint64_t, std::vector<long long>> sets;
+    for (long long d = 0; d < nd; ++d)
+        sets[ex.alpha_strings[ex.det_alpha[d]] & ~ex.beta_strings[ex.det_beta[d]]].push_back(d);
+    if ((long long)sets.size() > nd / 4) {
+        // covalent lists: every determinant alone
+        long long alone = 0;
+        for (const auto& s : sets) alone += s.second.size() == 1;
+        if (2 * alone > nd) return false;
+    }
+    std::vector<std::vector<long long>> groups;
+    std::vector<long long> singles;
+    for (auto& s : sets) {
+        if (s.second.size() == 1)
+            singles.push_back(s.second[0]);
+        else
+            groups.push_back(std::move(s.second));
+    }
+    std::vector<std::vector<int>> with_alpha(ex.n_alpha_strings);  // groups that hold an alpha string
+    std::vector<std::set<int>> betas(groups.size());
+    for (size_t g = 0; g < groups.size(); ++g) {
+        std::set<int> a;
+        for (long long d : groups[g]) {
+            a.insert(ex.det_alpha[d]);
+            betas[g].insert(ex.det_beta[d]);
+        }
+        for (int x : a) with_alpha[x].push_back((int)g);
+    }
+    for (long long d : singles) {
+        int best = -1;
+        for (int g : with_alpha[ex.det_alpha[d]])
+            if (betas[g].count(ex.det_beta[d]) && (best < 0 || groups[g].size() < groups[best].size())) best = g;
+        if (best >= 0)
+            groups[best].push_back(d);
+        else
+            groups.push_back({d});
+    }
+    DeterminantBlocks b;
+    std::vector<long long> sorted;
+    long long cells = 0;
+    int max_a = 0, max_b = 0;
+    b.first.push_back(0);
+    for (auto& g : groups) {
+        std::vector<int> as, bs;
+        for (long long d : g) {
+            as.push_back(ex.det_alpha[d]);
+            bs.push_back(ex.det_beta[d]);
+        }
+        for (std::vector<int>* v : {&as, &bs}) {
+            std::sort(v->begin(), v->end());
+            v->erase(std::unique(v->begin(), v->end()), v->end());
+        }
+        std::map<std::pair<int, int>, long long> at;
+        for (long long d : g)
+            if (!at.emplace(std::make_pair(ex.det_alpha[d], ex.det_beta[d]), d).second) return false;  // repeated
+        // chunks of nearly equal size
+        const int ca = ((int)as.size() + 7) / 8, cb = ((int)bs.size() + 7) / 8;
+        for (int x = 0; x < ca; ++x)
+            for (int y = 0; y < cb; ++y) {
+                const int a0 = (int)as.size() * x / ca, a1 = (int)as.size() * (x + 1) / ca;
+                const int b0 = (int)bs.size() * y / cb, b1 = (int)bs.size() * (y + 1) / cb;
+                BlockStrings block;
+                std::memset(&block, 0xFF, sizeof(block));
+                int count = 0;
+                for (int i = a0; i < a1; ++i)
+                    for (int k = b0; k < b1; ++k) {
+                        const auto it = at.find({as[i], bs[k]});
+                        if (it == at.end()) continue;
+                        block.cell[8 * (i - a0) + k - b0] = (unsigned char)count++;
+                        sorted.push_back(it->second);
+                    }
+                if (count == 0) continue;
+                for (int i = a0; i < a1; ++i) block.alpha[i - a0] = (uint16_t)as[i];
+                for (int k = b0; k < b1; ++k) block.beta[k - b0] = (uint16_t)bs[k];
+                cells += (long long)(a1 - a0) * (b1 - b0);
+                max_a = std::max(max_a, a1 - a0);
+                max_b = std::max(max_b, b1 - b0);
+                b.max_dets = std::max(b.max_dets, count);
+                b.strings.push_back(block);
+                b.first.push_back((int)sorted.size());
+                ++b.n;
+            }
+    }
+    b.max_a = max_a * max_a;
+    b.max_b = max_b * max_b;
+    if ((long long)sorted.size() != nd || 5 * nd < 2 * cells || nd < 10LL * b.n) return false;
+    *out = std::move(b);
+    *order = std::move(sorted);
+    return true;
+}
+
+vb_status upload_blocks(vb_hs_plan* p, const DeterminantBlocks& b) {
+    vb_status st = upload(p->ctx, p->blocks.first, b.first.data(), sizeof(int) * b.first.size());
+    if (st == VB_OK) st = upload(p->ctx, p->blocks.strings, b.strings.data(), sizeof(BlockStrings) * b.strings.size());
+    p->blocks.n = b.n;
+    p->blocks.max_a = b.max_a;
+    p->blocks.max_b = b.max_b;
+    p->blocks.max_dets = b.max_dets;
+    p->blocks.first_host = b.first;
+    return st;
+}
+
+BlockPairArgs block_args(const vb_hs_plan* p, const FullPairArgs& f) {
+    BlockPairArgs a{};
+    a.f = f;
+    a.first = p->blocks.first.as<int>();
+    a.strings = p->blocks.strings.as<BlockStrings>();
+    a.max_a = p->blocks.max_a;
+    a.max_b = p->blocks.max_b;
+    a.max_dets = p->blocks.max_dets;
+    const auto& first = p->blocks.first_host;
+    a.h0 = (int)(std::lower_bound(first.begin(), first.end(), (int)f.e0) - first.begin());
+    a.h1 = (int)(std::lower_bound(first.begin(), first.end(), (int)f.e1) - first.begin());
+    return a;
+}
+
 }  // namespace
 
 namespace vbcore {
@@ -157,32 +291,39 @@ vb_status vb_hs_plan_create(vb_context* ctx, const vb_expansion* ex, vb_hs_plan*
         if (ex->term_structure[t] < 0 || ex->term_structure[t] >= p->n_str)
             return fail(set_error(ctx, VB_ERR_INVALID, "term structure index out of range"));
 
-    // Determinant order.  Structures that share few determinants (ionic structures: determinants
-    // cluster by occupation pattern) leave each band-reduction structure group reading a row tile
+    // Determinant order.  Lists whose determinants fill blocks of (alpha strings) x (beta strings) are
+    // ordered by block (determinant_blocks): the pair kernel then works on whole blocks and the band
+    // reduction gathers the rows of each structure group.  Otherwise: structures that share few
+    // determinants (ionic structures: determinants cluster by occupation pattern) leave each
+    // band-reduction structure group reading a row tile
     // for a handful of its rows.  Placing every determinant at the first structure that uses it
     // makes the determinants of consecutive structures contiguous; the reorder is taken when it at
     // least halves the (structure group, row tile) segments.  Everything the plan computes is per
     // structure or per spin string, so only vb_hs_plan_determinant_pairs translates indices.
+    DeterminantBlocks blocks;
     std::vector<int32_t> r_alpha, r_beta, r_str;
     std::vector<int64_t> r_off;
     std::vector<double> r_coef;
     vb_expansion reordered;
     {
         const long long nd = p->n_det;
-        std::vector<long long> first(nd, (long long)p->n_str);
-        for (long long d = 0; d < nd; ++d)
-            for (long long t = ex->term_offsets[d]; t < ex->term_offsets[d + 1]; ++t)
-                first[d] = std::min<long long>(first[d], ex->term_structure[t]);
         std::vector<long long> order(nd);
         for (long long d = 0; d < nd; ++d) order[d] = d;
-        // within a structure group's range, determinants stay in alpha-major order (the spin-pair
-        // records of neighbouring determinant pairs stay neighbours)
-        std::stable_sort(order.begin(), order.end(), [&](long long x, long long y) {
-            const long long gx = first[x] / kBandGroup, gy = first[y] / kBandGroup;
-            if (gx != gy) return gx < gy;
-            if (ex->det_alpha[x] != ex->det_alpha[y]) return ex->det_alpha[x] < ex->det_alpha[y];
-            return ex->det_beta[x] < ex->det_beta[y];
-        });
+        const bool by_block = p->ka > 0 && p->kb > 0 && determinant_blocks(*ex, &blocks, &order);
+        if (!by_block) {
+            std::vector<long long> first(nd, (long long)p->n_str);
+            for (long long d = 0; d < nd; ++d)
+                for (long long t = ex->term_offsets[d]; t < ex->term_offsets[d + 1]; ++t)
+                    first[d] = std::min<long long>(first[d], ex->term_structure[t]);
+            // within a structure group's range, determinants stay in alpha-major order (the spin-pair
+            // records of neighbouring determinant pairs stay neighbours)
+            std::stable_sort(order.begin(), order.end(), [&](long long x, long long y) {
+                const long long gx = first[x] / kBandGroup, gy = first[y] / kBandGroup;
+                if (gx != gy) return gx < gy;
+                if (ex->det_alpha[x] != ex->det_alpha[y]) return ex->det_alpha[x] < ex->det_alpha[y];
+                return ex->det_beta[x] < ex->det_beta[y];
+            });
+        }
         std::vector<long long> pos(nd);
         for (long long i = 0; i < nd; ++i) pos[order[i]] = i;
         const long long tiles = (nd + kBandTileRows - 1) / kBandTileRows;
@@ -196,7 +337,7 @@ vb_status vb_hs_plan_create(vb_context* ctx, const vb_expansion* ex, vb_hs_plan*
             std::sort(keys.begin(), keys.end());
             return (long long)(std::unique(keys.begin(), keys.end()) - keys.begin());
         };
-        if (2 * segments(true) <= segments(false)) {
+        if (by_block || 2 * segments(true) <= segments(false)) {
             r_alpha.resize(nd);
             r_beta.resize(nd);
             r_off.assign(nd + 1, 0);
@@ -352,8 +493,19 @@ vb_status vb_hs_plan_create(vb_context* ctx, const vb_expansion* ex, vb_hs_plan*
     const size_t band_cap = std::min<size_t>((size_t)1 << 30, ctx->budget / 8);
     long long width = (long long)(band_cap / (16 * (size_t)p->n_det));
     width = std::max(32LL, std::min(width, p->n_det));
-    p->band_width = width;
     p->band_ld = (width + 31) / 32 * 32;
+    // band boundaries: every `width` columns, at block boundaries when the pair kernel works on blocks
+    p->bands.assign(1, 0);
+    if (blocks.n > 0) {
+        if ((st = upload_blocks(p, blocks)) != VB_OK) return fail(st);
+        p->band_ld = std::max(p->band_ld, (long long)64);
+        for (int h = 0; h < blocks.n; ++h)
+            if (blocks.first[h + 1] - p->bands.back() > p->band_ld) p->bands.push_back(blocks.first[h]);
+        p->bands.push_back(p->n_det);
+    } else {
+        for (long long e = width; e < p->n_det; e += width) p->bands.push_back(e);
+        p->bands.push_back(p->n_det);
+    }
     // the bands and the structure-reduce buffers (Z, W) are the context's execute scratch
     const size_t wbytes = sizeof(double) * (size_t)p->n_str * p->n_str;
     for (DeviceBuffer* b : {&p->Hout, &p->Sout})
@@ -377,52 +529,80 @@ vb_status vb_hs_plan_create(vb_context* ctx, const vb_expansion* ex, vb_hs_plan*
     if ((st = upload(ctx, p->str_coef, scoef.data(), sizeof(double) * std::max<size_t>(1, scoef.size()))) != VB_OK)
         return fail(st);
 
-    // band-reduction term segments: for every (structure group, row tile) the terms (row in the
-    // tile, coefficient) of the group's structures ordered by (warp, slot, determinant)
+    // band-reduction term segments: for every row tile of every structure group the terms (row in the
+    // tile, coefficient) of the group's structures ordered by (warp, slot, determinant).  The tiles of
+    // a group are its 64-row tiles of the determinant list that hold terms, or (blocks) the group's own
+    // rows 64 at a time.
     {
         BandSegments& b = p->segments;
         b.n_groups = (p->n_str + kBandGroup - 1) / kBandGroup;
-        b.n_tiles = (int)((p->n_det + kBandTileRows - 1) / kBandTileRows);
-        const size_t nseg = (size_t)b.n_groups * b.n_tiles;
-        std::vector<long long> off(nseg + 1, 0);
-        std::vector<unsigned char> meta(nseg * kBandMetaBytes, 0);
+        b.gather = blocks.n > 0;
+        std::vector<long long> off;
+        std::vector<unsigned char> meta;
         std::vector<double> coef;
         std::vector<unsigned char> row;
-        std::vector<long long> cur(soff.begin(), soff.end() - 1);  // next term of each structure
-        std::vector<int> tiles, tile_off(b.n_groups + 1, 0);
-        for (int g = 0; g < b.n_groups; ++g)
-            for (int t = 0; t < b.n_tiles; ++t) {
-                const size_t seg = (size_t)g * b.n_tiles + t;
-                off[seg] = (long long)coef.size();
-                unsigned char* m = meta.data() + seg * kBandMetaBytes;
-                const long long r0 = (long long)t * kBandTileRows, r1 = r0 + kBandTileRows;
+        std::vector<int> rows, first_row, last_row, tile_off(b.n_groups + 1, 0);
+        std::vector<int> local(p->n_det, -1);  // row of the group's tile that holds a determinant
+        for (int g = 0; g < b.n_groups; ++g) {
+            // determinants of the group, ascending
+            const int I0 = g * kBandGroup, I1 = std::min(p->n_str, I0 + kBandGroup);
+            std::vector<int> used;
+            for (long long t = soff[I0]; t < soff[I1]; ++t)
+                if (local[sdet[t]] < 0) {
+                    local[sdet[t]] = 0;
+                    used.push_back((int)sdet[t]);
+                }
+            std::sort(used.begin(), used.end());
+            std::vector<long long> cur(soff.begin() + I0, soff.begin() + I1);  // next term of each structure
+            for (size_t u0 = 0; u0 < used.size();) {
+                size_t u1 = u0;
+                const int t0 = used[u0] / kBandTileRows * kBandTileRows;
+                if (b.gather) {
+                    u1 = std::min(used.size(), u0 + kBandTileRows);
+                } else {
+                    while (u1 < used.size() && used[u1] < t0 + kBandTileRows) ++u1;
+                }
+                for (size_t u = u0; u < u1; ++u) local[used[u]] = b.gather ? (int)(u - u0) : used[u] - t0;
+                const int end = used[u1 - 1];
+                off.push_back((long long)coef.size());
+                const size_t m0 = meta.size();
+                meta.resize(m0 + kBandMetaBytes, 0);
                 int within = 0;
                 for (int w = 0; w < kBandWarps; ++w) {
                     const unsigned short start = (unsigned short)within;
-                    std::memcpy(m + kBandWarps * kBandSlots + 2 * w, &start, 2);
+                    std::memcpy(meta.data() + m0 + kBandWarps * kBandSlots + 2 * w, &start, 2);
                     for (int sl = 0; sl < kBandSlots; ++sl) {
-                        const int I = g * kBandGroup + sl * kBandWarps + w;
+                        const int I = I0 + sl * kBandWarps + w;
                         int cnt = 0;
-                        if (I < p->n_str)
-                            for (; cur[I] < soff[I + 1] && sdet[cur[I]] < r1; ++cur[I], ++cnt) {
-                                row.push_back((unsigned char)(sdet[cur[I]] - r0));
-                                coef.push_back(scoef[cur[I]]);
+                        if (I < I1)
+                            for (long long& c = cur[I - I0]; c < soff[I + 1] && sdet[c] <= end; ++c, ++cnt) {
+                                row.push_back((unsigned char)local[sdet[c]]);
+                                coef.push_back(scoef[c]);
                             }
-                        m[w * kBandSlots + sl] = (unsigned char)cnt;
+                        meta[m0 + w * kBandSlots + sl] = (unsigned char)cnt;
                         within += cnt;
                     }
                 }
-                if (within > 0) tiles.push_back(t);
-                tile_off[g + 1] = (int)tiles.size();
                 while (coef.size() % 16) {
                     coef.push_back(0.0);
                     row.push_back(0);
                 }
-                b.seg_max = std::max(b.seg_max, (int)((long long)coef.size() - off[seg]));
+                b.seg_max = std::max(b.seg_max, (int)((long long)coef.size() - off.back()));
+                first_row.push_back(b.gather ? used[u0] : t0);
+                last_row.push_back(b.gather ? end : t0 + kBandTileRows - 1);
+                if (b.gather)
+                    for (int q = 0; q < kBandTileRows; ++q) rows.push_back(u0 + q < u1 ? used[u0 + q] : -1);
+                u0 = u1;
             }
-        off[nseg] = (long long)coef.size();
-        if ((st = upload(ctx, b.tiles, tiles.data(), sizeof(int) * std::max<size_t>(1, tiles.size()))) != VB_OK)
+            for (int d : used) local[d] = -1;
+            tile_off[g + 1] = (int)first_row.size();
+        }
+        off.push_back((long long)coef.size());
+        if ((st = upload(ctx, b.first_row, first_row.data(), sizeof(int) * std::max<size_t>(1, first_row.size()))) != VB_OK)
             return fail(st);
+        if ((st = upload(ctx, b.last_row, last_row.data(), sizeof(int) * std::max<size_t>(1, last_row.size()))) != VB_OK)
+            return fail(st);
+        if (b.gather && (st = upload(ctx, b.rows, rows.data(), sizeof(int) * rows.size())) != VB_OK) return fail(st);
         if ((st = upload(ctx, b.tile_off, tile_off.data(), sizeof(int) * tile_off.size())) != VB_OK) return fail(st);
         if ((st = upload(ctx, b.off, off.data(), sizeof(long long) * off.size())) != VB_OK) return fail(st);
         if ((st = upload(ctx, b.meta, meta.data(), std::max<size_t>(16, meta.size()))) != VB_OK) return fail(st);
@@ -631,8 +811,8 @@ vb_status execute_impl(vb_hs_plan* p, const double* S, const double* h, const do
     }
     FullPairArgs fa = full_args(p);
     fa.flip = p->has_flip ? p->flip.as<int>() : nullptr;
-    for (long long e0 = 0; e0 < p->n_det; e0 += p->band_width) {
-        const long long e1 = std::min(p->n_det, e0 + p->band_width);
+    for (size_t band = 0; band + 1 < p->bands.size(); ++band) {
+        const long long e0 = p->bands[band], e1 = p->bands[band + 1];
         const long long B = e1 - e0;
         fa.e0 = e0;
         fa.e1 = e1;
@@ -641,7 +821,8 @@ vb_status execute_impl(vb_hs_plan* p, const double* S, const double* h, const do
         fa.Hb = scr[0];
         fa.Sb = scr[1];
         PhaseMark pairs(p, VB_PHASE_DETERMINANT_PAIRS);
-        cudaError_t err = launch_full_pairs(fa, s, &launches);
+        cudaError_t err = p->blocks.n > 0 ? launch_block_pairs(block_args(p, fa), s, &launches)
+                                          : launch_full_pairs(fa, s, &launches);
         if (err != cudaSuccess) return cuda_error(ctx, err, "full_pairs");
         pairs.close();
         PhaseMark reduce(p, VB_PHASE_BAND_REDUCE);
@@ -655,13 +836,14 @@ vb_status execute_impl(vb_hs_plan* p, const double* S, const double* h, const do
             ba.Sb = fa.Sb;
             ba.ldb = p->band_ld;
             ba.n_groups = p->segments.n_groups;
-            ba.n_tiles = p->segments.n_tiles;
             ba.seg_max = p->segments.seg_max;
             ba.seg_off = p->segments.off.as<long long>();
             ba.seg_meta = p->segments.meta.as<unsigned char>();
             ba.term_c = p->segments.coef.as<double>();
             ba.term_d = p->segments.row.as<unsigned char>();
-            ba.seg_tiles = p->segments.tiles.as<int>();
+            ba.seg_first = p->segments.first_row.as<int>();
+            ba.seg_last = p->segments.last_row.as<int>();
+            ba.seg_rows = p->segments.gather ? p->segments.rows.as<int>() : nullptr;
             ba.seg_tile_off = p->segments.tile_off.as<int>();
             ba.error = reinterpret_cast<int*>(p->counters.as<unsigned long long>() + 7);
             ba.spin_limit = ctx->barrier_spin_limit > 0 ? ctx->barrier_spin_limit : (1ll << 26);

@@ -67,13 +67,32 @@ struct FullPairArgs {
     const int* flip;      // spin-flip permutation of determinants (nullptr: no folding)
 };
 
+// Determinant pairs of one band by blocks of the determinant list: block h holds determinants
+// first[h] .. first[h + 1] - 1 of at most 8 alpha x 8 beta strings (0xFFFF beyond the last); the
+// determinant of cell (i, k) is first[h] + cell[8 i + k] (0xFF: none).  Blocks h0 .. h1 - 1 are the
+// band's columns, blocks g <= h its rows.
+struct BlockStrings {
+    uint16_t alpha[8], beta[8];
+    unsigned char cell[64];
+    unsigned char pad[32];
+};
+struct BlockPairArgs {
+    FullPairArgs f;
+    const int* first;
+    const BlockStrings* strings;
+    int h0, h1;
+    int max_a, max_b, max_dets;  // largest alpha and beta string pair counts and determinants of a block
+};
+
 // Band reduction Z = T^T U' (structure-major weights T, band U' upper triangle).  Rows of the
-// band are streamed in tiles of kBandTileRows; for every (structure group g, row tile t) the plan
-// holds one segment of (row-in-tile, coefficient) terms ordered by (warp, slot, determinant):
-// seg_off[g T + t] (a multiple of 16) indexes term_c / term_d, and seg_meta holds kBandMetaBytes
+// band are streamed in tiles of kBandTileRows; for every tile t of structure group g (t in
+// [seg_tile_off[g], seg_tile_off[g + 1]), rows ascending) the plan holds one segment of
+// (row-in-tile, coefficient) terms ordered by (warp, slot, determinant): seg_off[t] (a multiple of 16)
+// indexes term_c / term_d, and seg_meta holds kBandMetaBytes
 // per segment: the term count of each (warp, slot) (kBandWarps x kBandSlots bytes) followed by the
 // start of each warp's terms within the segment (kBandWarps uint16).  Structure of group g, warp
-// w, slot s: I = g * kBandGroup + s * kBandWarps + w.
+// w, slot s: I = g * kBandGroup + s * kBandWarps + w.  A tile holds the consecutive rows from
+// seg_first[t] on or, with seg_rows, the listed rows seg_rows[64 t ..] (-1 beyond the last).
 struct BandReduceArgs {
     long long n_det;
     int n_str;
@@ -81,14 +100,16 @@ struct BandReduceArgs {
     long long ldb;            // band row stride (elements, even)
     const double* Hb;
     const double* Sb;
-    int n_groups, n_tiles;
+    int n_groups;
     int seg_max;              // longest segment (terms, a multiple of 16)
     const long long* seg_off;
     const unsigned char* seg_meta;
     const double* term_c;
     const unsigned char* term_d;
-    const int* seg_tiles;     // row tiles whose segment has terms, per group ascending
-    const int* seg_tile_off;  // group g: seg_tiles[seg_tile_off[g] .. seg_tile_off[g + 1])
+    const int* seg_first;
+    const int* seg_last;
+    const int* seg_rows;
+    const int* seg_tile_off;
     double* Zh;  // n_str x n_det column-major: Z[e * n_str + I]
     double* Zs;
     int* error;  // set to 1 when a tile wait gives up (the results are then incomplete)
@@ -157,6 +178,7 @@ cudaError_t preload_frame_kernels();
 // kernel is otherwise loaded, and its code placed in device memory, at its first launch).
 cudaError_t preload_spin_pair_kernels();
 cudaError_t launch_full_pairs(const FullPairArgs& a, cudaStream_t stream, int* launches);
+cudaError_t launch_block_pairs(const BlockPairArgs& a, cudaStream_t stream, int* launches);
 cudaError_t launch_band_reduce(const BandReduceArgs& a, cudaStream_t stream, int* launches);
 cudaError_t launch_structure_reduce(const StructureReduceArgs& a, double* H, double* S, cudaStream_t stream,
                                     int* launches);

@@ -14,6 +14,8 @@
 //  * full_pairs_kernel: one thread per determinant pair (d <= e) of a band of columns:
 //    S = S_a S_b, H = H_a S_b + H_b S_a + sum_m sigma_m u_a[m] u_b[m] (evaluator.cpp:95-148,
 //    354-384 with the opposite-spin term in factored form), folded over the spin-flip orbit.
+//  * block_pairs_kernel: the same for lists ordered by blocks of alpha x beta strings, as products of
+//    the blocks' records on the FP64 tensor cores.
 #include <cuda_runtime.h>
 #include <math.h>
 
@@ -24,6 +26,7 @@
 
 #include "autotune.h"
 #include "device_algebra.cuh"
+#include "frame.cuh"
 #include "internal.h"
 #include "kernels.h"
 #include "pair_value.cuh"
@@ -535,6 +538,176 @@ __global__ void __launch_bounds__(512) full_pairs_kernel(FullPairArgs a) {
     }
 }
 
+// Determinant pairs by blocks (BlockPairArgs): one CTA per block pair (g <= h).  With the alpha records
+// of the string pairs (i, j), i in g and j in h, as rows and the beta records of (k, l) as columns,
+//   H[(i, k), (j, l)] = sum_m sigma_m u_a[ij][m] u_b[kl][m] + H_a[ij] S_b[kl] + S_a[ij] H_b[kl]
+// is one (up to 64) x (up to 64) x (R + 2) product on the FP64 tensor cores, and S the outer product of
+// the determinants: every record is read once per block pair and used by 7 x 7 determinant pairs (n =
+// 12, singly ionic), where one thread per pair gathers two records (640 bytes) for R multiply-adds.
+// The records arrive by cp.async, all in flight together (a warp per record, one after the other, left
+// the loads' latency exposed: 35 ms).  Each of the four warps owns M tiles w and w + 4 and all N tiles;
+// H goes through shared memory so that band rows are written in runs of a block's determinants.  Both
+// members of a spin-flip orbit are evaluated: blocks do not map to blocks under the flip.  Bound by the
+// product (2.3 ms at the DGEMM rate for 34,188 determinants) and the band it writes (9.3 GB); takes
+// 10.7 ms there, the gather form 27.3 ms.
+constexpr int kBlockWarps = 4;
+constexpr int kBlockEdge = 8;                        // strings per block and spin
+constexpr int kBlockCells = kBlockEdge * kBlockEdge;
+
+__host__ __device__ inline int block_k(int R) { return (R + 2 + 3) / 4 * 4; }
+// record stride in shared memory: 4 or 12 mod 16 doubles (conflict-free fragment loads)
+__host__ __device__ inline int block_ld(int R) { return block_k(R) % 8 == 4 ? block_k(R) : block_k(R) + 4; }
+inline size_t block_pairs_smem(int rows_a, int rows_b, int dets, int R) {
+    const size_t ra = (rows_a + 7) / 8 * 8, rb = (rows_b + 7) / 8 * 8;
+    return sizeof(double) * ((ra + rb) * block_ld(R) + (size_t)dets * (dets + 1));
+}
+
+__global__ void __launch_bounds__(32 * kBlockWarps) block_pairs_kernel(BlockPairArgs a) {
+    extern __shared__ __align__(16) double bsm[];
+    const int R = a.f.R, KD = block_k(R), LD = block_ld(R), r_pos = a.f.r_pos;
+    double* sA = bsm;                                    // [ij][record]
+    double* sB = sA + (a.max_a + 7) / 8 * 8 * LD;        // [kl][record]
+    double* sH = sB + (a.max_b + 7) / 8 * 8 * LD;        // [determinant of g][determinant of h]
+    const int OUT = a.max_dets + 1;
+    __shared__ __align__(16) BlockStrings s_desc[2];
+    __shared__ unsigned char s_i[2][kBlockCells], s_k[2][kBlockCells];  // determinant -> its strings
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, gr = lane >> 2, gc = lane & 3;
+    const int chunks = (R + 3) / 2;  // 16-byte pieces of a record up to the energy
+    // block pairs of the band: a rectangle (g < h0) and a triangle
+    const long long nh = a.h1 - a.h0, rect = nh * a.h0, total = rect + nh * (nh + 1) / 2;
+    auto decode = [&](long long t, int* g, int* h) {
+        if (t < rect) {
+            *g = (int)(t / nh);
+            *h = a.h0 + (int)(t % nh);
+            return;
+        }
+        const long long q = t - rect;
+        long long y = (long long)((sqrt(8.0 * (double)q + 1.0) - 1.0) * 0.5);
+        while (y * (y + 1) / 2 > q) --y;
+        while ((y + 1) * (y + 2) / 2 <= q) ++y;
+        *h = a.h0 + (int)y;
+        *g = a.h0 + (int)(q - y * (y + 1) / 2);
+    };
+    constexpr int kWords = sizeof(BlockStrings) / 4;  // one word per thread of the first two warps
+    static_assert(kWords == 32 && 2 * kBlockCells == 32 * kBlockWarps, "a descriptor per warp, a cell per thread");
+    int g = 0, h = 0;
+    unsigned word = 0;  // this thread's word of the next pair's descriptors
+    if (blockIdx.x < total) {
+        decode(blockIdx.x, &g, &h);
+        if (tid < 2 * kWords) word = __ldg(reinterpret_cast<const unsigned*>(a.strings + (tid < kWords ? g : h)) + tid % kWords);
+    }
+    for (long long t = blockIdx.x; t < total; t += gridDim.x) {
+        const int d0 = __ldg(a.first + g), nd = __ldg(a.first + g + 1) - d0;
+        const int e0 = __ldg(a.first + h), ne = __ldg(a.first + h + 1) - e0;
+        const bool diagonal = g == h;
+        __syncthreads();  // the previous pair's shared data is consumed
+        if (tid < 2 * kWords) reinterpret_cast<unsigned*>(s_desc)[tid] = word;
+        __syncthreads();
+        if (t + gridDim.x < total) {
+            decode(t + gridDim.x, &g, &h);
+            if (tid < 2 * kWords) word = __ldg(reinterpret_cast<const unsigned*>(a.strings + (tid < kWords ? g : h)) + tid % kWords);
+        }
+        int n_str[4];  // alpha strings of g and of h, beta strings of g and of h
+#pragma unroll
+        for (int w = 0; w < 4; ++w) {
+            const BlockStrings& b = s_desc[w & 1];
+            n_str[w] = 0;
+#pragma unroll
+            for (int q = 0; q < kBlockEdge; ++q) n_str[w] += (w < 2 ? b.alpha[q] : b.beta[q]) != 0xFFFF ? 1 : 0;
+        }
+        const int rows_a = n_str[0] * n_str[1], rows_b = n_str[2] * n_str[3];
+        for (int x = tid; x < (rows_a + rows_b) * chunks; x += blockDim.x) {
+            const int r = x / chunks, piece = x - r * chunks;
+            const bool beta = r >= rows_a;
+            const int q = beta ? r - rows_a : r, w = beta ? n_str[3] : n_str[1];
+            const int qi = q / w, qj = q - qi * w;
+            const int u = beta ? s_desc[0].beta[qi] : s_desc[0].alpha[qi];
+            const int v = beta ? s_desc[1].beta[qj] : s_desc[1].alpha[qj];
+            const long long at = record_index(min(u, v), max(u, v), beta ? a.f.Nb : a.f.Na);
+            const double* rec = (beta ? a.f.rec_b + at * a.f.stride_b : a.f.rec_a + at * a.f.stride_a) + 2 * piece;
+            const unsigned dst = (unsigned)__cvta_generic_to_shared((beta ? sB : sA) + q * LD + 2 * piece);
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(rec) : "memory");
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+        {
+            const int which = tid / kBlockCells, cell = tid % kBlockCells;
+            const unsigned char at = s_desc[which].cell[cell];
+            if (at != 0xFF) {
+                s_i[which][at] = (unsigned char)(cell / kBlockEdge);
+                s_k[which][at] = (unsigned char)(cell % kBlockEdge);
+            }
+        }
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
+        __syncthreads();
+        const int mt = (rows_a + 7) / 8, nt = (rows_b + 7) / 8;
+        if (warp < mt) {
+            double acc[2][kBlockEdge][2];
+#pragma unroll
+            for (int i = 0; i < 2; ++i)
+#pragma unroll
+                for (int j = 0; j < kBlockEdge; ++j) acc[i][j][0] = acc[i][j][1] = 0.0;
+            const bool two = warp + kBlockWarps < mt;
+            const double* pa = sA + (8 * warp + gr) * LD;
+            const double* pa2 = pa + (two ? 8 * kBlockWarps * LD : 0);
+            const double* pb = sB + gr * LD;
+            auto step = [&](int ka, int kb, bool on, bool negative) {
+                double a0 = pa[ka], a1 = pa2[ka];
+                if (negative) {
+                    a0 = -a0;
+                    a1 = -a1;
+                }
+                if (!on) a0 = a1 = 0.0;
+#pragma unroll
+                for (int j = 0; j < kBlockEdge; ++j) {
+                    if (j >= nt) break;
+                    const double b = on ? pb[8 * j * LD + kb] : 0.0;
+                    mma_f64(acc[0][j], a0, b);
+                    if (two) mma_f64(acc[1][j], a1, b);
+                }
+            };
+            int k = 0;
+            for (; k + 4 <= R; k += 4) step(k + gc, k + gc, true, k + gc >= r_pos);
+            for (; k < KD; k += 4) {
+                // the remaining factor columns, then H_a S_b and S_a H_b (a record holds [.. | S | H])
+                const int m = k + gc;
+                const bool on = m < R + 2;
+                const int mb = on ? m : 0;
+                step(m < R ? m : (on ? 2 * R + 1 - m : 0), mb, on, m < R && m >= r_pos);
+            }
+#pragma unroll
+            for (int i = 0; i < 2; ++i) {
+                const int r = 8 * (warp + kBlockWarps * i) + gr;
+                if (r >= rows_a) continue;
+                const int ii = r / n_str[1], jj = r - ii * n_str[1];
+#pragma unroll
+                for (int j = 0; j < kBlockEdge; ++j)
+#pragma unroll
+                    for (int x = 0; x < 2; ++x) {
+                        const int c = 8 * j + 2 * gc + x;
+                        if (c >= rows_b) continue;
+                        const int kk = c / n_str[3], ll = c - kk * n_str[3];
+                        const unsigned d = s_desc[0].cell[kBlockEdge * ii + kk], e = s_desc[1].cell[kBlockEdge * jj + ll];
+                        if (d != 0xFF && e != 0xFF) sH[d * OUT + e] = acc[i][j][x];
+                    }
+            }
+        }
+        __syncthreads();
+        for (int d = warp; d < nd; d += kBlockWarps) {
+            const int i = s_i[0][d] * n_str[1], k = s_k[0][d] * n_str[3];
+            double* H = a.f.Hb + (d0 + d) * a.f.ldb + (e0 - a.f.e0);
+            double* S = a.f.Sb + (d0 + d) * a.f.ldb + (e0 - a.f.e0);
+#pragma unroll 2
+            for (int e = lane; e < ne; e += 32) {
+                if (diagonal && e < d) continue;
+                const double w = diagonal && e == d ? 0.5 : 1.0;
+                const double sa = sA[(i + s_i[1][e]) * LD + R], sb = sB[(k + s_k[1][e]) * LD + R];
+                H[e] = w * sH[d * OUT + e];
+                S[e] = w * (sa * sb);
+            }
+        }
+    }
+}
+
 // Listed determinant pairs (d, e) in any order.
 __global__ void listed_pairs_kernel(FullPairArgs a, long long n_pairs, const long long* __restrict__ pairs,
                                     double* __restrict__ h_out, double* __restrict__ s_out) {
@@ -721,6 +894,21 @@ cudaError_t launch_full_pairs(const FullPairArgs& a, cudaStream_t stream, int* l
         {}, &err);
     ++*launches;
     return err;
+}
+
+cudaError_t launch_block_pairs(const BlockPairArgs& a, cudaStream_t stream, int* launches) {
+    const long long nh = a.h1 - a.h0, total = nh * a.h0 + nh * (nh + 1) / 2;
+    if (total <= 0) return cudaSuccess;
+    const size_t smem = block_pairs_smem(a.max_a, a.max_b, a.max_dets, a.f.R);
+    cudaError_t err = allow_dynamic_smem((const void*)block_pairs_kernel, smem);
+    if (err != cudaSuccess) return err;
+    int per_sm = 1;
+    err = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, block_pairs_kernel, 32 * kBlockWarps, smem);
+    if (err != cudaSuccess) return err;
+    const long long grid = (long long)kSms * (per_sm > 0 ? per_sm : 1);
+    block_pairs_kernel<<<(unsigned)(total < grid ? total : grid), 32 * kBlockWarps, smem, stream>>>(a);
+    ++*launches;
+    return cudaGetLastError();
 }
 
 cudaError_t launch_listed_pairs(const FullPairArgs& a, long long n_pairs, const long long* pairs, double* h_out,

@@ -11,12 +11,21 @@
 
 using namespace vbcore;
 
-// Term segments of the band reduction per (structure group, row tile) (see BandReduceArgs).
+// Term segments of the band reduction per row tile of every structure group (see BandReduceArgs).
 struct BandSegments {
-    int n_groups = 0, n_tiles = 0, seg_max = 0;
+    int n_groups = 0, seg_max = 0;
+    bool gather = false;  // tiles list their rows
     DeviceBuffer off, meta, coef, row;
-    // row tiles with terms, per group ascending (CSR: tile_off[g] .. tile_off[g + 1] index tiles)
-    DeviceBuffer tiles, tile_off;
+    // tiles of every group (CSR: tile_off[g] .. tile_off[g + 1]), their first and last rows and rows
+    DeviceBuffer first_row, last_row, rows, tile_off;
+};
+
+// Blocks of (alpha strings) x (beta strings) the determinant list is ordered by (see BlockPairArgs).
+struct PlanBlocks {
+    int n = 0;
+    int max_a = 0, max_b = 0, max_dets = 0;
+    DeviceBuffer first, strings;
+    std::vector<int> first_host;
 };
 
 constexpr int kPlanCounters = 10;
@@ -44,8 +53,9 @@ struct vb_hs_plan {
     DeviceBuffer lf, fwork, fcols, fsigns, fmeta;
     int* meta_host = nullptr;
     int R = 0, r_pos = 0;
-    long long band_width = 0;  // determinant columns per band (bands live in the context scratch)
-    long long band_ld = 0;     // band row stride (band_width rounded up to 32 elements)
+    std::vector<long long> bands;  // determinant columns of the bands (they live in the context scratch)
+    long long band_ld = 0;         // band row stride (a multiple of 32 elements)
+    PlanBlocks blocks;
     DeviceBuffer Hout, Sout;
     DeviceBuffer str_off, str_det, str_coef;
     // structure incidence by determinant (CSR) and the gradient's adjoint scratch

@@ -224,3 +224,26 @@ def test_frame_gradient_graded_overlaps(ctx, kw, n, nel, mult):
     fd = _richardson(lambda t: _energy(n, ex_o, S, h, workloads.pack_pair_kernel((F + t * dF) @ (F + t * dF).T)), 1e-4)
     assert abs(fd - np.sum(g["ri"] * dF)) < 1e-7 * max(1.0, abs(fd))
     plan.close()
+
+
+@pytest.mark.parametrize("kw,n,mult", [("COV", 12, 1), ("COV ION(1)", 7, 2), ("COV", 14, 1)])
+def test_frame_gradient_from_records_and_high_levels(ctx, kw, n, mult):
+    """Covalent singlets (one determinant per alpha string: adjoints read from the partners' records)
+    and lists without that property, with strings of 6 and 7 electrons whose pairs reach levels 6 and 7
+    through the inverse, or through the listed kernel where the overlaps are zero for one orbital.
+    Same comparison and bound as above."""
+    rng = np.random.default_rng(n)
+    S = workloads.active_space(n, 3 * n, 7 + n)[0]
+    S[0, 1:] = S[1:, 0] = 0.0
+    h = _sym(rng, n)
+    P = n * (n + 1) // 2
+    F = 0.05 * rng.standard_normal((P, P)) + 0.1 * np.eye(P)
+    eri = workloads.pack_pair_kernel(F @ F.T)
+    plan = vbcore.HsPlan(ctx, vbcore.expand_structures(vbcore.generate_structures(kw, n, n, mult), n, mult), n)
+    c = rng.standard_normal(plan.n_structures)
+    c /= np.linalg.norm(c)
+    a = plan.gradient(S, h, eri, c, -0.7, packed_eri=False, ri_factors=F)
+    b = plan.gradient(S, h, eri, c, -0.7, packed_eri=True, ri_factors=F)
+    for key in ("S", "h", "ri"):
+        assert np.abs(a[key] - b[key]).max() < 1e-8 * max(1e-3, np.abs(b[key]).max()), key
+    plan.close()

@@ -23,6 +23,14 @@ struct FrameAdjointArgs {
     const int* ebound;
     const double* adj;     // record adjoints, even stride: [u (R), determinant, energy]
     long long adj_stride;
+    // instead (weight not null): one determinant per string u, of weight weight[u] and with the opposite
+    // string partner[u] in the same table, and a spin-flip symmetric list; the adjoint of (u, v) is then
+    // 2 (1 + [u < v]) weight[u] weight[v] times [sigma u, H - lambda S, S] of the partners' record
+    const double* weight;
+    const int* partner;
+    const double* records;
+    long long rec_stride;
+    double lambda;
     unsigned long long* task_counter;   // zero
     unsigned long long* careful_count;  // zero; pairs left to the exact kernel
     unsigned long long* careful_list;

@@ -319,6 +319,7 @@ struct BackArgs {
     int R;
     const double* adj;
     int adj_stride;
+    int adj_listed;  // 1: row i of adj belongs to listed pair i (else to the pair's record)
     double* gS;  // n x n (index as read: S[L_c n + R_r])
     double* gh;  // n x n
     double* gG;  // gd x gd, [anti(L pair) gd + anti(R pair)]
@@ -566,7 +567,44 @@ __global__ void gather_adjoint_kernel(BackArgs a, long long idx_begin, long long
         const int m = (int)(e % a.R);
         long long u, v;
         careful_pair(a, idx_begin + i, all_pairs, &u, &v);
-        Ac[e] = a.adj[record_index(u, v, a.N) * a.adj_stride + m];
+        Ac[e] = a.adj[(a.adj_listed ? idx_begin + i : record_index(u, v, a.N)) * a.adj_stride + m];
+    }
+}
+
+// Weight and opposite string of every string's only determinant (weight 0 where there is none).
+__global__ void string_weights_kernel(int n_strings, const int* __restrict__ aoff, const int* __restrict__ adets,
+                                      const double* __restrict__ w, const int* __restrict__ det_beta,
+                                      double* __restrict__ weight, int* __restrict__ partner) {
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n_strings; i += gridDim.x * blockDim.x) {
+        const int k = __ldg(aoff + i);
+        const bool has = __ldg(aoff + i + 1) > k;
+        const int d = has ? __ldg(adets + k) : 0;
+        weight[i] = has ? __ldg(w + d) : 0.0;
+        partner[i] = has ? __ldg(det_beta + d) : 0;
+    }
+}
+
+// Adjoint rows of the listed pairs from the partners' records (FrameAdjointArgs::weight), a warp per row.
+__global__ void __launch_bounds__(256) listed_adjoint_kernel(FrameAdjointArgs f, long long count, int stride,
+                                                             double* __restrict__ out) {
+    const int lane = threadIdx.x & 31;
+    const long long nwarps = ((long long)gridDim.x * blockDim.x) >> 5;
+    for (long long i = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < count; i += nwarps) {
+        const unsigned long long w = f.careful_list[i];
+        const int u = (int)(w >> 32), v = (int)(w & 0xffffffffull);
+        const int x = __ldg(f.partner + u), y = __ldg(f.partner + v);
+        const double* rec = f.records + record_index(min(x, y), max(x, y), f.n_strings) * f.rec_stride;
+        const double omega = (u == v ? 2.0 : 4.0) * __ldg(f.weight + u) * __ldg(f.weight + v);
+        for (int m = lane; m < f.R + 2; m += 32) {
+            double val;
+            if (m < f.R)
+                val = m < f.r_pos ? __ldg(rec + m) : -__ldg(rec + m);
+            else if (m == f.R)
+                val = __ldg(rec + f.R + 1) - f.lambda * __ldg(rec + f.R);
+            else
+                val = __ldg(rec + f.R);
+            out[i * stride + m] = omega * val;
+        }
     }
 }
 
@@ -715,7 +753,7 @@ __global__ void __launch_bounds__(128) careful_backward_kernel(BackArgs a, long 
         careful_pair(a, idx, all_pairs, &u, &v);
         const long long t = record_index(u, v, N);
         const long long row = idx - idx_begin;
-        const double* adj = a.adj + t * a.adj_stride;
+        const double* adj = a.adj + (a.adj_listed ? idx : t) * a.adj_stride;
         const double aS = adj[a.R], aH = adj[a.R + 1];
         int L[KM], Rr[KM];
         for (int c = 0; c < k; ++c) {
@@ -963,7 +1001,10 @@ extern "C" vb_status vb_hs_plan_gradient(vb_hs_plan* p, const double* S, const d
     // the two-stage record adjoint when alpha strings carry four or more determinants on average
     const bool flip_adjoint = p->has_flip && p->shared_tables && p->ka > 0 && p->R <= 128;
     const int chunk = flip_adjoint && p->n_det >= 4LL * p->Na ? two_stage_chunk(p->Nb) : 0;
-    const size_t order_doubles = chunk ? (size_t)p->n_det + ((size_t)p->n_det + 1) / 2 : 0;
+    // one determinant per alpha string: the record adjoints are scaled records, read where they are
+    const bool direct = p->has_flip && p->shared_tables && p->ka > 0 && p->single_determinants && !deri_out &&
+                        p->tables_a.ptr && frame_adjoint_supported(n, p->ka, R);
+    const size_t order_doubles = chunk ? (size_t)p->n_det + ((size_t)p->n_det + 1) / 2 : (direct ? 2 * (size_t)p->Na : 0);
     if ((st = p->grad_acc.allocate(ctx, sizeof(double) * (acc_doubles + p->n_det + p->n_str + order_doubles))) !=
         VB_OK)
         return st;
@@ -974,8 +1015,24 @@ extern "C" vb_status vb_hs_plan_gradient(vb_hs_plan* p, const double* S, const d
     double* w = gL + n_gL;
     double* cdev = w + p->n_det;
     double* ws = cdev + p->n_str;
-    int* bs = reinterpret_cast<int*>(ws + p->n_det);
-    const long long adj_a_n = std::max(1LL, p->npairs_a) * adj_stride;
+    int* bs = reinterpret_cast<int*>(ws + (direct ? p->Na : p->n_det));
+    // blocks of the frame form for one spin table; without room for them (*got = false) the pair-by-pair
+    // form works in chunks
+    DeviceBuffer blocks, sums;
+    auto frame_blocks = [&](int beta, bool* got) -> vb_status {
+        const int k = beta ? p->kb : p->ka;
+        *got = false;
+        if (deri_out || !(beta ? p->tables_b : p->tables_a).ptr || !frame_adjoint_supported(n, k, R)) return VB_OK;
+        vb_status bst = blocks.allocate(ctx, sizeof(double) * frame_adjoint_block_doubles(n, k, R) * (beta ? p->Nb : p->Na));
+        if (bst == VB_OK)
+            bst = sums.allocate(ctx, sizeof(double) * kAdjointMaxParts * ((size_t)np * R + 2 * (size_t)n * n));
+        if (bst != VB_OK) blocks.release();
+        *got = bst == VB_OK;
+        return bst == VB_ERR_BUDGET ? VB_OK : bst;
+    };
+    bool from_records = false;
+    if (direct && (st = frame_blocks(0, &from_records)) != VB_OK) return st;
+    const long long adj_a_n = from_records ? 1 : std::max(1LL, p->npairs_a) * adj_stride;
     const long long adj_b_n = p->shared_tables ? 0 : std::max(1LL, p->npairs_b) * adj_stride;
     if ((st = p->adj_a.allocate(ctx, sizeof(double) * adj_a_n)) != VB_OK) return st;
     if (!p->shared_tables && p->kb > 0 && (st = p->adj_b.allocate(ctx, sizeof(double) * adj_b_n)) != VB_OK) return st;
@@ -997,7 +1054,11 @@ extern "C" vb_status vb_hs_plan_gradient(vb_hs_plan* p, const double* S, const d
     aa.adj_a = p->adj_a.as<double>();
     aa.adj_b = p->shared_tables ? p->adj_a.as<double>() : p->adj_b.as<double>();
     aa.adj_stride = adj_stride;
-    if (err == cudaSuccess) {
+    if (err == cudaSuccess && from_records) {
+        string_weights_kernel<<<(p->Na + 127) / 128, 128, 0, s>>>(p->Na, p->alpha_off.as<int>(), p->alpha_dets.as<int>(),
+                                                                 w, p->det_beta.as<int>(), ws, bs);
+        err = cudaGetLastError();
+    } else if (err == cudaSuccess) {
         if (chunk) {
             alpha_order_kernel<<<(unsigned)std::min<long long>(4096, (p->n_det + 255) / 256), 256, 0, s>>>(
                 p->n_det, p->alpha_dets.as<int>(), w, p->det_beta.as<int>(), ws, bs);
@@ -1050,25 +1111,15 @@ extern "C" vb_status vb_hs_plan_gradient(vb_hs_plan* p, const double* S, const d
         if (err != cudaSuccess) break;
         const bool fast = k <= 8 && frame_spin_supported(n, k, R);
         const DeviceBuffer& tables = beta ? p->tables_b : p->tables_a;
-        // the frame form (gradient_frame.cu) folds the same-spin two-electron energy into the factor
-        // columns; a gradient per packed integral keeps its table separate (the map from factor
-        // columns to integrals loses accuracy with the kernel's condition)
-        DeviceBuffer blocks, sums;
-        bool frame = !deri_out && tables.ptr && frame_adjoint_supported(n, k, R);
-        if (frame) {
-            st = blocks.allocate(ctx, sizeof(double) * frame_adjoint_block_doubles(n, k, R) * b.N);
-            if (st == VB_OK)
-                st = sums.allocate(ctx, sizeof(double) * kAdjointMaxParts * ((size_t)np * R + 2 * (size_t)n * n));
-            if (st != VB_OK && st != VB_ERR_BUDGET) return st;
-            if (st == VB_ERR_BUDGET) {  // no room for the blocks: the pair-by-pair form works in chunks
-                blocks.release();
-                frame = false;
-            }
-        }
         auto listed_pairs = [&](unsigned long long* listed) {
             cudaError_t e = cudaMemcpyAsync(listed, b.careful_count, sizeof(*listed), cudaMemcpyDeviceToHost, s);
             return e == cudaSuccess ? cudaStreamSynchronize(s) : e;
         };
+        // the frame form (gradient_frame.cu) folds the same-spin two-electron energy into the factor
+        // columns; a gradient per packed integral keeps its table separate (the map from factor
+        // columns to integrals loses accuracy with the kernel's condition)
+        bool frame = from_records;
+        if (!frame && (st = frame_blocks(beta, &frame)) != VB_OK) return st;
         if (frame) {
             FrameAdjointArgs f{};
             f.n = n;
@@ -1087,6 +1138,13 @@ extern "C" vb_status vb_hs_plan_gradient(vb_hs_plan* p, const double* S, const d
             f.ebound = (beta ? p->ebound_b : p->ebound_a).as<int>();
             f.adj = b.adj;
             f.adj_stride = adj_stride;
+            if (from_records) {
+                f.weight = ws;
+                f.partner = bs;
+                f.records = p->rec_a.as<double>();
+                f.rec_stride = record_stride(R);
+                f.lambda = eigenvalue;
+            }
             f.task_counter = p->counters.as<unsigned long long>() + 4 + beta;
             f.careful_count = b.careful_count;
             f.careful_list = b.careful_list;
@@ -1100,6 +1158,14 @@ extern "C" vb_status vb_hs_plan_gradient(vb_hs_plan* p, const double* S, const d
             unsigned long long listed = 0;
             if (err == cudaSuccess) err = listed_pairs(&listed);
             if (err != cudaSuccess) break;
+            DeviceBuffer rows;
+            if (from_records && listed > 0) {
+                if ((st = rows.allocate(ctx, sizeof(double) * adj_stride * listed)) != VB_OK) return st;
+                listed_adjoint_kernel<<<148 * 8, 256, 0, s>>>(f, (long long)listed, adj_stride, rows.as<double>());
+                if ((err = cudaGetLastError()) != cudaSuccess) break;
+                b.adj = rows.as<double>();
+                b.adj_listed = 1;
+            }
             if ((st = careful_chunks(ctx, b, (long long)listed, 0, partial.as<double>())) != VB_OK) return st;
         } else if (fast) {
             // chunks of whole work items (left string u, right strings v0 .. v0 + 127): per chunk
@@ -1165,6 +1231,8 @@ extern "C" vb_status vb_hs_plan_gradient(vb_hs_plan* p, const double* S, const d
             if ((st = careful_chunks(ctx, b, NN * (NN + 1) / 2, 1, partial.as<double>())) != VB_OK) return st;
         }
         err = cudaGetLastError();
+        blocks.release();
+        sums.release();
     }
     std::vector<double> hS(n_gS), hh(n_gS), hG(n_gG), hL(n_gL), hlf((size_t)np * np);
     if (err == cudaSuccess) err = cudaMemcpyAsync(hS.data(), gS, sizeof(double) * n_gS, cudaMemcpyDeviceToHost, s);

@@ -21,11 +21,16 @@
 //  * frame_tables_adjoint<K>: per left string, the reverse of frame_tables back to S, h and the
 //    factor columns, accumulated per CTA in shared memory; frame_adjoint_reduce sums the CTAs in a
 //    fixed order.
-// Levels E >= 6 (1.5 % of the pairs at K = 7) and strings whose S_LL is near singular are listed for
-// the exact kernel of gradient.cu.  The former path took the K x K inverse of every pair with
-// C(K, 2)^2 shared-memory atomics, and an SVD per thread for the uncertified ones: 14 stretched
-// hydrogen atoms (5.9 M pairs, 4.9 M of them uncertified), 48.7 + 170 ms and 24 ms of contractions,
-// against 6.9 + 1.2 ms here and 3.2 ms for the listed pairs.
+// Uncertified pairs at levels E >= 6 (1.5 % of the pairs are at these levels at K = 7) and strings whose
+// S_LL is near singular are listed for the exact kernel of gradient.cu; certified ones take the inverse
+// of B.  When every alpha string carries one determinant (covalent singlets) and the list is spin-flip
+// symmetric, the adjoint of record (u, v) is the record of the partners' beta strings times one weight:
+// the rows w are then read from the records themselves, and no adjoint buffer is built or read (5.2 GB
+// at K = 7, 3.8 ms).  The pair-by-pair path takes the K x K inverse of every pair with C(K, 2)^2
+// shared-memory atomics, and an SVD per thread for the uncertified ones: 14 stretched hydrogen atoms
+// (5.9 M pairs, 4.9 M of them uncertified), 48.7 + 170 ms and 24 ms of contractions, against 7.0 + 1.2 ms
+// here and 2.9 ms for the listed pairs.  Bound by latency: eight warps per SM (255 registers, 190 KB of
+// shared memory), tables re-read from shared memory for every pair tile.
 #include <cuda_runtime.h>
 #include <math.h>
 #include <stdint.h>
@@ -44,7 +49,8 @@ namespace {
 // than the pair-by-pair inverse of the listed path.
 constexpr double kAdjointCondition2 = 1.0e12;
 
-constexpr int kStagePairs = 16;  // pairs whose adjoint rows are staged at a time
+// pairs whose adjoint rows are staged at a time (two stages of 8 MT doubles per pair)
+constexpr int stage_pairs(int MT) { return MT <= 6 ? 32 : 16; }
 
 // Adjoint block of one left string (doubles).
 struct AdjointLayout {
@@ -240,27 +246,169 @@ __device__ __forceinline__ double backward_minors(const double* __restrict__ blk
     return D * fma(detb, s, fma(aH, quad, at));
 }
 
+// The same at levels E >= 6 through W = B^-1 (Gauss-Jordan with partial pivoting), for certified pairs;
+// *ok = false for the others.  With T(i, j) = tau, q = quad / det B and N = dq / dW:
+//   f = D det B c,  c = s + tr(T W) + a_H q,
+//   df/dB(i, j) = D det B [ W(j, i) c - (W (T + a_H N) W)(j, i) ].
+// Rare (50 of 3432 pairs per string at K = 7): out of line, with its small matrices in local memory.
+template <int K, int E>
+__device__ __noinline__ double backward_inverse(const double* __restrict__ blk, const FrameLayout* Fp, unsigned desc,
+                                                double s, double aH, double* ts, double* as, double* __restrict__ gq,
+                                                double* dd, bool* ok) {
+    constexpr int CP = fr_cp(K);
+    const FrameLayout& F = *Fp;
+    int hc[E], pb[E], lab[E];
+    {
+        unsigned h = desc & 0xFFu, pm = (desc >> 8) & 0xFFu;
+#pragma unroll
+        for (int j = 0; j < E; ++j) {
+            hc[j] = __ffs(h) - 1;
+            h &= h - 1;
+            pb[j] = __ffs(pm) - 1;
+            pm &= pm - 1;
+            lab[j] = j;
+        }
+    }
+    const double* P = blk + F.o_p;
+    double x[E][E];
+#pragma unroll
+    for (int i = 0; i < E; ++i)
+#pragma unroll
+        for (int j = 0; j < E; ++j) x[i][j] = P[pb[i] * K + hc[j]];
+    double detb = 1.0;
+#pragma unroll
+    for (int st = 0; st < E; ++st) {
+        int p = st;
+        double best = fabs(x[st][st]);
+#pragma unroll
+        for (int i = st + 1; i < E; ++i) {
+            const double av = fabs(x[i][st]);
+            if (av > best) {
+                best = av;
+                p = i;
+            }
+        }
+#pragma unroll
+        for (int i = st + 1; i < E; ++i) {
+            const bool sw = (p == i);
+#pragma unroll
+            for (int j = 0; j < E; ++j) {
+                const double a0 = x[st][j], a1 = x[i][j];
+                x[st][j] = sw ? a1 : a0;
+                x[i][j] = sw ? a0 : a1;
+            }
+            const int l0 = lab[st], l1 = lab[i];
+            lab[st] = sw ? l1 : l0;
+            lab[i] = sw ? l0 : l1;
+        }
+        if (p != st) detb = -detb;
+        const double piv = x[st][st];
+        detb *= piv;
+        const double ip = 1.0 / piv;
+        x[st][st] = 1.0;
+#pragma unroll
+        for (int j = 0; j < E; ++j) x[st][j] *= ip;
+#pragma unroll
+        for (int i = 0; i < E; ++i) {
+            if (i == st) continue;
+            const double f = x[i][st];
+            x[i][st] = 0.0;
+#pragma unroll
+            for (int j = 0; j < E; ++j) x[i][j] = fma(-f, x[st][j], x[i][j]);
+        }
+    }
+    double na2 = 0.0;
+#pragma unroll
+    for (int j = 0; j < E; ++j)
+#pragma unroll
+        for (int q = 0; q < E; ++q) {
+            as[j * E + lab[q]] = x[j][q];  // W(j, i) at as[j E + i]
+            na2 = fma(detb * x[j][q], detb * x[j][q], na2);
+        }
+    *ok = frame_certificate<K, E>(blk, F, hc, pb, na2, detb);
+    *dd = 0.0;
+    if (!*ok) return 0.0;
+    const double D = ((desc >> 16) & 1u ? -1.0 : 1.0) * blk[F.o_scal], scale = D * detb;
+    const double* Q = blk + F.o_q;
+    double M[E][E];  // T + a_H N
+    double c = s, q = 0.0;
+#pragma unroll 1
+    for (int i = 0; i < E; ++i)
+#pragma unroll 1
+        for (int j = 0; j < E; ++j) {
+            M[i][j] = ts[j * E + i];
+            c = fma(as[j * E + i], M[i][j], c);
+        }
+#pragma unroll 1
+    for (int i2 = 1; i2 < E; ++i2)
+#pragma unroll 1
+        for (int i1 = 0; i1 < i2; ++i1) {
+            const int qrow = (pb[i2] * (pb[i2] - 1) / 2 + pb[i1]) * CP;
+#pragma unroll 1
+            for (int j2 = 1; j2 < E; ++j2)
+#pragma unroll 1
+                for (int j1 = 0; j1 < j2; ++j1) {
+                    const int at = qrow + hc[j2] * (hc[j2] - 1) / 2 + hc[j1];
+                    const double w11 = as[j1 * E + i1], w12 = as[j1 * E + i2], w21 = as[j2 * E + i1], w22 = as[j2 * E + i2];
+                    const double minor = fma(w11, w22, -w12 * w21), qv = Q[at], g = aH * qv;
+                    q = fma(qv, minor, q);
+                    M[i1][j1] = fma(g, w22, M[i1][j1]);
+                    M[i2][j2] = fma(g, w11, M[i2][j2]);
+                    M[i2][j1] = fma(-g, w21, M[i2][j1]);
+                    M[i1][j2] = fma(-g, w12, M[i1][j2]);
+                    if (aH != 0.0) atomicAdd(gq + at, scale * aH * minor);
+                }
+        }
+    c = fma(aH, q, c);
+#pragma unroll 1
+    for (int j = 0; j < E; ++j) {
+        double y[E];  // row j of W M
+#pragma unroll 1
+        for (int b = 0; b < E; ++b) {
+            double acc = 0.0;
+            for (int i = 0; i < E; ++i) acc = fma(as[j * E + i], M[i][b], acc);
+            y[b] = acc;
+        }
+#pragma unroll 1
+        for (int i = 0; i < E; ++i) {
+            double acc = as[j * E + i] * c;
+            for (int b = 0; b < E; ++b) acc = fma(-y[b], as[b * E + i], acc);
+            ts[j * E + i] = scale * acc;
+        }
+    }
+#pragma unroll 1
+    for (int i = 0; i < E * E; ++i) as[i] *= scale;
+    *dd = scale;
+    return scale * c;
+}
+
 template <int K>
 __device__ __forceinline__ double backward_dispatch(int e, const double* blk, const FrameLayout& F, unsigned desc,
                                                     double s, double aH, double* ts, double* as, double* gq,
-                                                    double* dd) {
+                                                    double* dd, bool* ok) {
+    *ok = true;
+#define VB_BACKWARD_CASE(E_)                                                                          \
+    case E_:                                                                                          \
+        if constexpr (E_ <= K) {                                                                      \
+            if constexpr (E_ <= kMinorsEMax)                                                          \
+                return backward_minors<K, E_>(blk, F, desc, s, aH, ts, as, gq, dd);                   \
+            else                                                                                      \
+                return backward_inverse<K, E_>(blk, &F, desc, s, aH, ts, as, gq, dd, ok);             \
+        }                                                                                             \
+        break;
     switch (e) {
-        case 0: return backward_minors<K, 0>(blk, F, desc, s, aH, ts, as, gq, dd);
-        case 1: return backward_minors<K, 1>(blk, F, desc, s, aH, ts, as, gq, dd);
-        case 2:
-            if constexpr (K >= 2) return backward_minors<K, 2>(blk, F, desc, s, aH, ts, as, gq, dd);
-            break;
-        case 3:
-            if constexpr (K >= 3) return backward_minors<K, 3>(blk, F, desc, s, aH, ts, as, gq, dd);
-            break;
-        case 4:
-            if constexpr (K >= 4) return backward_minors<K, 4>(blk, F, desc, s, aH, ts, as, gq, dd);
-            break;
-        case 5:
-            if constexpr (K >= 5) return backward_minors<K, 5>(blk, F, desc, s, aH, ts, as, gq, dd);
-            break;
+        VB_BACKWARD_CASE(0)
+        VB_BACKWARD_CASE(1)
+        VB_BACKWARD_CASE(2)
+        VB_BACKWARD_CASE(3)
+        VB_BACKWARD_CASE(4)
+        VB_BACKWARD_CASE(5)
+        VB_BACKWARD_CASE(6)
+        VB_BACKWARD_CASE(7)
+        VB_BACKWARD_CASE(8)
         default: break;
     }
+#undef VB_BACKWARD_CASE
     *dd = 0.0;
     return 0.0;
 }
@@ -273,12 +421,13 @@ struct BackwardShape {
     static constexpr int kThreads = 32 * kWarps;
     static constexpr int kPairs = 32 * kWarps;  // pairs per round
     static constexpr int kLdw = 8 * MT + 4;     // = 4 mod 16: fragment loads without bank conflicts
+    static constexpr int kStage = stage_pairs(MT);
     static_assert(MT % 2 == 0, "staged row stride");
     __host__ __device__ static int table_rows(int R) { return (R + 2 + 3) / 4 * 4; }
     static size_t bytes(int n, int R) {
         const FrameLayout F = frame_layout(n, K, R);
         const size_t d = (size_t)table_rows(R) * fr_kfs(K) + (F.total - F.o_q) + 2 * (size_t)kPairs * kCompactSlot +
-                         2 * (size_t)kPairs + 2 * (size_t)kStagePairs * kLdw;
+                         2 * (size_t)kPairs + 2 * (size_t)kStage * kLdw;
         return sizeof(double) * d + (size_t)kPairs * (sizeof(long long) + 3 * sizeof(unsigned)) + kPairs;
     }
 };
@@ -296,7 +445,7 @@ __global__ void __launch_bounds__(32 * (K + 1), 1) frame_backward_pairs(FrameAdj
     double* sRest = sTab + trows * KFS;
     const double* blk = sRest - F.o_q;  // parts of the block from o_q on, at their usual offsets
     double* sW = sRest + (F.total - F.o_q);  // even offsets: the staged rows start 16-byte aligned
-    double* sA = sW + 2 * kStagePairs * LDW;
+    double* sA = sW + 2 * Shape::kStage * LDW;
     double* sT = sA + PAIRS * kCompactSlot;
     double* sD = sT + PAIRS * kCompactSlot;
     double* sTr = sD + PAIRS;
@@ -309,8 +458,11 @@ __global__ void __launch_bounds__(32 * (K + 1), 1) frame_backward_pairs(FrameAdj
     __shared__ double s_f[K + 1];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, gr = lane >> 2, gc = lane & 3;
     const long long N = a.n_strings;
-    const long long stride = a.adj_stride;
-    const int chunks16 = (int)(stride / 2);  // 16-byte pieces of an adjoint row
+    const bool direct = a.weight != nullptr;
+    const double* const rows = direct ? a.records : a.adj;
+    const long long stride = direct ? a.rec_stride : a.adj_stride;
+    const int hrow = direct ? R : R + 1;      // source row that weights the h + linear table row
+    const int chunks16 = (R + 2 + 1) / 2;     // 16-byte pieces of a source row
     for (;;) {
         if (tid == 0) s_task = (int)atomicAdd(a.task_counter, 1ull);
         __syncthreads();
@@ -324,10 +476,12 @@ __global__ void __launch_bounds__(32 * (K + 1), 1) frame_backward_pairs(FrameAdj
         for (int i = tid; i < trows * KFS; i += Shape::kThreads) {
             const int r = i / KFS, c = i % KFS;
             double v = 0.0;
-            if (r < R)
+            if (r < R) {
                 v = __ldg(src + (2 + r) * KFS + c);
-            else if (r == R + 1)
+                if (direct && r >= a.r_pos) v = -v;
+            } else if (r == hrow) {
                 v = __ldg(src + c) + __ldg(src + KFS + c);
+            }
             sTab[i] = v;
         }
         for (int i = tid; i < F.total - F.o_q; i += Shape::kThreads) sRest[i] = __ldg(src + F.o_q + i);
@@ -336,13 +490,12 @@ __global__ void __launch_bounds__(32 * (K + 1), 1) frame_backward_pairs(FrameAdj
         __syncthreads();
         const long long base = record_index(u, u, N);
         const bool sound = blk[F.o_scal + 1] * blk[F.o_scal + 2] < kAdjointCondition2;
-        constexpr int EM = K < kMinorsEMax ? K : kMinorsEMax;
-        // pairs left to the exact kernel
-        const int list0 = sound ? bound[EM + 1] : 0;
-        for (int i = list0 + tid; i < bound[K + 1]; i += Shape::kThreads) {
+        auto list = [&](int v) {
             const unsigned long long at = atomicAdd(a.careful_count, 1ull);
-            a.careful_list[at] = ((unsigned long long)u << 32) | (unsigned long long)__ldg(a.rlist + base + i);
-        }
+            a.careful_list[at] = ((unsigned long long)u << 32) | (unsigned long long)v;
+        };
+        if (!sound)
+            for (int i = tid; i < bound[K + 1]; i += Shape::kThreads) list(__ldg(a.rlist + base + i));
         if (!sound) {
             if (tid == 0) out[G.o_f + 1] = 0.0;
             __syncthreads();
@@ -350,7 +503,9 @@ __global__ void __launch_bounds__(32 * (K + 1), 1) frame_backward_pairs(FrameAdj
         }
         int nchunks = 0;
 #pragma unroll
-        for (int e = 0; e <= EM; ++e) nchunks += (bound[e + 1] - bound[e] + 31) / 32;
+        for (int e = 0; e <= K; ++e) nchunks += (bound[e + 1] - bound[e] + compact_chunk_pairs(e) - 1) / compact_chunk_pairs(e);
+        const double weight_u = direct ? __ldg(a.weight + u) : 0.0;
+        const int partner_u = direct ? __ldg(a.partner + u) : 0;
         double acc[MT][2];
 #pragma unroll
         for (int m = 0; m < MT; ++m) acc[m][0] = acc[m][1] = 0.0;
@@ -359,19 +514,32 @@ __global__ void __launch_bounds__(32 * (K + 1), 1) frame_backward_pairs(FrameAdj
             // ---- a lane per pair -------------------------------------------------------------
             int e = 0, start = 0, cnt = 0, left = c0 + warp;
 #pragma unroll
-            for (int ee = EM; ee >= 0; --ee) {
-                const int c = (bound[ee + 1] - bound[ee] + 31) / 32;
+            for (int ee = K; ee >= 0; --ee) {
+                const int cs = compact_chunk_pairs(ee), c = (bound[ee + 1] - bound[ee] + cs - 1) / cs;
                 if (left >= 0 && left < c) {
                     e = ee;
-                    start = bound[ee] + 32 * left;
-                    cnt = min(32, bound[ee + 1] - start);
+                    start = bound[ee] + cs * left;
+                    cnt = min(cs, bound[ee + 1] - start);
                 }
                 left -= c;
             }
             const bool valid = lane < cnt;
             const int pair0 = 32 * warp, pair = pair0 + lane;
             const unsigned desc = valid ? __ldg(a.rdesc + base + start + lane) : 0u;
-            const long long rec = valid ? record_index(u, __ldg(a.rlist + base + start + lane), N) : -1;
+            const int v = valid ? __ldg(a.rlist + base + start + lane) : u;
+            // source row of the pair's adjoint and its weight
+            long long rec = -1;
+            double omega = 1.0;
+            if (valid && direct) {
+                const int partner = __ldg(a.partner + v);
+                rec = record_index(min(partner_u, partner), max(partner_u, partner), N);
+                omega = (v == u ? 2.0 : 4.0) * weight_u * __ldg(a.weight + v);
+            } else if (valid) {
+                rec = record_index(u, v, N);
+            }
+            const int slot = compact_slot(e);
+            double* const as = sA + pair0 * kCompactSlot + lane * slot;
+            double* const ts = sT + pair0 * kCompactSlot + lane * slot;
             unsigned hmap = 0xFFFFFFFFu, pmap = 0xFFFFFFFFu;
             {
                 unsigned h = desc & 0xFFu, p = (desc >> 8) & 0xFFu;
@@ -392,81 +560,110 @@ __global__ void __launch_bounds__(32 * (K + 1), 1) frame_backward_pairs(FrameAdj
             if ((lane & 3) == 0) sUnion[pair >> 2] = un;
             double aS = 0.0, aH = 0.0;
             if (valid) {
-                aS = __ldg(a.adj + rec * stride + R);
-                aH = __ldg(a.adj + rec * stride + R + 1);
+                aS = __ldg(rows + rec * stride + R);
+                aH = __ldg(rows + rec * stride + R + 1);
+                if (direct) {  // a record holds the determinant, then the energy
+                    const double sb = aS;
+                    aS = omega * fma(-a.lambda, sb, aH);
+                    aH = omega * sb;
+                }
             }
-            // tau and tr_w, one 8-pair tile at a time
+            // tau and tr_w, one 8-pair tile at a time; the loads of a tile's rows (48 at a time) are all
+            // in flight together, the first ones issued while the tile before is multiplied
             const int tiles = (cnt + 7) / 8;
+            constexpr int kBatch = 12;
+            double wv[kBatch];
+            auto load_rows = [&](int mt, int r0) {
+                const long long rg = __shfl_sync(0xffffffffu, rec, (8 * mt + gr) & 31);
+                const double* w = rows + (rg < 0 ? 0 : rg) * stride + r0 + gc;
+#pragma unroll
+                for (int q = 0; q < kBatch; ++q)
+                    wv[q] = (rg >= 0 && r0 + 4 * q + gc < R + 2) ? __ldg(w + 4 * q) : 0.0;
+            };
+            if (tiles > 0) load_rows(0, 0);
 #pragma unroll 1
             for (int mt = 0; mt < tiles; ++mt) {
                 const int owner = 8 * mt + gr;
-                const long long rec_g = __shfl_sync(0xffffffffu, rec, owner);
+                const double omega_g = __shfl_sync(0xffffffffu, omega, owner);
                 const unsigned hmap_g = __shfl_sync(0xffffffffu, hmap, owner);
                 const unsigned pmap_g = __shfl_sync(0xffffffffu, pmap, owner);
                 const unsigned uh = __reduce_or_sync(0xffffffffu, (lane >> 3) == mt ? (desc & 0xFFu) : 0u);
-                const double* w = a.adj + (rec_g < 0 ? 0 : rec_g) * stride + gc;
                 double t[K][2], tr = 0.0;
 #pragma unroll
                 for (int c = 0; c < K; ++c) t[c][0] = t[c][1] = 0.0;
 #pragma unroll 1
-                for (int r0 = 0; r0 < trows; r0 += 16) {
-                    double wv[4];
+                for (int r0 = 0; r0 < trows; r0 += 4 * kBatch) {
+                    double wc[kBatch];
 #pragma unroll
-                    for (int q = 0; q < 4; ++q) wv[q] = (rec_g >= 0 && r0 + 4 * q + gc < R + 2) ? __ldg(w + r0 + 4 * q) : 0.0;
+                    for (int q = 0; q < kBatch; ++q) wc[q] = wv[q];
+                    if (r0 + 4 * kBatch < trows)
+                        load_rows(mt, r0 + 4 * kBatch);
+                    else if (mt + 1 < tiles)
+                        load_rows(mt + 1, 0);
 #pragma unroll
-                    for (int q = 0; q < 4; ++q) {
+                    for (int q = 0; q < kBatch; ++q) {
                         if (r0 + 4 * q >= trows) break;
                         const double* row = sTab + (r0 + 4 * q + gc) * KFS;
-                        tr = fma(wv[q], row[8 * K], tr);
+                        tr = fma(wc[q], row[8 * K], tr);
 #pragma unroll
                         for (int c = 0; c < K; ++c)
-                            if ((uh >> c) & 1u) mma_f64(t[c], wv[q], row[8 * c + gr]);
+                            if ((uh >> c) & 1u) mma_f64(t[c], wc[q], row[8 * c + gr]);
                     }
                 }
                 tr += __shfl_xor_sync(0xffffffffu, tr, 1);
                 tr += __shfl_xor_sync(0xffffffffu, tr, 2);
-                if (gc == 0) sTr[pair0 + owner] = tr;
-                double* ts = sT + (pair0 + owner) * kCompactSlot;
+                if (gc == 0) sTr[pair0 + owner] = omega_g * tr;
+                double* to = sT + pair0 * kCompactSlot + owner * slot;
 #pragma unroll
                 for (int c = 0; c < K; ++c) {
                     const unsigned jh = (hmap_g >> (4 * c)) & 0xFu;
 #pragma unroll
                     for (int x = 0; x < 2; ++x) {
                         const unsigned ip = (pmap_g >> (4 * (2 * gc + x))) & 0xFu;
-                        if (jh < (unsigned)e && ip < (unsigned)e) ts[jh * e + ip] = t[c][x];
+                        if (jh < (unsigned)e && ip < (unsigned)e) to[jh * e + ip] = omega_g * t[c][x];
                     }
                 }
             }
             __syncwarp();
             double dd = 0.0;
-            if (valid)
-                fsum += backward_dispatch<K>(e, blk, F, desc, aS + sTr[pair], aH, sT + pair * kCompactSlot,
-                                             sA + pair * kCompactSlot, out + G.o_q, &dd);
+            if (valid) {
+                bool ok;
+                fsum += backward_dispatch<K>(e, blk, F, desc, aS + sTr[pair], aH, ts, as, out + G.o_q, &dd, &ok);
+                if (!ok) {
+                    list(v);
+                    sH[pair] = 0xFFFFFFFFu;  // no hole: the pair adds nothing below
+                }
+                if (direct && ok) {
+                    // the staged rows are records: their weight goes with D adj B
+                    for (int i = 0; i < e * e; ++i) as[i] *= omega;
+                    dd *= omega;
+                }
+            }
             sD[pair] = dd;
             __syncthreads();
             // ---- adjoints of the tables ------------------------------------------------------
             const int used = min(PAIRS, 32 * (nchunks - c0));  // pairs of the warps that have a chunk
             auto stage = [&](int p0, int buf) {
-                for (int i = tid; i < kStagePairs * chunks16; i += Shape::kThreads) {
+                for (int i = tid; i < Shape::kStage * chunks16; i += Shape::kThreads) {
                     const int p = i / chunks16, q = i % chunks16;
                     const long long r = sRec[p0 + p];
-                    copy_async16(sW + (buf * kStagePairs + p) * LDW + 2 * q, a.adj + (r < 0 ? 0 : r) * stride + 2 * q, r >= 0);
+                    copy_async16(sW + (buf * Shape::kStage + p) * LDW + 2 * q, rows + (r < 0 ? 0 : r) * stride + 2 * q, r >= 0);
                 }
                 asm volatile("cp.async.commit_group;" ::: "memory");
             };
             stage(0, 0);
-            for (int p0 = 0; p0 < used; p0 += kStagePairs) {
-                const int buf = (p0 / kStagePairs) & 1;
-                if (p0 + kStagePairs < used) {
-                    stage(p0 + kStagePairs, buf ^ 1);
+            for (int p0 = 0; p0 < used; p0 += Shape::kStage) {
+                const int buf = (p0 / Shape::kStage) & 1;
+                if (p0 + Shape::kStage < used) {
+                    stage(p0 + Shape::kStage, buf ^ 1);
                     asm volatile("cp.async.wait_group 1;" ::: "memory");
                 } else {
                     asm volatile("cp.async.wait_group 0;" ::: "memory");
                 }
                 __syncthreads();
-                const double* w = sW + buf * kStagePairs * LDW;
+                const double* w = sW + buf * Shape::kStage * LDW;
 #pragma unroll
-                for (int g4 = 0; g4 < kStagePairs / 4; ++g4) {
+                for (int g4 = 0; g4 < Shape::kStage / 4; ++g4) {
                     const int p = p0 + 4 * g4 + gc;
                     double y = 0.0;
                     if (warp < K) {
@@ -474,8 +671,9 @@ __global__ void __launch_bounds__(32 * (K + 1), 1) frame_backward_pairs(FrameAdj
                         const unsigned le = sE[p];
                         const unsigned jh = (sH[p] >> (4 * warp)) & 0xFu, ip = (sPm[p] >> (4 * gr)) & 0xFu;
                         if (jh < le && ip < le) {
-                            y = sA[p * kCompactSlot + jh * le + ip];
-                            gp += sT[p * kCompactSlot + jh * le + ip];
+                            const int at = (p & ~31) * kCompactSlot + (p & 31) * compact_slot(le) + jh * le + ip;
+                            y = sA[at];
+                            gp += sT[at];
                         }
                     } else {
                         y = gr == 0 ? sD[p] : 0.0;
@@ -493,12 +691,15 @@ __global__ void __launch_bounds__(32 * (K + 1), 1) frame_backward_pairs(FrameAdj
         for (int m = 0; m < MT; ++m)
 #pragma unroll
             for (int x = 0; x < 2; ++x) {
-                const int r = 8 * m + gr, c = 2 * gc + x;
-                if (r >= R + 2) continue;
+                const int q = 8 * m + gr, c = 2 * gc + x;
+                if (q >= R + 2) continue;
+                // block rows are in adjoint order: a record's determinant and energy are the other way round
+                const int r = direct && q >= R ? 2 * R + 1 - q : q;
+                const double v = direct && q < R && q >= a.r_pos ? -acc[m][x] : acc[m][x];
                 if (warp < K)
-                    out[r * KFS + 8 * warp + c] = acc[m][x];
+                    out[r * KFS + 8 * warp + c] = v;
                 else if (c == 0)
-                    out[r * KFS + 8 * K] = acc[m][x];
+                    out[r * KFS + 8 * K] = v;
             }
         gp += __shfl_xor_sync(0xffffffffu, gp, 1);
         gp += __shfl_xor_sync(0xffffffffu, gp, 2);

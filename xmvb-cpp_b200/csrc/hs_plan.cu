@@ -472,6 +472,7 @@ vb_status vb_hs_plan_create(vb_context* ctx, const vb_expansion* ex, vb_hs_plan*
             // determinants grouped by alpha string, for the gradient's per-record adjoint sums
             std::vector<int> aoff(p->Na + 1, 0), adets(p->n_det);
             for (long long d = 0; d < p->n_det; ++d) ++aoff[ex->det_alpha[d] + 1];
+            p->single_determinants = *std::max_element(aoff.begin(), aoff.end()) <= 1;
             for (int i = 0; i < p->Na; ++i) aoff[i + 1] += aoff[i];
             std::vector<int> next(aoff.begin(), aoff.end() - 1);
             for (long long d = 0; d < p->n_det; ++d) adets[next[ex->det_alpha[d]]++] = (int)d;

@@ -70,6 +70,7 @@ struct vb_hs_plan {
     // determinants by alpha string (CSR: alpha_off[i] .. alpha_off[i + 1] index alpha_dets)
     DeviceBuffer alpha_off, alpha_dets;
     bool has_flip = false;
+    bool single_determinants = false;  // (has_flip) no alpha string carries two determinants
     // internal position of each determinant of the caller's list when the plan reorders them
     // (empty: the caller's order), host copy and device copy
     std::vector<long long> det_position;

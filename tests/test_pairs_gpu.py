@@ -332,3 +332,49 @@ def test_block_ordered_determinants_match_oracle(ctx, kw, n, nel, mult):
         y = S[np.ix_(b[e], b[d])]
         ref = np.linalg.det(x) * np.linalg.det(y)
         assert abs(so[q] - ref) < 1e-11 * max(1.0, abs(ref))
+
+
+@pytest.mark.parametrize("n,mult", [(4, 1), (5, 2), (6, 1), (6, 3), (7, 4), (8, 1), (9, 2), (10, 3), (11, 2), (12, 1), (13, 2)])
+@pytest.mark.parametrize("overlap", ["random", "orthogonal", "dependent"])
+def test_covalent_pairs_match_records(ctx, n, mult, overlap):
+    """Covalent lists take both spins of a determinant pair in one kernel; the same matrices from the
+    spin-pair records (the listed determinant pairs of the same plan, all of them, contracted with the
+    expansion here).  Closed and open shells, one pair per spin-flip orbit and all of them, levels 0 ..
+    6, regular overlaps, overlaps of 0 (every excited block singular, the highest levels listed) and two
+    nearly dependent orbitals (strings that hold both have kappa(S_LL) near 1e8 and are listed with all
+    their pairs, or certified just below it).  Both forms add the same terms in another order, 1e-11 of
+    the largest element; dependent orbitals: a certified block carries eps kappa_F < 2.2e-16 1e8 = 2.2e-8,
+    and the two forms take a pair from either of its strings."""
+    rng = np.random.default_rng(10 * n + mult)
+    S, h, eri = workloads.active_space(n, 3 * n, 90 + n)
+    if overlap == "orthogonal":
+        S = np.eye(n)
+    elif overlap == "dependent":
+        C = np.eye(n) + 0.05 * rng.standard_normal((n, n))
+        C[:, 1] = C[:, 0] + 1e-4 * C[:, 1]
+        S = C.T @ C
+        d = 1.0 / np.sqrt(np.diag(S))
+        S = d[:, None] * S * d[None, :]
+    tol = 2.2e-8 if overlap == "dependent" else 1e-11
+    rows = vbcore.generate_structures("COV", n, n, mult)
+    ex = vbcore.expand_structures(rows, n, mult)
+    plan = vbcore.HsPlan(ctx, ex, n)
+    H, So = plan.execute(S, h, eri)
+    assert np.array_equal(H, H.T) and np.array_equal(So, So.T)
+    oex = O.expand(O.generate_structures("COV", n, n, mult), n, mult)
+    if n <= 8:
+        Hr, Sr, _ = O.structure_matrices(n, oex, S, h, eri)
+        assert _rel(H, Hr) < max(REL, tol) and _rel(So, Sr) < max(REL, tol)
+    nd = ex.n_determinants
+    pairs = np.array([(d, e) for d in range(nd) for e in range(d, nd)], dtype=np.int64)
+    hd, sd = plan.determinant_pairs(S, h, eri, pairs)
+    Hd = np.zeros((nd, nd))
+    Sd = np.zeros((nd, nd))
+    Hd[pairs[:, 0], pairs[:, 1]] = Hd[pairs[:, 1], pairs[:, 0]] = hd
+    Sd[pairs[:, 0], pairs[:, 1]] = Sd[pairs[:, 1], pairs[:, 0]] = sd
+    T = np.zeros((nd, plan.n_structures))
+    off = ex.term_offsets
+    for d in range(nd):
+        T[d, ex.term_structure[off[d]:off[d + 1]]] = ex.term_coefficient[off[d]:off[d + 1]]
+    assert _rel(H, T.T @ Hd @ T) < tol and _rel(So, T.T @ Sd @ T) < tol
+    plan.close()

@@ -69,24 +69,48 @@ __device__ __forceinline__ uint64_t occ_mask(uint64_t w, int k) {
     return m;
 }
 
+// One left string's block: with its electron count at compile time, or chosen per thread.
+template <int K>
+struct FrameView {
+    const double* blk;
+    const FrameLayout& F;
+    __device__ static constexpr int k() { return K; }
+    __device__ static constexpr int cp() { return fr_cp(K); }
+    __device__ const double* p() const { return blk + F.o_p; }
+    __device__ const double* q() const { return blk + F.o_q; }
+    __device__ const double* rowsq() const { return blk + F.o_rowsq; }
+    __device__ const double* prow2() const { return blk + F.o_prow2; }
+    __device__ const double* scal() const { return blk + F.o_scal; }
+};
+struct FrameViewAny {
+    const double* rest;  // the block from Q on
+    int kk, o_p, o_rowsq, o_prow2, o_scal;
+    __device__ int k() const { return kk; }
+    __device__ int cp() const { return kk * (kk - 1) / 2; }
+    __device__ const double* p() const { return rest + o_p; }
+    __device__ const double* q() const { return rest; }
+    __device__ const double* rowsq() const { return rest + o_rowsq; }
+    __device__ const double* prow2() const { return rest + o_prow2; }
+    __device__ const double* scal() const { return rest + o_scal; }
+};
+
 // The certificate of kernels.h for X = P[R, :] S_LL with B^-1 = A / detb, without the division:
 // ||X||_F^2 from the row norms, ||X^-1||_F <= ||S_LL^-1||_F ||P[R, :]^-1||_F and
 // ||P[R, :]^-1||_F^2 <= (K - E) + ||B^-1||_F^2 (1 + sum_i ||P[p_i, :]||^2).
-template <int K, int E>
-__device__ __forceinline__ bool frame_certificate(const double* __restrict__ blk, const FrameLayout& F,
-                                                  const int (&hc)[E > 0 ? E : 1], const int (&pb)[E > 0 ? E : 1],
-                                                  double na2, double detb) {
-    const double* scal = blk + F.o_scal;
-    const double* rowsq = blk + F.o_rowsq;
-    const double* prow2 = blk + F.o_prow2;
+template <int E, class View>
+__device__ __forceinline__ bool frame_certificate(const View& f, const int (&hc)[E > 0 ? E : 1],
+                                                  const int (&pb)[E > 0 ? E : 1], double na2, double detb) {
+    const double* scal = f.scal();
+    const double* rowsq = f.rowsq();
+    const double* prow2 = f.prow2();
     double nx2 = scal[2], pr = 0.0;
 #pragma unroll
     for (int j = 0; j < E; ++j) {
-        nx2 += rowsq[K + pb[j]] - rowsq[hc[j]];
+        nx2 += rowsq[f.k() + pb[j]] - rowsq[hc[j]];
         pr += prow2[pb[j]];
     }
     const double det2 = detb * detb;
-    const double lhs = nx2 * scal[1] * ((double)(K - E) * det2 + na2 * (1.0 + pr));
+    const double lhs = nx2 * scal[1] * ((double)(f.k() - E) * det2 + na2 * (1.0 + pr));
     return isfinite(lhs) && det2 > 0.0 && lhs < kCertificate2 * det2;
 }
 

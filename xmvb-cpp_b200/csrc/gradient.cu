@@ -986,10 +986,11 @@ extern "C" vb_status vb_hs_plan_gradient(vb_hs_plan* p, const double* S, const d
     int launches = 0;
     const double *dS = nullptr, *dh = nullptr, *deri = nullptr;
     vb_status st = VB_OK;
-    if (records_match(p, S, h, eri, mem_space)) {
+    if (inputs_match(p, S, h, eri, mem_space)) {
         dS = p->S_in.as<double>();
         dh = p->h_in.as<double>();
         deri = p->eri_in.as<double>();
+        if (!p->records_current && (st = evaluate_spin_records(p, dS, dh, deri, &launches)) != VB_OK) return st;
     } else if ((st = prepare_spin_records(p, S, h, eri, mem_space, &dS, &dh, &deri, &launches)) != VB_OK) {
         return st;
     }

@@ -325,7 +325,7 @@ __device__ __noinline__ double backward_inverse(const double* __restrict__ blk, 
             as[j * E + lab[q]] = x[j][q];  // W(j, i) at as[j E + i]
             na2 = fma(detb * x[j][q], detb * x[j][q], na2);
         }
-    *ok = frame_certificate<K, E>(blk, F, hc, pb, na2, detb);
+    *ok = frame_certificate<E>(FrameView<K>{blk, F}, hc, pb, na2, detb);
     *dd = 0.0;
     if (!*ok) return 0.0;
     const double D = ((desc >> 16) & 1u ? -1.0 : 1.0) * blk[F.o_scal], scale = D * detb;

@@ -216,6 +216,80 @@ vb_status upload_blocks(vb_hs_plan* p, const DeterminantBlocks& b) {
     return st;
 }
 
+// Pair lists of a covalent list: every orbital singly occupied, one determinant per alpha string, frame
+// tables for both spins and, where these are one table, spin-flip symmetric.  Without room for them the
+// records path needs none.
+vb_status covalent_lists(vb_hs_plan* p, const vb_expansion* ex) {
+    const int n = p->n;
+    if (p->ka < p->kb || p->ka + p->kb != n || p->n_det != p->Na || p->n_det != p->Nb || !p->tables_a.ptr ||
+        (p->shared_tables ? !p->has_flip : !p->tables_b.ptr) || !covalent_pairs_supported(n, p->ka, p->kb, 0))
+        return VB_OK;
+    const uint64_t all = n >= 64 ? ~0ull : (1ull << n) - 1;
+    std::vector<int> det(p->Na, -1), beta(p->Na, -1);
+    for (long long d = 0; d < p->n_det; ++d) {
+        const int u = ex->det_alpha[d], x = ex->det_beta[d];
+        if ((ex->alpha_strings[u] ^ ex->beta_strings[x]) != all || det[u] >= 0) return VB_OK;
+        det[u] = (int)d;
+        beta[u] = x;
+    }
+    CovalentPlan& c = p->covalent;
+    const size_t pairs = (size_t)std::max(1LL, p->npairs_a);
+    vb_status st = upload(p->ctx, c.det, det.data(), sizeof(int) * det.size());
+    if (st == VB_OK) st = upload(p->ctx, c.beta, beta.data(), sizeof(int) * beta.size());
+    if (st == VB_OK) st = c.desc.allocate(p->ctx, sizeof(unsigned) * pairs);
+    if (st == VB_OK) st = c.bounds.allocate(p->ctx, sizeof(int) * (size_t)p->Na * (p->ka + 2));
+    if (st == VB_OK) st = c.listed.allocate(p->ctx, sizeof(unsigned long long) * pairs);
+    if (st == VB_OK) st = c.list.allocate(p->ctx, sizeof(int) * pairs);
+    if (st == VB_ERR_BUDGET) {
+        for (DeviceBuffer* b : {&c.det, &c.beta, &c.desc, &c.bounds, &c.listed, &c.list}) b->release();
+        return VB_OK;
+    }
+    if (st != VB_OK) return st;
+    CovalentArgs a{};
+    a.n = n;
+    a.ka = p->ka;
+    a.kb = p->kb;
+    a.n_strings = p->Na;
+    a.fold = p->shared_tables;
+    a.beta = c.beta.as<int>();
+    const cudaError_t err = launch_sort_covalent_pairs(a, p->occ_a.as<uint64_t>(), c.list.as<int>(), c.desc.as<unsigned>(),
+                                                       c.bounds.as<int>(), p->ctx->stream);
+    return err == cudaSuccess ? VB_OK : cuda_error(p->ctx, err, "sort_covalent_pairs");
+}
+
+CovalentArgs covalent_args(const vb_hs_plan* p, const FullPairArgs& f) {
+    const CovalentPlan& c = p->covalent;
+    auto* counters = p->counters.as<unsigned long long>();
+    CovalentArgs a{};
+    a.n = p->n;
+    a.ka = p->ka;
+    a.kb = p->kb;
+    a.n_strings = p->Na;
+    a.R = p->R;
+    a.r_pos = p->r_pos;
+    a.fold = p->shared_tables;
+    a.det = c.det.as<int>();
+    a.beta = c.beta.as<int>();
+    a.tables_a = p->tables_a.as<double>();
+    a.tables_b = (p->shared_tables ? p->tables_a : p->tables_b).as<double>();
+    a.list = c.list.as<int>();
+    a.desc = c.desc.as<unsigned>();
+    a.bounds = c.bounds.as<int>();
+    a.Hb = f.Hb;
+    a.Sb = f.Sb;
+    a.ldb = f.ldb;
+    a.task_counter = counters + 4;
+    a.uncertified_a = counters + 8;
+    a.uncertified_b = counters + (p->shared_tables ? 8 : 9);
+    a.count_a = counters;
+    a.count_b = counters + (p->shared_tables ? 0 : 1);
+    a.list_a = p->list_a.as<unsigned long long>();
+    a.list_b = (p->shared_tables ? p->list_a : p->list_b).as<unsigned long long>();
+    a.listed_count = counters + 10;
+    a.listed = c.listed.as<unsigned long long>();
+    return a;
+}
+
 BlockPairArgs block_args(const vb_hs_plan* p, const FullPairArgs& f) {
     BlockPairArgs a{};
     a.f = f;
@@ -488,6 +562,7 @@ vb_status vb_hs_plan_create(vb_context* ctx, const vb_expansion* ex, vb_hs_plan*
         }
     }
 
+    if ((st = covalent_lists(p, ex)) != VB_OK) return fail(st);
     if (!p->has_flip) p->det_pair_evaluations = p->n_det * (p->n_det + 1) / 2;
 
     // band of determinant columns: keep the two band buffers within ~1 GB and 1/8 of the budget
@@ -678,8 +753,8 @@ FullPairArgs full_args(vb_hs_plan* p) {
 }
 
 // Stage inputs and evaluate the spin-pair records of every distinct table.
-bool records_match(const vb_hs_plan* p, const double* S, const double* h, const double* eri, int mem) {
-    if (mem != VB_MEM_HOST || !p->records_current) return false;
+bool inputs_match(const vb_hs_plan* p, const double* S, const double* h, const double* eri, int mem) {
+    if (mem != VB_MEM_HOST || !p->tables_current) return false;
     const size_t n2 = (size_t)p->n * p->n, ne = (size_t)p->np * (p->np + 1) / 2;
     if (p->last_inputs.size() != 2 * n2 + ne) return false;
     return std::memcmp(p->last_inputs.data(), S, sizeof(double) * n2) == 0 &&
@@ -687,13 +762,13 @@ bool records_match(const vb_hs_plan* p, const double* S, const double* h, const 
            std::memcmp(p->last_inputs.data() + 2 * n2, eri, sizeof(double) * ne) == 0;
 }
 
-vb_status prepare_spin_records(vb_hs_plan* p, const double* S, const double* h, const double* eri, int mem,
+vb_status prepare_frame_tables(vb_hs_plan* p, const double* S, const double* h, const double* eri, int mem,
                                const double** dS, const double** dh, const double** deri, int* launches) {
     vb_context* ctx = p->ctx;
     cudaStream_t s = ctx->stream;
     const size_t n2 = sizeof(double) * p->n * p->n;
     const size_t ne = sizeof(double) * (size_t)p->np * (p->np + 1) / 2;
-    p->records_current = false;
+    p->tables_current = p->records_current = false;
     if (mem == VB_MEM_HOST) {
         const size_t a = (size_t)p->n * p->n, b = (size_t)p->np * (p->np + 1) / 2;
         p->last_inputs.resize(2 * a + b);
@@ -756,29 +831,42 @@ vb_status prepare_spin_records(vb_hs_plan* p, const double* S, const double* h, 
             if (err != cudaSuccess) return cuda_error(ctx, err, "frame tables (beta)");
         }
     }
+    p->tables_current = mem == VB_MEM_HOST;
+    return VB_OK;
+}
+
+vb_status evaluate_spin_records(vb_hs_plan* p, const double* dS, const double* dh, const double* deri, int* launches) {
+    vb_context* ctx = p->ctx;
+    cudaStream_t s = ctx->stream;
     PhaseMark spin(p, VB_PHASE_SPIN_PAIRS);
-    err = cudaMemsetAsync(p->counters.ptr, 0, kPlanCounters * sizeof(unsigned long long), s);
+    cudaError_t err = cudaMemsetAsync(p->counters.ptr, 0, kPlanCounters * sizeof(unsigned long long), s);
     if (err != cudaSuccess) return cuda_error(ctx, err, "cudaMemsetAsync");
     if (p->ka > 0) {
-        err = launch_spin_pairs(table_args(p, false, *dS, *dh, *deri), p->tables_a.as<double>(), s, launches);
+        err = launch_spin_pairs(table_args(p, false, dS, dh, deri), p->tables_a.as<double>(), s, launches);
         if (err != cudaSuccess) return cuda_error(ctx, err, "spin_pairs (alpha)");
     }
     if (p->kb > 0 && !p->shared_tables) {
-        err = launch_spin_pairs(table_args(p, true, *dS, *dh, *deri), p->tables_b.as<double>(), s, launches);
+        err = launch_spin_pairs(table_args(p, true, dS, dh, deri), p->tables_b.as<double>(), s, launches);
         if (err != cudaSuccess) return cuda_error(ctx, err, "spin_pairs (beta)");
     }
     spin.close();
     PhaseMark exact(p, VB_PHASE_EXACT_PAIRS);
     if (p->ka > 0) {
-        err = launch_spin_pairs_exact(table_args(p, false, *dS, *dh, *deri), s, launches);
+        err = launch_spin_pairs_exact(table_args(p, false, dS, dh, deri), s, launches);
         if (err != cudaSuccess) return cuda_error(ctx, err, "spin_pairs exact (alpha)");
     }
     if (p->kb > 0 && !p->shared_tables) {
-        err = launch_spin_pairs_exact(table_args(p, true, *dS, *dh, *deri), s, launches);
+        err = launch_spin_pairs_exact(table_args(p, true, dS, dh, deri), s, launches);
         if (err != cudaSuccess) return cuda_error(ctx, err, "spin_pairs exact (beta)");
     }
-    p->records_current = mem == VB_MEM_HOST;
+    p->records_current = p->tables_current;
     return VB_OK;
+}
+
+vb_status prepare_spin_records(vb_hs_plan* p, const double* S, const double* h, const double* eri, int mem,
+                               const double** dS, const double** dh, const double** deri, int* launches) {
+    const vb_status st = prepare_frame_tables(p, S, h, eri, mem, dS, dh, deri, launches);
+    return st == VB_OK ? evaluate_spin_records(p, *dS, *dh, *deri, launches) : st;
 }
 
 }  // namespace vbcore
@@ -789,15 +877,21 @@ namespace {
 
 // Inputs in `mem`; outputs: H_out/S_out in `mem`, or (H_out == nullptr) left in the plan's
 // device buffers Hout/Sout.
-vb_status execute_impl(vb_hs_plan* p, const double* S, const double* h, const double* eri, int mem, double* H_out,
-                       double* S_out) {
+// keep_records: leave the spin-pair records for a gradient at the same inputs
+vb_status execute_impl(vb_hs_plan* p, const double* S, const double* h, const double* eri, int mem, bool keep_records,
+                       double* H_out, double* S_out) {
     vb_context* ctx = p->ctx;
     cudaSetDevice(ctx->device);
     cudaStream_t s = ctx->stream;
     int launches = 0;
     const double *dS, *dh, *deri;
-    vb_status st = prepare_spin_records(p, S, h, eri, mem, &dS, &dh, &deri, &launches);
+    vb_status st = prepare_frame_tables(p, S, h, eri, mem, &dS, &dh, &deri, &launches);
     if (st != VB_OK) return st;
+    // Covalent lists go from the frame tables straight to the determinant pairs, unless a gradient that
+    // reads the records follows.
+    const bool covalent = !keep_records && p->covalent.list.ptr && p->bands.size() == 2 &&
+                          covalent_pairs_supported(p->n, p->ka, p->kb, p->R);
+    if (!covalent && (st = evaluate_spin_records(p, dS, dh, deri, &launches)) != VB_OK) return st;
     // execute scratch of the context: bands [n_det x width] and Z [n_det x n_str] (H, S), W [n_str^2] (H, S)
     double* scr[6];
     {
@@ -821,9 +915,21 @@ vb_status execute_impl(vb_hs_plan* p, const double* S, const double* h, const do
         fa.ldb = p->band_ld;
         fa.Hb = scr[0];
         fa.Sb = scr[1];
+        if (covalent) {
+            PhaseMark spin(p, VB_PHASE_SPIN_PAIRS);
+            cudaError_t cerr = cudaMemsetAsync(p->counters.ptr, 0, kPlanCounters * sizeof(unsigned long long), s);
+            if (cerr == cudaSuccess) cerr = launch_covalent_pairs(covalent_args(p, fa), s, &launches);
+            if (cerr != cudaSuccess) return cuda_error(ctx, cerr, "covalent_pairs");
+            spin.close();
+            PhaseMark exact(p, VB_PHASE_EXACT_PAIRS);
+            for (int beta = 0; beta < (p->shared_tables ? 1 : 2) && cerr == cudaSuccess; ++beta)
+                cerr = launch_spin_pairs_exact(table_args(p, beta != 0, dS, dh, deri), s, &launches);
+            if (cerr != cudaSuccess) return cuda_error(ctx, cerr, "spin_pairs exact");
+        }
         PhaseMark pairs(p, VB_PHASE_DETERMINANT_PAIRS);
-        cudaError_t err = p->blocks.n > 0 ? launch_block_pairs(block_args(p, fa), s, &launches)
-                                          : launch_full_pairs(fa, s, &launches);
+        cudaError_t err = covalent         ? launch_listed_covalent_pairs(covalent_args(p, fa), fa, s, &launches)
+                          : p->blocks.n > 0 ? launch_block_pairs(block_args(p, fa), s, &launches)
+                                            : launch_full_pairs(fa, s, &launches);
         if (err != cudaSuccess) return cuda_error(ctx, err, "full_pairs");
         pairs.close();
         PhaseMark reduce(p, VB_PHASE_BAND_REDUCE);
@@ -909,7 +1015,7 @@ vb_status vb_hs_plan_execute(vb_hs_plan* p, const double* S, const double* h, co
     vb_context* ctx = p->ctx;
     if (!S || !h || !eri || !H_out || !S_out) return set_error(ctx, VB_ERR_INVALID, "vb_hs_plan_execute: null pointer");
     if (mem != VB_MEM_HOST && mem != VB_MEM_DEVICE) return set_error(ctx, VB_ERR_INVALID, "bad memory space");
-    return execute_impl(p, S, h, eri, mem, H_out, S_out);
+    return execute_impl(p, S, h, eri, mem, false, H_out, S_out);
 }
 
 vb_status vb_hs_plan_root_gradient(vb_hs_plan* p, const double* S, const double* h, const double* eri,
@@ -919,7 +1025,7 @@ vb_status vb_hs_plan_root_gradient(vb_hs_plan* p, const double* S, const double*
     vb_context* ctx = p->ctx;
     if (!S || !h || !eri || !energy)
         return set_error(ctx, VB_ERR_INVALID, "vb_hs_plan_root_gradient: null pointer");
-    vb_status st = execute_impl(p, S, h, eri, VB_MEM_HOST, nullptr, nullptr);
+    vb_status st = execute_impl(p, S, h, eri, VB_MEM_HOST, dS_out && dh_out, nullptr, nullptr);
     if (st == VB_OK) st = band_status(p);
     if (st != VB_OK) return st;
     const int ns = p->n_str;

@@ -67,6 +67,29 @@ struct FullPairArgs {
     const int* flip;      // spin-flip permutation of determinants (nullptr: no folding)
 };
 
+// Determinant pairs of a covalent list from the frame tables (covalent_pairs.cu): alpha string u has the
+// determinant det[u] with the beta string beta[u], its complement.
+struct CovalentArgs {
+    int n, ka, kb;      // ka >= kb, n = ka + kb
+    int n_strings;      // of alpha; the beta table has as many
+    int R, r_pos;
+    bool fold;          // one table for both spins and a spin-flip symmetric list: one pair per orbit is listed
+    const int* det;
+    const int* beta;
+    const double* tables_a;
+    const double* tables_b;
+    const int* list;        // as SpinTableArgs::rlist, rdesc (with the beta parity << 17), ebound
+    const unsigned* desc;
+    const int* bounds;
+    double* Hb;             // upper triangle, row stride ldb
+    double* Sb;
+    long long ldb;
+    unsigned long long* task_counter;                 // zero
+    unsigned long long *uncertified_a, *uncertified_b;
+    unsigned long long *count_a, *count_b, *list_a, *list_b;  // records for the exact path (as careful_list)
+    unsigned long long *listed_count, *listed;        // and their determinant pairs, (u << 32) | v
+};
+
 // Determinant pairs of one band by blocks of the determinant list: block h holds determinants
 // first[h] .. first[h + 1] - 1 of at most 8 alpha x 8 beta strings (0xFFFF beyond the last); the
 // determinant of cell (i, k) is first[h] + cell[8 i + k] (0xFF: none).  Blocks h0 .. h1 - 1 are the
@@ -179,6 +202,11 @@ cudaError_t preload_frame_kernels();
 cudaError_t preload_spin_pair_kernels();
 cudaError_t launch_full_pairs(const FullPairArgs& a, cudaStream_t stream, int* launches);
 cudaError_t launch_block_pairs(const BlockPairArgs& a, cudaStream_t stream, int* launches);
+bool covalent_pairs_supported(int n, int ka, int kb, int R);
+cudaError_t launch_sort_covalent_pairs(const CovalentArgs& a, const uint64_t* occ, int* list, unsigned* desc, int* bounds,
+                                       cudaStream_t stream);
+cudaError_t launch_covalent_pairs(const CovalentArgs& a, cudaStream_t stream, int* launches);
+cudaError_t launch_listed_covalent_pairs(const CovalentArgs& a, const FullPairArgs& f, cudaStream_t stream, int* launches);
 cudaError_t launch_band_reduce(const BandReduceArgs& a, cudaStream_t stream, int* launches);
 cudaError_t launch_structure_reduce(const StructureReduceArgs& a, double* H, double* S, cudaStream_t stream,
                                     int* launches);

@@ -28,7 +28,12 @@ struct PlanBlocks {
     std::vector<int> first_host;
 };
 
-constexpr int kPlanCounters = 10;
+// Pair lists of a covalent determinant list (CovalentArgs); empty where it is not one.
+struct CovalentPlan {
+    DeviceBuffer det, beta, list, desc, bounds, listed;
+};
+
+constexpr int kPlanCounters = 11;
 
 struct vb_hs_plan {
     vb_context* ctx = nullptr;
@@ -63,8 +68,9 @@ struct vb_hs_plan {
     DeviceBuffer adj_a, adj_b, grad_acc;
     // host inputs of the last host-pointer evaluation whose records are still resident
     std::vector<double> last_inputs;
-    bool records_current = false;
+    bool tables_current = false, records_current = false;
     BandSegments segments;
+    CovalentPlan covalent;
     // spin-flip map of the determinant list (folds the determinant-pair work in half)
     DeviceBuffer flip;
     // determinants by alpha string (CSR: alpha_off[i] .. alpha_off[i + 1] index alpha_dets)
@@ -102,9 +108,11 @@ FullPairArgs full_args(vb_hs_plan* p);
 // Uploads host inputs (mem == VB_MEM_HOST), builds the integral tables and the pair-kernel
 // factorization, and evaluates every spin-pair record; *dS, *dh, *deri receive the device
 // copies of the inputs.
-// True when the resident spin-pair records were evaluated from exactly these host inputs.
-bool records_match(const vb_hs_plan* p, const double* S, const double* h, const double* eri, int mem);
+// True when the resident inputs and frame tables are those of exactly these host inputs.
+bool inputs_match(const vb_hs_plan* p, const double* S, const double* h, const double* eri, int mem);
 vb_status prepare_spin_records(vb_hs_plan* p, const double* S, const double* h, const double* eri, int mem,
                                const double** dS, const double** dh, const double** deri, int* launches);
+// The second half of it: the records, from the frame tables.
+vb_status evaluate_spin_records(vb_hs_plan* p, const double* dS, const double* dh, const double* deri, int* launches);
 
 }  // namespace vbcore

@@ -16,11 +16,13 @@
 #include <mutex>
 
 #include "internal.h"
+#include "frame.cuh"
 #include "kernels.h"
 
 namespace vbcore {
 namespace {
 
+constexpr int kSms = 148;
 constexpr int kTileBytes = kBandTileRows * kBandColumns * 8;  // one band tile (H or S)
 constexpr long long kDrainPolls = 1ll << 22;  // bound on waiting for copies in flight (~seconds)
 constexpr int kZPad = kBandColumns + 1;
@@ -29,10 +31,6 @@ __device__ __forceinline__ unsigned smem_addr(const void* p) { return (unsigned)
 
 __device__ __forceinline__ void mbar_init(unsigned long long* bar, unsigned arrivals) {
     asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_addr(bar)), "r"(arrivals) : "memory");
-}
-
-__device__ __forceinline__ void copy_async16(void* dst, const void* src) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_addr(dst)), "l"(src) : "memory");
 }
 
 __device__ __forceinline__ void mbar_expect_tx(unsigned long long* bar, unsigned bytes) {
@@ -87,13 +85,6 @@ __device__ __forceinline__ void bulk_load(void* dst, const void* src, unsigned b
 // Tiles that reach below the diagonal have their entries d > e zeroed in shared memory first,
 // so the term loop carries no mask.  The accumulators then pass through shared memory so that
 // Z is written in coalesced runs of structures.
-//
-// GATHER (block-ordered determinant lists): a structure group's rows lie anywhere, so a tile is a list
-// of 64 of them, copied by cp.async (16 bytes per thread and copy; completion through the stage's
-// mbarrier, one arrival per thread).  The n = 12 covalent + ionic groups have 252 to 504 rows each, 4 to
-// 8 full tiles; with rows only grouped by structure a group met 30 partly used ones.  Both forms take
-// 10.1 to 10.4 ms there; a bulk copy per 256-byte row ran at 110 cycles a copy (16.7 ms).
-template <bool GATHER>
 __global__ void __launch_bounds__(kBandWarps * 32, 3)
     band_reduce_kernel(const __grid_constant__ CUtensorMap map_h, const __grid_constant__ CUtensorMap map_s,
                        BandReduceArgs a, int stage_bytes) {
@@ -124,46 +115,29 @@ __global__ void __launch_bounds__(kBandWarps * 32, 3)
         nt = lo;
     }
 
-    // stage st <- the i-th tile: thread 0 by TMA, or (GATHER) every thread its share of the rows
-    constexpr int kRowChunks = kBandColumns * 8 / 16;  // 16-byte pieces of a row
+    // stage st <- the i-th tile
     auto issue = [&](int i, int st) {
         const int t = t_begin + i;
         unsigned char* base = bsm + (size_t)st * stage_bytes;
-        if (GATHER) {
-            for (int q = tid; q < kBandTileRows * kRowChunks; q += kBandWarps * 32) {
-                const int row = a.seg_rows[(long long)t * kBandTileRows + q / kRowChunks], piece = q % kRowChunks;
-                if (row < 0) continue;
-                const long long at = row * a.ldb + col0 + 2 * piece;
-                copy_async16(base + 16 * q, a.Hb + at);
-                copy_async16(base + kTileBytes + 16 * q, a.Sb + at);
-            }
-            asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(smem_addr(&full[st])) : "memory");
-            if (tid != 0) return;
-        }
         const long long o0 = a.seg_off[t];
         const unsigned len = (unsigned)(a.seg_off[t + 1] - o0);
-        mbar_expect_tx(&full[st], (GATHER ? 0u : 2u * kTileBytes) + 9u * len + kBandMetaBytes);
-        if (!GATHER) {
-            tma_band_tile(base, &map_h, (int)col0, a.seg_first[t], &full[st]);
-            tma_band_tile(base + kTileBytes, &map_s, (int)col0, a.seg_first[t], &full[st]);
-        }
+        mbar_expect_tx(&full[st], 2u * kTileBytes + 9u * len + kBandMetaBytes);
+        tma_band_tile(base, &map_h, (int)col0, a.seg_first[t], &full[st]);
+        tma_band_tile(base + kTileBytes, &map_s, (int)col0, a.seg_first[t], &full[st]);
         if (len) {
             bulk_load(base + 2 * kTileBytes, a.term_c + o0, 8u * len, &full[st]);
             bulk_load(base + 2 * kTileBytes + 8 * seg_max, a.term_d + o0, len, &full[st]);
         }
         bulk_load(base + 2 * kTileBytes + 9 * seg_max, a.seg_meta + (long long)t * kBandMetaBytes, kBandMetaBytes, &full[st]);
     };
-    const bool issuer = GATHER || tid == 0;
-
     if (tid == 0) {
-        // thread 0 arrives with the expected bytes, and (GATHER) every thread when its copies landed
-        mbar_init(&full[0], GATHER ? 1 + kBandWarps * 32 : 1);
-        mbar_init(&full[1], GATHER ? 1 + kBandWarps * 32 : 1);
+        mbar_init(&full[0], 1);
+        mbar_init(&full[1], 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     __syncthreads();
-    int issued = 0;  // tiles issued so far (the issuing threads)
-    if (issuer && nt > 0) {
+    int issued = 0;  // tiles issued so far (thread 0)
+    if (tid == 0 && nt > 0) {
         issue(0, 0);
         if (nt > 1) issue(1, 1);
         issued = nt > 1 ? 2 : 1;
@@ -187,10 +161,9 @@ __global__ void __launch_bounds__(kBandWarps * 32, 3)
             // rows below the diagonal of this column block hold no data: zero them
             double* zH = reinterpret_cast<double*>(base);
             double* zS = zH + kBandTileRows * kBandColumns;
-            const int* listed = GATHER ? a.seg_rows + (long long)(t_begin + i) * kBandTileRows : nullptr;
             for (int q = tid; q < kBandTileRows * kBandColumns; q += blockDim.x) {
                 const int dl = q / kBandColumns, l = q % kBandColumns;
-                if ((GATHER ? listed[dl] : r0 + dl) > a.e0 + col0 + l) {
+                if (r0 + dl > a.e0 + col0 + l) {
                     zH[q] = 0.0;
                     zS[q] = 0.0;
                 }
@@ -221,7 +194,7 @@ __global__ void __launch_bounds__(kBandWarps * 32, 3)
         }
         const bool next = i + 1 >= nt || mbar_wait(&full[st ^ 1], (unsigned)((i + 1) >> 1) & 1u, limit);
         ok = __syncthreads_and(next) != 0;
-        if (ok && issuer && i + 2 < nt) {
+        if (ok && tid == 0 && i + 2 < nt) {
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
             issue(i + 2, st);
             ++issued;
@@ -230,7 +203,6 @@ __global__ void __launch_bounds__(kBandWarps * 32, 3)
     if (!ok) {
         // a tile never landed: flag it, let the copies still in flight land (a generous bound of
         // its own: no copy may outlive the CTA), and leave
-        if (GATHER) asm volatile("cp.async.wait_all;" ::: "memory");
         if (tid == 0) {
             atomicExch(a.error, 1);
             for (int u = i; u < issued; ++u) mbar_wait(&full[u & 1], (unsigned)(u >> 1) & 1u, kDrainPolls);
@@ -255,6 +227,143 @@ __global__ void __launch_bounds__(kBandWarps * 32, 3)
         const long long col = a.e0 + col0 + l;
         a.Zh[col * a.n_str + gbegin + li] = zh[li * kZPad + l];
         a.Zs[col * a.n_str + gbegin + li] = zs[li * kZPad + l];
+    }
+}
+
+// The same as a product on the FP64 tensor cores, for lists ordered by determinant blocks: their
+// structure groups share few rows (42 structures of one doubly occupied and one empty orbital have 252
+// determinants at n = 12), so that all of a group's rows fit shared memory and T is 13 % dense.  A CTA
+// keeps one group: warp w holds the coefficients of its 8 structures over all rows as A fragments in
+// registers (up to 64 k-steps) and walks column tiles of 16, whose rows arrive by cp.async (128 bytes of
+// H and of S each, rows past the diagonal as zeros) while the tile before is multiplied.
+// The tensor cores' share is 3.2 ms (216 M products for 34,188 determinants); takes 8.2 ms there, with
+// one CTA per SM and three barriers per tile.  The tiled form above takes 36.7 ms on such a list, and
+// 10.1 ms with 64-row tiles gathered from each group's own rows: one shared-memory load per nonzero and
+// column and 25 instructions around it.
+constexpr int kDenseWarps = 12;    // 6 structure tiles x 2 column halves
+constexpr int kDenseColumns = 16;
+constexpr int kDenseLd = 2 * kDenseColumns + 4;  // 4 mod 16: fragment loads without bank conflicts
+constexpr int kDenseZ = kDenseStructures + 1;
+constexpr int kDenseSteps = kDenseRows / 4;
+
+static int dense_rows(int rows) { return (rows + 31) / 32 * 32; }
+static size_t dense_smem_bytes(int rows) {
+    // the coefficients pass through the tile buffers first
+    const size_t tiles = 2 * (size_t)dense_rows(rows) * kDenseLd, coefficients = (size_t)kDenseStructures * (kDenseRows + 4);
+    return sizeof(double) * ((tiles > coefficients ? tiles : coefficients) + 2 * kDenseColumns * kDenseZ) +
+           sizeof(int) * (size_t)rows;
+}
+
+__global__ void __launch_bounds__(32 * kDenseWarps, 1) dense_reduce_kernel(BandReduceArgs a, int parts, int tile_doubles,
+                                                                           int z_at) {
+    extern __shared__ __align__(16) double rsm[];
+    constexpr int C = kDenseColumns, LD = kDenseLd, kThreads = 32 * kDenseWarps;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, gr = lane >> 2, gc = lane & 3;
+    const int mt = warp % 6, ch = warp / 6;  // structure tile, column half
+    double* zbuf = rsm + z_at;
+    int* rows = reinterpret_cast<int*>(zbuf + 2 * C * kDenseZ);
+    const int nb = (int)((a.width + C - 1) / C);
+    const int4 grp = __ldg(a.groups + blockIdx.x / parts);  // first row entry, rows, first structure, structures
+    const int n_rows = grp.y, n_str = grp.w;
+    for (int i = tid; i < n_rows; i += kThreads) rows[i] = __ldg(a.rows + grp.x + i);
+    double coef[kDenseSteps];
+    {
+        constexpr int LDT = kDenseRows + 4;
+        for (int i = tid; i < kDenseStructures * LDT; i += kThreads) rsm[i] = 0.0;
+        __syncthreads();
+        for (int s = warp; s < n_str; s += kDenseWarps) {
+            const long long t0 = __ldg(a.seg_off + grp.z + s), t1 = __ldg(a.seg_off + grp.z + s + 1);
+            for (long long q = t0 + lane; q < t1; q += 32) rsm[s * LDT + __ldg(a.term_row + q)] = __ldg(a.term_c + q);
+        }
+        __syncthreads();
+#pragma unroll
+        for (int k = 0; k < kDenseSteps; ++k) coef[k] = rsm[(8 * mt + gr) * LDT + 4 * k + gc];
+        __syncthreads();
+    }
+    // this CTA's column tiles: blockIdx.x % parts, + parts, ...
+    const int piece = tid % 16, half = piece / 8, x = 2 * (piece % 8);
+    const double* src = (half ? a.Sb : a.Hb) + x;
+    double* const own = rsm + half * C + x;
+    // rows of a tile: those up to its last column come first
+    auto valid_rows = [&](int b, int from) {
+        const long long last = a.e0 + (long long)b * C + C - 1;
+        while (from < n_rows && rows[from] <= last) ++from;
+        return from;
+    };
+    auto issue = [&](int b, int buf, int valid) {
+        const double* from = src + (long long)b * C;
+        double* dst = own + buf * tile_doubles;
+        for (int r = tid / 16; r < (valid + 31) / 32 * 32; r += kThreads / 16) {
+            const long long at = r < valid ? rows[r] * a.ldb : 0;
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_addr(dst + r * LD)), "l"(from + at),
+                         "r"(r < valid ? 16 : 0)
+                         : "memory");
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    int b = blockIdx.x % parts, buf = 0, valid = 0;
+    {
+        // first tile: by bisection
+        const long long last = a.e0 + (long long)b * C + C - 1;
+        int hi = n_rows;
+        while (valid < hi) {
+            const int mid = (valid + hi) >> 1;
+            if (rows[mid] <= last)
+                valid = mid + 1;
+            else
+                hi = mid;
+        }
+    }
+    issue(b, 0, valid);
+    for (; b < nb; b += parts, buf ^= 1) {
+        int next = valid;
+        if (b + parts < nb) {
+            next = valid_rows(b + parts, valid);
+            issue(b + parts, buf ^ 1, next);
+            asm volatile("cp.async.wait_group 1;" ::: "memory");
+        } else {
+            asm volatile("cp.async.wait_group 0;" ::: "memory");
+        }
+        const long long col0 = (long long)b * C, first = a.e0 + col0;
+        double* tile = rsm + buf * tile_doubles;
+        if (valid > 0 && rows[valid - 1] > first) {
+            // the band holds no data below the diagonal: a thread clears its own copies there
+            double* dst = own + buf * tile_doubles;
+            for (int r = tid / 16; r < valid; r += kThreads / 16) {
+                const long long below = rows[r] - first;
+                if (below > x) dst[r * LD] = 0.0;
+                if (below > x + 1) dst[r * LD + 1] = 0.0;
+            }
+        }
+        __syncthreads();
+        if (8 * mt < n_str) {
+            double h[2][2] = {}, s[2][2] = {};
+            const double* p = tile + gc * LD + 8 * ch + gr;
+            const int steps = (valid + 3) / 4;
+#pragma unroll
+            for (int k0 = 0; k0 < kDenseSteps; k0 += 8) {
+                if (k0 >= steps) break;
+#pragma unroll
+                for (int k = k0; k < k0 + 8; ++k) {
+                    mma_f64(h[k & 1], coef[k], p[4 * k * LD]);
+                    mma_f64(s[k & 1], coef[k], p[4 * k * LD + C]);
+                }
+            }
+#pragma unroll
+            for (int i = 0; i < 2; ++i) {
+                const int col = 8 * ch + 2 * gc + i;
+                zbuf[col * kDenseZ + 8 * mt + gr] = h[0][i] + h[1][i];
+                zbuf[(C + col) * kDenseZ + 8 * mt + gr] = s[0][i] + s[1][i];
+            }
+        }
+        __syncthreads();
+        for (int l = warp; l < 2 * C; l += kDenseWarps) {
+            const long long col = col0 + l % C;
+            if (col >= a.width) continue;
+            double* Z = (l < C ? a.Zh : a.Zs) + (a.e0 + col) * a.n_str + grp.z;
+            for (int q = lane; q < n_str; q += 32) Z[q] = zbuf[l * kDenseZ + q];
+        }
+        valid = next;
     }
 }
 
@@ -302,8 +411,9 @@ __global__ void __launch_bounds__(512) structure_reduce_kernel(StructureReduceAr
             }
         }
         if (valid) {
-            a.Wh[(long long)J * a.n_str + I] = wh0 + wh1;
-            a.Ws[(long long)J * a.n_str + I] = ws0 + ws1;
+            const long long at = (long long)J * a.n_str + (a.order ? __ldg(a.order + I) : I);
+            a.Wh[at] = wh0 + wh1;
+            a.Ws[at] = ws0 + ws1;
         }
     }
 }
@@ -362,15 +472,28 @@ cudaError_t launch_band_reduce(const BandReduceArgs& a, cudaStream_t stream, int
     if (a.width <= 0 || a.n_str <= 0) return cudaSuccess;
     if (a.ldb % 2 != 0 || (reinterpret_cast<uintptr_t>(a.Hb) & 15) || (reinterpret_cast<uintptr_t>(a.Sb) & 15))
         return cudaErrorInvalidValue;
+    if (a.groups) {
+        // column tiles of a group in strides of `parts`, about six CTAs per SM one after the other
+        const size_t smem = dense_smem_bytes(a.group_rows);
+        cudaError_t err = allow_dynamic_smem((const void*)dense_reduce_kernel, smem);
+        if (err != cudaSuccess) return err;
+        const long long nb = (a.width + kDenseColumns - 1) / kDenseColumns;
+        long long parts = (6 * kSms + a.n_groups - 1) / a.n_groups;
+        parts = parts > nb ? nb : parts;
+        const int tile_doubles = dense_rows(a.group_rows) * kDenseLd;
+        const int z_at = (int)((smem - sizeof(int) * a.group_rows) / sizeof(double)) - 2 * kDenseColumns * kDenseZ;
+        dense_reduce_kernel<<<(unsigned)(parts * a.n_groups), 32 * kDenseWarps, smem, stream>>>(a, (int)parts, tile_doubles, z_at);
+        ++*launches;
+        return cudaGetLastError();
+    }
     CUtensorMap mh, ms;
     if (!band_tensor_map(&mh, a.Hb, a.width, a.n_det, a.ldb) || !band_tensor_map(&ms, a.Sb, a.width, a.n_det, a.ldb))
         return cudaErrorInvalidValue;
     const size_t smem = band_reduce_smem_bytes(a.seg_max);
-    const auto kernel = a.seg_rows ? band_reduce_kernel<true> : band_reduce_kernel<false>;
-    cudaError_t err = allow_dynamic_smem((const void*)kernel, smem);
+    cudaError_t err = allow_dynamic_smem((const void*)band_reduce_kernel, smem);
     if (err != cudaSuccess) return err;
     const long long blocks = (a.width + kBandColumns - 1) / kBandColumns * a.n_groups;
-    kernel<<<(unsigned)blocks, kBandWarps * 32, smem, stream>>>(mh, ms, a, band_stage_bytes(a.seg_max));
+    band_reduce_kernel<<<(unsigned)blocks, kBandWarps * 32, smem, stream>>>(mh, ms, a, band_stage_bytes(a.seg_max));
     ++*launches;
     return cudaGetLastError();
 }

@@ -186,6 +186,8 @@ bool determinant_blocks(const vb_expansion& ex, DeterminantBlocks* out, std::vec
                         sorted.push_back(it->second);
                     }
                 if (count == 0) continue;
+                block.n_alpha = (unsigned char)(a1 - a0);
+                block.n_beta = (unsigned char)(b1 - b0);
                 for (int i = a0; i < a1; ++i) block.alpha[i - a0] = (uint16_t)as[i];
                 for (int k = b0; k < b1; ++k) block.beta[k - b0] = (uint16_t)bs[k];
                 cells += (long long)(a1 - a0) * (b1 - b0);
@@ -202,6 +204,76 @@ bool determinant_blocks(const vb_expansion& ex, DeterminantBlocks* out, std::vec
     if ((long long)sorted.size() != nd || 5 * nd < 2 * cells || nd < 10LL * b.n) return false;
     *out = std::move(b);
     *order = std::move(sorted);
+    return true;
+}
+
+// Structure groups whose rows fit shared memory together (BandReduceArgs::groups): up to kDenseStructures
+// structures and kDenseRows rows.  Structures with the same doubly occupied and empty orbitals share their
+// determinants, so they are taken one after the other: order[i] is the caller's index of structure i, and
+// off, coef and term_row list the terms in this order.
+struct ResidentGroups {
+    std::vector<int4> groups;
+    std::vector<int> rows, order;
+    std::vector<long long> off;
+    std::vector<double> coef;
+    std::vector<unsigned short> term_row;
+    int max_rows = 0;
+};
+
+// false where a structure alone has too many rows, or where the groups together read the rows so often
+// (four times each on average) that the tiled form, whose groups always hold kBandGroup structures, reads
+// less.
+bool resident_groups(const vb_expansion& ex, int n_str, const std::vector<long long>& off, const std::vector<long long>& det,
+                     const std::vector<double>& coef, ResidentGroups* out) {
+    ResidentGroups r;
+    std::vector<std::pair<uint64_t, uint64_t>> key(n_str);  // doubly occupied, occupied orbitals
+    for (int I = 0; I < n_str; ++I)
+        if (off[I] < off[I + 1]) {
+            const uint64_t a = ex.alpha_strings[ex.det_alpha[det[off[I]]]], b = ex.beta_strings[ex.det_beta[det[off[I]]]];
+            key[I] = {a & b, a | b};
+        }
+    r.order.resize(n_str);
+    for (int i = 0; i < n_str; ++i) r.order[i] = i;
+    std::stable_sort(r.order.begin(), r.order.end(), [&](int x, int y) { return key[x] < key[y]; });
+    std::vector<int> owner(ex.n_determinants, -1);  // group that last took the determinant
+    r.off.push_back(0);
+    for (int i0 = 0; i0 < n_str;) {
+        const int g = (int)r.groups.size();
+        std::vector<int> used;
+        int i1 = i0;
+        for (; i1 < n_str && i1 - i0 < kDenseStructures; ++i1) {
+            const int I = r.order[i1];
+            const size_t before = used.size();
+            for (long long t = off[I]; t < off[I + 1]; ++t) {
+                if (t > off[I] && det[t] == det[t - 1]) return false;  // one coefficient per structure and determinant
+                if (owner[det[t]] != g) {
+                    owner[det[t]] = g;
+                    used.push_back((int)det[t]);
+                }
+            }
+            if (used.size() > (size_t)kDenseRows) {
+                if (i1 == i0) return false;
+                used.resize(before);
+                break;
+            }
+        }
+        std::sort(used.begin(), used.end());
+        for (int i = i0; i < i1; ++i) {
+            const int I = r.order[i];
+            for (long long t = off[I]; t < off[I + 1]; ++t) {
+                r.term_row.push_back(
+                    (unsigned short)(std::lower_bound(used.begin(), used.end(), (int)det[t]) - used.begin()));
+                r.coef.push_back(coef[t]);
+            }
+            r.off.push_back((long long)r.coef.size());
+        }
+        r.groups.push_back(make_int4((int)r.rows.size(), (int)used.size(), i0, i1 - i0));
+        r.rows.insert(r.rows.end(), used.begin(), used.end());
+        r.max_rows = std::max(r.max_rows, (int)used.size());
+        i0 = i1;
+    }
+    if ((long long)r.rows.size() > 4 * ex.n_determinants) return false;
+    *out = std::move(r);
     return true;
 }
 
@@ -607,17 +679,28 @@ vb_status vb_hs_plan_create(vb_context* ctx, const vb_expansion* ex, vb_hs_plan*
 
     // band-reduction term segments: for every row tile of every structure group the terms (row in the
     // tile, coefficient) of the group's structures ordered by (warp, slot, determinant).  The tiles of
-    // a group are its 64-row tiles of the determinant list that hold terms, or (blocks) the group's own
-    // rows 64 at a time.
-    {
+    // a group are its 64-row tiles of the determinant list that hold terms.  Lists ordered by blocks
+    // take groups whose rows fit shared memory together, where they can be formed.
+    ResidentGroups resident;
+    if (blocks.n > 0 && resident_groups(*ex, p->n_str, soff, sdet, scoef, &resident)) {
+        BandSegments& b = p->segments;
+        b.n_groups = (int)resident.groups.size();
+        b.group_rows = resident.max_rows;
+        if ((st = upload(ctx, b.groups, resident.groups.data(), sizeof(int4) * resident.groups.size())) != VB_OK ||
+            (st = upload(ctx, b.rows, resident.rows.data(), sizeof(int) * resident.rows.size())) != VB_OK ||
+            (st = upload(ctx, b.order, resident.order.data(), sizeof(int) * resident.order.size())) != VB_OK ||
+            (st = upload(ctx, b.off, resident.off.data(), sizeof(long long) * resident.off.size())) != VB_OK ||
+            (st = upload(ctx, b.coef, resident.coef.data(), sizeof(double) * resident.coef.size())) != VB_OK ||
+            (st = upload(ctx, b.term_row, resident.term_row.data(), sizeof(unsigned short) * resident.term_row.size())) != VB_OK)
+            return fail(st);
+    } else {
         BandSegments& b = p->segments;
         b.n_groups = (p->n_str + kBandGroup - 1) / kBandGroup;
-        b.gather = blocks.n > 0;
         std::vector<long long> off;
         std::vector<unsigned char> meta;
         std::vector<double> coef;
         std::vector<unsigned char> row;
-        std::vector<int> rows, first_row, last_row, tile_off(b.n_groups + 1, 0);
+        std::vector<int> first_row, last_row, tile_off(b.n_groups + 1, 0);
         std::vector<int> local(p->n_det, -1);  // row of the group's tile that holds a determinant
         for (int g = 0; g < b.n_groups; ++g) {
             // determinants of the group, ascending
@@ -633,12 +716,8 @@ vb_status vb_hs_plan_create(vb_context* ctx, const vb_expansion* ex, vb_hs_plan*
             for (size_t u0 = 0; u0 < used.size();) {
                 size_t u1 = u0;
                 const int t0 = used[u0] / kBandTileRows * kBandTileRows;
-                if (b.gather) {
-                    u1 = std::min(used.size(), u0 + kBandTileRows);
-                } else {
-                    while (u1 < used.size() && used[u1] < t0 + kBandTileRows) ++u1;
-                }
-                for (size_t u = u0; u < u1; ++u) local[used[u]] = b.gather ? (int)(u - u0) : used[u] - t0;
+                while (u1 < used.size() && used[u1] < t0 + kBandTileRows) ++u1;
+                for (size_t u = u0; u < u1; ++u) local[used[u]] = used[u] - t0;
                 const int end = used[u1 - 1];
                 off.push_back((long long)coef.size());
                 const size_t m0 = meta.size();
@@ -664,10 +743,8 @@ vb_status vb_hs_plan_create(vb_context* ctx, const vb_expansion* ex, vb_hs_plan*
                     row.push_back(0);
                 }
                 b.seg_max = std::max(b.seg_max, (int)((long long)coef.size() - off.back()));
-                first_row.push_back(b.gather ? used[u0] : t0);
-                last_row.push_back(b.gather ? end : t0 + kBandTileRows - 1);
-                if (b.gather)
-                    for (int q = 0; q < kBandTileRows; ++q) rows.push_back(u0 + q < u1 ? used[u0 + q] : -1);
+                first_row.push_back(t0);
+                last_row.push_back(t0 + kBandTileRows - 1);
                 u0 = u1;
             }
             for (int d : used) local[d] = -1;
@@ -678,7 +755,6 @@ vb_status vb_hs_plan_create(vb_context* ctx, const vb_expansion* ex, vb_hs_plan*
             return fail(st);
         if ((st = upload(ctx, b.last_row, last_row.data(), sizeof(int) * std::max<size_t>(1, last_row.size()))) != VB_OK)
             return fail(st);
-        if (b.gather && (st = upload(ctx, b.rows, rows.data(), sizeof(int) * rows.size())) != VB_OK) return fail(st);
         if ((st = upload(ctx, b.tile_off, tile_off.data(), sizeof(int) * tile_off.size())) != VB_OK) return fail(st);
         if ((st = upload(ctx, b.off, off.data(), sizeof(long long) * off.size())) != VB_OK) return fail(st);
         if ((st = upload(ctx, b.meta, meta.data(), std::max<size_t>(16, meta.size()))) != VB_OK) return fail(st);
@@ -946,11 +1022,16 @@ vb_status execute_impl(vb_hs_plan* p, const double* S, const double* h, const do
             ba.seg_max = p->segments.seg_max;
             ba.seg_off = p->segments.off.as<long long>();
             ba.seg_meta = p->segments.meta.as<unsigned char>();
+            if (p->segments.groups.ptr) {
+                ba.groups = p->segments.groups.as<int4>();
+                ba.rows = p->segments.rows.as<int>();
+                ba.term_row = p->segments.term_row.as<unsigned short>();
+                ba.group_rows = p->segments.group_rows;
+            }
             ba.term_c = p->segments.coef.as<double>();
             ba.term_d = p->segments.row.as<unsigned char>();
             ba.seg_first = p->segments.first_row.as<int>();
             ba.seg_last = p->segments.last_row.as<int>();
-            ba.seg_rows = p->segments.gather ? p->segments.rows.as<int>() : nullptr;
             ba.seg_tile_off = p->segments.tile_off.as<int>();
             ba.error = reinterpret_cast<int*>(p->counters.as<unsigned long long>() + 7);
             ba.spin_limit = ctx->barrier_spin_limit > 0 ? ctx->barrier_spin_limit : (1ll << 26);
@@ -966,6 +1047,7 @@ vb_status execute_impl(vb_hs_plan* p, const double* S, const double* h, const do
     ra.str_off = p->str_off.as<long long>();
     ra.str_det = p->str_det.as<long long>();
     ra.str_coef = p->str_coef.as<double>();
+    ra.order = p->segments.groups.ptr ? p->segments.order.as<int>() : nullptr;
     ra.Zh = scr[2];
     ra.Zs = scr[3];
     ra.Wh = scr[4];

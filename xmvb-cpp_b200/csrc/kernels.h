@@ -97,7 +97,8 @@ struct CovalentArgs {
 struct BlockStrings {
     uint16_t alpha[8], beta[8];
     unsigned char cell[64];
-    unsigned char pad[32];
+    unsigned char n_alpha, n_beta;
+    unsigned char pad[30];
 };
 struct BlockPairArgs {
     FullPairArgs f;
@@ -115,7 +116,11 @@ struct BlockPairArgs {
 // per segment: the term count of each (warp, slot) (kBandWarps x kBandSlots bytes) followed by the
 // start of each warp's terms within the segment (kBandWarps uint16).  Structure of group g, warp
 // w, slot s: I = g * kBandGroup + s * kBandWarps + w.  A tile holds the consecutive rows from
-// seg_first[t] on or, with seg_rows, the listed rows seg_rows[64 t ..] (-1 beyond the last).
+// seg_first[t] on.
+// With `groups` instead (block-ordered lists), group g is {first entry of `rows`, rows, first structure,
+// structures}: at most kDenseRows ascending rows and kDenseStructures structures, in an order of the
+// plan's own.  Structure i of this order has the terms seg_off[i] .. seg_off[i + 1] - 1 of term_c, term t
+// in row term_row[t] of its group, and is row i of Z.
 struct BandReduceArgs {
     long long n_det;
     int n_str;
@@ -131,8 +136,11 @@ struct BandReduceArgs {
     const unsigned char* term_d;
     const int* seg_first;
     const int* seg_last;
-    const int* seg_rows;
     const int* seg_tile_off;
+    const int4* groups;
+    const int* rows;
+    const unsigned short* term_row;
+    int group_rows;  // largest of any group
     double* Zh;  // n_str x n_det column-major: Z[e * n_str + I]
     double* Zs;
     int* error;  // set to 1 when a tile wait gives up (the results are then incomplete)
@@ -145,6 +153,7 @@ struct StructureReduceArgs {
     const long long* str_off;  // CSC by structure
     const long long* str_det;
     const double* str_coef;
+    const int* order;          // structure of every row of Z (nullptr: its own)
     const double* Zh;
     const double* Zs;
     double* Wh;  // n_str x n_str column-major
@@ -164,6 +173,9 @@ constexpr int kBandSlots = 8;        // structures per warp (register accumulato
 constexpr int kBandGroup = kBandWarps * kBandSlots;
 constexpr int kBandColumns = 32;     // band columns per CTA (one per lane)
 constexpr int kBandTileRows = 64;    // band rows per staged tile
+// structure groups of the dense form
+constexpr int kDenseRows = 256;
+constexpr int kDenseStructures = 48;
 constexpr int kBandMetaBytes = kBandWarps * kBandSlots + 2 * kBandWarps;
 constexpr int kSpinBlock = 128;    // right strings per fast-kernel item (threads per CTA)
 

@@ -545,120 +545,147 @@ __global__ void __launch_bounds__(512) full_pairs_kernel(FullPairArgs a) {
 // the determinants: every record is read once per block pair and used by 7 x 7 determinant pairs (n =
 // 12, singly ionic), where one thread per pair gathers two records (640 bytes) for R multiply-adds.
 // The records arrive by cp.async, all in flight together (a warp per record, one after the other, left
-// the loads' latency exposed: 35 ms).  Each of the four warps owns M tiles w and w + 4 and all N tiles;
-// H goes through shared memory so that band rows are written in runs of a block's determinants.  Both
+// the loads' latency exposed: 35 ms).  Each of the eight warps owns M tiles w and w + 4 (w = 0 .. 3) and
+// half of the N tiles; H goes through shared memory so that band rows are written in runs of a block's determinants.  Both
 // members of a spin-flip orbit are evaluated: blocks do not map to blocks under the flip.  Bound by the
-// product (2.3 ms at the DGEMM rate for 34,188 determinants) and the band it writes (9.3 GB); takes
-// 10.7 ms there, the gather form 27.3 ms.
-constexpr int kBlockWarps = 4;
+// product (1.7 ms at the tensor cores' rate for 34,188 determinants) and the band it writes (9.3 GB, 1.4 ms);
+// takes 9.0 ms there (10.7 ms with record addresses and determinant cells divided out per element, four
+// warps and four barriers), the gather form 27.3 ms.  A block pair is 2.4 us of loads, products and stores
+// one after the other on 3 CTAs per SM; a second record buffer with one CTA per SM: 11.7 ms.
+constexpr int kBlockWarps = 8;
 constexpr int kBlockEdge = 8;                        // strings per block and spin
 constexpr int kBlockCells = kBlockEdge * kBlockEdge;
 
 __host__ __device__ inline int block_k(int R) { return (R + 2 + 3) / 4 * 4; }
 // record stride in shared memory: 4 or 12 mod 16 doubles (conflict-free fragment loads)
 __host__ __device__ inline int block_ld(int R) { return block_k(R) % 8 == 4 ? block_k(R) : block_k(R) + 4; }
+__host__ __device__ inline int block_rows(int rows) { return (rows + 7) / 8 * 8; }
 inline size_t block_pairs_smem(int rows_a, int rows_b, int dets, int R) {
-    const size_t ra = (rows_a + 7) / 8 * 8, rb = (rows_b + 7) / 8 * 8;
-    return sizeof(double) * ((ra + rb) * block_ld(R) + (size_t)dets * (dets + 1));
+    return sizeof(double) * ((size_t)(block_rows(rows_a) + block_rows(rows_b)) * block_ld(R) + (size_t)dets * (dets + 1));
 }
 
-__global__ void __launch_bounds__(32 * kBlockWarps) block_pairs_kernel(BlockPairArgs a) {
+__global__ void __launch_bounds__(32 * kBlockWarps, 3) block_pairs_kernel(BlockPairArgs a) {
     extern __shared__ __align__(16) double bsm[];
     const int R = a.f.R, KD = block_k(R), LD = block_ld(R), r_pos = a.f.r_pos;
     double* sA = bsm;                                    // [ij][record]
-    double* sB = sA + (a.max_a + 7) / 8 * 8 * LD;        // [kl][record]
-    double* sH = sB + (a.max_b + 7) / 8 * 8 * LD;        // [determinant of g][determinant of h]
+    double* sB = sA + block_rows(a.max_a) * LD;          // [kl][record]
+    double* sH = sB + block_rows(a.max_b) * LD;          // [determinant of g][determinant of h]
     const int OUT = a.max_dets + 1;
-    __shared__ __align__(16) BlockStrings s_desc[2];
+    __shared__ __align__(16) BlockStrings s_desc[2][2];
     __shared__ unsigned char s_i[2][kBlockCells], s_k[2][kBlockCells];  // determinant -> its strings
+    // first cells of block g and of block h of record row ij (alpha) and of record column kl (beta)
+    __shared__ unsigned char s_row[2][kBlockCells], s_col[2][kBlockCells];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, gr = lane >> 2, gc = lane & 3;
     const int chunks = (R + 3) / 2;  // 16-byte pieces of a record up to the energy
     // block pairs of the band: a rectangle (g < h0) and a triangle
     const long long nh = a.h1 - a.h0, rect = nh * a.h0, total = rect + nh * (nh + 1) / 2;
-    auto decode = [&](long long t, int* g, int* h) {
-        if (t < rect) {
-            *g = (int)(t / nh);
-            *h = a.h0 + (int)(t % nh);
+    auto decode = [&](unsigned t, int* g, int* h) {
+        if (t < (unsigned)rect) {
+            *g = (int)(t / (unsigned)nh);
+            *h = a.h0 + (int)(t - (unsigned)*g * (unsigned)nh);
             return;
         }
-        const long long q = t - rect;
-        long long y = (long long)((sqrt(8.0 * (double)q + 1.0) - 1.0) * 0.5);
+        const int q = (int)(t - (unsigned)rect);
+        int y = (int)((sqrtf(8.0f * (float)q + 1.0f) - 1.0f) * 0.5f);
         while (y * (y + 1) / 2 > q) --y;
         while ((y + 1) * (y + 2) / 2 <= q) ++y;
-        *h = a.h0 + (int)y;
-        *g = a.h0 + (int)(q - y * (y + 1) / 2);
+        *h = a.h0 + y;
+        *g = a.h0 + (q - y * (y + 1) / 2);
     };
     constexpr int kWords = sizeof(BlockStrings) / 4;  // one word per thread of the first two warps
-    static_assert(kWords == 32 && 2 * kBlockCells == 32 * kBlockWarps, "a descriptor per warp, a cell per thread");
-    int g = 0, h = 0;
-    unsigned word = 0;  // this thread's word of the next pair's descriptors
-    if (blockIdx.x < total) {
-        decode(blockIdx.x, &g, &h);
-        if (tid < 2 * kWords) word = __ldg(reinterpret_cast<const unsigned*>(a.strings + (tid < kWords ? g : h)) + tid % kWords);
-    }
-    for (long long t = blockIdx.x; t < total; t += gridDim.x) {
-        const int d0 = __ldg(a.first + g), nd = __ldg(a.first + g + 1) - d0;
-        const int e0 = __ldg(a.first + h), ne = __ldg(a.first + h + 1) - e0;
-        const bool diagonal = g == h;
-        __syncthreads();  // the previous pair's shared data is consumed
-        if (tid < 2 * kWords) reinterpret_cast<unsigned*>(s_desc)[tid] = word;
-        __syncthreads();
-        if (t + gridDim.x < total) {
-            decode(t + gridDim.x, &g, &h);
-            if (tid < 2 * kWords) word = __ldg(reinterpret_cast<const unsigned*>(a.strings + (tid < kWords ? g : h)) + tid % kWords);
-        }
-        int n_str[4];  // alpha strings of g and of h, beta strings of g and of h
-#pragma unroll
-        for (int w = 0; w < 4; ++w) {
-            const BlockStrings& b = s_desc[w & 1];
-            n_str[w] = 0;
-#pragma unroll
-            for (int q = 0; q < kBlockEdge; ++q) n_str[w] += (w < 2 ? b.alpha[q] : b.beta[q]) != 0xFFFF ? 1 : 0;
-        }
-        const int rows_a = n_str[0] * n_str[1], rows_b = n_str[2] * n_str[3];
-        for (int x = tid; x < (rows_a + rows_b) * chunks; x += blockDim.x) {
-            const int r = x / chunks, piece = x - r * chunks;
+    static_assert(kWords == 32 && 2 * kBlockCells <= 32 * kBlockWarps, "a descriptor per warp, a cell per thread");
+    auto descriptor_word = [&](int g, int h) {
+        return __ldg(reinterpret_cast<const unsigned*>(a.strings + (tid < kWords ? g : h)) + tid % kWords);
+    };
+    // a warp copies the records warp, warp + 8, ... of a block pair: lane q addresses the q-th of them
+    auto load_records = [&](const BlockStrings* desc) {
+        const int wa = desc[1].n_alpha, wb = desc[1].n_beta;
+        const int rows_a = desc[0].n_alpha * wa, rows = rows_a + desc[0].n_beta * wb;
+        const double* rec = nullptr;
+        const int r = warp + kBlockWarps * lane;
+        if (r < rows) {
             const bool beta = r >= rows_a;
-            const int q = beta ? r - rows_a : r, w = beta ? n_str[3] : n_str[1];
+            const int q = beta ? r - rows_a : r, w = beta ? wb : wa;
             const int qi = q / w, qj = q - qi * w;
-            const int u = beta ? s_desc[0].beta[qi] : s_desc[0].alpha[qi];
-            const int v = beta ? s_desc[1].beta[qj] : s_desc[1].alpha[qj];
+            const int u = beta ? desc[0].beta[qi] : desc[0].alpha[qi];
+            const int v = beta ? desc[1].beta[qj] : desc[1].alpha[qj];
             const long long at = record_index(min(u, v), max(u, v), beta ? a.f.Nb : a.f.Na);
-            const double* rec = (beta ? a.f.rec_b + at * a.f.stride_b : a.f.rec_a + at * a.f.stride_a) + 2 * piece;
-            const unsigned dst = (unsigned)__cvta_generic_to_shared((beta ? sB : sA) + q * LD + 2 * piece);
-            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(rec) : "memory");
+            rec = beta ? a.f.rec_b + at * a.f.stride_b : a.f.rec_a + at * a.f.stride_a;
+        }
+        for (int it = 0, y = warp; y < rows; ++it, y += kBlockWarps) {
+            const double* src =
+                reinterpret_cast<const double*>(__shfl_sync(0xffffffffu, reinterpret_cast<unsigned long long>(rec), it));
+            const unsigned dst = (unsigned)__cvta_generic_to_shared(y < rows_a ? sA + y * LD : sB + (y - rows_a) * LD);
+            for (int piece = lane; piece < chunks; piece += 32)
+                asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + 16 * piece), "l"(src + 2 * piece) : "memory");
         }
         asm volatile("cp.async.commit_group;" ::: "memory");
-        {
+    };
+    // fragment tiles of this warp: M tiles wm and wm + 4, N tiles wn to wn + 3
+    const int wm = warp & 3, wn = 4 * (warp >> 2);
+    int g = 0, h = 0, g1 = 0, h1 = 0;  // blocks of this pair and of the next
+    unsigned word = 0;                 // this thread's word of the pair after next
+    long long t = blockIdx.x;
+    if (t < total) {
+        decode(t, &g, &h);
+        if (tid < 2 * kWords) reinterpret_cast<unsigned*>(s_desc[0])[tid] = descriptor_word(g, h);
+        if (t + gridDim.x < total) {
+            decode(t + gridDim.x, &g1, &h1);
+            if (tid < 2 * kWords) word = descriptor_word(g1, h1);
+        }
+    }
+    __syncthreads();
+    for (int parity = 0; t < total; t += gridDim.x, parity ^= 1) {
+        const int d0 = __ldg(a.first + g), nd = __ldg(a.first + g + 1) - d0;
+        const int e0 = __ldg(a.first + h), ne = __ldg(a.first + h + 1) - e0;
+        const bool diagonal = g == h, more = t + gridDim.x < total;
+        const BlockStrings* desc = s_desc[parity];
+        __syncthreads();  // the previous pair's shared data is consumed
+        load_records(desc);
+        if (tid < 2 * kWords && more) reinterpret_cast<unsigned*>(s_desc[parity ^ 1])[tid] = word;
+        const int wa = desc[1].n_alpha, wb = desc[1].n_beta;
+        const int rows_a = desc[0].n_alpha * wa, rows_b = desc[0].n_beta * wb;
+        if (tid < 2 * kBlockCells) {
             const int which = tid / kBlockCells, cell = tid % kBlockCells;
-            const unsigned char at = s_desc[which].cell[cell];
+            const unsigned char at = desc[which].cell[cell];
             if (at != 0xFF) {
                 s_i[which][at] = (unsigned char)(cell / kBlockEdge);
                 s_k[which][at] = (unsigned char)(cell % kBlockEdge);
             }
+        } else if (tid < 4 * kBlockCells) {
+            const bool beta = tid >= 3 * kBlockCells;
+            const int q = tid % kBlockCells, w = beta ? wb : wa, qi = q / w;
+            if (q < (beta ? rows_b : rows_a)) {
+                (beta ? s_col[0] : s_row[0])[q] = (unsigned char)(beta ? qi : kBlockEdge * qi);
+                (beta ? s_col[1] : s_row[1])[q] = (unsigned char)(beta ? q - qi * w : kBlockEdge * (q - qi * w));
+            }
+        }
+        g = g1;
+        h = h1;
+        if (t + 2 * (long long)gridDim.x < total) {
+            decode(t + 2 * (long long)gridDim.x, &g1, &h1);
+            if (tid < 2 * kWords) word = descriptor_word(g1, h1);
         }
         asm volatile("cp.async.wait_group 0;" ::: "memory");
         __syncthreads();
-        const int mt = (rows_a + 7) / 8, nt = (rows_b + 7) / 8;
-        if (warp < mt) {
-            double acc[2][kBlockEdge][2];
+        const int mt = (rows_a + 7) / 8, nt = (rows_b + 7) / 8 - wn;
+        if (wm < mt && nt > 0) {
+            double acc[2][4][2];
 #pragma unroll
             for (int i = 0; i < 2; ++i)
 #pragma unroll
-                for (int j = 0; j < kBlockEdge; ++j) acc[i][j][0] = acc[i][j][1] = 0.0;
-            const bool two = warp + kBlockWarps < mt;
-            const double* pa = sA + (8 * warp + gr) * LD;
-            const double* pa2 = pa + (two ? 8 * kBlockWarps * LD : 0);
-            const double* pb = sB + gr * LD;
-            auto step = [&](int ka, int kb, bool on, bool negative) {
-                double a0 = pa[ka], a1 = pa2[ka];
-                if (negative) {
-                    a0 = -a0;
-                    a1 = -a1;
-                }
-                if (!on) a0 = a1 = 0.0;
+                for (int j = 0; j < 4; ++j) acc[i][j][0] = acc[i][j][1] = 0.0;
+            const bool two = wm + 4 < mt;
+            const double* pa = sA + (8 * wm + gr) * LD;
+            const double* pa2 = pa + (two ? 32 * LD : 0);
+            const double* pb = sB + (8 * wn + gr) * LD;
+            // sign of the factor columns from r_pos on
+            auto signed_value = [](double x, bool negative) {
+                return __hiloint2double(__double2hiint(x) ^ (negative ? 0x80000000 : 0), __double2loint(x));
+            };
+            auto products = [&](double a0, double a1, int kb, bool on) {
 #pragma unroll
-                for (int j = 0; j < kBlockEdge; ++j) {
+                for (int j = 0; j < 4; ++j) {
                     if (j >= nt) break;
                     const double b = on ? pb[8 * j * LD + kb] : 0.0;
                     mma_f64(acc[0][j], a0, b);
@@ -666,34 +693,38 @@ __global__ void __launch_bounds__(32 * kBlockWarps) block_pairs_kernel(BlockPair
                 }
             };
             int k = 0;
-            for (; k + 4 <= R; k += 4) step(k + gc, k + gc, true, k + gc >= r_pos);
+#pragma unroll 2
+            for (; k + 4 <= R; k += 4) {
+                const bool negative = k + gc >= r_pos;
+                products(signed_value(pa[k + gc], negative), signed_value(pa2[k + gc], negative), k + gc, true);
+            }
             for (; k < KD; k += 4) {
                 // the remaining factor columns, then H_a S_b and S_a H_b (a record holds [.. | S | H])
                 const int m = k + gc;
-                const bool on = m < R + 2;
-                const int mb = on ? m : 0;
-                step(m < R ? m : (on ? 2 * R + 1 - m : 0), mb, on, m < R && m >= r_pos);
+                const bool on = m < R + 2, negative = m < R && m >= r_pos;
+                const int ma = m < R ? m : (on ? 2 * R + 1 - m : 0);
+                products(on ? signed_value(pa[ma], negative) : 0.0, on ? signed_value(pa2[ma], negative) : 0.0, on ? m : 0, on);
             }
 #pragma unroll
             for (int i = 0; i < 2; ++i) {
-                const int r = 8 * (warp + kBlockWarps * i) + gr;
+                const int r = 8 * (wm + 4 * i) + gr;
                 if (r >= rows_a) continue;
-                const int ii = r / n_str[1], jj = r - ii * n_str[1];
+                const unsigned char* cg = desc[0].cell + s_row[0][r];
+                const unsigned char* ch = desc[1].cell + s_row[1][r];
 #pragma unroll
-                for (int j = 0; j < kBlockEdge; ++j)
+                for (int j = 0; j < 4; ++j)
 #pragma unroll
                     for (int x = 0; x < 2; ++x) {
-                        const int c = 8 * j + 2 * gc + x;
+                        const int c = 8 * (wn + j) + 2 * gc + x;
                         if (c >= rows_b) continue;
-                        const int kk = c / n_str[3], ll = c - kk * n_str[3];
-                        const unsigned d = s_desc[0].cell[kBlockEdge * ii + kk], e = s_desc[1].cell[kBlockEdge * jj + ll];
+                        const unsigned d = cg[s_col[0][c]], e = ch[s_col[1][c]];
                         if (d != 0xFF && e != 0xFF) sH[d * OUT + e] = acc[i][j][x];
                     }
             }
         }
         __syncthreads();
         for (int d = warp; d < nd; d += kBlockWarps) {
-            const int i = s_i[0][d] * n_str[1], k = s_k[0][d] * n_str[3];
+            const int i = s_i[0][d] * wa, k = s_k[0][d] * wb;
             double* H = a.f.Hb + (d0 + d) * a.f.ldb + (e0 - a.f.e0);
             double* S = a.f.Sb + (d0 + d) * a.f.ldb + (e0 - a.f.e0);
 #pragma unroll 2
@@ -900,13 +931,14 @@ cudaError_t launch_block_pairs(const BlockPairArgs& a, cudaStream_t stream, int*
     const long long nh = a.h1 - a.h0, total = nh * a.h0 + nh * (nh + 1) / 2;
     if (total <= 0) return cudaSuccess;
     const size_t smem = block_pairs_smem(a.max_a, a.max_b, a.max_dets, a.f.R);
-    cudaError_t err = allow_dynamic_smem((const void*)block_pairs_kernel, smem);
+    const auto kernel = block_pairs_kernel;
+    cudaError_t err = allow_dynamic_smem((const void*)kernel, smem);
     if (err != cudaSuccess) return err;
     int per_sm = 1;
-    err = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, block_pairs_kernel, 32 * kBlockWarps, smem);
+    err = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, 32 * kBlockWarps, smem);
     if (err != cudaSuccess) return err;
     const long long grid = (long long)kSms * (per_sm > 0 ? per_sm : 1);
-    block_pairs_kernel<<<(unsigned)(total < grid ? total : grid), 32 * kBlockWarps, smem, stream>>>(a);
+    kernel<<<(unsigned)(total < grid ? total : grid), 32 * kBlockWarps, smem, stream>>>(a);
     ++*launches;
     return cudaGetLastError();
 }

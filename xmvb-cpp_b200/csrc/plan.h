@@ -14,10 +14,12 @@ using namespace vbcore;
 // Term segments of the band reduction per row tile of every structure group (see BandReduceArgs).
 struct BandSegments {
     int n_groups = 0, seg_max = 0;
-    bool gather = false;  // tiles list their rows
     DeviceBuffer off, meta, coef, row;
-    // tiles of every group (CSR: tile_off[g] .. tile_off[g + 1]), their first and last rows and rows
-    DeviceBuffer first_row, last_row, rows, tile_off;
+    // tiles of every group (CSR: tile_off[g] .. tile_off[g + 1]), their first and last rows
+    DeviceBuffer first_row, last_row, tile_off;
+    // instead (groups not empty): rows of every group together, terms by structure in the groups' order
+    DeviceBuffer groups, rows, order, term_row;
+    int group_rows = 0;
 };
 
 // Blocks of (alpha strings) x (beta strings) the determinant list is ordered by (see BlockPairArgs).

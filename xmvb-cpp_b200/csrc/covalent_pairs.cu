@@ -18,12 +18,14 @@
 // at a level above five) are listed: both records go to the exact path, and listed_covalent_pairs
 // combines them.
 //
-// 14 orbitals, 2.9 M orbits: 1428 us, against 1280 us for the records and 537 us for the pairs gathered
+// 14 orbitals, 2.9 M orbits: 1361 us (1428 us with a test per row tile in the product), against 1280 us for the records and 537 us for the pairs gathered
 // from them; 12-orbital triplet: 160 us, against 235 us.  Bound by instruction issue (50 %) and the FP64
 // tensor cores (45 %): one CTA of up to 16 warps per SM, the two blocks and the warps' adj B slots in
 // shared memory.
 #include <cuda_runtime.h>
 #include <stdint.h>
+
+#include <type_traits>
 
 #include "device_algebra.cuh"
 #include "frame.cuh"
@@ -284,24 +286,24 @@ __global__ void __launch_bounds__(32 * kCovalentMaxWarps, 1) covalent_pairs(Cova
                 const unsigned i0 = (pmap >> (4 * tq)) & 0xFu, i1 = (pmap >> (4 * (tq + 4))) & 0xFu;
                 const bool pad_trace = e >= 1 && pad;
                 double dot = 0.0, ha = 0.0, hb = 0.0;
-#pragma unroll 1
-                for (int p = 0; p < passes; ++p) {
-                    const int nt0 = p * per_pass, nt = min(per_pass, NT - nt0);
+                // one pass over nt tiles of table rows from nt0 on (nt at compile time: no test per tile)
+                auto pass = [&](auto tiles_of_pass, int nt0) {
+                    constexpr int T = decltype(tiles_of_pass)::value;
                     const double* rowA = tabA + (8 * nt0 + g) * KFS + tq;
                     const double* rowB = tabB + (8 * nt0 + g) * KFS + tq;
-                    double ua[kCovalentTiles][2], ub[kCovalentTiles][2];
+                    double ua[T][2], ub[T][2];
 #pragma unroll
-                    for (int j = 0; j < kCovalentTiles; ++j) ua[j][0] = ua[j][1] = ub[j][0] = ub[j][1] = 0.0;
+                    for (int j = 0; j < T; ++j) ua[j][0] = ua[j][1] = ub[j][0] = ub[j][1] = 0.0;
                     auto step = [&](double fa, double fb, int col) {
 #pragma unroll
-                        for (int j = 0; j < kCovalentTiles; ++j) {
-                            if (j >= nt) break;
+                        for (int j = 0; j < T; ++j) {
                             mma_f64(ua[j], fa, rowA[8 * j * KFS + col]);
                             mma_f64(ub[j], fb, rowB[8 * j * KFS + col]);
                         }
                     };
                     if (!pad_trace) step(tq == 0 && ok ? deta : 0.0, tq == 0 && ok ? detb : 0.0, 8 * K);
                     unsigned rest = uh;
+#pragma unroll 1
                     while (rest) {
                         const int c = __ffs(rest) - 1;
                         rest &= rest - 1;
@@ -321,18 +323,28 @@ __global__ void __launch_bounds__(32 * kCovalentMaxWarps, 1) covalent_pairs(Cova
                     }
                     // columns 2 tq and 2 tq + 1 of pair g: table rows 0 = h, 1 = two-electron linear, 2 + m
 #pragma unroll
-                    for (int j = 0; j < kCovalentTiles; ++j) {
-                        if (j >= nt) break;
+                    for (int j = 0; j < T; ++j)
 #pragma unroll
                         for (int i = 0; i < 2; ++i) {
                             const int m = 8 * (nt0 + j) + 2 * tq + i - 2;
                             const double prod = ua[j][i] * ub[j][i];
                             if (m >= 0 && m < R) dot += m < a.r_pos ? prod : -prod;
                         }
-                    }
-                    if (p == 0) {
+                    if (nt0 == 0) {
                         ha = ua[0][0] + ua[0][1];
                         hb = ub[0][0] + ub[0][1];
+                    }
+                };
+#pragma unroll 1
+                for (int nt0 = 0; nt0 < NT; nt0 += per_pass) {
+                    switch (min(per_pass, NT - nt0)) {
+                        case 1: pass(std::integral_constant<int, 1>{}, nt0); break;
+                        case 2: pass(std::integral_constant<int, 2>{}, nt0); break;
+                        case 3: pass(std::integral_constant<int, 3>{}, nt0); break;
+                        case 4: pass(std::integral_constant<int, 4>{}, nt0); break;
+                        case 5: pass(std::integral_constant<int, 5>{}, nt0); break;
+                        case 6: pass(std::integral_constant<int, 6>{}, nt0); break;
+                        default: pass(std::integral_constant<int, 7>{}, nt0); break;
                     }
                 }
                 dot += __shfl_xor_sync(0xffffffffu, dot, 1);

@@ -12,7 +12,8 @@
 //   3. bc_trailing_kernel: A_22 -= U_12^T U_12 over the upper 64 x 64 tiles from the row block after
 //      the next one on.
 // The chain of 1 and 2 bounds the factorization (n = 2048: 32 panels, 1.88 ms before the panel's
-// pivots moved into one warp and the next panel's updates into these two kernels, 1.31 ms now); it
+// pivots moved into one warp and the next panel's updates into these two kernels, 1.31 ms after it,
+// 1.16 ms with the row kernel launched beside the panel kernel: its update needs earlier panels only); it
 // runs on a high-priority auxiliary stream while the trailing updates run one panel behind it on
 // the caller's stream.
 // Inverse U^-1 (optional): the panel kernels leave U_JJ^-1 on the diagonal blocks; then for block
@@ -271,6 +272,8 @@ __global__ void __launch_bounds__(kThreadsB) bc_panel_kernel(double* __restrict_
     double* sX = psm + kNB * kPL;   // the inverse
     double* sT = sX + kNB * kPL;    // scratch of the inverse
     __shared__ int s_bad;
+    // the row kernel of this panel may start its own update (it waits for this kernel's results)
+    asm volatile("griddepcontrol.launch_dependents;");
     if (failed(status)) return;
     const int t = threadIdx.x, warp = t >> 5, lane = t & 31, gr = lane >> 2, gc = lane & 3;
     const int jb = min(kNB, n - j0);
@@ -380,8 +383,7 @@ __global__ void __launch_bounds__(kThreadsB) bc_panel_kernel(double* __restrict_
 // update of this row block), then U_12 = U_11^-T A_12 in place.  Doing the update here (and that of
 // the diagonal block in the panel kernel) takes the trailing kernel of panel j0 - 64 off the chain of
 // panels, which needs the trailing update of panel j0 - 128 only.
-__global__ void __launch_bounds__(kThreadsB) bc_panel_row_kernel(double* __restrict__ U, const double* __restrict__ Ub,
-                                                                 int n, int j0, const int* status) {
+__global__ void __launch_bounds__(kThreadsB) bc_panel_row_kernel(double* __restrict__ U, const double* Ub, int n, int j0, const int* status) {
     extern __shared__ double smem[];
     const int jb = min(kNB, n - j0), j1 = j0 + jb;
     const int c0 = j1 + blockIdx.x * kNB;
@@ -399,6 +401,8 @@ __global__ void __launch_bounds__(kThreadsB) bc_panel_row_kernel(double* __restr
         const Opnd P{U + j0 - kNB, n, n, kNB};
         tile_product<true, true>(P, P, j0, c0, 0, kNB, smem, acc);
     }
+    // everything so far is older than the panel kernel, which this kernel was launched beside
+    asm volatile("griddepcontrol.wait;" ::: "memory");
     if (failed(status)) return;
     // the updated tile as the k-contiguous B operand and U_11^-T as the A operand, two 32-deep halves each
 #pragma unroll
@@ -413,7 +417,7 @@ __global__ void __launch_bounds__(kThreadsB) bc_panel_row_kernel(double* __restr
             }
     for (int e = threadIdx.x; e < kNB * kNB; e += kThreadsB) {
         const int k = e % kNB, i = e / kNB;
-        smem[(k >> 5) * kTileDoubles + i * kStrideKC + (k & 31)] = Ub[e];
+        smem[(k >> 5) * kTileDoubles + i * kStrideKC + (k & 31)] = __ldcg(Ub + e);
     }
     __syncthreads();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, gr = lane >> 2, gc = lane & 3;
@@ -612,7 +616,20 @@ cudaError_t blocked_cholesky(const double* M, int n, double* U, double* Ui, void
         bc_panel_kernel<<<1, kThreadsB, kPanelSmem, aux.stream>>>(U, Ub, Ui, n, j0, status);
         const int j1 = j0 + kNB;
         if (j1 >= n) break;
-        bc_panel_row_kernel<<<(n - j1 + kNB - 1) / kNB, kThreadsB, kProductSmem, aux.stream>>>(U, Ub, n, j0, status);
+        // programmatic dependent launch: the row kernel's update of its block by the previous panel runs
+        // beside the panel kernel
+        cudaLaunchAttribute beside{};
+        beside.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        beside.val.programmaticStreamSerializationAllowed = 1;
+        cudaLaunchConfig_t row{};
+        row.gridDim = dim3((n - j1 + kNB - 1) / kNB);
+        row.blockDim = dim3(kThreadsB);
+        row.dynamicSmemBytes = kProductSmem;
+        row.stream = aux.stream;
+        row.attrs = &beside;
+        row.numAttrs = 1;
+        err = cudaLaunchKernelEx(&row, bc_panel_row_kernel, U, (const double*)Ub, n, j0, (const int*)status);
+        if (err != cudaSuccess) break;
         const int m = n - j1 - kNB;
         if (m > 0) {
             if ((err = cudaEventRecord(aux.row_done, aux.stream)) != cudaSuccess) break;

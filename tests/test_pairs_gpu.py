@@ -378,3 +378,25 @@ def test_covalent_pairs_match_records(ctx, n, mult, overlap):
         T[d, ex.term_structure[off[d]:off[d + 1]]] = ex.term_coefficient[off[d]:off[d + 1]]
     assert _rel(H, T.T @ Hd @ T) < tol and _rel(So, T.T @ Sd @ T) < tol
     plan.close()
+
+
+@pytest.mark.parametrize("n", [2, 3, 7, 8, 10, 11, 13, 14, 15, 16, 17])
+@pytest.mark.parametrize("kernel", ["definite", "indefinite", "low_rank", "tied"])
+def test_pair_kernel_factorization_sizes(ctx, n, kernel):
+    """Two electrons: H_de holds (ij|kl) itself through the factored pair kernel, sum_m sigma_m l_m l_m^T.
+    Row counts 3 .. 153 at the edges of the factorization's launch classes (32, 64, 96, 128, 152 rows and
+    the general form), pivots of both signs, early stop and equal diagonals."""
+    P = n * (n + 1) // 2
+    rng = np.random.default_rng(n)
+    S, h, _ = workloads.active_space(n, 3 * n, 60 + n)
+    B = rng.standard_normal((P, P))
+    K = {"definite": lambda: B @ B.T / P, "indefinite": lambda: 0.5 * (B + B.T),
+         "low_rank": lambda: B[:, :n] @ B[:, :n].T / n,
+         "tied": lambda: np.eye(P) + 0.01 * np.sign(np.triu(B, 1) + np.triu(B, 1).T)}[kernel]()
+    eri = workloads.pack_pair_kernel(K)
+    plan, ex = _plan(ctx, "COV", n, 2)
+    H, So = plan.execute(S, h, eri)
+    Hr, Sr, _ = O.structure_matrices(n, ex, S, h, eri)
+    assert _rel(H, Hr) < REL and _rel(So, Sr) < REL
+    assert plan.stats()["factor_columns"] == (n if kernel == "low_rank" else P)
+    plan.close()

@@ -17,6 +17,7 @@
 //  * block_pairs_kernel: the same for lists ordered by blocks of alpha x beta strings, as products of
 //    the blocks' records on the FP64 tensor cores.
 #include <cuda_runtime.h>
+#include <limits.h>
 #include <math.h>
 
 #include <algorithm>
@@ -75,20 +76,143 @@ __global__ void prepare_tables_kernel(int n, const double* __restrict__ eri, dou
     }
 }
 
-// Pivoted LDL^T of the unpacked pair kernel with diagonal (complete) pivoting, one CTA, in the
-// left-looking form.  Thread t owns rows t, t + nt, ... (at most kFactorRows) and keeps their
-// diagonal in registers.  Step m: with the pivot p and its value known, every owned row forms its
-// entry of the Schur-complement column, K[i, p] - sum_{m' < m} sigma_m' l_m'[p] l_m'[i], scales it
+// Pivoted LDL^T of the unpacked pair kernel with diagonal (complete) pivoting, K = sum_m sigma_m l_m l_m^T.
+// Stops when the largest remaining |diagonal| falls to rel_tol times the largest initial one; the dropped
+// remainder then perturbs any opposite-spin energy by at most rel_tol * max|K_pp| * ||p_a||_1 ||p_b||_1.
+// Columns are emitted positive-sign first.
+//
+// factor_pair_registers (np <= 32 B): one CTA of W warps, right-looking, the Schur complement in
+// registers: entry (i, j) with i = W a + warp and j = 32 b + lane in s[a][b].  Per pivot the warp that
+// owns row p scales it into shared memory, one barrier, and every thread updates its entries.  Each warp
+// keeps all diagonals (dg[b], updated from the same row) and finds the next pivot by itself, by integer
+// reductions over the high and low words of |diagonal|: no second barrier and no published maxima.  Bound
+// by the chain pivot search - rsqrt - row - barrier - update, one per factor column: 24 us for 36 columns
+// of 78 rows (n = 12) and 10 us for 18 of 21 (n = 6).  The left-looking form below, which gathers m products
+// per row, publishes warp maxima and compares them in every thread, took 66 us at n = 12, and a one-warp
+// form that read K from global memory in every step 22 us at n = 6.
+template <int W, int B>
+__global__ void __launch_bounds__(32 * W) factor_pair_registers(int np, const double* __restrict__ kfull,
+                                                                int* __restrict__ signs, double* __restrict__ lf, int ld,
+                                                                int* __restrict__ meta, double rel_tol) {
+    constexpr int A = 32 * B / W;
+    extern __shared__ double L[];  // column m of the factor at L[m np ..]
+    __shared__ double s_row[2][32 * B];
+    __shared__ int s_sign[32 * B], s_slot[32 * B];
+    const unsigned full = 0xffffffffu;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    double s[A][B], dg[B];
+    unsigned used = 0;  // bit b: row 32 b + lane is a pivot already (or past the end)
+#pragma unroll
+    for (int a = 0; a < A; ++a)
+#pragma unroll
+        for (int b = 0; b < B; ++b) {
+            const int i = W * a + warp, j = 32 * b + lane;
+            s[a][b] = i < np && j < np ? __ldg(kfull + (long long)i * np + j) : 0.0;
+        }
+#pragma unroll
+    for (int b = 0; b < B; ++b) {
+        const int j = 32 * b + lane;
+        dg[b] = j < np ? __ldg(kfull + (long long)j * np + j) : 0.0;
+        if (j >= np) used |= 1u << b;
+    }
+    // largest |diagonal| of the rows left, the smallest index on ties; *p = -1 when there is none
+    auto search = [&](int* p, double* piv) {
+        double best = -1.0, bd = 0.0;
+        int bi = INT_MAX;
+#pragma unroll
+        for (int b = 0; b < B; ++b)
+            if (!((used >> b) & 1u) && fabs(dg[b]) > best) {
+                best = fabs(dg[b]);
+                bd = dg[b];
+                bi = 32 * b + lane;
+            }
+        // every lane takes part in every reduction
+        bool in = bi != INT_MAX;
+        const unsigned hi = in ? (unsigned)__double2hiint(best) : 0u;
+        const unsigned top = __reduce_max_sync(full, hi);
+        in = in && hi == top;
+        const unsigned lo = in ? (unsigned)__double2loint(best) : 0u;
+        const unsigned low = __reduce_max_sync(full, lo);
+        in = in && lo == low;
+        const int at = __reduce_min_sync(full, in ? bi : INT_MAX);
+        *piv = __shfl_sync(full, bd, at & 31);
+        *p = at == INT_MAX ? -1 : at;
+    };
+    int p;
+    double piv;
+    search(&p, &piv);
+    const double cut = rel_tol * fabs(piv);
+    int m = 0;
+    for (; m < np; ++m) {
+        if (p < 0 || !(fabs(piv) > cut) || piv == 0.0) break;
+        const double inv = rsqrt(fabs(piv));
+        const double sgn = piv > 0.0 ? 1.0 : -1.0;
+        double* row = s_row[m & 1];
+        if (warp == p % W) {
+            const int ap = p / W;
+#pragma unroll
+            for (int b = 0; b < B; ++b) {
+                double v = 0.0;
+#pragma unroll
+                for (int a = 0; a < A; ++a) v = a == ap ? s[a][b] : v;
+                v = (used >> b) & 1u ? 0.0 : v * inv;
+                const int j = 32 * b + lane;
+                row[j] = v;
+                if (j < np) L[m * np + j] = v;
+            }
+        }
+        if (lane == (p & 31)) used |= 1u << (p >> 5);
+        if (tid == 0) {
+            s_sign[m] = (int)sgn;
+            signs[m] = (int)sgn;
+        }
+        __syncthreads();
+        double lj[B];
+#pragma unroll
+        for (int b = 0; b < B; ++b) {
+            lj[b] = row[32 * b + lane];
+            dg[b] = fma(-sgn * lj[b], lj[b], dg[b]);
+        }
+#pragma unroll
+        for (int a = 0; a < A; ++a) {
+            const double li = -sgn * row[W * a + warp];
+#pragma unroll
+            for (int b = 0; b < B; ++b) s[a][b] = fma(li, lj[b], s[a][b]);
+        }
+        search(&p, &piv);
+    }
+    // slots: the columns with positive sign first
+    if (warp == 0) {
+        int pos = 0;
+        for (int c0 = 0; c0 < m; c0 += 32) pos += __popc(__ballot_sync(full, c0 + lane < m && s_sign[c0 + lane] > 0));
+        int ip = 0, in = pos;
+        for (int c0 = 0; c0 < m; c0 += 32) {
+            const bool here = c0 + lane < m, plus = here && s_sign[c0 + lane] > 0;
+            const unsigned bp = __ballot_sync(full, plus), bn = __ballot_sync(full, here && !plus);
+            const unsigned below = (1u << lane) - 1u;
+            if (here) s_slot[plus ? ip + __popc(bp & below) : in + __popc(bn & below)] = c0 + lane;
+            ip += __popc(bp);
+            in += __popc(bn);
+        }
+        if (lane == 0) {
+            meta[0] = pos;
+            meta[1] = m - pos;
+        }
+    }
+    __syncthreads();
+    for (int q = warp; q < np; q += W)
+        for (int slot = lane; slot < ld; slot += 32)
+            lf[(long long)q * ld + slot] = slot < m ? L[s_slot[slot] * np + q] : 0.0;
+}
+
+// Larger pair kernels, one CTA, left-looking.  Thread t owns rows t, t + nt, ... (at most kFactorRows) and
+// keeps their diagonal in registers.  Step m: with the pivot p and its value known, every owned row forms
+// its entry of the Schur-complement column, K[i, p] - sum_{m' < m} sigma_m' l_m'[p] l_m'[i], scales it
 // into l_m[i] and updates its diagonal; each warp then reduces its rows' largest |diagonal| and
 // one barrier publishes the warp results, from which every thread picks the next pivot.
-// Stops when the largest remaining |diagonal| falls to rel_tol times the largest initial one;
-// the dropped remainder then perturbs any opposite-spin energy by at most
-// rel_tol * max|K_pp| * ||p_a||_1 ||p_b||_1.  Columns are emitted positive-sign first.
-// K and the columns l_m (l_m[i] at [m np + i]) sit in shared memory when they fit (in_smem),
-// else K is read from `kfull` and the columns live in `cols`.  `work_g` is not used.
+// The columns l_m (l_m[i] at [m np + i]) live in `cols`.  `work_g` is not used.
 constexpr int kFactorRows = 4;
 
-template <bool in_smem>  // compile-time, so that the shared-memory path uses shared loads
 __global__ void __launch_bounds__(1024) factor_pair_kernel(int np, const double* __restrict__ kfull,
                                                            double* __restrict__ work_g, double* __restrict__ cols,
                                                            int* __restrict__ signs, double* __restrict__ lf, int ld,
@@ -97,14 +221,11 @@ __global__ void __launch_bounds__(1024) factor_pair_kernel(int np, const double*
     extern __shared__ double fsm[];
     double* sig = fsm;                                        // np
     int* slot_col = reinterpret_cast<int*>(sig + np);         // np (+1 pad)
-    double* Ks = sig + np + (np + 2) / 2;                     // np^2 when in_smem
-    const double* K = in_smem ? Ks : kfull;
-    double* L = in_smem ? Ks + (size_t)np * np : cols;
+    const double* K = kfull;
+    double* L = cols;
     __shared__ double red_v[2][32], red_d[2][32];
     __shared__ int red_i[2][32];
     const int tid = threadIdx.x, nt = blockDim.x, lane = tid & 31, warp = tid >> 5, nwarps = nt >> 5;
-    if (in_smem)
-        for (long long i = tid; i < (long long)np * np; i += nt) Ks[i] = __ldg(kfull + i);
     double dg[kFactorRows];
     bool used[kFactorRows];
 #pragma unroll
@@ -212,74 +333,6 @@ __global__ void __launch_bounds__(1024) factor_pair_kernel(int np, const double*
     for (int q = warp; q < np; q += nwarps)
         for (int slot = lane; slot < ld; slot += 32)
             lf[(long long)q * ld + slot] = slot < m ? L[(long long)slot_col[slot] * np + q] : 0.0;
-}
-
-// The same factorization for np <= 32 (active spaces of up to 7 orbitals) in one warp: lane i
-// owns row i, the pivot search is a shuffle reduction and the steps need no block barrier.
-__global__ void __launch_bounds__(32) factor_pair_warp_kernel(int np, const double* __restrict__ kfull,
-                                                             int* __restrict__ signs, double* __restrict__ lf,
-                                                             int ld, int* __restrict__ meta, double rel_tol) {
-    __shared__ double sL[32][33];  // column m of the factor in sL[m][.]
-    __shared__ double sig[32];
-    __shared__ int slot_col[32];
-    const int lane = threadIdx.x;
-    double dg = lane < np ? __ldg(kfull + (long long)lane * np + lane) : 0.0;
-    bool used = lane >= np;
-    auto argmax = [&](int* p, double* piv) {
-        double best = used ? -1.0 : fabs(dg), bd = dg;
-        int bi = used ? -1 : lane;
-        for (int o = 16; o > 0; o >>= 1) {
-            const double ov = __shfl_xor_sync(0xffffffffu, best, o);
-            const double od = __shfl_xor_sync(0xffffffffu, bd, o);
-            const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
-            if (ov > best || (ov == best && oi >= 0 && (bi < 0 || oi < bi))) {
-                best = ov;
-                bd = od;
-                bi = oi;
-            }
-        }
-        *p = bi;
-        *piv = bd;
-    };
-    int p;
-    double piv;
-    argmax(&p, &piv);
-    const double cut = rel_tol * fmax(fabs(piv), 0.0);
-    int m = 0;
-    for (; m < np; ++m) {
-        if (p < 0 || !(fabs(piv) > cut) || piv == 0.0) break;
-        const double inv = rsqrt(fabs(piv));
-        const double sgn = piv > 0.0 ? 1.0 : -1.0;
-        double v = 0.0;
-        if (!used) {
-            double acc = __ldg(kfull + (long long)p * np + lane);
-            for (int q = 0; q < m; ++q) acc = fma(-sig[q] * sL[q][p], sL[q][lane], acc);
-            v = acc * inv;
-            if (lane == p)
-                used = true;
-            else
-                dg = fma(-sgn * v, v, dg);
-        }
-        sL[m][lane] = v;
-        if (lane == 0) {
-            sig[m] = sgn;
-            signs[m] = (int)sgn;
-        }
-        __syncwarp();
-        argmax(&p, &piv);
-    }
-    if (lane == 0) {
-        int pos = 0;
-        for (int c = 0; c < m; ++c) pos += sig[c] > 0.0 ? 1 : 0;
-        int ip = 0, in = pos;
-        for (int c = 0; c < m; ++c) slot_col[sig[c] > 0.0 ? ip++ : in++] = c;
-        meta[0] = pos;
-        meta[1] = m - pos;
-    }
-    __syncwarp();
-    for (int q = 0; q < np; ++q)
-        for (int slot = lane; slot < ld; slot += 32)
-            lf[(long long)q * ld + slot] = slot < m ? sL[slot_col[slot]][q] : 0.0;
 }
 
 // Listed blocks (or all blocks): one thread per block resolves it by the exact path; its first
@@ -799,27 +852,27 @@ __global__ void same_spin_list_kernel(int n, int k, long long batch, const int* 
 
 cudaError_t launch_factor_pair_kernel(int np, const double* kfull, double* work, double* cols, int* signs, double* lf,
                                       int ld, int* meta, cudaStream_t stream) {
-    if (np <= 32) {
-        factor_pair_warp_kernel<<<1, 32, 0, stream>>>(np, kfull, signs, lf, ld, meta, factor_tolerance(np));
+    const double tol = factor_tolerance(np);
+    // up to 152 rows (16 orbitals) the columns fit shared memory and the Schur complement registers
+    const size_t columns = sizeof(double) * (size_t)np * np;
+    auto registers = [&](auto kernel, int warps) {
+        const cudaError_t err = allow_dynamic_smem((const void*)kernel, columns);
+        if (err != cudaSuccess) return err;
+        kernel<<<1, 32 * warps, columns, stream>>>(np, kfull, signs, lf, ld, meta, tol);
         return cudaGetLastError();
-    }
+    };
+    if (np <= 32) return registers(factor_pair_registers<4, 1>, 4);
+    if (np <= 64) return registers(factor_pair_registers<8, 2>, 8);
+    if (np <= 96) return registers(factor_pair_registers<16, 3>, 16);
+    if (np <= 128) return registers(factor_pair_registers<16, 4>, 16);
+    if (np <= 152) return registers(factor_pair_registers<16, 5>, 16);
     int threads = (np + 31) / 32 * 32;
-    threads = threads < 64 ? 64 : (threads > 1024 ? 1024 : threads);
+    threads = threads > 1024 ? 1024 : threads;
     if (np > threads * kFactorRows) return cudaErrorInvalidValue;
-    const size_t aux_bytes = sizeof(double) * ((size_t)np + (np + 2) / 2);
-    const size_t in_smem_bytes = aux_bytes + 2 * sizeof(double) * (size_t)np * np;
-    const int in_smem = in_smem_bytes <= 200 * 1024 ? 1 : 0;
-    const size_t smem = in_smem ? in_smem_bytes : aux_bytes;
-    cudaError_t err = allow_dynamic_smem(in_smem ? (const void*)factor_pair_kernel<true>
-                                                 : (const void*)factor_pair_kernel<false>,
-                                         (int)smem);
+    const size_t smem = sizeof(double) * ((size_t)np + (np + 2) / 2);
+    cudaError_t err = allow_dynamic_smem((const void*)factor_pair_kernel, (int)smem);
     if (err != cudaSuccess) return err;
-    if (in_smem)
-        factor_pair_kernel<true><<<1, threads, smem, stream>>>(np, kfull, work, cols, signs, lf, ld, meta,
-                                                               factor_tolerance(np));
-    else
-        factor_pair_kernel<false><<<1, threads, smem, stream>>>(np, kfull, work, cols, signs, lf, ld, meta,
-                                                                factor_tolerance(np));
+    factor_pair_kernel<<<1, threads, smem, stream>>>(np, kfull, work, cols, signs, lf, ld, meta, tol);
     return cudaGetLastError();
 }
 
@@ -843,8 +896,10 @@ size_t exact_stack_bytes() {
 
 cudaError_t preload_spin_pair_kernels() {
     // cudaFuncGetAttributes loads a function that lazy module loading has not loaded yet
-    const void* fns[] = {(const void*)prepare_tables_kernel, (const void*)factor_pair_kernel<true>,
-                         (const void*)factor_pair_kernel<false>, (const void*)factor_pair_warp_kernel,
+    const void* fns[] = {(const void*)prepare_tables_kernel, (const void*)factor_pair_kernel,
+                         (const void*)factor_pair_registers<4, 1>, (const void*)factor_pair_registers<8, 2>,
+                         (const void*)factor_pair_registers<16, 3>, (const void*)factor_pair_registers<16, 4>,
+                         (const void*)factor_pair_registers<16, 5>,
                          (const void*)spin_pairs_exact<7, 7>, (const void*)spin_pairs_exact<8, 0>,
                          (const void*)spin_pairs_exact<dev::KMAX, 0>};
     for (const void* f : fns) {

@@ -236,8 +236,8 @@ __global__ void __launch_bounds__(kBandWarps * 32, 3)
 // keeps one group: warp w holds the coefficients of its 8 structures over all rows as A fragments in
 // registers (up to 64 k-steps) and walks column tiles of 16, whose rows arrive by cp.async (128 bytes of
 // H and of S each, rows past the diagonal as zeros) while the tile before is multiplied.
-// The tensor cores' share is 3.2 ms (216 M products for 34,188 determinants); takes 8.2 ms there, with
-// one CTA per SM and three barriers per tile.  The tiled form above takes 36.7 ms on such a list, and
+// The tensor cores' share is 3.2 ms (216 M products for 34,188 determinants); takes 8.1 ms there
+// (8.3 ms with a second barrier per tile before Z is written), one CTA of 12 warps per SM.  The tiled form above takes 36.7 ms on such a list, and
 // 10.1 ms with 64-row tiles gathered from each group's own rows: one shared-memory load per nonzero and
 // column and 25 instructions around it.
 constexpr int kDenseWarps = 12;    // 6 structure tiles x 2 column halves
@@ -250,7 +250,7 @@ static int dense_rows(int rows) { return (rows + 31) / 32 * 32; }
 static size_t dense_smem_bytes(int rows) {
     // the coefficients pass through the tile buffers first
     const size_t tiles = 2 * (size_t)dense_rows(rows) * kDenseLd, coefficients = (size_t)kDenseStructures * (kDenseRows + 4);
-    return sizeof(double) * ((tiles > coefficients ? tiles : coefficients) + 2 * kDenseColumns * kDenseZ) +
+    return sizeof(double) * ((tiles > coefficients ? tiles : coefficients) + 4 * kDenseColumns * kDenseZ) +
            sizeof(int) * (size_t)rows;
 }
 
@@ -261,7 +261,7 @@ __global__ void __launch_bounds__(32 * kDenseWarps, 1) dense_reduce_kernel(BandR
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, gr = lane >> 2, gc = lane & 3;
     const int mt = warp % 6, ch = warp / 6;  // structure tile, column half
     double* zbuf = rsm + z_at;
-    int* rows = reinterpret_cast<int*>(zbuf + 2 * C * kDenseZ);
+    int* rows = reinterpret_cast<int*>(zbuf + 4 * C * kDenseZ);  // after the Z of two tiles
     const int nb = (int)((a.width + C - 1) / C);
     const int4 grp = __ldg(a.groups + blockIdx.x / parts);  // first row entry, rows, first structure, structures
     const int n_rows = grp.y, n_str = grp.w;
@@ -301,6 +301,14 @@ __global__ void __launch_bounds__(32 * kDenseWarps, 1) dense_reduce_kernel(BandR
         }
         asm volatile("cp.async.commit_group;" ::: "memory");
     };
+    auto store = [&](int b, const double* z) {
+        for (int l = warp; l < 2 * C; l += kDenseWarps) {
+            const long long col = (long long)b * C + l % C;
+            if (col >= a.width) continue;
+            double* Z = (l < C ? a.Zh : a.Zs) + (a.e0 + col) * a.n_str + grp.z;
+            for (int q = lane; q < n_str; q += 32) Z[q] = z[l * kDenseZ + q];
+        }
+    };
     int b = blockIdx.x % parts, buf = 0, valid = 0;
     {
         // first tile: by bisection
@@ -315,17 +323,13 @@ __global__ void __launch_bounds__(32 * kDenseWarps, 1) dense_reduce_kernel(BandR
         }
     }
     issue(b, 0, valid);
+    // one barrier per tile: past it every warp is done with the tile before, whose buffer takes the next
+    // one and whose Z goes out while the products run
     for (; b < nb; b += parts, buf ^= 1) {
-        int next = valid;
-        if (b + parts < nb) {
-            next = valid_rows(b + parts, valid);
-            issue(b + parts, buf ^ 1, next);
-            asm volatile("cp.async.wait_group 1;" ::: "memory");
-        } else {
-            asm volatile("cp.async.wait_group 0;" ::: "memory");
-        }
-        const long long col0 = (long long)b * C, first = a.e0 + col0;
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
+        const long long first = a.e0 + (long long)b * C;
         double* tile = rsm + buf * tile_doubles;
+        double* z = zbuf + buf * 2 * C * kDenseZ;
         if (valid > 0 && rows[valid - 1] > first) {
             // the band holds no data below the diagonal: a thread clears its own copies there
             double* dst = own + buf * tile_doubles;
@@ -336,6 +340,12 @@ __global__ void __launch_bounds__(32 * kDenseWarps, 1) dense_reduce_kernel(BandR
             }
         }
         __syncthreads();
+        int next = valid;
+        if (b + parts < nb) {
+            next = valid_rows(b + parts, valid);
+            issue(b + parts, buf ^ 1, next);
+        }
+        if (b >= parts) store(b - parts, zbuf + (buf ^ 1) * 2 * C * kDenseZ);
         if (8 * mt < n_str) {
             double h[2][2] = {}, s[2][2] = {};
             const double* p = tile + gc * LD + 8 * ch + gr;
@@ -352,19 +362,14 @@ __global__ void __launch_bounds__(32 * kDenseWarps, 1) dense_reduce_kernel(BandR
 #pragma unroll
             for (int i = 0; i < 2; ++i) {
                 const int col = 8 * ch + 2 * gc + i;
-                zbuf[col * kDenseZ + 8 * mt + gr] = h[0][i] + h[1][i];
-                zbuf[(C + col) * kDenseZ + 8 * mt + gr] = s[0][i] + s[1][i];
+                z[col * kDenseZ + 8 * mt + gr] = h[0][i] + h[1][i];
+                z[(C + col) * kDenseZ + 8 * mt + gr] = s[0][i] + s[1][i];
             }
-        }
-        __syncthreads();
-        for (int l = warp; l < 2 * C; l += kDenseWarps) {
-            const long long col = col0 + l % C;
-            if (col >= a.width) continue;
-            double* Z = (l < C ? a.Zh : a.Zs) + (a.e0 + col) * a.n_str + grp.z;
-            for (int q = lane; q < n_str; q += 32) Z[q] = zbuf[l * kDenseZ + q];
         }
         valid = next;
     }
+    __syncthreads();
+    if (b >= parts) store(b - parts, zbuf + (buf ^ 1) * 2 * C * kDenseZ);
 }
 
 // W[I, J] = sum_{(e, c) in J} c Z[I, e]; one CTA per J, threads over I.  The terms of J are
@@ -481,7 +486,7 @@ cudaError_t launch_band_reduce(const BandReduceArgs& a, cudaStream_t stream, int
         long long parts = (6 * kSms + a.n_groups - 1) / a.n_groups;
         parts = parts > nb ? nb : parts;
         const int tile_doubles = dense_rows(a.group_rows) * kDenseLd;
-        const int z_at = (int)((smem - sizeof(int) * a.group_rows) / sizeof(double)) - 2 * kDenseColumns * kDenseZ;
+        const int z_at = (int)((smem - sizeof(int) * a.group_rows) / sizeof(double)) - 4 * kDenseColumns * kDenseZ;
         dense_reduce_kernel<<<(unsigned)(parts * a.n_groups), 32 * kDenseWarps, smem, stream>>>(a, (int)parts, tile_doubles, z_at);
         ++*launches;
         return cudaGetLastError();

@@ -3,7 +3,7 @@
 // In a covalent list every orbital is singly occupied: the beta string of a determinant is the
 // complement x of its alpha string u, every alpha string carries one determinant, and each spin-pair
 // record is used by exactly one determinant pair (two that are equal, with spin-flip symmetry).  Writing
-// the records (R + 4 doubles a pair: 5.2 GB for the 5.9 M pairs of 14 orbitals) and gathering them again
+// the records (R + 4 doubles a pair: 2.2 GB for the 5.9 M pairs of 14 orbitals) and gathering them again
 // took as long as the products behind them.  covalent_pairs takes both spins of a determinant pair in the
 // same warp and keeps the two u-vectors in tensor-core accumulators until they are multiplied.
 //
@@ -380,10 +380,11 @@ size_t covalent_smem(int n, int kb, int R, int warps) {
 
 constexpr size_t kCovalentSmemMax = 226 * 1024;
 
-// Warps per CTA: enough for a left string's chunks (16 pairs each) in four rounds, within shared memory.
+// Warps per CTA: enough for a left string's chunks (16 pairs each) in four rounds, at least four to load the
+// blocks, within shared memory (6 orbitals: 18 us with two warps, 12.5 us with four).
 template <int K>
 int covalent_warps(const CovalentArgs& a) {
-    int warps = 2;
+    int warps = 4;
     while (warps < kCovalentMaxWarps && warps * 64 < a.n_strings) warps *= 2;
     while (warps > 2 && covalent_smem<K>(a.n, a.kb, a.R, warps) > kCovalentSmemMax) warps /= 2;
     return warps;

@@ -3,14 +3,16 @@
 //  * prepare_tables: the unpacked pair kernel K[p][q] = (p|q) over packed orbital pairs and the
 //    antisymmetrized same-spin table Gamma[(i<k)][(j<l)] = (ij|kl) - (il|kj) used by the
 //    same-spin two-electron sum (hamiltonian.cpp:83-123 sums exactly these differences).
-//  * factor_pair_kernel: pivoted LDL^T of the pair kernel, K = sum_m sigma_m l_m l_m^T.
+//  * factor_pair_registers, factor_pair_kernel: pivoted LDL^T of the pair kernel, K = sum_m sigma_m l_m l_m^T.
 //  * the register-resident spin-pair path lives in spin_frame.cu (left-string frame kernels); a
 //    block is accepted there only under the conditioning certificate (kCertificate2): then the
 //    last pivot of a complete-pivoting LU is at least 1 / ||X^{-1}||_F and the first at most
 //    ||X||_F, so their ratio stays far above 1e-12 and the reference's FullPivLU would also find
-//    full rank (overlap.cpp:60-71).  Every other block is appended to a list for the exact kernel.
+//    full rank (overlap.cpp:60-71).  Other blocks are evaluated there by polynomials at excitation levels
+//    up to 5 when the left string's frame is sound, or appended to a list for the exact kernel.
 //  * spin_pairs_exact<KM>: complete-pivoting LU / Jacobi SVD with the reference semantics
 //    (device_algebra.cuh) for listed blocks, one thread per block, local arrays bounded by KM.
+//  * determinant pairs of covalent lists: covalent_pairs.cu, without records.
 //  * full_pairs_kernel: one thread per determinant pair (d <= e) of a band of columns:
 //    S = S_a S_b, H = H_a S_b + H_b S_a + sum_m sigma_m u_a[m] u_b[m] (evaluator.cpp:95-148,
 //    354-384 with the opposite-spin term in factored form), folded over the spin-flip orbit.
@@ -955,7 +957,10 @@ cudaError_t launch_spin_pairs_exact(const SpinTableArgs& a, cudaStream_t stream,
         err = allow_dynamic_smem((const void*)exact, (int)slot_bytes);
         if (err != cudaSuccess) return err;
     }
-    exact<<<kSms * 8, 64, slot_bytes, stream>>>(b);
+    // at most one warp per pair of the table: the list is usually empty, and a full grid of CTAs that only
+    // read its length takes 6 us
+    const long long grid = (a.n_pairs + 1) / 2;
+    exact<<<(unsigned)(grid < kSms * 8 ? grid : kSms * 8), 64, slot_bytes, stream>>>(b);
     ++*launches;
     return cudaGetLastError();
 }

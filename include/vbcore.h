@@ -55,8 +55,8 @@ vb_status vb_context_destroy(vb_context* ctx);
  * stream order). */
 vb_status vb_context_set_stream(vb_context* ctx, void* cuda_stream);
 vb_status vb_context_synchronize(vb_context* ctx);
-/* Polls a grid-barrier wait of the cooperative eigensolver kernels (vb_generalized_eigh, and
- * vb_metric_cholesky up to n = 96; the blocked Cholesky used above that size and for the Davidson
+/* Polls a grid-barrier wait of the cooperative eigensolver kernels (vb_generalized_eigh above 160
+ * structures, and vb_metric_cholesky up to n = 96; the blocked Cholesky used above that size and for the Davidson
  * shift-invert factor has no grid barrier) makes before it gives up: the kernel
  * then ends and the call returns VB_ERR_TIMEOUT, with the context still usable.  0 restores the
  * built-in default (2^26 polls, seconds).  No reference counterpart: the reference's solvers are
@@ -155,8 +155,9 @@ vb_status vb_hs_plan_stats(const vb_hs_plan* plan, vb_hs_stats* stats);
  * execute records events around its phases; vb_hs_plan_phase_times synchronizes and returns
  * the milliseconds of the last execute per phase: [0] integral tables (pair-kernel factorization
  * and the per-left-string frame tables), [1] spin-pair records of the register path (frame
- * kernel), [2] determinant pairs (all bands), [3] band reduction, [4] structure reduction +
- * symmetrization, [5] spin-pair records of the exact path (listed blocks).  Phases [2] and [3] sum over bands. */
+ * kernel) or, for covalent lists evaluated without records, the determinant pairs, [2] determinant
+ * pairs from records (all bands), [3] band reduction, [4] structure reduction + symmetrization,
+ * [5] spin-pair records of the exact path (listed blocks).  Phases [2] and [3] sum over bands. */
 enum { VB_PHASE_TABLES = 0, VB_PHASE_SPIN_PAIRS = 1, VB_PHASE_DETERMINANT_PAIRS = 2, VB_PHASE_BAND_REDUCE = 3,
        VB_PHASE_STRUCTURE_REDUCE = 4, VB_PHASE_EXACT_PAIRS = 5, VB_PHASE_COUNT = 6 };
 vb_status vb_hs_plan_enable_phase_timing(vb_hs_plan* plan, int enable);

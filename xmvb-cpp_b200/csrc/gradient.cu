@@ -14,8 +14,10 @@
 //      the same with a <-> b.  With a spin-flip symmetric determinant list the scatter is grouped
 //      by alpha record (det_pair_adjoint_flip_kernel, no atomics), and in two stages through a
 //      per-alpha-string table in shared memory when alpha strings carry several determinants
-//      (det_pair_adjoint_two_stage_kernel).
-//   2. spin_backward_kernel<K>: per spin pair, with X = S[R, L], B = X^-1 and d = det X:
+//      (det_pair_adjoint_two_stage_kernel).  Covalent singlets (one determinant per alpha string) need no
+//      scatter: the adjoints are the partners' records times a weight.
+//   2. with RI factors, the reverse of the frame kernels (gradient_frame.cu); for a gradient per packed
+//      integral spin_backward_kernel<K>: per spin pair, with X = S[R, L], B = X^-1 and d = det X:
 //      det = d, A = d B^T, H_1 = <h[R, L], A>, H_2 = d q(B) (q: the same-spin two-electron form
 //      in B), u[m] = <l_m[pair(R, L)], A>.  The adjoint with respect to X is
 //        d ( s B^T - (B M B)^T ),  s = adj_det + <G_A, B^T> + adj_H q,  M = G_A + adj_H Q^T,

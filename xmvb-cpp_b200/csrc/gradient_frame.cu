@@ -25,7 +25,7 @@
 // S_LL is near singular are listed for the exact kernel of gradient.cu; certified ones take the inverse
 // of B.  When every alpha string carries one determinant (covalent singlets) and the list is spin-flip
 // symmetric, the adjoint of record (u, v) is the record of the partners' beta strings times one weight:
-// the rows w are then read from the records themselves, and no adjoint buffer is built or read (5.2 GB
+// the rows w are then read from the records themselves, and no adjoint buffer is built or read (2.1 GB
 // at K = 7, 3.8 ms).  The pair-by-pair path takes the K x K inverse of every pair with C(K, 2)^2
 // shared-memory atomics, and an SVD per thread for the uncertified ones: 14 stretched hydrogen atoms
 // (5.9 M pairs, 4.9 M of them uncertified), 48.7 + 170 ms and 24 ms of contractions, against 7.0 + 1.2 ms

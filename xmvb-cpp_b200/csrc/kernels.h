@@ -165,7 +165,8 @@ struct StructureReduceArgs {
 // of X is 1 / (an entry of the permuted X^-1) >= 1 / ||X^-1||_F and the first complete-pivoting
 // pivot is max|x_ij| <= ||X||_F, so the smallest pivot ratio of the reference's complete-pivoting
 // LU stays >= ~1 / (c_k kappa_F) with c_k modest for k <= 16: far above its 1e-12 rank threshold,
-// so these blocks are full rank under the reference semantics.  Others take the exact path.
+// so these blocks are full rank under the reference semantics.  Others are evaluated by polynomials in the
+// frame (kFrameCondition2) or take the exact path.
 constexpr double kCertificate2 = 1.0e16;
 
 constexpr int kBandWarps = 8;        // warps per band-reduction CTA

@@ -997,10 +997,20 @@ cudaError_t launch_block_pairs(const BlockPairArgs& a, cudaStream_t stream, int*
     int per_sm = 1;
     err = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, 32 * kBlockWarps, smem);
     if (err != cudaSuccess) return err;
-    const long long grid = (long long)kSms * (per_sm > 0 ? per_sm : 1);
-    kernel<<<(unsigned)(total < grid ? total : grid), 32 * kBlockWarps, smem, stream>>>(a);
+    // launch variants (CTAs per SM: as many as fit, or one less), chosen by the autotuner per list
+    if (per_sm < 1) per_sm = 1;
+    const int fewer = per_sm > 1 ? per_sm - 1 : 1;
+    const std::string key = "full_pairs_kernel (blocks) R=" + std::to_string(a.f.R) + " ndet=" + std::to_string(a.f.n_det);
+    autotune_run(
+        key, 2, stream,
+        [&](int v) {
+            const long long grid = (long long)kSms * (v ? fewer : per_sm);
+            kernel<<<(unsigned)(total < grid ? total : grid), 32 * kBlockWarps, smem, stream>>>(a);
+            return cudaGetLastError();
+        },
+        {}, &err);
     ++*launches;
-    return cudaGetLastError();
+    return err;
 }
 
 cudaError_t launch_listed_pairs(const FullPairArgs& a, long long n_pairs, const long long* pairs, double* h_out,

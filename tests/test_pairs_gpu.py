@@ -400,3 +400,20 @@ def test_pair_kernel_factorization_sizes(ctx, n, kernel):
     assert _rel(H, Hr) < REL and _rel(So, Sr) < REL
     assert plan.stats()["factor_columns"] == (n if kernel == "low_rank" else P)
     plan.close()
+
+
+@pytest.mark.parametrize("n,mult", [(8, 1), (10, 3)])
+def test_small_budget_takes_records_and_exact_path(ctx, n, mult):
+    """A budget without room for the covalent pair lists (and an open shell's frame tables) beside what
+    later calls may take: the plan works from records; same matrices (same bound as above)."""
+    S, h, eri = workloads.active_space(n, 3 * n, n)
+    plan, _ = _plan(ctx, "COV", n, n, mult)
+    H, So = plan.execute(S, h, eri)
+    small = vbcore.Context(0, 200 << 20)
+    try:
+        tight, _ = _plan(small, "COV", n, n, mult)
+        H2, S2 = tight.execute(S, h, eri)
+        assert _rel(H2, H) < 1e-11 and _rel(S2, So) < 1e-11
+        tight.close()
+    finally:
+        small.close()

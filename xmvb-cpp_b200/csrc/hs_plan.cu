@@ -288,6 +288,17 @@ vb_status upload_blocks(vb_hs_plan* p, const DeterminantBlocks& b) {
     return st;
 }
 
+// Whether `bytes` more leave the budget what evaluations and gradients of the plan may still take (records at
+// the largest factor rank and their adjoints, bands, Z, W and outputs): tables that only save time are
+// built where they cannot make a later call run out.
+bool room_for(const vb_hs_plan* p, size_t bytes) {
+    const vb_context* ctx = p->ctx;
+    const double records = 8.0 * record_stride(p->np) * (double)(p->npairs_a + p->npairs_b);
+    const double scratch = (double)std::min<size_t>((size_t)1 << 30, ctx->budget / 8) + 16.0 * p->n_str * (double)p->n_det +
+                           48.0 * p->n_str * (double)p->n_str;
+    return (double)ctx->current + (double)bytes + 3.0 * records + scratch + (256 << 20) <= (double)ctx->budget;
+}
+
 // Pair lists of a covalent list: every orbital singly occupied, one determinant per alpha string, frame
 // tables for both spins and, where these are one table, spin-flip symmetric.  Without room for them the
 // records path needs none.
@@ -306,6 +317,8 @@ vb_status covalent_lists(vb_hs_plan* p, const vb_expansion* ex) {
     }
     CovalentPlan& c = p->covalent;
     const size_t pairs = (size_t)std::max(1LL, p->npairs_a);
+    if (!room_for(p, (2 * sizeof(int) + sizeof(unsigned long long)) * pairs + sizeof(int) * (size_t)p->Na * (p->ka + 4)))
+        return VB_OK;
     vb_status st = upload(p->ctx, c.det, det.data(), sizeof(int) * det.size());
     if (st == VB_OK) st = upload(p->ctx, c.beta, beta.data(), sizeof(int) * beta.size());
     if (st == VB_OK) st = c.desc.allocate(p->ctx, sizeof(unsigned) * pairs);
@@ -551,6 +564,9 @@ vb_status vb_hs_plan_create(vb_context* ctx, const vb_expansion* ex, vb_hs_plan*
         DeviceBuffer& rd = beta ? p->rdesc_b : p->rdesc_a;
         DeviceBuffer& eb = beta ? p->ebound_b : p->ebound_a;
         DeviceBuffer& tb = beta ? p->tables_b : p->tables_a;
+        if (frame_wide_complement(n, k) &&
+            !room_for(p, 8 * ((size_t)N * (N + 1) / 2) + sizeof(double) * frame_table_doubles(n, k, p->np) * N))
+            continue;  // as below
         st = rl.allocate(ctx, sizeof(int) * (size_t)std::max(1LL, N * (N + 1) / 2));
         if (st == VB_OK) st = rd.allocate(ctx, sizeof(unsigned) * (size_t)std::max(1LL, N * (N + 1) / 2));
         if (st == VB_OK) st = eb.allocate(ctx, sizeof(int) * (size_t)N * (k + 2));

@@ -387,9 +387,10 @@ def run_vbcore(args):
     n_strings = len(ex.alpha_strings)
     spin_units = n_strings * (n_strings + 1) // 2
     det_units = stats["determinant_pairs"]  # orbit representatives under the alpha/beta exchange
+    # covalent lists: one kernel takes both spins of a determinant pair and combines them (spin-pair phase;
+    # the determinant-pair phase holds the few pairs of the exact path)
     kernels = {
-        "spin_pairs": ("spin_pairs_frame", spin_units * flops_spin_pair(k), spin_units),
-        "determinant_pairs": ("full_pairs_kernel", det_units * flops_full_pair(k, k), det_units),
+        "spin_pairs": ("covalent_pairs", spin_units * flops_spin_pair(k) + det_units * flops_full_pair(k, k), det_units),
     }
     dominant = max(kernels, key=lambda name: mean_phase[name])
     kname, flops, units = kernels[dominant]

@@ -604,7 +604,7 @@ __global__ void __launch_bounds__(512) full_pairs_kernel(FullPairArgs a) {
 // half of the N tiles; H goes through shared memory so that band rows are written in runs of a block's determinants.  Both
 // members of a spin-flip orbit are evaluated: blocks do not map to blocks under the flip.  Bound by the
 // product (1.7 ms at the tensor cores' rate for 34,188 determinants) and the band it writes (9.3 GB, 1.4 ms);
-// takes 9.0 ms there (10.7 ms with record addresses and determinant cells divided out per element, four
+// takes 8.7 to 9.0 ms there (10.7 with record addresses and determinant cells divided out per element, four
 // warps and four barriers), the gather form 27.3 ms.  A block pair is 2.4 us of loads, products and stores
 // one after the other on 3 CTAs per SM; a second record buffer with one CTA per SM: 11.7 ms.
 constexpr int kBlockWarps = 8;
@@ -997,19 +997,20 @@ cudaError_t launch_block_pairs(const BlockPairArgs& a, cudaStream_t stream, int*
     int per_sm = 1;
     err = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, 32 * kBlockWarps, smem);
     if (err != cudaSuccess) return err;
-    // launch variants (CTAs per SM: as many as fit, or one less), chosen by the autotuner per list
+    // launch variants (CTAs per SM: as many as fit, or one less), chosen by the autotuner per list on a band
+    // that fills the chip sixteen times over (the first bands of a large list are too short to tell: tuned
+    // there, 34,188 determinants took 10.3 ms instead of 8.7)
     if (per_sm < 1) per_sm = 1;
     const int fewer = per_sm > 1 ? per_sm - 1 : 1;
-    const std::string key = "full_pairs_kernel (blocks) R=" + std::to_string(a.f.R) + " ndet=" + std::to_string(a.f.n_det);
-    autotune_run(
-        key, 2, stream,
-        [&](int v) {
-            const long long grid = (long long)kSms * (v ? fewer : per_sm);
-            kernel<<<(unsigned)(total < grid ? total : grid), 32 * kBlockWarps, smem, stream>>>(a);
-            return cudaGetLastError();
-        },
-        {}, &err);
+    auto launch = [&](int v) {
+        const long long grid = (long long)kSms * (v ? fewer : per_sm);
+        kernel<<<(unsigned)(total < grid ? total : grid), 32 * kBlockWarps, smem, stream>>>(a);
+        return cudaGetLastError();
+    };
     ++*launches;
+    if (total < 16ll * kSms * per_sm) return launch(0);
+    autotune_run("full_pairs_kernel (blocks) R=" + std::to_string(a.f.R) + " ndet=" + std::to_string(a.f.n_det), 2, stream,
+                 launch, {}, &err);
     return err;
 }
 

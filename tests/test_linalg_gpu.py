@@ -247,3 +247,33 @@ def test_tridiagonal_eigh_sizes_and_clusters(ctx, n, spectrum):
     assert np.all(np.diff(w) >= 0)
     assert np.abs(C.T @ S @ C - np.eye(n)).max() < 1e-10
     assert np.abs(H @ C - S @ C * w).max() < 1e-10 * scale * max(1.0, np.abs(C).max())
+
+
+def test_tridiagonal_eigh_beside_other_solves(ctx):
+    """The reduction's four CTAs exchange sums through each other's shared memory: solves of several threads
+    with contexts of their own, all at once, give the bits of a solve alone."""
+    import threading
+
+    n, workers = 150, 6
+    problems = [(_random_symmetric(n, 900 + i), O.conditioned_metric(n, 1e3, seed=950 + i)) for i in range(workers)]
+    alone = [vbcore.generalized_eigh(ctx, H, S) for H, S in problems]
+    wrong = []
+
+    def work(i):
+        own = vbcore.Context(0)
+        try:
+            for _ in range(10):
+                w, C = vbcore.generalized_eigh(own, *problems[i])
+                if not (np.array_equal(w, alone[i][0]) and np.array_equal(C, alone[i][1])):
+                    wrong.append(i)
+        except Exception as e:  # reported below: an exception in a thread does not fail the test
+            wrong.append((i, e))
+        finally:
+            own.close()
+
+    threads = [threading.Thread(target=work, args=(i,)) for i in range(workers)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not wrong

@@ -149,6 +149,7 @@ __global__ void __cluster_dims__(kReduceCtas, 1, 1) __launch_bounds__(32 * kRedu
     double x[kCols];  // row s
 #pragma unroll
     for (int j = 0; j < kCols; ++j) x[j] = lane + 32 * j < n ? __ldg(A + (long long)(lane + 32 * j) * n) : 0.0;
+    cluster.sync();  // no CTA writes to another one's shared memory before that one runs
     // one of five registers, without a dynamic index
     auto pick = [](int q, double y0, double y1, double y2, double y3, double y4) {
         return q < 2 ? (q == 0 ? y0 : y1) : (q == 2 ? y2 : (q == 3 ? y3 : y4));

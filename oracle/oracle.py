@@ -816,3 +816,84 @@ class VbscfOracle:
         res = scipy.optimize.minimize(fun, x0, jac=True, method="L-BFGS-B",
                                       options={"maxcor": 100, "gtol": gtol, "ftol": 1e-15, "maxiter": maxiter})
         return res.fun, unpack(res.x), res
+
+
+# ---- gradient of c^T (H - root S) c in extended precision ------------------------------------
+
+
+def _batched_inverse(X):
+    """Determinants and inverses of X[..., k, k] by Gauss-Jordan elimination with partial pivoting, in the
+    arrays' own type (no LAPACK: it has no extended precision)."""
+    k = X.shape[-1]
+    lead = X.shape[:-2]
+    A = np.concatenate([X, np.broadcast_to(np.eye(k, dtype=X.dtype), X.shape)], axis=-1).reshape(-1, k, 2 * k)
+    det = np.ones(len(A), dtype=X.dtype)
+    rows = np.arange(len(A))
+    for s in range(k):
+        p = s + np.argmax(np.abs(A[:, s:, s]), axis=1)
+        top = A[:, s].copy()
+        A[:, s] = A[rows, p]
+        A[rows, p] = top
+        pivot = A[:, s, s].copy()
+        det *= np.where(p == s, pivot, -pivot)
+        A[:, s] /= pivot[:, None]
+        factor = A[:, :, s].copy()
+        factor[:, s] = 0
+        A -= factor[:, :, None] * A[:, None, s]
+    return det.reshape(lead), A[:, :, k:].reshape(X.shape)
+
+
+def functional_gradient(n, expansion, S, h, F, c, root):
+    """Gradients of c^T (H - root S) c, at fixed c and root, with respect to S, h (symmetric) and the pair
+    factors F of the packed pair kernel K = F F^T: every block inverted by itself, in the platform's extended
+    precision (64-bit significands here).  Regular blocks only.  Formulas of the active-space backward files
+    (src/vbscf/derivatives/gradient/active_space/evaluator.cpp:1046-1133)."""
+    real = np.longdouble
+    S, h, F, c = (np.asarray(x, dtype=real) for x in (S, h, F, c))
+    pair = np.array([[pair_index(i, j) for j in range(n)] for i in range(n)]).reshape(-1)
+    K = (F @ F.T)[pair][:, pair]  # (ij|kl) as [n n, n n]
+    exchange = K.reshape(n, n, n, n).transpose(0, 3, 2, 1).reshape(n * n, n * n)
+    anti = K - exchange
+
+    def table(strings):
+        occ = np.array([_occ(int(s)) for s in strings])
+        N, k = occ.shape
+        X = S[occ[None, :, :, None], occ[:, None, None, :]]  # [u, v, row of v, column of u]
+        det, inv = _batched_inverse(X)
+        G = np.zeros((N, N, n, n), dtype=real)
+        u, v = np.meshgrid(np.arange(N), np.arange(N), indexing="ij")
+        for r in range(k):
+            for q in range(k):
+                G[u, v, occ[v, r], occ[u, q]] = inv[:, :, q, r]
+        G = G.reshape(N, N, n * n)
+        energy = G @ h.reshape(-1) + ((G @ anti) * G).sum(-1) / 2
+        return occ, det, inv, G, energy
+
+    ta, tb = table(expansion.alpha_strings), table(expansion.beta_strings)
+    W = np.zeros((len(ta[0]), len(tb[0])), dtype=real)
+    np.add.at(W, (expansion.det_alpha, expansion.det_beta), expansion.coefficient_matrix().astype(real) @ c)
+    gS, gh = np.zeros((n, n), dtype=real), np.zeros(n * n, dtype=real)
+    gK = np.zeros((n * n, n * n), dtype=real)
+    for own, other, w, first in ((ta, tb, W, True), (tb, ta, W.T, False)):
+        occ, det, inv, G, energy = own
+        N, k = occ.shape
+        aH = w @ other[1] @ w.T
+        aS = w @ (other[1] * other[4]) @ w.T - real(root) * aH
+        aA = (w @ (other[1][..., None] * other[3]).transpose(2, 0, 1) @ w.T).transpose(1, 2, 0)
+        if first:  # the opposite-spin energy holds K once
+            gK += np.einsum("uvp,uvq->pq", det[..., None] * G, aA)
+        aA = aA @ K
+        s = aS + aH * energy + (aA * G).sum(-1)
+        M = (aA + aH[..., None] * (h.reshape(-1) + G @ anti)).reshape(N, N, n, n)
+        u, v = np.meshgrid(np.arange(N), np.arange(N), indexing="ij")
+        local = M[u[..., None, None], v[..., None, None], occ[None, :, :, None], occ[:, None, None, :]]  # [u, v, r, q]
+        gX = det[..., None, None] * (s[..., None, None] * inv - inv @ local @ inv).transpose(0, 1, 3, 2)
+        np.add.at(gS, (np.broadcast_to(occ[None, :, :, None], gX.shape), np.broadcast_to(occ[:, None, None, :], gX.shape)), gX)
+        weight = aH * det
+        gh += (weight[..., None] * G).sum((0, 1))
+        same = np.einsum("uvp,uvq->pq", weight[..., None] * G, G) / 2
+        gK += same - same.reshape(n, n, n, n).transpose(0, 3, 2, 1).reshape(n * n, n * n)
+    gP = np.zeros((n * (n + 1) // 2,) * 2, dtype=real)
+    np.add.at(gP, (pair[:, None], pair[None, :]), gK)
+    gh = gh.reshape(n, n)
+    return {"S": (gS + gS.T) / 2, "h": (gh + gh.T) / 2, "ri": (gP + gP.T) @ F}

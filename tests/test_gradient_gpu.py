@@ -247,3 +247,45 @@ def test_frame_gradient_from_records_and_high_levels(ctx, kw, n, mult):
     for key in ("S", "h", "ri"):
         assert np.abs(a[key] - b[key]).max() < 1e-8 * max(1e-3, np.abs(b[key]).max()), key
     plan.close()
+
+
+def _nearly_dependent(n, separation, seed):
+    """Overlaps of orbitals close to orthogonal, but for the second one: the first one plus `separation` times
+    another."""
+    rng = np.random.default_rng(seed)
+    C = np.eye(n) + 0.05 * rng.standard_normal((n, n))
+    C[:, 1] = C[:, 0] + separation * C[:, 1]
+    S = C.T @ C
+    d = 1.0 / np.sqrt(np.diag(S))
+    return d[:, None] * S * d[None, :]
+
+
+@pytest.mark.parametrize("kw,n,nel,mult", [("COV", 6, 6, 1), ("COV ION(1)", 6, 6, 1), ("COV", 7, 7, 2), ("COV", 8, 8, 1)])
+@pytest.mark.parametrize("separation", [0.3, 0.1, 0.03, 0.01, 3e-3, 1e-3])
+def test_gradient_of_nearly_dependent_orbitals(ctx, kw, n, nel, mult, separation):
+    """Two nearly dependent orbitals: strings that hold both have an ill-conditioned S_LL (kappa up to 4e6).
+    Against every block inverted by itself in extended precision.  Bound: a block's 64-bit inverse enters its
+    derivative twice, against det X of order 1 / kappa, and leaves up to kappa^2 eps / 600 here (measured),
+    so kappa^2 eps / 256; the frame of such a string would leave kappa^2 eps / 50 and more.  5e-14 for what
+    does not depend on the dependent pair."""
+    S = _nearly_dependent(n, separation, n)
+    rng = np.random.default_rng(n)
+    h = _sym(rng, n)
+    P = n * (n + 1) // 2
+    F = 0.05 * rng.standard_normal((P, P)) + 0.1 * np.eye(P)
+    eri = workloads.pack_pair_kernel(F @ F.T)
+    plan = vbcore.HsPlan(ctx, vbcore.expand_structures(vbcore.generate_structures(kw, n, nel, mult), nel, mult), n)
+    ex = O.expand(O.generate_structures(kw, n, nel, mult), nel, mult)
+    c = rng.standard_normal(plan.n_structures)
+    c /= np.linalg.norm(c)
+    ref = O.functional_gradient(n, ex, S, h, F, c, -1.3)
+    kappa2 = 1.0
+    for strings in (ex.alpha_strings, ex.beta_strings):
+        occ = np.array([[i for i in range(n) if (s >> i) & 1] for s in strings])
+        X = S[occ[:, :, None], occ[:, None, :]]
+        kappa2 = max(kappa2, (np.linalg.norm(X, axis=(1, 2)) * np.linalg.norm(np.linalg.inv(X), axis=(1, 2))).max() ** 2)
+    got = plan.gradient(S, h, eri, c, -1.3, packed_eri=False, ri_factors=F)
+    for key in ("S", "h", "ri"):
+        err = float(np.abs(got[key] - ref[key]).max() / np.abs(ref[key]).max())
+        assert err < 5e-14 + 2.2e-16 * kappa2 / 256, (key, kappa2, err)
+    plan.close()

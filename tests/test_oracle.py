@@ -184,3 +184,31 @@ def test_ri_pair_factor_frame_restatement():
     a = O.ri_pair_factors_frame(O.ri_pair_factors_frame(B, Q), Q, 2, dB, K)
     b = O.ri_pair_factors_frame(B, Q, 1, dB, -Q @ K)
     assert np.abs(a - b).max() < 1e-12
+
+
+@pytest.mark.parametrize("kw,n,nel,mult", [("COV", 6, 6, 1), ("COV ION(1)", 5, 4, 1), ("COV", 7, 7, 2)])
+def test_extended_precision_gradient_matches_differences(kw, n, nel, mult):
+    """c^T (H - root S) c is a polynomial in every input; Richardson differences at 1e-3 leave 1e-9."""
+    rng = np.random.default_rng(n)
+    S = np.eye(n) + 0.1 * rng.standard_normal((n, n))
+    S = S.T @ S / n + np.eye(n)
+    h = rng.standard_normal((n, n))
+    h = h + h.T
+    P = n * (n + 1) // 2
+    F = 0.05 * rng.standard_normal((P, P)) + 0.1 * np.eye(P)
+    ex = O.expand(O.generate_structures(kw, n, nel, mult), nel, mult)
+    c = rng.standard_normal(ex.n_structures)
+
+    def value(S, h, F):
+        K = F @ F.T
+        H, Sm, _ = O.structure_matrices(n, ex, S, h, K[np.tril_indices(P)])
+        return c @ (H + 0.7 * Sm) @ c
+
+    g = O.functional_gradient(n, ex, S, h, F, c, -0.7)
+    dS, dh, dF = rng.standard_normal((n, n)), rng.standard_normal((n, n)), rng.standard_normal(F.shape)
+    dS, dh = dS + dS.T, dh + dh.T
+    for key, f, d in (("S", lambda t: value(S + t * dS, h, F), dS), ("h", lambda t: value(S, h + t * dh, F), dh),
+                      ("ri", lambda t: value(S, h, F + t * dF), dF)):
+        d1, d2 = (f(1e-3) - f(-1e-3)) / 2e-3, (f(5e-4) - f(-5e-4)) / 1e-3
+        fd = (4 * d2 - d1) / 3
+        assert abs(float((g[key] * d).sum()) - fd) < 1e-8 * max(1.0, abs(fd)), key

@@ -114,10 +114,18 @@ __device__ __forceinline__ bool frame_certificate(const View& f, const int (&hc)
     return isfinite(lhs) && det2 > 0.0 && lhs < kCertificate2 * det2;
 }
 
-// An uncertified pair is still evaluated here, by polynomials in the entries of B, when the frame is
-// sound: kappa_F(S_LL)^2 below this bound leaves P = S[:, L] S_LL^-1 with an error near 1e4 eps at
-// worst (of order eps for the near-orthogonal orbitals of a stretched geometry).
-constexpr double kFrameCondition2 = 1.0e8;
+// kappa_F(S_LL)^2 below which a left string's frame is sound.  Uncertified pairs are then still evaluated
+// in it, by polynomials in the entries of B (P = S[:, L] S_LL^-1 carries 0.03 kappa eps), and the gradient
+// takes the string's pairs through the reverse of its tables, which loses kappa^2 eps / 50: the adjoints are
+// multiplied by S_LL^-1 more than once.  Largest error of dE/dS for two nearly dependent orbitals, relative,
+// against the blocks inverted one by one (6 to 8 electrons, extended precision as the reference):
+//   kappa^2 = 3e3: 2e-15 against 6e-16, 1.4e4: 2e-15 against 2e-15, 2e5: 3e-13 against 3e-14, 2e7: 1e-10
+//   against 5e-13, 2e9: 4e-9 against 9e-11.
+// Hydrogen chains stay below 2.3e3 (14 atoms 0.7 A apart) and near-orthogonal orbitals below 60.
+constexpr double kFrameCondition2 = 1.0e4;
+// Strings from here on have all their pairs differentiated through singular values: the blocks' own
+// inverses lose 1e-7 of the gradient there.
+constexpr double kSingularCondition2 = 1.0e12;
 
 __host__ __device__ constexpr int pair_slot(int x, int y) { return x < y ? y * (y - 1) / 2 + x : x * (x - 1) / 2 + y; }
 // n-th element of {0, 1, ...} without i1 < i2

@@ -34,6 +34,8 @@ struct FrameAdjointArgs {
     unsigned long long* task_counter;   // zero
     unsigned long long* careful_count;  // zero; pairs left to the exact kernel
     unsigned long long* careful_list;
+    unsigned long long* unsound_count;  // zero; strings left to the pair-by-pair kernels (kFrameCondition2)
+    int* unsound;                       // n_strings
     double* out;      // n_strings blocks of frame_adjoint_block_doubles
     double* partial;  // kAdjointMaxParts x (np R + 2 n^2)
     double* gL;       // [pair * ld + m], added to

@@ -319,21 +319,24 @@ struct BackArgs {
     const double* lf;
     int ld;
     int R;
+    // adjoint rows: of every record, of the listed pairs (adj_listed) or, for spin_backward_kernel, of the
+    // chunk's items
     const double* adj;
     int adj_stride;
-    int adj_listed;  // 1: row i of adj belongs to listed pair i (else to the pair's record)
+    int adj_listed;
     double* gS;  // n x n (index as read: S[L_c n + R_r])
     double* gh;  // n x n
     double* gG;  // gd x gd, [anti(L pair) gd + anti(R pair)]
     double* gL;  // [pair q * ld + m]
     unsigned long long* careful_count;
     unsigned long long* careful_list;
-    // chunked fast path: items [item_begin, item_end) own records [record_base, ...)
+    // chunked fast path: items [item_begin, item_end), item i with the rows item_row[i] - row_base, ...
     const int2* items;
+    const long long* item_row;
     int item_begin, item_end;
-    long long record_base;
-    const double* Q;  // [record - record_base][np]: adj_u . l_m at each packed pair
-    double* Pout;     // [record - record_base][np]: A scattered onto packed pairs (zeroed)
+    long long row_base;
+    const double* Q;  // [row][np]: adj_u . l_m at each packed pair
+    double* Pout;     // [row][np]: A scattered onto packed pairs (zeroed)
 };
 
 template <int K>
@@ -386,9 +389,8 @@ __global__ void __launch_bounds__(128) spin_backward_kernel(BackArgs a) {
         }
         const long long v = (long long)it.y + threadIdx.x;
         if (v >= N) continue;
-        const long long t = record_index(u, v, N);
-        const long long tl = t - a.record_base;
-        const double* adj = a.adj + t * a.adj_stride;
+        const long long tl = a.item_row[item] - a.row_base + threadIdx.x;
+        const double* adj = a.adj + tl * a.adj_stride;
         const double aS = adj[a.R], aH = adj[a.R + 1];
         int Rr[K];
         {
@@ -586,28 +588,48 @@ __global__ void string_weights_kernel(int n_strings, const int* __restrict__ aof
     }
 }
 
-// Adjoint rows of the listed pairs from the partners' records (FrameAdjointArgs::weight), a warp per row.
+// Adjoint row of the pair (u, v), from the partners' record (FrameAdjointArgs::weight) or from the table.
+__device__ __forceinline__ void adjoint_row(const FrameAdjointArgs& f, int u, int v, int lane, double* __restrict__ out) {
+    if (!f.weight) {
+        const double* row = f.adj + record_index(u, v, f.n_strings) * f.adj_stride;
+        for (int m = lane; m < f.R + 2; m += 32) out[m] = __ldg(row + m);
+        return;
+    }
+    const int x = __ldg(f.partner + u), y = __ldg(f.partner + v);
+    const double* rec = f.records + record_index(min(x, y), max(x, y), f.n_strings) * f.rec_stride;
+    const double omega = (u == v ? 2.0 : 4.0) * __ldg(f.weight + u) * __ldg(f.weight + v);
+    for (int m = lane; m < f.R + 2; m += 32) {
+        double val;
+        if (m < f.R)
+            val = m < f.r_pos ? __ldg(rec + m) : -__ldg(rec + m);
+        else if (m == f.R)
+            val = __ldg(rec + f.R + 1) - f.lambda * __ldg(rec + f.R);
+        else
+            val = __ldg(rec + f.R);
+        out[m] = omega * val;
+    }
+}
+
+// Adjoint rows of the listed pairs, a warp per row.
 __global__ void __launch_bounds__(256) listed_adjoint_kernel(FrameAdjointArgs f, long long count, int stride,
                                                              double* __restrict__ out) {
     const int lane = threadIdx.x & 31;
     const long long nwarps = ((long long)gridDim.x * blockDim.x) >> 5;
     for (long long i = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < count; i += nwarps) {
         const unsigned long long w = f.careful_list[i];
-        const int u = (int)(w >> 32), v = (int)(w & 0xffffffffull);
-        const int x = __ldg(f.partner + u), y = __ldg(f.partner + v);
-        const double* rec = f.records + record_index(min(x, y), max(x, y), f.n_strings) * f.rec_stride;
-        const double omega = (u == v ? 2.0 : 4.0) * __ldg(f.weight + u) * __ldg(f.weight + v);
-        for (int m = lane; m < f.R + 2; m += 32) {
-            double val;
-            if (m < f.R)
-                val = m < f.r_pos ? __ldg(rec + m) : -__ldg(rec + m);
-            else if (m == f.R)
-                val = __ldg(rec + f.R + 1) - f.lambda * __ldg(rec + f.R);
-            else
-                val = __ldg(rec + f.R);
-            out[i * stride + m] = omega * val;
-        }
+        adjoint_row(f, (int)(w >> 32), (int)(w & 0xffffffffull), lane, out + i * stride);
     }
+}
+
+// Adjoint rows of the pairs of the items [begin, end), a block per item.
+__global__ void __launch_bounds__(256) item_adjoint_kernel(FrameAdjointArgs f, const int2* __restrict__ items,
+                                                           const long long* __restrict__ item_row, int begin,
+                                                           long long row_base, int stride, double* __restrict__ out) {
+    const int lane = threadIdx.x & 31, item = begin + blockIdx.x;
+    const int2 it = items[item];
+    const int rows = min(kSpinBlock, f.n_strings - it.y);
+    for (int r = threadIdx.x >> 5; r < rows; r += blockDim.x >> 5)
+        adjoint_row(f, it.x, it.y + r, lane, out + (item_row[item] - row_base + r) * stride);
 }
 
 // Product of the singular values outside the index set `skip` (bit mask).
@@ -1021,7 +1043,7 @@ extern "C" vb_status vb_hs_plan_gradient(vb_hs_plan* p, const double* S, const d
     int* bs = reinterpret_cast<int*>(ws + (direct ? p->Na : p->n_det));
     // blocks of the frame form for one spin table; without room for them (*got = false) the pair-by-pair
     // form works in chunks
-    DeviceBuffer blocks, sums;
+    DeviceBuffer blocks, sums, unsound;
     auto frame_blocks = [&](int beta, bool* got) -> vb_status {
         const int k = beta ? p->kb : p->ka;
         *got = false;
@@ -1029,7 +1051,11 @@ extern "C" vb_status vb_hs_plan_gradient(vb_hs_plan* p, const double* S, const d
         vb_status bst = blocks.allocate(ctx, sizeof(double) * frame_adjoint_block_doubles(n, k, R) * (beta ? p->Nb : p->Na));
         if (bst == VB_OK)
             bst = sums.allocate(ctx, sizeof(double) * kAdjointMaxParts * ((size_t)np * R + 2 * (size_t)n * n));
-        if (bst != VB_OK) blocks.release();
+        if (bst == VB_OK) bst = unsound.allocate(ctx, sizeof(int) * (size_t)(beta ? p->Nb : p->Na));
+        if (bst != VB_OK) {
+            blocks.release();
+            sums.release();
+        }
         *got = bst == VB_OK;
         return bst == VB_ERR_BUDGET ? VB_OK : bst;
     };
@@ -1114,9 +1140,80 @@ extern "C" vb_status vb_hs_plan_gradient(vb_hs_plan* p, const double* S, const d
         if (err != cudaSuccess) break;
         const bool fast = k <= 8 && frame_spin_supported(n, k, R);
         const DeviceBuffer& tables = beta ? p->tables_b : p->tables_a;
-        auto listed_pairs = [&](unsigned long long* listed) {
-            cudaError_t e = cudaMemcpyAsync(listed, b.careful_count, sizeof(*listed), cudaMemcpyDeviceToHost, s);
+        auto read_count = [&](const unsigned long long* from, unsigned long long* to) {
+            cudaError_t e = cudaMemcpyAsync(to, from, sizeof(*to), cudaMemcpyDeviceToHost, s);
             return e == cudaSuccess ? cudaStreamSynchronize(s) : e;
+        };
+        // Certified pairs of all left strings, or of the given ones (ascending), pair by pair; the others are
+        // listed.  Chunks of whole work items (left string u, right strings v0 .. v0 + 127): per chunk
+        // Q = L_f^T adj_U (the u-adjoint contracted with every factor column at every packed pair), the
+        // backward kernel (writes P = A scattered onto packed pairs), then gL += adj_U P^T -- the two
+        // contractions over the R factor columns as FP64 GEMMs.  Given strings: the chunk's adjoint rows are
+        // gathered first (f).
+        auto pair_by_pair = [&](const std::vector<int>* strings, const FrameAdjointArgs* f) -> vb_status {
+            const long long NN = b.N;
+            std::vector<int2> items;
+            std::vector<long long> rec_off;  // first row of each item, then the total
+            long long tot = 0;
+            for (long long i = 0; i < (strings ? (long long)strings->size() : NN); ++i)
+                for (long long u = strings ? (*strings)[i] : i, v0 = u; v0 < NN; v0 += kSpinBlock) {
+                    items.push_back(make_int2((int)u, (int)v0));
+                    rec_off.push_back(tot);
+                    tot += std::min<long long>(kSpinBlock, NN - v0);
+                }
+            rec_off.push_back(tot);
+            const long long cap = std::max<long long>(kSpinBlock, ((long long)256 << 20) / (8LL * np));
+            DeviceBuffer ditems, drows, qbuf, pbuf, abuf;
+            vb_status pst = upload(ctx, ditems, items.data(), sizeof(int2) * items.size());
+            const long long rows_max = std::min<long long>(cap + kSpinBlock, tot);
+            if (pst == VB_OK) pst = upload(ctx, drows, rec_off.data(), sizeof(long long) * rec_off.size());
+            if (pst == VB_OK) pst = qbuf.allocate(ctx, sizeof(double) * (size_t)np * rows_max);
+            if (pst == VB_OK) pst = pbuf.allocate(ctx, sizeof(double) * (size_t)np * rows_max);
+            if (pst == VB_OK && strings) pst = abuf.allocate(ctx, sizeof(double) * (size_t)adj_stride * rows_max);
+            if (pst != VB_OK) return pst;
+            BackArgs c = b;
+            c.items = ditems.as<int2>();
+            c.item_row = drows.as<long long>();
+            c.Q = qbuf.as<double>();
+            c.Pout = pbuf.as<double>();
+            cudaError_t e = cudaSuccess;
+            for (size_t i0 = 0; i0 < items.size() && e == cudaSuccess;) {
+                size_t i1 = i0;
+                while (i1 < items.size() && rec_off[i1 + 1] - rec_off[i0] <= cap) ++i1;
+                if (i1 == i0) ++i1;
+                const long long tb = rec_off[i0], rows = rec_off[i1] - tb;
+                if (strings) {
+                    item_adjoint_kernel<<<(unsigned)(i1 - i0), 256, 0, s>>>(*f, c.items, c.item_row, (int)i0, tb, adj_stride,
+                                                                           abuf.as<double>());
+                    e = cudaGetLastError();
+                    c.adj = abuf.as<double>();
+                } else {
+                    c.adj = b.adj + tb * adj_stride;
+                }
+                if (e == cudaSuccess)
+                    e = launch_factor_project(np, R, b.lf, np, c.adj, adj_stride, rows, qbuf.as<double>(), np, s);
+                if (e == cudaSuccess) e = cudaMemsetAsync(pbuf.ptr, 0, sizeof(double) * (size_t)np * rows, s);
+                if (e != cudaSuccess) break;
+                c.item_begin = (int)i0;
+                c.item_end = (int)i1;
+                c.row_base = tb;
+                switch (k) {
+                    case 1: e = launch_backward<1>(c, s); break;
+                    case 2: e = launch_backward<2>(c, s); break;
+                    case 3: e = launch_backward<3>(c, s); break;
+                    case 4: e = launch_backward<4>(c, s); break;
+                    case 5: e = launch_backward<5>(c, s); break;
+                    case 6: e = launch_backward<6>(c, s); break;
+                    case 7: e = launch_backward<7>(c, s); break;
+                    case 8: e = launch_backward<8>(c, s); break;
+                    default: break;
+                }
+                if (e == cudaSuccess)
+                    e = launch_factor_outer(np, R, c.adj, adj_stride, pbuf.as<double>(), np, rows, gL, np,
+                                            partial.as<double>(), s);
+                i0 = i1;
+            }
+            return e == cudaSuccess ? VB_OK : cuda_error(ctx, e, "vb_hs_plan_gradient (pair by pair)");
         };
         // the frame form (gradient_frame.cu) folds the same-spin two-electron energy into the factor
         // columns; a gradient per packed integral keeps its table separate (the map from factor
@@ -1156,11 +1253,26 @@ extern "C" vb_status vb_hs_plan_gradient(vb_hs_plan* p, const double* S, const d
             f.gL = gL;
             f.gS = gS;
             f.gh = gh;
+            f.unsound_count = p->counters.as<unsigned long long>() + 11 + beta;
+            f.unsound = unsound.as<int>();
             err = cudaMemsetAsync(f.task_counter, 0, sizeof(unsigned long long), s);
+            if (err == cudaSuccess) err = cudaMemsetAsync(f.unsound_count, 0, sizeof(unsigned long long), s);
             if (err == cudaSuccess) err = launch_frame_adjoint(f, s);
-            unsigned long long listed = 0;
-            if (err == cudaSuccess) err = listed_pairs(&listed);
+            unsigned long long left = 0, listed = 0;
+            if (err == cudaSuccess) err = cudaMemcpyAsync(&left, f.unsound_count, sizeof(left), cudaMemcpyDeviceToHost, s);
+            if (err == cudaSuccess) err = read_count(b.careful_count, &listed);
             if (err != cudaSuccess) break;
+            if (left > 0) {
+                std::vector<int> strings(left);
+                err = cudaMemcpyAsync(strings.data(), f.unsound, sizeof(int) * left, cudaMemcpyDeviceToHost, s);
+                if (err == cudaSuccess) err = cudaStreamSynchronize(s);
+                if (err != cudaSuccess) break;
+                std::sort(strings.begin(), strings.end());
+                blocks.release();
+                sums.release();
+                if ((st = pair_by_pair(&strings, &f)) != VB_OK) return st;
+                if ((err = read_count(b.careful_count, &listed)) != cudaSuccess) break;
+            }
             DeviceBuffer rows;
             if (from_records && listed > 0) {
                 if ((st = rows.allocate(ctx, sizeof(double) * adj_stride * listed)) != VB_OK) return st;
@@ -1171,62 +1283,9 @@ extern "C" vb_status vb_hs_plan_gradient(vb_hs_plan* p, const double* S, const d
             }
             if ((st = careful_chunks(ctx, b, (long long)listed, 0, partial.as<double>())) != VB_OK) return st;
         } else if (fast) {
-            // chunks of whole work items (left string u, right strings v0 .. v0 + 127): per chunk
-            // Q = L_f^T adj_U (the u-adjoint contracted with every factor column at every packed
-            // pair), the backward kernel (writes P = A scattered onto packed pairs), then
-            // gL += adj_U P^T -- the two contractions over the R factor columns as FP64 GEMMs
-            const long long NN = b.N;
-            std::vector<int2> items;
-            std::vector<long long> rec_off;  // first record of each item, then the total
-            long long tot = 0;
-            for (long long u = 0; u < NN; ++u)
-                for (long long v0 = u; v0 < NN; v0 += kSpinBlock) {
-                    items.push_back(make_int2((int)u, (int)v0));
-                    rec_off.push_back(tot);
-                    tot += std::min<long long>(kSpinBlock, NN - v0);
-                }
-            rec_off.push_back(tot);
-            const long long cap = std::max<long long>(kSpinBlock, ((long long)256 << 20) / (8LL * np));
-            DeviceBuffer ditems, qbuf, pbuf;
-            if ((st = upload(ctx, ditems, items.data(), sizeof(int2) * items.size())) != VB_OK) return st;
-            const long long rows_max = std::min<long long>(cap + kSpinBlock, tot);
-            if ((st = qbuf.allocate(ctx, sizeof(double) * (size_t)np * rows_max)) != VB_OK) return st;
-            if ((st = pbuf.allocate(ctx, sizeof(double) * (size_t)np * rows_max)) != VB_OK) return st;
-            b.items = ditems.as<int2>();
-            b.Q = qbuf.as<double>();
-            b.Pout = pbuf.as<double>();
-            for (size_t i0 = 0; i0 < items.size() && err == cudaSuccess;) {
-                size_t i1 = i0;
-                while (i1 < items.size() && rec_off[i1 + 1] - rec_off[i0] <= cap) ++i1;
-                if (i1 == i0) ++i1;
-                const long long tb = rec_off[i0], rows = rec_off[i1] - tb;
-                const double* A = b.adj + tb * adj_stride;
-                err = launch_factor_project(np, R, b.lf, np, A, adj_stride, rows, qbuf.as<double>(), np, s);
-                if (err == cudaSuccess) err = cudaMemsetAsync(pbuf.ptr, 0, sizeof(double) * (size_t)np * rows, s);
-                if (err != cudaSuccess) break;
-                b.item_begin = (int)i0;
-                b.item_end = (int)i1;
-                b.record_base = tb;
-                switch (k) {
-                    case 1: err = launch_backward<1>(b, s); break;
-                    case 2: err = launch_backward<2>(b, s); break;
-                    case 3: err = launch_backward<3>(b, s); break;
-                    case 4: err = launch_backward<4>(b, s); break;
-                    case 5: err = launch_backward<5>(b, s); break;
-                    case 6: err = launch_backward<6>(b, s); break;
-                    case 7: err = launch_backward<7>(b, s); break;
-                    case 8: err = launch_backward<8>(b, s); break;
-                    default: break;
-                }
-                if (err != cudaSuccess) break;
-                err = launch_factor_outer(np, R, A, adj_stride, pbuf.as<double>(), np, rows, gL, np,
-                                          partial.as<double>(), s);
-                if (err != cudaSuccess) break;
-                i0 = i1;
-            }
-            if (err != cudaSuccess) break;
+            if ((st = pair_by_pair(nullptr, nullptr)) != VB_OK) return st;
             unsigned long long listed = 0;
-            err = listed_pairs(&listed);
+            err = read_count(b.careful_count, &listed);
             if (err != cudaSuccess) break;
             if ((st = careful_chunks(ctx, b, (long long)listed, 0, partial.as<double>())) != VB_OK) return st;
         } else {
@@ -1236,6 +1295,7 @@ extern "C" vb_status vb_hs_plan_gradient(vb_hs_plan* p, const double* S, const d
         err = cudaGetLastError();
         blocks.release();
         sums.release();
+        unsound.release();
     }
     std::vector<double> hS(n_gS), hh(n_gS), hG(n_gG), hL(n_gL), hlf((size_t)np * np);
     if (err == cudaSuccess) err = cudaMemcpyAsync(hS.data(), gS, sizeof(double) * n_gS, cudaMemcpyDeviceToHost, s);

@@ -21,9 +21,9 @@
 //  * frame_tables_adjoint<K>: per left string, the reverse of frame_tables back to S, h and the
 //    factor columns, accumulated per CTA in shared memory; frame_adjoint_reduce sums the CTAs in a
 //    fixed order.
-// Uncertified pairs at levels E >= 6 (1.5 % of the pairs are at these levels at K = 7) and strings whose
-// S_LL is near singular are listed for the exact kernel of gradient.cu; certified ones take the inverse
-// of B.  When every alpha string carries one determinant (covalent singlets) and the list is spin-flip
+// Uncertified pairs at levels E >= 6 (1.5 % of the pairs are at these levels at K = 7) are listed for the
+// exact kernel of gradient.cu; certified ones take the inverse of B.  Strings outside kFrameCondition2 are
+// listed: their pairs take the pair-by-pair kernels (all the exact one outside kSingularCondition2).  When every alpha string carries one determinant (covalent singlets) and the list is spin-flip
 // symmetric, the adjoint of record (u, v) is the record of the partners' beta strings times one weight:
 // the rows w are then read from the records themselves, and no adjoint buffer is built or read (2.1 GB
 // at K = 7, 3.8 ms).  The pair-by-pair path takes the K x K inverse of every pair with C(K, 2)^2
@@ -44,10 +44,6 @@
 
 namespace vbcore {
 namespace {
-
-// kappa_F(S_LL)^2 above which a left string's pairs are listed: the frame's inverse then loses more
-// than the pair-by-pair inverse of the listed path.
-constexpr double kAdjointCondition2 = 1.0e12;
 
 // pairs whose adjoint rows are staged at a time (two stages of 8 MT doubles per pair)
 constexpr int stage_pairs(int MT) { return MT <= 6 ? 32 : 16; }
@@ -489,15 +485,19 @@ __global__ void __launch_bounds__(32 * (K + 1), 1) frame_backward_pairs(FrameAdj
         __threadfence();
         __syncthreads();
         const long long base = record_index(u, u, N);
-        const bool sound = blk[F.o_scal + 1] * blk[F.o_scal + 2] < kAdjointCondition2;
+        const double kappa2 = blk[F.o_scal + 1] * blk[F.o_scal + 2];
+        const bool sound = kappa2 < kFrameCondition2, invertible = kappa2 < kSingularCondition2;
         auto list = [&](int v) {
             const unsigned long long at = atomicAdd(a.careful_count, 1ull);
             a.careful_list[at] = ((unsigned long long)u << 32) | (unsigned long long)v;
         };
-        if (!sound)
-            for (int i = tid; i < bound[K + 1]; i += Shape::kThreads) list(__ldg(a.rlist + base + i));
         if (!sound) {
-            if (tid == 0) out[G.o_f + 1] = 0.0;
+            if (!invertible)
+                for (int i = tid; i < bound[K + 1]; i += Shape::kThreads) list(__ldg(a.rlist + base + i));
+            if (tid == 0) {
+                out[G.o_f + 1] = 0.0;
+                if (invertible) a.unsound[atomicAdd(a.unsound_count, 1ull)] = u;
+            }
             __syncthreads();
             continue;
         }
@@ -762,7 +762,7 @@ __global__ void __launch_bounds__(kAdjThreads) frame_tables_adjoint(FrameAdjoint
     for (long long u = blockIdx.x; u < a.n_strings; u += gridDim.x) {
         const double* tab = a.tables + u * F.total;
         const double* adj = a.out + u * G.total;
-        if (adj[G.o_f + 1] == 0.0) continue;  // uniform: the string's pairs were listed
+        if (adj[G.o_f + 1] == 0.0) continue;  // uniform: the string is not in the frame form
         __syncthreads();
         if (tid < 8) {
             const uint64_t w0 = __ldg(a.occ + 2 * u);

@@ -35,7 +35,7 @@ struct CovalentPlan {
     DeviceBuffer det, beta, list, desc, bounds, listed;
 };
 
-constexpr int kPlanCounters = 11;
+constexpr int kPlanCounters = 13;
 
 struct vb_hs_plan {
     vb_context* ctx = nullptr;
@@ -50,7 +50,8 @@ struct vb_hs_plan {
     long long npairs_a = 0, npairs_b = 0;
     // counters: [0, 1] listed (exact-path) spin pairs alpha/beta, [2, 3] the gradient's listed
     // pairs, [4, 5] the frame kernel's task counters alpha/beta, [7] the band reduction's
-    // timeout flag, [8, 9] pairs the frame kernel evaluated outside the certificate alpha/beta
+    // timeout flag, [8, 9] pairs the frame kernel evaluated outside the certificate alpha/beta,
+    // [10] listed covalent determinant pairs, [11, 12] the gradient's strings outside the frame form
     DeviceBuffer counters, list_a, list_b;
     // right strings of each left string bucketed by hole set (see SpinTableArgs::rlist)
     DeviceBuffer rlist_a, rlist_b, rdesc_a, rdesc_b, ebound_a, ebound_b;

@@ -334,6 +334,47 @@ def test_block_ordered_determinants_match_oracle(ctx, kw, n, nel, mult):
         assert abs(so[q] - ref) < 1e-11 * max(1.0, abs(ref))
 
 
+def _full_blocks(n, holders):
+    """An expansion over n orbitals whose determinants fill 8 x 8 blocks but for the diagonal: for each of
+    the last `holders` orbitals x, the alpha strings {x, c} and the beta strings (orbitals 0 .. 7 without e),
+    c != e; structures of one to three random determinants."""
+    rng = np.random.default_rng(n)
+    alpha = sorted((1 << (n - 1 - x)) | (1 << c) for x in range(holders) for c in range(8))
+    beta = sorted(0xFF ^ (1 << e) for e in range(8))
+    dets = sorted((i, k) for i, a in enumerate(alpha) for k, b in enumerate(beta) if bin(a & b).count("1") == 1)
+    per_det = [[] for _ in dets]
+    n_str = len(dets)
+    for I in range(n_str):
+        for d in {I, *rng.integers(0, len(dets), size=2).tolist()}:
+            per_det[d].append((I, float(rng.choice([-1.0, 1.0]))))
+    offsets = np.cumsum([0] + [len(t) for t in per_det]).astype(np.int64)
+    ts = np.array([t[0] for d in per_det for t in sorted(d)], dtype=np.int32)
+    tc = np.array([t[1] for d in per_det for t in sorted(d)])
+    da, db = (np.array([d[q] for d in dets], dtype=np.int32) for q in (0, 1))
+    ex = vbcore.Expansion(n_str, 2, 7, np.array(alpha, dtype=np.uint64), np.array(beta, dtype=np.uint64), da, db,
+                          offsets, ts, tc)
+    ref = O.Expansion(n_str, 2, 7, alpha, beta, da, db, offsets, ts, tc)
+    ref.det_alpha_occ, ref.det_beta_occ = ex.occupations(), ex.occupations(beta=True)
+    return ex, ref
+
+
+@pytest.mark.parametrize("n", [18, 19, 20])
+def test_block_ordered_lists_of_any_factor_rank(ctx, n):
+    """Full-rank pair kernels of 171, 190 and 210 columns: the records of a pair of 8 x 8 blocks fit shared
+    memory up to 186 columns (190 with 7 of 8 cells taken)."""
+    ex, ref = _full_blocks(n, 10)
+    S, h, _ = workloads.active_space(n, n, 40 + n)
+    P = n * (n + 1) // 2
+    B = 0.2 * np.random.default_rng(n).standard_normal((P, P))
+    eri = workloads.pack_pair_kernel(B @ B.T / P + 0.01 * np.eye(P))
+    plan = vbcore.HsPlan(ctx, ex, n)
+    H, So = plan.execute(S, h, eri)
+    assert plan.stats()["factor_columns"] == P
+    Hr, Sr, _ = O.structure_matrices(n, ref, S, h, eri, threads=8)
+    assert _rel(H, Hr) < REL and _rel(So, Sr) < REL
+    plan.close()
+
+
 @pytest.mark.parametrize("n,mult", [(4, 1), (5, 2), (6, 1), (6, 3), (7, 4), (8, 1), (9, 2), (10, 3), (11, 2), (12, 1), (13, 2)])
 @pytest.mark.parametrize("overlap", ["random", "orthogonal", "dependent"])
 def test_covalent_pairs_match_records(ctx, n, mult, overlap):

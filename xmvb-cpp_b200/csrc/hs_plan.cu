@@ -998,6 +998,7 @@ vb_status execute_impl(vb_hs_plan* p, const double* S, const double* h, const do
     }
     FullPairArgs fa = full_args(p);
     fa.flip = p->has_flip ? p->flip.as<int>() : nullptr;
+    const bool by_block = p->blocks.n > 0 && block_pairs_supported(p->blocks.max_a, p->blocks.max_b, p->blocks.max_dets, p->R);
     for (size_t band = 0; band + 1 < p->bands.size(); ++band) {
         const long long e0 = p->bands[band], e1 = p->bands[band + 1];
         const long long B = e1 - e0;
@@ -1019,9 +1020,9 @@ vb_status execute_impl(vb_hs_plan* p, const double* S, const double* h, const do
             if (cerr != cudaSuccess) return cuda_error(ctx, cerr, "spin_pairs exact");
         }
         PhaseMark pairs(p, VB_PHASE_DETERMINANT_PAIRS);
-        cudaError_t err = covalent         ? launch_listed_covalent_pairs(covalent_args(p, fa), fa, s, &launches)
-                          : p->blocks.n > 0 ? launch_block_pairs(block_args(p, fa), s, &launches)
-                                            : launch_full_pairs(fa, s, &launches);
+        cudaError_t err = covalent   ? launch_listed_covalent_pairs(covalent_args(p, fa), fa, s, &launches)
+                          : by_block ? launch_block_pairs(block_args(p, fa), s, &launches)
+                                     : launch_full_pairs(fa, s, &launches);
         if (err != cudaSuccess) return cuda_error(ctx, err, "full_pairs");
         pairs.close();
         PhaseMark reduce(p, VB_PHASE_BAND_REDUCE);

@@ -214,6 +214,9 @@ cudaError_t preload_frame_kernels();
 // kernel is otherwise loaded, and its code placed in device memory, at its first launch).
 cudaError_t preload_spin_pair_kernels();
 cudaError_t launch_full_pairs(const FullPairArgs& a, cudaStream_t stream, int* launches);
+// Records of a block pair and its determinant pairs fit shared memory at factor rank R (full 8 x 8 blocks:
+// up to R = 186, any kernel of 18 orbitals); lists of larger ones take launch_full_pairs.
+bool block_pairs_supported(int max_a, int max_b, int max_dets, int R);
 cudaError_t launch_block_pairs(const BlockPairArgs& a, cudaStream_t stream, int* launches);
 bool covalent_pairs_supported(int n, int ka, int kb, int R);
 cudaError_t launch_sort_covalent_pairs(const CovalentArgs& a, const uint64_t* occ, int* list, unsigned* desc, int* bounds,

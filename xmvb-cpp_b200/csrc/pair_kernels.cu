@@ -987,6 +987,11 @@ cudaError_t launch_full_pairs(const FullPairArgs& a, cudaStream_t stream, int* l
     return err;
 }
 
+bool block_pairs_supported(int max_a, int max_b, int max_dets, int R) {
+    // of the 227 KB a CTA may have, the kernel's static arrays take one
+    return block_pairs_smem(max_a, max_b, max_dets, R) <= 226 * 1024;
+}
+
 cudaError_t launch_block_pairs(const BlockPairArgs& a, cudaStream_t stream, int* launches) {
     const long long nh = a.h1 - a.h0, total = nh * a.h0 + nh * (nh + 1) / 2;
     if (total <= 0) return cudaSuccess;

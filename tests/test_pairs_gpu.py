@@ -375,6 +375,29 @@ def test_block_ordered_lists_of_any_factor_rank(ctx, n):
     plan.close()
 
 
+@pytest.mark.parametrize("n,mult,budget_mb", [(8, 1, 16), (8, 1, 24), (9, 2, 128), (10, 1, 400)])
+def test_block_ordered_determinants_in_bands(ctx, n, mult, budget_mb):
+    """Block-ordered lists over several bands of determinant columns (a small budget): bands end at block
+    boundaries, 65 to 512 columns and not multiples of 16 apart.  A column of the determinant matrix and its
+    sums do not depend on the band it is in: the bits of one band, and the oracle's matrices."""
+    S, h, eri = workloads.active_space(n, 2 * n, 30 + n)
+    plan, ex = _plan(ctx, "COV ION(1)", n, n, mult)
+    H, So = plan.execute(S, h, eri)
+    one = plan.stats()["kernel_launches"]
+    small = vbcore.Context(0, budget_mb << 20)
+    try:
+        banded, _ = _plan(small, "COV ION(1)", n, n, mult)
+        H2, S2 = banded.execute(S, h, eri)
+        assert banded.stats()["kernel_launches"] >= one + 4  # two kernels a band
+        assert np.array_equal(H, H2) and np.array_equal(So, S2)
+        banded.close()
+    finally:
+        small.close()
+    Hr, Sr, _ = O.structure_matrices(n, ex, S, h, eri, threads=8)
+    assert _rel(H2, Hr) < REL and _rel(S2, Sr) < REL
+    plan.close()
+
+
 @pytest.mark.parametrize("n,mult", [(4, 1), (5, 2), (6, 1), (6, 3), (7, 4), (8, 1), (9, 2), (10, 3), (11, 2), (12, 1), (13, 2)])
 @pytest.mark.parametrize("overlap", ["random", "orthogonal", "dependent"])
 def test_covalent_pairs_match_records(ctx, n, mult, overlap):

@@ -444,6 +444,32 @@ def test_covalent_pairs_match_records(ctx, n, mult, overlap):
     plan.close()
 
 
+@pytest.mark.parametrize("n,mult", [(4, 1), (6, 1), (7, 2), (8, 1), (8, 3), (10, 1), (12, 1)])
+def test_covalent_diagnostics_count_every_record_once(ctx, n, mult):
+    """careful_spin_pairs: with orthogonal orbitals every pair of different strings has a singular block.  With
+    two of them nearly dependent (kappa = 2e6) the strings that hold both list all their pairs, and with each
+    the record of the other spin, which alone would be evaluated; no record is counted for both."""
+    _, h, eri = workloads.active_space(n, 3 * n, 10 + n)
+    rows = vbcore.generate_structures("COV", n, n, mult)
+    ex = vbcore.expand_structures(rows, n, mult)
+    plan = vbcore.HsPlan(ctx, ex, n)
+    S = np.eye(n)
+    plan.execute(S, h, eri)
+    st = plan.stats()
+    tables = [ex.alpha_strings] if mult == 1 else [ex.alpha_strings, ex.beta_strings]
+    assert st["spin_pairs"] == sum(len(t) * (len(t) + 1) // 2 for t in tables)
+    assert st["careful_spin_pairs"] == sum(len(t) * (len(t) - 1) // 2 for t in tables)
+    S[0, 1] = S[1, 0] = 1.0 - 1e-6
+    plan.execute(S, h, eri)
+    singular = 0
+    for t in tables:
+        occ = [[i for i in range(n) if (int(s) >> i) & 1] for s in t]
+        singular += sum(np.linalg.det(S[np.ix_(occ[u], occ[v])]) == 0.0 for u in range(len(t)) for v in range(u, len(t))) \
+            if len(t) < 300 else 0
+    assert singular <= plan.stats()["careful_spin_pairs"] <= st["spin_pairs"]
+    plan.close()
+
+
 @pytest.mark.parametrize("n", [2, 3, 7, 8, 10, 11, 13, 14, 15, 16, 17])
 @pytest.mark.parametrize("kernel", ["definite", "indefinite", "low_rank", "tied"])
 def test_pair_kernel_factorization_sizes(ctx, n, kernel):

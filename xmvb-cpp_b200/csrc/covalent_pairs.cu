@@ -66,7 +66,7 @@ __device__ __forceinline__ unsigned excitation_parity(uint64_t mL, uint64_t mR) 
 
 // One warp per alpha string u: its partners v >= u (with flip, one of each orbit) by hole set, in order
 // of excitation level, then hole mask, then v.  Descriptor: hole mask, particle mask << 8, alpha parity
-// << 16, beta parity << 17.
+// << 16, beta parity << 17, and << 19 whether the orbit is its own flip (both spins hold the same record).
 constexpr int kSortWarps = 4;
 __global__ void __launch_bounds__(32 * kSortWarps) sort_covalent_pairs(CovalentArgs a, const uint64_t* __restrict__ occ,
                                                                        int* __restrict__ list, unsigned* __restrict__ desc,
@@ -92,6 +92,10 @@ __global__ void __launch_bounds__(32 * kSortWarps) sort_covalent_pairs(CovalentA
         int hm = 0;
         for (int c = 0; c < K; ++c) hm |= ((mR >> ((wL >> (8 * c)) & 0xFFu)) & 1ull) ? 0 : (1 << c);
         return hm;
+    };
+    auto own = [&](int v) -> unsigned {
+        const int y = __ldg(a.beta + v);
+        return a.fold && min(x, y) == u && max(x, y) == v;
     };
     for (int v0 = u; v0 < N; v0 += 32) {
         const int hm = holes(v0 + lane);
@@ -127,7 +131,7 @@ __global__ void __launch_bounds__(32 * kSortWarps) sort_covalent_pairs(CovalentA
             for (uint64_t p = mR & ~mL; p; p &= p - 1) pm |= 1u << __popcll(~mL & ((p & (~p + 1)) - 1));
             list[base + pos] = v;
             desc[base + pos] = (unsigned)hm | (pm << 8) | (excitation_parity(mL, mR) << 16) |
-                               (excitation_parity(all & ~mL, all & ~mR) << 17);
+                               (excitation_parity(all & ~mL, all & ~mR) << 17) | (own(v) << 19);
             if (lane == __ffs(same) - 1) cur[hm] += __popc(same);
         }
         __syncwarp();
@@ -252,8 +256,8 @@ __global__ void __launch_bounds__(32 * kCovalentMaxWarps, 1) covalent_pairs(Cova
             unsigned desc = d_next;
             if (e < 0) break;
             claim(&e_next, &cnt_next, &v_next, &d_next);
-            const unsigned hm = desc & 0xFFu;
-            if (beta) desc = ((desc >> 8) & 0xFFu) | (hm << 8) | ((desc >> 1) & 0x10000u);
+            const unsigned hm = desc & 0x800FFu;  // holes, and bit 19
+            if (beta) desc = ((desc >> 8) & 0xFFu) | ((desc & 0xFFu) << 8) | ((desc >> 1) & 0x10000u);
             const int slot = compact_slot(e);
             FramePair o{};
             o.hmap = o.pmap = 0xFFFFFFFFu;
@@ -261,7 +265,9 @@ __global__ void __launch_bounds__(32 * kCovalentMaxWarps, 1) covalent_pairs(Cova
             // slots of the alpha pairs, then of the beta pairs
             if (valid) o = frame_pair_dispatch<K>(e, view, desc, yw + ((lane & 15) + (beta ? covalent_chunk(e) : 0)) * slot);
             const unsigned okbits = __ballot_sync(0xffffffffu, o.ok), both = okbits & (okbits >> 16);
-            const unsigned poly = __ballot_sync(0xffffffffu, o.ok && !o.certified);
+            // pairs evaluated outside the certificate, every record once: listed ones are counted by the list,
+            // and an orbit that is its own flip holds one record
+            const unsigned poly = __ballot_sync(0xffffffffu, o.ok && !o.certified && !(beta && (hm >> 19))) & (both | (both << 16));
             if (lane == 0 && (poly & 0xFFFFu)) atomicAdd(a.uncertified_a, (unsigned long long)__popc(poly & 0xFFFFu));
             if (lane == 0 && (poly >> 16)) atomicAdd(a.uncertified_b, (unsigned long long)__popc(poly >> 16));
             if (valid && !beta && !((both >> lane) & 1u)) {
@@ -275,7 +281,7 @@ __global__ void __launch_bounds__(32 * kCovalentMaxWarps, 1) covalent_pairs(Cova
             const int tiles = (covalent_chunk(e) + 7) / 8;
 #pragma unroll 1
             for (int mt = 0; mt < tiles; ++mt) {
-                const unsigned uh = __reduce_or_sync(0xffffffffu, (lane >> 3) == mt ? hm : 0u);
+                const unsigned uh = __reduce_or_sync(0xffffffffu, (lane >> 3) == mt ? hm & 0xFFu : 0u);
                 if (((both >> (8 * mt)) & 0xFFu) == 0) continue;
                 const int owner = 8 * mt + g;
                 const double deta = __shfl_sync(0xffffffffu, o.detb, owner), detb = __shfl_sync(0xffffffffu, o.detb, owner + 16);

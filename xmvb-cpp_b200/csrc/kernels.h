@@ -78,7 +78,7 @@ struct CovalentArgs {
     const int* beta;
     const double* tables_a;
     const double* tables_b;
-    const int* list;        // as SpinTableArgs::rlist, rdesc (with the beta parity << 17), ebound
+    const int* list;        // as SpinTableArgs::rlist, rdesc (with the beta parity << 17, own flip << 19), ebound
     const unsigned* desc;
     const int* bounds;
     double* Hb;             // upper triangle, row stride ldb

@@ -375,6 +375,26 @@ def test_block_ordered_lists_of_any_factor_rank(ctx, n):
     plan.close()
 
 
+@pytest.mark.parametrize("n,mult,budget_mb", [(8, 1, 0), (9, 2, 128), (10, 1, 0)])
+def test_block_ordered_lists_with_the_tiled_reduction(ctx, n, mult, budget_mb):
+    """Every term given twice with half its coefficient: the dense groups do not take repeated terms, so block
+    pairs feed the tiled reduction, over one band and several."""
+    S, h, eri = workloads.active_space(n, 2 * n, 50 + n)
+    ref = O.expand(O.generate_structures("COV ION(1)", n, n, mult), n, mult)
+    ex = vbcore.expand_structures(vbcore.generate_structures("COV ION(1)", n, n, mult), n, mult)
+    ex.term_offsets = 2 * ex.term_offsets
+    ex.term_structure = np.repeat(ex.term_structure, 2)
+    ex.term_coefficient = 0.5 * np.repeat(ex.term_coefficient, 2)
+    own = vbcore.Context(0, budget_mb << 20) if budget_mb else ctx
+    plan = vbcore.HsPlan(own, ex, n)
+    H, So = plan.execute(S, h, eri)
+    Hr, Sr, _ = O.structure_matrices(n, ref, S, h, eri, threads=8)
+    assert _rel(H, Hr) < REL and _rel(So, Sr) < REL
+    plan.close()
+    if budget_mb:
+        own.close()
+
+
 @pytest.mark.parametrize("n,mult,budget_mb", [(8, 1, 16), (8, 1, 24), (9, 2, 128), (10, 1, 400)])
 def test_block_ordered_determinants_in_bands(ctx, n, mult, budget_mb):
     """Block-ordered lists over several bands of determinant columns (a small budget): bands end at block

@@ -10,12 +10,11 @@
 // (src/vbscf/structures/assembly/hamiltonian_overlap.hpp:70-107 in the reference).
 #include <algorithm>
 #include <cstring>
-#include <map>
 #include <new>
-#include <set>
 #include <string>
 #include <vector>
 
+#include "determinant_order.h"
 #include "device_algebra.cuh"
 #include "internal.h"
 #include "kernels.h"
@@ -97,185 +96,6 @@ struct PhaseMark {
     }
     ~PhaseMark() { close(); }
 };
-
-// Blocks of (at most 8 alpha strings) x (at most 8 beta strings) that the determinant list fills (see
-// BlockPairArgs); block h holds determinants first[h] .. first[h + 1] - 1 of the new order.
-struct DeterminantBlocks {
-    int n = 0, max_a = 0, max_b = 0, max_dets = 0;
-    std::vector<int> first;
-    std::vector<BlockStrings> strings;
-};
-
-// Determinants with the same alpha-only orbitals (alpha minus beta) pair a set of alpha strings with a
-// set of beta strings: for singly ionic structures X + {d} with the complement of X minus {e}, every
-// d != e, n - |X| strings of each spin.  Determinants alone in their set (the covalent ones, d = e)
-// join a set that holds both their strings.  Sets are cut into blocks; the blocks are taken when they
-// are dense enough that the padding of their pair products stays below the gathers they replace (40 %
-// filled, ten determinants per block on average) and the list is not tiny.
-bool determinant_blocks(const vb_expansion& ex, DeterminantBlocks* out, std::vector<long long>* order) {
-    const long long nd = ex.n_determinants;
-    if (nd < 512 || ex.n_alpha_strings >= 0xFFFF || ex.n_beta_strings >= 0xFFFF) return false;
-    std::map<uint64_t, std::vector<long long>> sets;
-    for (long long d = 0; d < nd; ++d)
-        sets[ex.alpha_strings[ex.det_alpha[d]] & ~ex.beta_strings[ex.det_beta[d]]].push_back(d);
-    if ((long long)sets.size() > nd / 4) {
-        // covalent lists: every determinant alone
-        long long alone = 0;
-        for (const auto& s : sets) alone += s.second.size() == 1;
-        if (2 * alone > nd) return false;
-    }
-    std::vector<std::vector<long long>> groups;
-    std::vector<long long> singles;
-    for (auto& s : sets) {
-        if (s.second.size() == 1)
-            singles.push_back(s.second[0]);
-        else
-            groups.push_back(std::move(s.second));
-    }
-    std::vector<std::vector<int>> with_alpha(ex.n_alpha_strings);  // groups that hold an alpha string
-    std::vector<std::set<int>> betas(groups.size());
-    for (size_t g = 0; g < groups.size(); ++g) {
-        std::set<int> a;
-        for (long long d : groups[g]) {
-            a.insert(ex.det_alpha[d]);
-            betas[g].insert(ex.det_beta[d]);
-        }
-        for (int x : a) with_alpha[x].push_back((int)g);
-    }
-    for (long long d : singles) {
-        int best = -1;
-        for (int g : with_alpha[ex.det_alpha[d]])
-            if (betas[g].count(ex.det_beta[d]) && (best < 0 || groups[g].size() < groups[best].size())) best = g;
-        if (best >= 0)
-            groups[best].push_back(d);
-        else
-            groups.push_back({d});
-    }
-    DeterminantBlocks b;
-    std::vector<long long> sorted;
-    long long cells = 0;
-    int max_a = 0, max_b = 0;
-    b.first.push_back(0);
-    for (auto& g : groups) {
-        std::vector<int> as, bs;
-        for (long long d : g) {
-            as.push_back(ex.det_alpha[d]);
-            bs.push_back(ex.det_beta[d]);
-        }
-        for (std::vector<int>* v : {&as, &bs}) {
-            std::sort(v->begin(), v->end());
-            v->erase(std::unique(v->begin(), v->end()), v->end());
-        }
-        std::map<std::pair<int, int>, long long> at;
-        for (long long d : g)
-            if (!at.emplace(std::make_pair(ex.det_alpha[d], ex.det_beta[d]), d).second) return false;  // repeated
-        // chunks of nearly equal size
-        const int ca = ((int)as.size() + 7) / 8, cb = ((int)bs.size() + 7) / 8;
-        for (int x = 0; x < ca; ++x)
-            for (int y = 0; y < cb; ++y) {
-                const int a0 = (int)as.size() * x / ca, a1 = (int)as.size() * (x + 1) / ca;
-                const int b0 = (int)bs.size() * y / cb, b1 = (int)bs.size() * (y + 1) / cb;
-                BlockStrings block;
-                std::memset(&block, 0xFF, sizeof(block));
-                int count = 0;
-                for (int i = a0; i < a1; ++i)
-                    for (int k = b0; k < b1; ++k) {
-                        const auto it = at.find({as[i], bs[k]});
-                        if (it == at.end()) continue;
-                        block.cell[8 * (i - a0) + k - b0] = (unsigned char)count++;
-                        sorted.push_back(it->second);
-                    }
-                if (count == 0) continue;
-                block.n_alpha = (unsigned char)(a1 - a0);
-                block.n_beta = (unsigned char)(b1 - b0);
-                for (int i = a0; i < a1; ++i) block.alpha[i - a0] = (uint16_t)as[i];
-                for (int k = b0; k < b1; ++k) block.beta[k - b0] = (uint16_t)bs[k];
-                cells += (long long)(a1 - a0) * (b1 - b0);
-                max_a = std::max(max_a, a1 - a0);
-                max_b = std::max(max_b, b1 - b0);
-                b.max_dets = std::max(b.max_dets, count);
-                b.strings.push_back(block);
-                b.first.push_back((int)sorted.size());
-                ++b.n;
-            }
-    }
-    b.max_a = max_a * max_a;
-    b.max_b = max_b * max_b;
-    if ((long long)sorted.size() != nd || 5 * nd < 2 * cells || nd < 10LL * b.n) return false;
-    *out = std::move(b);
-    *order = std::move(sorted);
-    return true;
-}
-
-// Structure groups whose rows fit shared memory together (BandReduceArgs::groups): up to kDenseStructures
-// structures and kDenseRows rows.  Structures with the same doubly occupied and empty orbitals share their
-// determinants, so they are taken one after the other: order[i] is the caller's index of structure i, and
-// off, coef and term_row list the terms in this order.
-struct ResidentGroups {
-    std::vector<int4> groups;
-    std::vector<int> rows, order;
-    std::vector<long long> off;
-    std::vector<double> coef;
-    std::vector<unsigned short> term_row;
-    int max_rows = 0;
-};
-
-// false where a structure alone has too many rows, or where the groups together read the rows so often
-// (four times each on average) that the tiled form, whose groups always hold kBandGroup structures, reads
-// less.
-bool resident_groups(const vb_expansion& ex, int n_str, const std::vector<long long>& off, const std::vector<long long>& det,
-                     const std::vector<double>& coef, ResidentGroups* out) {
-    ResidentGroups r;
-    std::vector<std::pair<uint64_t, uint64_t>> key(n_str);  // doubly occupied, occupied orbitals
-    for (int I = 0; I < n_str; ++I)
-        if (off[I] < off[I + 1]) {
-            const uint64_t a = ex.alpha_strings[ex.det_alpha[det[off[I]]]], b = ex.beta_strings[ex.det_beta[det[off[I]]]];
-            key[I] = {a & b, a | b};
-        }
-    r.order.resize(n_str);
-    for (int i = 0; i < n_str; ++i) r.order[i] = i;
-    std::stable_sort(r.order.begin(), r.order.end(), [&](int x, int y) { return key[x] < key[y]; });
-    std::vector<int> owner(ex.n_determinants, -1);  // group that last took the determinant
-    r.off.push_back(0);
-    for (int i0 = 0; i0 < n_str;) {
-        const int g = (int)r.groups.size();
-        std::vector<int> used;
-        int i1 = i0;
-        for (; i1 < n_str && i1 - i0 < kDenseStructures; ++i1) {
-            const int I = r.order[i1];
-            const size_t before = used.size();
-            for (long long t = off[I]; t < off[I + 1]; ++t) {
-                if (t > off[I] && det[t] == det[t - 1]) return false;  // one coefficient per structure and determinant
-                if (owner[det[t]] != g) {
-                    owner[det[t]] = g;
-                    used.push_back((int)det[t]);
-                }
-            }
-            if (used.size() > (size_t)kDenseRows) {
-                if (i1 == i0) return false;
-                used.resize(before);
-                break;
-            }
-        }
-        std::sort(used.begin(), used.end());
-        for (int i = i0; i < i1; ++i) {
-            const int I = r.order[i];
-            for (long long t = off[I]; t < off[I + 1]; ++t) {
-                r.term_row.push_back(
-                    (unsigned short)(std::lower_bound(used.begin(), used.end(), (int)det[t]) - used.begin()));
-                r.coef.push_back(coef[t]);
-            }
-            r.off.push_back((long long)r.coef.size());
-        }
-        r.groups.push_back(make_int4((int)r.rows.size(), (int)used.size(), i0, i1 - i0));
-        r.rows.insert(r.rows.end(), used.begin(), used.end());
-        r.max_rows = std::max(r.max_rows, (int)used.size());
-        i0 = i1;
-    }
-    if ((long long)r.rows.size() > 4 * ex.n_determinants) return false;
-    *out = std::move(r);
-    return true;
-}
 
 vb_status upload_blocks(vb_hs_plan* p, const DeterminantBlocks& b) {
     vb_status st = upload(p->ctx, p->blocks.first, b.first.data(), sizeof(int) * b.first.size());
@@ -450,53 +270,20 @@ vb_status vb_hs_plan_create(vb_context* ctx, const vb_expansion* ex, vb_hs_plan*
         if (ex->term_structure[t] < 0 || ex->term_structure[t] >= p->n_str)
             return fail(set_error(ctx, VB_ERR_INVALID, "term structure index out of range"));
 
-    // Determinant order.  Lists whose determinants fill blocks of (alpha strings) x (beta strings) are
-    // ordered by block (determinant_blocks): the pair kernel then works on whole blocks and the band
-    // reduction gathers the rows of each structure group.  Otherwise: structures that share few
-    // determinants (ionic structures: determinants cluster by occupation pattern) leave each
-    // band-reduction structure group reading a row tile
-    // for a handful of its rows.  Placing every determinant at the first structure that uses it
-    // makes the determinants of consecutive structures contiguous; the reorder is taken when it at
-    // least halves the (structure group, row tile) segments.  Everything the plan computes is per
-    // structure or per spin string, so only vb_hs_plan_determinant_pairs translates indices.
-    DeterminantBlocks blocks;
+    // Determinant order (determinant_order.h).  Everything the plan computes is per structure or per spin
+    // string, so only vb_hs_plan_determinant_pairs translates indices.
+    DeterminantOrder chosen = determinant_order(*ex);
+    const DeterminantBlocks& blocks = chosen.blocks;
     std::vector<int32_t> r_alpha, r_beta, r_str;
     std::vector<int64_t> r_off;
     std::vector<double> r_coef;
     vb_expansion reordered;
     {
         const long long nd = p->n_det;
-        std::vector<long long> order(nd);
-        for (long long d = 0; d < nd; ++d) order[d] = d;
-        const bool by_block = p->ka > 0 && p->kb > 0 && determinant_blocks(*ex, &blocks, &order);
-        if (!by_block) {
-            std::vector<long long> first(nd, (long long)p->n_str);
-            for (long long d = 0; d < nd; ++d)
-                for (long long t = ex->term_offsets[d]; t < ex->term_offsets[d + 1]; ++t)
-                    first[d] = std::min<long long>(first[d], ex->term_structure[t]);
-            // within a structure group's range, determinants stay in alpha-major order (the spin-pair
-            // records of neighbouring determinant pairs stay neighbours)
-            std::stable_sort(order.begin(), order.end(), [&](long long x, long long y) {
-                const long long gx = first[x] / kBandGroup, gy = first[y] / kBandGroup;
-                if (gx != gy) return gx < gy;
-                if (ex->det_alpha[x] != ex->det_alpha[y]) return ex->det_alpha[x] < ex->det_alpha[y];
-                return ex->det_beta[x] < ex->det_beta[y];
-            });
-        }
-        std::vector<long long> pos(nd);
-        for (long long i = 0; i < nd; ++i) pos[order[i]] = i;
-        const long long tiles = (nd + kBandTileRows - 1) / kBandTileRows;
-        auto segments = [&](bool moved) {
-            std::vector<long long> keys;
-            keys.reserve((size_t)n_terms);
-            for (long long d = 0; d < nd; ++d)
-                for (long long t = ex->term_offsets[d]; t < ex->term_offsets[d + 1]; ++t)
-                    keys.push_back((long long)(ex->term_structure[t] / kBandGroup) * tiles +
-                                   (moved ? pos[d] : d) / kBandTileRows);
-            std::sort(keys.begin(), keys.end());
-            return (long long)(std::unique(keys.begin(), keys.end()) - keys.begin());
-        };
-        if (by_block || 2 * segments(true) <= segments(false)) {
+        const std::vector<long long>& order = chosen.order;
+        if (!order.empty()) {
+            std::vector<long long> pos(nd);
+            for (long long i = 0; i < nd; ++i) pos[order[i]] = i;
             r_alpha.resize(nd);
             r_beta.resize(nd);
             r_off.assign(nd + 1, 0);
@@ -676,17 +463,8 @@ vb_status vb_hs_plan_create(vb_context* ctx, const vb_expansion* ex, vb_hs_plan*
         if ((st = b->allocate(ctx, wbytes)) != VB_OK) return fail(st);
 
     // structure-major incidence (CSC of T)
-    std::vector<long long> soff(p->n_str + 1, 0);
-    for (long long t = 0; t < n_terms; ++t) ++soff[ex->term_structure[t] + 1];
-    for (int I = 0; I < p->n_str; ++I) soff[I + 1] += soff[I];
-    std::vector<long long> sdet(n_terms), next(soff.begin(), soff.end() - 1);
-    std::vector<double> scoef(n_terms);
-    for (long long d = 0; d < p->n_det; ++d)
-        for (long long t = ex->term_offsets[d]; t < ex->term_offsets[d + 1]; ++t) {
-            const long long pos = next[ex->term_structure[t]]++;
-            sdet[pos] = d;
-            scoef[pos] = ex->term_coefficient[t];
-        }
+    const std::vector<long long>&soff = chosen.terms.off, &sdet = chosen.terms.det;
+    const std::vector<double>& scoef = chosen.terms.coef;
     if ((st = upload(ctx, p->str_off, soff.data(), sizeof(long long) * soff.size())) != VB_OK) return fail(st);
     if ((st = upload(ctx, p->str_det, sdet.data(), sizeof(long long) * std::max<size_t>(1, sdet.size()))) != VB_OK)
         return fail(st);
@@ -697,12 +475,13 @@ vb_status vb_hs_plan_create(vb_context* ctx, const vb_expansion* ex, vb_hs_plan*
     // tile, coefficient) of the group's structures ordered by (warp, slot, determinant).  The tiles of
     // a group are its 64-row tiles of the determinant list that hold terms.  Lists ordered by blocks
     // take groups whose rows fit shared memory together, where they can be formed.
-    ResidentGroups resident;
-    if (blocks.n > 0 && resident_groups(*ex, p->n_str, soff, sdet, scoef, &resident)) {
+    const ResidentGroups& resident = chosen.groups;
+    if (!resident.groups.empty()) {
         BandSegments& b = p->segments;
+        static_assert(sizeof(RowGroup) == sizeof(int4), "a group as the kernel reads it");
         b.n_groups = (int)resident.groups.size();
         b.group_rows = resident.max_rows;
-        if ((st = upload(ctx, b.groups, resident.groups.data(), sizeof(int4) * resident.groups.size())) != VB_OK ||
+        if ((st = upload(ctx, b.groups, resident.groups.data(), sizeof(RowGroup) * resident.groups.size())) != VB_OK ||
             (st = upload(ctx, b.rows, resident.rows.data(), sizeof(int) * resident.rows.size())) != VB_OK ||
             (st = upload(ctx, b.order, resident.order.data(), sizeof(int) * resident.order.size())) != VB_OK ||
             (st = upload(ctx, b.off, resident.off.data(), sizeof(long long) * resident.off.size())) != VB_OK ||

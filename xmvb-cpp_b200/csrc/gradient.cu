@@ -1043,15 +1043,17 @@ extern "C" vb_status vb_hs_plan_gradient(vb_hs_plan* p, const double* S, const d
     int* bs = reinterpret_cast<int*>(ws + (direct ? p->Na : p->n_det));
     // blocks of the frame form for one spin table; without room for them (*got = false) the pair-by-pair
     // form works in chunks
-    DeviceBuffer blocks, sums, unsound;
+    DeviceBuffer blocks, sums;
+    auto block_doubles = [&](int k, long long N) { return frame_adjoint_block_doubles(n, k, R) * (size_t)N; };
     auto frame_blocks = [&](int beta, bool* got) -> vb_status {
         const int k = beta ? p->kb : p->ka;
         *got = false;
         if (deri_out || !(beta ? p->tables_b : p->tables_a).ptr || !frame_adjoint_supported(n, k, R)) return VB_OK;
-        vb_status bst = blocks.allocate(ctx, sizeof(double) * frame_adjoint_block_doubles(n, k, R) * (beta ? p->Nb : p->Na));
+        const long long N = beta ? p->Nb : p->Na;
+        // the strings' blocks, then the list of those outside the frame form
+        vb_status bst = blocks.allocate(ctx, sizeof(double) * block_doubles(k, N) + sizeof(int) * (size_t)N);
         if (bst == VB_OK)
             bst = sums.allocate(ctx, sizeof(double) * kAdjointMaxParts * ((size_t)np * R + 2 * (size_t)n * n));
-        if (bst == VB_OK) bst = unsound.allocate(ctx, sizeof(int) * (size_t)(beta ? p->Nb : p->Na));
         if (bst != VB_OK) {
             blocks.release();
             sums.release();
@@ -1134,14 +1136,16 @@ extern "C" vb_status vb_hs_plan_gradient(vb_hs_plan* p, const double* S, const d
         b.gh = gh;
         b.gG = gG;
         b.gL = gL;
-        b.careful_count = p->counters.as<unsigned long long>() + 2 + beta;
+        // counters: listed pairs, strings outside the frame form, the frame kernel's task counter
+        b.careful_count = p->counters.as<unsigned long long>() + 11 + 3 * beta;
         b.careful_list = beta ? p->list_b.as<unsigned long long>() : p->list_a.as<unsigned long long>();
-        err = cudaMemsetAsync(b.careful_count, 0, sizeof(unsigned long long), s);
+        err = cudaMemsetAsync(b.careful_count, 0, 3 * sizeof(unsigned long long), s);
         if (err != cudaSuccess) break;
         const bool fast = k <= 8 && frame_spin_supported(n, k, R);
         const DeviceBuffer& tables = beta ? p->tables_b : p->tables_a;
-        auto read_count = [&](const unsigned long long* from, unsigned long long* to) {
-            cudaError_t e = cudaMemcpyAsync(to, from, sizeof(*to), cudaMemcpyDeviceToHost, s);
+        unsigned long long counts[2] = {0, 0};  // listed pairs, strings outside the frame form
+        auto read_counts = [&] {
+            cudaError_t e = cudaMemcpyAsync(counts, b.careful_count, sizeof(counts), cudaMemcpyDeviceToHost, s);
             return e == cudaSuccess ? cudaStreamSynchronize(s) : e;
         };
         // Certified pairs of all left strings, or of the given ones (ascending), pair by pair; the others are
@@ -1245,7 +1249,6 @@ extern "C" vb_status vb_hs_plan_gradient(vb_hs_plan* p, const double* S, const d
                 f.rec_stride = record_stride(R);
                 f.lambda = eigenvalue;
             }
-            f.task_counter = p->counters.as<unsigned long long>() + 4 + beta;
             f.careful_count = b.careful_count;
             f.careful_list = b.careful_list;
             f.out = blocks.as<double>();
@@ -1253,41 +1256,38 @@ extern "C" vb_status vb_hs_plan_gradient(vb_hs_plan* p, const double* S, const d
             f.gL = gL;
             f.gS = gS;
             f.gh = gh;
-            f.unsound_count = p->counters.as<unsigned long long>() + 11 + beta;
-            f.unsound = unsound.as<int>();
-            err = cudaMemsetAsync(f.task_counter, 0, sizeof(unsigned long long), s);
-            if (err == cudaSuccess) err = cudaMemsetAsync(f.unsound_count, 0, sizeof(unsigned long long), s);
-            if (err == cudaSuccess) err = launch_frame_adjoint(f, s);
-            unsigned long long left = 0, listed = 0;
-            if (err == cudaSuccess) err = cudaMemcpyAsync(&left, f.unsound_count, sizeof(left), cudaMemcpyDeviceToHost, s);
-            if (err == cudaSuccess) err = read_count(b.careful_count, &listed);
+            f.unsound_count = b.careful_count + 1;
+            f.task_counter = b.careful_count + 2;
+            f.unsound = reinterpret_cast<int*>(f.out + block_doubles(k, b.N));
+            err = launch_frame_adjoint(f, s);
+            if (err == cudaSuccess) err = read_counts();
             if (err != cudaSuccess) break;
-            if (left > 0) {
-                std::vector<int> strings(left);
-                err = cudaMemcpyAsync(strings.data(), f.unsound, sizeof(int) * left, cudaMemcpyDeviceToHost, s);
+            if (counts[1] > 0) {
+                std::vector<int> strings(counts[1]);
+                err = cudaMemcpyAsync(strings.data(), f.unsound, sizeof(int) * strings.size(), cudaMemcpyDeviceToHost, s);
                 if (err == cudaSuccess) err = cudaStreamSynchronize(s);
                 if (err != cudaSuccess) break;
                 std::sort(strings.begin(), strings.end());
                 blocks.release();
                 sums.release();
                 if ((st = pair_by_pair(&strings, &f)) != VB_OK) return st;
-                if ((err = read_count(b.careful_count, &listed)) != cudaSuccess) break;
+                if ((err = read_counts()) != cudaSuccess) break;
             }
+            const long long listed = (long long)counts[0];
             DeviceBuffer rows;
             if (from_records && listed > 0) {
                 if ((st = rows.allocate(ctx, sizeof(double) * adj_stride * listed)) != VB_OK) return st;
-                listed_adjoint_kernel<<<148 * 8, 256, 0, s>>>(f, (long long)listed, adj_stride, rows.as<double>());
+                listed_adjoint_kernel<<<148 * 8, 256, 0, s>>>(f, listed, adj_stride, rows.as<double>());
                 if ((err = cudaGetLastError()) != cudaSuccess) break;
                 b.adj = rows.as<double>();
                 b.adj_listed = 1;
             }
-            if ((st = careful_chunks(ctx, b, (long long)listed, 0, partial.as<double>())) != VB_OK) return st;
+            if ((st = careful_chunks(ctx, b, listed, 0, partial.as<double>())) != VB_OK) return st;
         } else if (fast) {
             if ((st = pair_by_pair(nullptr, nullptr)) != VB_OK) return st;
-            unsigned long long listed = 0;
-            err = read_count(b.careful_count, &listed);
+            err = read_counts();
             if (err != cudaSuccess) break;
-            if ((st = careful_chunks(ctx, b, (long long)listed, 0, partial.as<double>())) != VB_OK) return st;
+            if ((st = careful_chunks(ctx, b, (long long)counts[0], 0, partial.as<double>())) != VB_OK) return st;
         } else {
             const long long NN = b.N;
             if ((st = careful_chunks(ctx, b, NN * (NN + 1) / 2, 1, partial.as<double>())) != VB_OK) return st;
@@ -1295,7 +1295,6 @@ extern "C" vb_status vb_hs_plan_gradient(vb_hs_plan* p, const double* S, const d
         err = cudaGetLastError();
         blocks.release();
         sums.release();
-        unsound.release();
     }
     std::vector<double> hS(n_gS), hh(n_gS), hG(n_gG), hL(n_gL), hlf((size_t)np * np);
     if (err == cudaSuccess) err = cudaMemcpyAsync(hS.data(), gS, sizeof(double) * n_gS, cudaMemcpyDeviceToHost, s);

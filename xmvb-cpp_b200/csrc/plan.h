@@ -35,7 +35,7 @@ struct CovalentPlan {
     DeviceBuffer det, beta, list, desc, bounds, listed;
 };
 
-constexpr int kPlanCounters = 13;
+constexpr int kPlanCounters = 17;
 
 struct vb_hs_plan {
     vb_context* ctx = nullptr;
@@ -48,10 +48,10 @@ struct vb_hs_plan {
     DeviceBuffer rec_a, rec_b, tables_a, tables_b;
     int stride_a = 0, stride_b = 0;
     long long npairs_a = 0, npairs_b = 0;
-    // counters: [0, 1] listed (exact-path) spin pairs alpha/beta, [2, 3] the gradient's listed
-    // pairs, [4, 5] the frame kernel's task counters alpha/beta, [7] the band reduction's
+    // counters: [0, 1] listed (exact-path) spin pairs alpha/beta, [4, 5] the frame kernel's task counters alpha/beta, [7] the band reduction's
     // timeout flag, [8, 9] pairs the frame kernel evaluated outside the certificate alpha/beta,
-    // [10] listed covalent determinant pairs, [11, 12] the gradient's strings outside the frame form
+    // [10] listed covalent determinant pairs, [11 .. 13, 14 .. 16] the gradient's listed pairs, strings
+    // outside the frame form and task counter alpha/beta
     DeviceBuffer counters, list_a, list_b;
     // right strings of each left string bucketed by hole set (see SpinTableArgs::rlist)
     DeviceBuffer rlist_a, rlist_b, rdesc_a, rdesc_b, ebound_a, ebound_b;

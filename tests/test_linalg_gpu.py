@@ -277,3 +277,15 @@ def test_tridiagonal_eigh_beside_other_solves(ctx):
     for t in threads:
         t.join()
     assert not wrong
+
+
+@pytest.mark.parametrize("n", [33, 100, 160])
+@pytest.mark.parametrize("power", [-1000, -700, -520, 500, 600])
+def test_tridiagonal_eigh_at_any_scale(ctx, n, power):
+    """H scaled by a power of two: the same vectors and scaled roots, to the bit (squares of the elements leave
+    the range of the exponent from 2^-511 and 2^511 on)."""
+    H = _random_symmetric(n, n)
+    S = O.conditioned_metric(n, 1e3, seed=n)
+    w, C = vbcore.generalized_eigh(ctx, H, S)
+    w2, C2 = vbcore.generalized_eigh(ctx, np.ldexp(H, power), S)
+    assert np.array_equal(w2, np.ldexp(w, power)) and np.array_equal(C, C2)

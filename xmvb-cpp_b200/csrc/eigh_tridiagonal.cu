@@ -128,7 +128,9 @@ __global__ void __launch_bounds__(32) td_product(int n, const double* __restrict
 // that takes row s to e[s] e_{s+1}; every warp forms v and the scalars itself (from the same values in
 // the same order), p = A v and the next row before its update go to all four CTAs' shared memory,
 // one cluster barrier, then A -= v w^T + w v^T with w = tau p - (tau^2 v^T p / 2) v, and every warp
-// updates the next row for itself.  Bound by the chain of n steps (barrier, two warp sums, a square
+// updates the next row for itself.  The matrix is scaled by a power of two to a largest element in [1, 2)
+// (squares neither overflow nor vanish at any scale of H); diag and off are left scaled, the exponent goes
+// to tau[n].  Bound by the chain of n steps (barrier, two warp sums, a square
 // root, two divisions): 222 us at n = 132, 555 us in one CTA of 20 warps, where the matrix spilled.
 __global__ void __cluster_dims__(kReduceCtas, 1, 1) __launch_bounds__(32 * kReduceWarps, 1)
     td_reduce(int n, const double* __restrict__ A, double* __restrict__ diag, double* __restrict__ off,
@@ -149,7 +151,28 @@ __global__ void __cluster_dims__(kReduceCtas, 1, 1) __launch_bounds__(32 * kRedu
     double x[kCols];  // row s
 #pragma unroll
     for (int j = 0; j < kCols; ++j) x[j] = lane + 32 * j < n ? __ldg(A + (long long)(lane + 32 * j) * n) : 0.0;
-    cluster.sync();  // no CTA writes to another one's shared memory before that one runs
+    double big = 0.0;
+#pragma unroll
+    for (int i = 0; i < kCols; ++i)
+#pragma unroll
+        for (int j = 0; j < kCols; ++j) big = fmax(big, fabs(a[i][j]));
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) big = fmax(big, __shfl_xor_sync(0xffffffffu, big, o));
+    __shared__ double s_big[kReduceWarps];
+    if (lane == 0) s_big[threadIdx.x >> 5] = big;
+    cluster.sync();  // no CTA addresses another one's shared memory before that one runs
+    for (int i = lane; i < kReduceCtas * kReduceWarps; i += 32)
+        big = fmax(big, cluster.map_shared_rank(s_big, i / kReduceWarps)[i % kReduceWarps]);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) big = fmax(big, __shfl_xor_sync(0xffffffffu, big, o));
+    const int exponent = big > 0.0 && isfinite(big) ? ilogb(big) : 0;
+#pragma unroll
+    for (int j = 0; j < kCols; ++j) {
+        x[j] = scalbn(x[j], -exponent);
+#pragma unroll
+        for (int i = 0; i < kCols; ++i) a[i][j] = scalbn(a[i][j], -exponent);
+    }
+    if (base == 0 && lane == 0) tau_out[n] = (double)exponent;
     // one of five registers, without a dynamic index
     auto pick = [](int q, double y0, double y1, double y2, double y3, double y4) {
         return q < 2 ? (q == 0 ? y0 : y1) : (q == 2 ? y2 : (q == 3 ? y3 : y4));
@@ -281,6 +304,7 @@ __global__ void __launch_bounds__(32) td_vectors(int n, const double* __restrict
         hi = fmax(hi, __shfl_xor_sync(0xffffffffu, hi, o));
     }
     const double norm = fmax(fmax(fabs(lo), fabs(hi)), 1e-280);
+    const int exponent = (int)__ldg(tau + n);
     const double inv = 1.0 / norm;
     for (int i = lane; i < n; i += 32) {
         sd[i] *= inv;
@@ -328,8 +352,8 @@ __global__ void __launch_bounds__(32) td_vectors(int n, const double* __restrict
     }
     const double lambda = 0.5 * (lo + hi);
     if (lane == 0) {
-        values[j] = lambda * norm;
-        if (j == 0) *norm_out = norm;
+        values[j] = scalbn(lambda * norm, exponent);
+        if (j == 0) *norm_out = scalbn(norm, exponent);
         const double tiny = 2.3e-16;
         auto away = [&](double v) { return fabs(v) < tiny ? (v < 0.0 ? -tiny : tiny) : v; };
         double cd = sd[0] - lambda, ce = se[0];

@@ -490,6 +490,28 @@ def test_covalent_diagnostics_count_every_record_once(ctx, n, mult):
     plan.close()
 
 
+@pytest.mark.parametrize("n,mult", [(8, 1), (10, 1), (10, 3), (11, 2), (12, 1)])
+def test_covalent_pairs_list_only_the_side_that_fails(ctx, n, mult):
+    """Two nearly dependent orbitals: a string that holds both leaves its uncertified pairs to the exact path,
+    the complement's record is evaluated in its own frame.  No more records outside the certificate than the
+    records path has (its frames are those of the lower string of every pair: 10 %), where listing both sides
+    gave nearly twice as many."""
+    rng = np.random.default_rng(n)
+    C = np.eye(n) + 0.05 * rng.standard_normal((n, n))
+    C[:, 1] = C[:, 0] + 2e-3 * C[:, 1]
+    S = C.T @ C
+    d = 1.0 / np.sqrt(np.diag(S))
+    S = d[:, None] * S * d[None, :]
+    _, h, eri = workloads.active_space(n, 3 * n, 90 + n)
+    plan, _ = _plan(ctx, "COV", n, n, mult)
+    plan.execute(S, h, eri)
+    covalent = plan.stats()["careful_spin_pairs"]
+    plan.determinant_pairs(S, h, eri, np.array([[0, 0]]))
+    records = plan.stats()["careful_spin_pairs"]
+    assert records > 0 and covalent <= 1.1 * records + 10
+    plan.close()
+
+
 @pytest.mark.parametrize("n", [2, 3, 7, 8, 10, 11, 13, 14, 15, 16, 17])
 @pytest.mark.parametrize("kernel", ["definite", "indefinite", "low_rank", "tied"])
 def test_pair_kernel_factorization_sizes(ctx, n, kernel):

@@ -14,9 +14,10 @@
 // hole set are also the beta side's particle set and both products walk the same k-steps.
 //
 // With spin-flip symmetry one member of each orbit {(d, e), (flip d, flip e)} is evaluated and written to
-// both places.  Pairs of which either side cannot be evaluated here (near-singular S_LL, or uncertified
-// at a level above five) are listed: both records go to the exact path, and listed_covalent_pairs
-// combines them.
+// both places.  Pairs of which a side cannot be evaluated here (uncertified in an ill-conditioned frame or at
+// a level above five) are listed: that side's record goes to the exact path, and listed_covalent_pairs
+// evaluates the other side and combines them.  (Both records in the exact path, 14 orbitals of which two
+// are nearly dependent: 520,853 of them in 8.7 ms, against 291,373 and 6.2 ms for the records alone.)
 //
 // 14 orbitals, 2.9 M orbits: 1361 us (1428 us with a test per row tile in the product), against 1280 us for the records and 537 us for the pairs gathered
 // from them; 12-orbital triplet: 160 us, against 235 us.  Bound by instruction issue (50 %) and the FP64
@@ -158,6 +159,17 @@ __device__ __forceinline__ void covalent_store(const CovalentArgs& a, int u, int
     }
 }
 
+// Appends the values of the lanes that have one, with one atomic per warp (all lanes call).
+__device__ __forceinline__ void append(unsigned long long* list, unsigned long long* count, bool has,
+                                       unsigned long long value, int lane) {
+    const unsigned mask = __ballot_sync(0xffffffffu, has);
+    if (mask == 0) return;
+    unsigned long long at = 0;
+    if (lane == 0) at = atomicAdd(count, (unsigned long long)__popc(mask));
+    at = __shfl_sync(0xffffffffu, at, 0);
+    if (has) list[at + __popc(mask & ((1u << lane) - 1u))] = value;
+}
+
 // Doubles of a block from Q on.
 __host__ __device__ inline int covalent_rest(const FrameLayout& F) { return F.total - F.o_q; }
 
@@ -265,17 +277,23 @@ __global__ void __launch_bounds__(32 * kCovalentMaxWarps, 1) covalent_pairs(Cova
             // slots of the alpha pairs, then of the beta pairs
             if (valid) o = frame_pair_dispatch<K>(e, view, desc, yw + ((lane & 15) + (beta ? covalent_chunk(e) : 0)) * slot);
             const unsigned okbits = __ballot_sync(0xffffffffu, o.ok), both = okbits & (okbits >> 16);
-            // pairs evaluated outside the certificate, every record once: listed ones are counted by the list,
-            // and an orbit that is its own flip holds one record
-            const unsigned poly = __ballot_sync(0xffffffffu, o.ok && !o.certified && !(beta && (hm >> 19))) & (both | (both << 16));
+            // pairs evaluated outside the certificate, every record once (an orbit that is its own flip holds
+            // one, listed unless both sides are evaluated)
+            const unsigned poly = __ballot_sync(
+                0xffffffffu, o.ok && !o.certified && (!(hm >> 19) || (!beta && ((both >> lane) & 1u))));
             if (lane == 0 && (poly & 0xFFFFu)) atomicAdd(a.uncertified_a, (unsigned long long)__popc(poly & 0xFFFFu));
             if (lane == 0 && (poly >> 16)) atomicAdd(a.uncertified_b, (unsigned long long)__popc(poly >> 16));
-            if (valid && !beta && !((both >> lane) & 1u)) {
-                a.listed[atomicAdd(a.listed_count, 1ull)] = ((unsigned long long)u << 32) | (unsigned long long)v;
-                a.list_a[atomicAdd(a.count_a, 1ull)] = ((unsigned long long)u << 32) | (unsigned long long)v;
-                const int x = __ldg(a.beta + u), y = __ldg(a.beta + v), lo = min(x, y), hi = max(x, y);
-                if (!a.fold || lo != u || hi != v)
-                    a.list_b[atomicAdd(a.count_b, 1ull)] = ((unsigned long long)lo << 32) | (unsigned long long)hi;
+            const unsigned fail = __ballot_sync(0xffffffffu, valid) & ~both & 0xFFFFu;
+            if (fail) {
+                // bit 0: alpha evaluated in its frame, bit 1: beta
+                const unsigned sides = hm >> 19 ? 0u : ((okbits >> (lane & 15)) & 1u) | ((okbits >> (15 + (lane & 15))) & 2u);
+                const bool mine = (fail >> lane) & 1u;
+                const unsigned long long pair = ((unsigned long long)u << 32) | (unsigned long long)v;
+                const int x = __ldg(a.beta + u), y = __ldg(a.beta + v);
+                append(a.listed, a.listed_count, mine, pair | ((unsigned long long)sides << 30), lane);
+                append(a.list_a, a.count_a, mine && !(sides & 1u), pair, lane);
+                append(a.list_b, a.count_b, mine && !(sides & 2u) && !(hm >> 19),
+                       ((unsigned long long)min(x, y) << 32) | (unsigned long long)max(x, y), lane);
             }
             __syncwarp();
             const int tiles = (covalent_chunk(e) + 7) / 8;
@@ -366,14 +384,108 @@ __global__ void __launch_bounds__(32 * kCovalentMaxWarps, 1) covalent_pairs(Cova
     }
 }
 
-__global__ void __launch_bounds__(128) listed_covalent_pairs(CovalentArgs a, FullPairArgs f) {
-    const long long count = (long long)*a.listed_count;
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < count; i += (long long)gridDim.x * blockDim.x) {
-        const unsigned long long w = a.listed[i];
-        const int u = (int)(w >> 32), v = (int)(w & 0xffffffffull);
-        double H, S;
-        pair_value(f, __ldg(a.det + u), __ldg(a.det + v), &H, &S);
-        covalent_store(a, u, v, H, S);
+// Listed pairs: a warp takes up to 32 of them.  A lane per pair runs the algebra of the side that is evaluated
+// in its frame (read from the tables in place), then the warp forms that side's u-vector row by row, lanes
+// over rows, against the other side's record; without such a side it multiplies the two records.
+constexpr int kListedWarps = 4;
+// doubles of a pair's adj B (odd stride)
+__host__ __device__ inline int listed_slot(int ka) { return (ka * ka) | 1; }
+
+__global__ void __launch_bounds__(32 * kListedWarps, 3) listed_covalent_pairs(CovalentArgs a, FullPairArgs f) {
+    extern __shared__ __align__(16) double smem[];
+    const long long count = (long long)*a.listed_count, N = a.n_strings;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, R = a.R;
+    const long long nwarps = (long long)gridDim.x * kListedWarps;
+    long long chunk = (count + nwarps - 1) / nwarps;
+    chunk = chunk < 1 ? 1 : (chunk > 32 ? 32 : chunk);
+    const FrameLayout FA = frame_layout(a.n, a.ka, R), FB = frame_layout(a.n, a.kb, R);
+    const uint64_t all = a.n >= 64 ? ~0ull : (1ull << a.n) - 1;
+    const int slot = listed_slot(a.ka);
+    double* slots = smem + (size_t)warp * 32 * slot;
+    for (long long base = ((long long)blockIdx.x * kListedWarps + warp) * chunk; base < count; base += nwarps * chunk) {
+        const int cnt = (int)(count - base < chunk ? count - base : chunk);
+        const unsigned long long w = lane < cnt ? a.listed[base + lane] : 0ull;
+        const int u = (int)(w >> 32), v = (int)(w & 0x3fffffffull);
+        const unsigned sides = (unsigned)(w >> 30) & 3u;
+        const bool beta = sides & 2u;
+        unsigned desc = 0;
+        FramePair o{};
+        if (sides) {
+            const uint64_t wL = __ldg(a.occ + 2 * (long long)u), mL = occ_mask(wL, a.ka);
+            const uint64_t mR = occ_mask(__ldg(a.occ + 2 * (long long)v), a.ka);
+            unsigned hm = 0, pm = 0;
+            for (uint64_t h = mL & ~mR; h; h &= h - 1) hm |= 1u << __popcll(mL & ((h & (~h + 1)) - 1));
+            for (uint64_t p = mR & ~mL; p; p &= p - 1) pm |= 1u << __popcll(~mL & ((p & (~p + 1)) - 1));
+            desc = beta ? pm | (hm << 8) | (excitation_parity(all & ~mL, all & ~mR) << 16)
+                        : hm | (pm << 8) | (excitation_parity(mL, mR) << 16);
+            const FrameLayout& F = beta ? FB : FA;
+            const double* blk = beta ? a.tables_b + (long long)__ldg(a.beta + u) * F.total : a.tables_a + (long long)u * F.total;
+            const FrameViewAny view{blk + F.o_q, beta ? a.kb : a.ka, F.o_p - F.o_q, F.o_rowsq - F.o_q, F.o_prow2 - F.o_q,
+                                    F.o_scal - F.o_q};
+            o = frame_pair_dispatch<8>(__popc(desc & 0xFFu), view, desc, slots + lane * slot);
+        }
+        __syncwarp();
+        for (int j = 0; j < cnt; ++j) {
+            const int uj = __shfl_sync(0xffffffffu, u, j), vj = __shfl_sync(0xffffffffu, v, j);
+            const unsigned sj = __shfl_sync(0xffffffffu, sides, j), dj = __shfl_sync(0xffffffffu, desc, j);
+            const double d = __shfl_sync(0xffffffffu, o.d, j), detb = __shfl_sync(0xffffffffu, o.detb, j);
+            const double quad = __shfl_sync(0xffffffffu, o.quad, j);
+            const int x = __ldg(a.beta + uj), y = __ldg(a.beta + vj);
+            const double* ra = f.rec_a + record_index(uj, vj, N) * f.stride_a;
+            const double* rb = f.rec_b + record_index(min(x, y), max(x, y), N) * f.stride_b;
+            const FrameLayout& F = sj & 2u ? FB : FA;
+            const double* blk = sj & 2u ? a.tables_b + (long long)x * F.total : a.tables_a + (long long)uj * F.total;
+            const int k = sj & 2u ? a.kb : a.ka;
+            const double* rec = sj & 1u ? rb : ra;  // a side of the exact path
+            double dot = 0.0, energy = 0.0;         // energy: h and two-electron linear rows
+            if (sj) {
+                // rows r0 + lane and r0 + lane + 32 of the frame side's table, a hole's block of eight columns
+                // at a time (the adj B of columns without a particle is zero)
+                const unsigned pm = (dj >> 8) & 0xFFu;
+                const int e = __popc(pm);
+                for (int r0 = 0; r0 < R + 2; r0 += 64) {
+                    const int ra0 = min(r0 + lane, R + 1), ra1 = min(r0 + lane + 32, R + 1);
+                    const double *t0 = blk + (long long)ra0 * F.kfs, *t1 = blk + (long long)ra1 * F.kfs;
+                    double v0 = detb * __ldg(t0 + 8 * k), v1 = detb * __ldg(t1 + 8 * k);
+                    const double* yj = slots + j * slot;
+#pragma unroll 1
+                    for (unsigned h = dj & 0xFFu; h; h &= h - 1, yj += e) {
+                        const int c = 8 * (__ffs(h) - 1);
+                        const double2 *b0 = reinterpret_cast<const double2*>(t0 + c), *b1 = reinterpret_cast<const double2*>(t1 + c);
+                        double2 x0[4], x1[4];
+#pragma unroll
+                        for (int q = 0; q < 4; ++q) {
+                            x0[q] = __ldg(b0 + q);
+                            x1[q] = __ldg(b1 + q);
+                        }
+#pragma unroll
+                        for (int b = 0; b < 8; ++b) {
+                            const double y = (pm >> b) & 1u ? yj[__popc(pm & ((1u << b) - 1u))] : 0.0;
+                            v0 = fma(y, b & 1 ? x0[b / 2].y : x0[b / 2].x, v0);
+                            v1 = fma(y, b & 1 ? x1[b / 2].y : x1[b / 2].x, v1);
+                        }
+                    }
+#pragma unroll
+                    for (int q = 0; q < 2; ++q) {
+                        const int r = r0 + lane + 32 * q, m = r - 2;
+                        const double v = d * (q ? v1 : v0);
+                        if (r < 2) energy = v;
+                        if (m >= 0 && m < R) dot = fma(m < a.r_pos ? v : -v, rec[m], dot);
+                    }
+                }
+            } else {
+                for (int m = lane; m < R; m += 32) dot = fma(m < a.r_pos ? ra[m] : -ra[m], rb[m], dot);
+            }
+#pragma unroll
+            for (int s = 16; s > 0; s >>= 1) dot += __shfl_xor_sync(0xffffffffu, dot, s);
+            energy += __shfl_xor_sync(0xffffffffu, energy, 1);
+            if (lane == 0) {
+                const double s1 = rec[R], h1 = rec[R + 1];
+                const double s2 = sj ? d * detb : rb[R], h2 = sj ? fma(d, quad, energy) : rb[R + 1];
+                covalent_store(a, uj, vj, fma(h1, s2, fma(h2, s1, dot)), s1 * s2);
+            }
+        }
+        __syncwarp();
     }
 }
 
@@ -449,7 +561,12 @@ cudaError_t launch_covalent_pairs(const CovalentArgs& a, cudaStream_t stream, in
 }
 
 cudaError_t launch_listed_covalent_pairs(const CovalentArgs& a, const FullPairArgs& f, cudaStream_t stream, int* launches) {
-    listed_covalent_pairs<<<kSms, 128, 0, stream>>>(a, f);
+    const size_t smem = sizeof(double) * kListedWarps * 32 * listed_slot(a.ka);
+    const cudaError_t err = allow_dynamic_smem((const void*)listed_covalent_pairs, smem);
+    if (err != cudaSuccess) return err;
+    // at most a warp per four pairs of the table: the list is usually empty
+    const long long pairs = (long long)a.n_strings * (a.n_strings + 1) / 2, grid = (pairs + 4 * kListedWarps - 1) / (4 * kListedWarps);
+    listed_covalent_pairs<<<(unsigned)(grid < 3 * kSms ? grid : 3 * kSms), 32 * kListedWarps, smem, stream>>>(a, f);
     ++*launches;
     return cudaGetLastError();
 }

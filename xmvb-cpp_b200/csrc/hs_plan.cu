@@ -173,6 +173,7 @@ CovalentArgs covalent_args(const vb_hs_plan* p, const FullPairArgs& f) {
     a.R = p->R;
     a.r_pos = p->r_pos;
     a.fold = p->shared_tables;
+    a.occ = p->occ_a.as<uint64_t>();
     a.det = c.det.as<int>();
     a.beta = c.beta.as<int>();
     a.tables_a = p->tables_a.as<double>();

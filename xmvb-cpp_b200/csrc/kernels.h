@@ -74,6 +74,7 @@ struct CovalentArgs {
     int n_strings;      // of alpha; the beta table has as many
     int R, r_pos;
     bool fold;          // one table for both spins and a spin-flip symmetric list: one pair per orbit is listed
+    const uint64_t* occ;  // alpha strings, as SpinTableArgs::occ
     const int* det;
     const int* beta;
     const double* tables_a;
@@ -87,7 +88,9 @@ struct CovalentArgs {
     unsigned long long* task_counter;                 // zero
     unsigned long long *uncertified_a, *uncertified_b;
     unsigned long long *count_a, *count_b, *list_a, *list_b;  // records for the exact path (as careful_list)
-    unsigned long long *listed_count, *listed;        // and their determinant pairs, (u << 32) | v
+    // determinant pairs with a record of the exact path: (u << 32) | v, bits 30 and 31 set where the alpha
+    // or beta record is evaluated in its frame
+    unsigned long long *listed_count, *listed;
 };
 
 // Determinant pairs of one band by blocks of the determinant list: block h holds determinants

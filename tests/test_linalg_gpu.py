@@ -289,3 +289,39 @@ def test_tridiagonal_eigh_at_any_scale(ctx, n, power):
     w, C = vbcore.generalized_eigh(ctx, H, S)
     w2, C2 = vbcore.generalized_eigh(ctx, np.ldexp(H, power), S)
     assert np.array_equal(w2, np.ldexp(w, power)) and np.array_equal(C, C2)
+
+
+def test_problems_the_tridiagonal_path_does_not_settle(ctx):
+    """33 <= n <= 160 take a path without a grid barrier; what it does not settle (here a NaN in H) goes on to the
+    block Jacobi, whose barrier gives up under a limit of one poll.  Vectors may lie over H: they are not
+    written before everything is settled, so that Jacobi finds H as it was."""
+    import ctypes
+
+    import torch
+
+    n = 120
+    c = vbcore.Context(0)
+    lib = vbcore.load_library()
+    try:
+        c.set_barrier_spin_limit(1)
+        H = _random_symmetric(n, 3)
+        S = O.conditioned_metric(n, 1e3, seed=4)
+        wr, Cr = vbcore.generalized_eigh(c, H, S)
+        for spoilt in (False, True):
+            Hd = torch.tensor(H, device="cuda")
+            if spoilt:
+                Hd[5, 3] = Hd[3, 5] = float("nan")
+            before = Hd.cpu().numpy().copy()
+            Sd, w = torch.tensor(S, device="cuda"), torch.empty(n, dtype=torch.float64, device="cuda")
+            info = ctypes.c_int(0)
+            torch.cuda.synchronize()
+            st = lib.vb_generalized_eigh(c.handle, *(ctypes.c_void_p(t.data_ptr()) for t in (Hd, Sd)), n,
+                                         vbcore.VB_MEM_DEVICE, ctypes.c_void_p(w.data_ptr()),
+                                         ctypes.c_void_p(Hd.data_ptr()), ctypes.byref(info))
+            if spoilt:
+                assert st == 6 and np.array_equal(Hd.cpu().numpy(), before, equal_nan=True)
+            else:
+                assert st == 0 and np.array_equal(w.cpu().numpy(), wr)
+                assert np.array_equal(Hd.cpu().numpy().T, Cr)
+    finally:
+        c.close()

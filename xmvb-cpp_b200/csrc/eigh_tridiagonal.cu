@@ -60,12 +60,14 @@ __device__ __forceinline__ void halve(double (&p)[kCols], bool up, int o) {
 //   2: G = X^T X          (likewise); status bit 1 when |G - I| > 0.1 somewhere
 //   3: Y = X (3 I - G) / 2
 //   4: C = Ui Y
+// 3 and 4 only when everything is settled: C may lie over H or S, which Jacobi then still needs.
 template <int MODE>
 __global__ void __launch_bounds__(32) td_product(int n, const double* __restrict__ A, const double* __restrict__ B,
                                                  double* __restrict__ C, int* __restrict__ status) {
     const int lane = threadIdx.x, gr = lane >> 2, gc = lane & 3;
     const int r0 = 16 * blockIdx.x, c0 = 16 * blockIdx.y;
     constexpr bool kMirror = MODE == 1 || MODE == 2;
+    if (MODE >= 3 && *status != 0) return;
     if (kMirror && r0 > c0) return;
     const long long ld = n;
     auto a_elem = [&](int r, int k) -> double {

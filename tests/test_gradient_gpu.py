@@ -289,3 +289,31 @@ def test_gradient_of_nearly_dependent_orbitals(ctx, kw, n, nel, mult, separation
         err = float(np.abs(got[key] - ref[key]).max() / np.abs(ref[key]).max())
         assert err < 5e-14 + 2.2e-16 * kappa2 / 256, (key, kappa2, err)
     plan.close()
+
+
+@pytest.mark.parametrize("n,mult,budget_mb", [(10, 1, 45), (10, 3, 70)])
+def test_gradient_of_nearly_dependent_orbitals_in_a_small_budget(n, mult, budget_mb):
+    """The pair-by-pair form of the ill-conditioned strings in as many chunks as the budget leaves room for
+    (50 and 80 MB hold one)."""
+    kw, nel = "COV", n
+    S = _nearly_dependent(n, 0.03, n)
+    rng = np.random.default_rng(n)
+    h = _sym(rng, n)
+    P = n * (n + 1) // 2
+    F = 0.05 * rng.standard_normal((P, P)) + 0.1 * np.eye(P)
+    eri = workloads.pack_pair_kernel(F @ F.T)
+    ex = vbcore.expand_structures(vbcore.generate_structures(kw, n, nel, mult), nel, mult)
+    c = rng.standard_normal(ex.n_structures)
+    c /= np.linalg.norm(c)
+    got = []
+    for budget in (0, budget_mb << 20):
+        own = vbcore.Context(0, budget) if budget else vbcore.Context(0)
+        try:
+            plan = vbcore.HsPlan(own, ex, n)
+            got.append(plan.gradient(S, h, eri, c, -1.3, packed_eri=False, ri_factors=F))
+            plan.close()
+        finally:
+            own.close()
+    # the sums over pairs are atomic: their order differs
+    for key in ("S", "h", "ri"):
+        assert np.abs(got[0][key] - got[1][key]).max() < 1e-10 * np.abs(got[0][key]).max(), key

@@ -1166,15 +1166,22 @@ extern "C" vb_status vb_hs_plan_gradient(vb_hs_plan* p, const double* S, const d
                     tot += std::min<long long>(kSpinBlock, NN - v0);
                 }
             rec_off.push_back(tot);
-            const long long cap = std::max<long long>(kSpinBlock, ((long long)256 << 20) / (8LL * np));
             DeviceBuffer ditems, drows, qbuf, pbuf, abuf;
             vb_status pst = upload(ctx, ditems, items.data(), sizeof(int2) * items.size());
-            const long long rows_max = std::min<long long>(cap + kSpinBlock, tot);
             if (pst == VB_OK) pst = upload(ctx, drows, rec_off.data(), sizeof(long long) * rec_off.size());
-            if (pst == VB_OK) pst = qbuf.allocate(ctx, sizeof(double) * (size_t)np * rows_max);
-            if (pst == VB_OK) pst = pbuf.allocate(ctx, sizeof(double) * (size_t)np * rows_max);
-            if (pst == VB_OK && strings) pst = abuf.allocate(ctx, sizeof(double) * (size_t)adj_stride * rows_max);
             if (pst != VB_OK) return pst;
+            // chunk buffers of 256 MB each, or less where the budget has no room for them
+            long long cap = std::max<long long>(kSpinBlock, ((long long)256 << 20) / (8LL * np));
+            for (;; cap = std::max<long long>(kSpinBlock, cap / 4)) {
+                const long long rows_max = std::min<long long>(cap + kSpinBlock, tot);
+                pst = qbuf.allocate(ctx, sizeof(double) * (size_t)np * rows_max);
+                if (pst == VB_OK) pst = pbuf.allocate(ctx, sizeof(double) * (size_t)np * rows_max);
+                if (pst == VB_OK && strings) pst = abuf.allocate(ctx, sizeof(double) * (size_t)adj_stride * rows_max);
+                if (pst == VB_OK) break;
+                if (pst != VB_ERR_BUDGET || cap == kSpinBlock) return pst;
+                qbuf.release();
+                pbuf.release();
+            }
             BackArgs c = b;
             c.items = ditems.as<int2>();
             c.item_row = drows.as<long long>();

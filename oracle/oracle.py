@@ -843,13 +843,26 @@ def _batched_inverse(X):
     return det.reshape(lead), A[:, :, k:].reshape(X.shape)
 
 
-def functional_gradient(n, expansion, S, h, F, c, root):
+def functional_gradient(n, expansion, S, h, F, c, root, digits=0):
     """Gradients of c^T (H - root S) c, at fixed c and root, with respect to S, h (symmetric) and the pair
     factors F of the packed pair kernel K = F F^T: every block inverted by itself, in the platform's extended
-    precision (64-bit significands here).  Regular blocks only.  Formulas of the active-space backward files
+    precision (64-bit significands here) or, for blocks of any condition number, with `digits` decimal digits.
+    Regular blocks only.  Formulas of the active-space backward files
     (src/vbscf/derivatives/gradient/active_space/evaluator.cpp:1046-1133)."""
-    real = np.longdouble
-    S, h, F, c = (np.asarray(x, dtype=real) for x in (S, h, F, c))
+    if digits:
+        import mpmath
+
+        mpmath.mp.dps = digits
+        real, number = object, mpmath.mpf
+    else:
+        real = number = np.longdouble
+
+    def convert(x):
+        x = np.asarray(x, dtype=np.float64)
+        return np.array([number(float(v)) for v in x.reshape(-1)], dtype=real).reshape(x.shape)
+
+    S, h, F, c = (convert(x) for x in (S, h, F, c))
+    root = number(float(root))
     pair = np.array([[pair_index(i, j) for j in range(n)] for i in range(n)]).reshape(-1)
     K = (F @ F.T)[pair][:, pair]  # (ij|kl) as [n n, n n]
     exchange = K.reshape(n, n, n, n).transpose(0, 3, 2, 1).reshape(n * n, n * n)
@@ -871,14 +884,14 @@ def functional_gradient(n, expansion, S, h, F, c, root):
 
     ta, tb = table(expansion.alpha_strings), table(expansion.beta_strings)
     W = np.zeros((len(ta[0]), len(tb[0])), dtype=real)
-    np.add.at(W, (expansion.det_alpha, expansion.det_beta), expansion.coefficient_matrix().astype(real) @ c)
+    np.add.at(W, (expansion.det_alpha, expansion.det_beta), convert(expansion.coefficient_matrix()) @ c)
     gS, gh = np.zeros((n, n), dtype=real), np.zeros(n * n, dtype=real)
     gK = np.zeros((n * n, n * n), dtype=real)
     for own, other, w, first in ((ta, tb, W, True), (tb, ta, W.T, False)):
         occ, det, inv, G, energy = own
         N, k = occ.shape
         aH = w @ other[1] @ w.T
-        aS = w @ (other[1] * other[4]) @ w.T - real(root) * aH
+        aS = w @ (other[1] * other[4]) @ w.T - root * aH
         aA = (w @ (other[1][..., None] * other[3]).transpose(2, 0, 1) @ w.T).transpose(1, 2, 0)
         if first:  # the opposite-spin energy holds K once
             gK += np.einsum("uvp,uvq->pq", det[..., None] * G, aA)
@@ -896,4 +909,5 @@ def functional_gradient(n, expansion, S, h, F, c, root):
     gP = np.zeros((n * (n + 1) // 2,) * 2, dtype=real)
     np.add.at(gP, (pair[:, None], pair[None, :]), gK)
     gh = gh.reshape(n, n)
-    return {"S": (gS + gS.T) / 2, "h": (gh + gh.T) / 2, "ri": (gP + gP.T) @ F}
+    out = {"S": (gS + gS.T) / 2, "h": (gh + gh.T) / 2, "ri": (gP + gP.T) @ F}
+    return {k: v.astype(np.float64) for k, v in out.items()} if digits else out

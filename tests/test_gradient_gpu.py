@@ -264,10 +264,9 @@ def _nearly_dependent(n, separation, seed):
 @pytest.mark.parametrize("separation", [0.3, 0.1, 0.03, 0.01, 3e-3, 1e-3])
 def test_gradient_of_nearly_dependent_orbitals(ctx, kw, n, nel, mult, separation):
     """Two nearly dependent orbitals: strings that hold both have an ill-conditioned S_LL (kappa up to 4e6).
-    Against every block inverted by itself in extended precision.  Bound: a block's 64-bit inverse enters its
-    derivative twice, against det X of order 1 / kappa, and leaves up to kappa^2 eps / 600 here (measured),
-    so kappa^2 eps / 256; the frame of such a string would leave kappa^2 eps / 50 and more.  5e-14 for what
-    does not depend on the dependent pair."""
+    Against every block inverted by itself in extended precision.  Bound: the inputs themselves are known to
+    kappa eps of the gradient, four times that; 5e-14 for pairs that take their own inverse
+    (kappa(X)^2 < 1e6, kappa^2 eps / 500 of it).  The frame of such a string would leave kappa^2 eps / 50 and more."""
     S = _nearly_dependent(n, separation, n)
     rng = np.random.default_rng(n)
     h = _sym(rng, n)
@@ -287,14 +286,47 @@ def test_gradient_of_nearly_dependent_orbitals(ctx, kw, n, nel, mult, separation
     got = plan.gradient(S, h, eri, c, -1.3, packed_eri=False, ri_factors=F)
     for key in ("S", "h", "ri"):
         err = float(np.abs(got[key] - ref[key]).max() / np.abs(ref[key]).max())
-        assert err < 5e-14 + 2.2e-16 * kappa2 / 256, (key, kappa2, err)
+        assert err < 5e-14 + 4 * 2.2e-16 * kappa2 ** 0.5, (key, kappa2, err)
     plan.close()
 
 
-@pytest.mark.parametrize("n,mult,budget_mb", [(10, 1, 45), (10, 3, 70)])
+@pytest.mark.parametrize("kw,n,nel,mult", [("COV", 4, 4, 1), ("COV", 5, 5, 2), ("COV ION(1)", 5, 4, 1)])
+@pytest.mark.parametrize("rate", [1.0, 3.0])
+@pytest.mark.parametrize("separation", [1.0, 0.1, 0.01])
+def test_gradient_of_graded_and_nearly_dependent_orbitals(ctx, kw, n, nel, mult, rate, separation):
+    """Overlaps exp(-rate |i - j|^2) (down to 1e-33), the second orbital close to the first one: blocks that are
+    tiny, ill conditioned or both, of strings in and outside the frame form.  Against blocks inverted one by one
+    with 100 digits; same bound (a block's own inverse up to the forward value's certificate would leave
+    2e-8)."""
+    dist = np.abs(np.subtract.outer(np.arange(n), np.arange(n))).astype(float)
+    C = np.eye(n)
+    C[:, 1] = (C[:, 0] if separation < 1.0 else 0.0) + separation * C[:, 1]
+    S = C.T @ np.exp(-rate * dist ** 2) @ C
+    d = 1.0 / np.sqrt(np.diag(S))
+    S = d[:, None] * S * d[None, :]
+    S = 0.5 * (S + S.T)
+    rng = np.random.default_rng(n)
+    h = _sym(rng, n)
+    P = n * (n + 1) // 2
+    F = 0.05 * rng.standard_normal((P, P)) + 0.1 * np.eye(P)
+    eri = workloads.pack_pair_kernel(F @ F.T)
+    plan = vbcore.HsPlan(ctx, vbcore.expand_structures(vbcore.generate_structures(kw, n, nel, mult), nel, mult), n)
+    ex = O.expand(O.generate_structures(kw, n, nel, mult), nel, mult)
+    c = rng.standard_normal(plan.n_structures)
+    c /= np.linalg.norm(c)
+    ref = O.functional_gradient(n, ex, S, h, F, c, -1.3, digits=100)
+    got = plan.gradient(S, h, eri, c, -1.3, packed_eri=False, ri_factors=F)
+    kappa = np.linalg.cond(S)
+    for key in ("S", "h", "ri"):
+        err = np.abs(got[key] - ref[key]).max() / np.abs(ref[key]).max()
+        assert err < 5e-14 + 4 * 2.2e-16 * kappa, (key, kappa, err)
+    plan.close()
+
+
+@pytest.mark.parametrize("n,mult,budget_mb", [(10, 1, 50), (10, 3, 70)])
 def test_gradient_of_nearly_dependent_orbitals_in_a_small_budget(n, mult, budget_mb):
     """The pair-by-pair form of the ill-conditioned strings in as many chunks as the budget leaves room for
-    (50 and 80 MB hold one)."""
+    (70 and 100 MB hold one)."""
     kw, nel = "COV", n
     S = _nearly_dependent(n, 0.03, n)
     rng = np.random.default_rng(n)

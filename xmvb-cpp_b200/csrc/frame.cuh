@@ -13,8 +13,8 @@ namespace vbcore {
 // The (hole position x particle) grid and the 8-bit particle masks hold up to eight complement
 // orbitals.  A block is laid out for fr_nbmin(K) of them (a closed shell's n - K = K fits) or, for
 // more, for all eight: an open shell's minority spin has n - K > K.  On the exact path the 5
-// beta electrons of a 12-orbital triplet took 1895 us of the evaluation's 2290 us; here the
-// whole evaluation takes 528 us.
+// beta electrons of a 12-orbital triplet took 1895 us of the evaluation's 2290 us; with frame tables for
+// them the whole evaluation takes 528 us from records and 366 us through covalent_pairs.cu.
 constexpr int kFrameMaxComplement = 8;
 __host__ __device__ constexpr int fr_nbmin(int K) { return K <= 4 ? K + 4 : K; }
 __host__ __device__ constexpr bool fr_wide(int n, int K) { return n - K > fr_nbmin(K); }
@@ -123,8 +123,14 @@ __device__ __forceinline__ bool frame_certificate(const View& f, const int (&hc)
 //   against 5e-13, 2e9: 4e-9 against 9e-11.
 // Hydrogen chains stay below 2.3e3 (14 atoms 0.7 A apart) and near-orthogonal orbitals below 60.
 constexpr double kFrameCondition2 = 1.0e4;
-// Strings from here on have all their pairs differentiated through singular values: the blocks' own
-// inverses lose 1e-7 of the gradient there.
+// Pairs of the other strings take their own inverses below this kappa_F(X)^2, which lose kappa(X)^2 eps /
+// 500 (1e-13 at worst), and singular values above, which lose kappa(S_LL) eps: 4e-12 instead of 9e-11 at
+// kappa(S_LL)^2 = 2e9, and 3e-14 instead of 2e-8 for graded overlaps of which two are nearly dependent.
+// Singular values take 58 ns a pair at seven electrons, four times an inverse (3432 strings, of which a
+// quarter holds the dependent orbitals, kappa^2 = 2e5 to 2e9: 68 to 96 ms per gradient, 47 to 51 with
+// inverses up to the certificate of the forward value, 134 with inverses for all strings).
+constexpr double kOwnInverseCondition2 = 1.0e6;
+// Strings from here on have all their pairs differentiated through singular values.
 constexpr double kSingularCondition2 = 1.0e12;
 
 __host__ __device__ constexpr int pair_slot(int x, int y) { return x < y ? y * (y - 1) / 2 + x : x * (x - 1) / 2 + y; }

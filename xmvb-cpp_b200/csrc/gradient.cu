@@ -42,6 +42,7 @@
 #include <vector>
 
 #include "device_algebra.cuh"
+#include "frame.cuh"
 #include "frame_adjoint.h"
 #include "internal.h"
 #include "kernels.h"
@@ -330,6 +331,7 @@ struct BackArgs {
     double* gL;  // [pair q * ld + m]
     unsigned long long* careful_count;
     unsigned long long* careful_list;
+    double certificate2;  // spin_backward_kernel lists blocks with kappa_F(X)^2 above this
     // chunked fast path: items [item_begin, item_end), item i with the rows item_row[i] - row_base, ...
     const int2* items;
     const long long* item_row;
@@ -458,7 +460,7 @@ __global__ void __launch_bounds__(128) spin_backward_kernel(BackArgs a) {
         for (int r = 0; r < K; ++r)
 #pragma unroll
             for (int c = 0; c < K; ++c) ni2 = fma(x[r][c], x[r][c], ni2);
-        if (!(isfinite(det) && det != 0.0 && nx2 * ni2 < kCertificate2)) {
+        if (!(isfinite(det) && det != 0.0 && nx2 * ni2 < a.certificate2)) {
             const unsigned long long slot = atomicAdd(a.careful_count, 1ull);
             a.careful_list[slot] = ((unsigned long long)u << 32) | (unsigned long long)v;
             continue;
@@ -880,21 +882,23 @@ vb_status careful_chunks(vb_context* ctx, BackArgs b, long long count, int all_p
     if (count <= 0) return VB_OK;
     cudaStream_t s = ctx->stream;
     const int np = b.ld, R = b.R;
-    // chunk buffers: up to 768 MB, at most half of what the context budget has left
-    const size_t left = ctx->budget > ctx->current ? ctx->budget - ctx->current : 0;
-    const size_t target = std::max<size_t>((size_t)16 << 20, std::min<size_t>((size_t)768 << 20, left / 2));
-    const long long chunk = std::min<long long>(
-        count, std::max<long long>(1024, (long long)(target / (8ULL * (2 * np + R + 1)))));
+    auto left = [&] { return ctx->budget > ctx->current ? ctx->budget - ctx->current : (size_t)0; };
     // per-block slots (two-electron table, S and h adjoints), summed once after the last chunk
     const size_t slot_bytes = sizeof(double) * ((size_t)b.gd * b.gd + 2 * (size_t)b.n * b.n);
     auto kernel = b.k == 7 ? careful_backward_kernel<7, 7>
                            : (b.k <= 8 ? careful_backward_kernel<8, 0> : careful_backward_kernel<dev::KMAX, 0>);
     int per_sm = 4;
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, 128, 0) != cudaSuccess || per_sm < 1) per_sm = 4;
-    const int grid = 148 * std::min(per_sm, 8);  // one wave of resident blocks
+    int grid = 148 * std::min(per_sm, 8);  // one wave of resident blocks, fewer in a tight budget
+    while (grid > 1 && slot_bytes * grid > left() / 2) grid /= 2;
     DeviceBuffer acb, qb, pb, slots;
     vb_status st;
     if ((st = slots.allocate(ctx, slot_bytes * grid)) != VB_OK) return st;
+    // chunk buffers: up to 768 MB, at most half of what the context budget has left, or up to 16 MB of the
+    // last of it
+    const size_t target = std::min<size_t>((size_t)768 << 20, std::max<size_t>(left() / 2, std::min<size_t>((size_t)16 << 20, left() / 8 * 7)));
+    const long long chunk = std::min<long long>(
+        count, std::max<long long>(128, (long long)(target / (8ULL * (2 * np + R + 1)))));
     if (cudaMemsetAsync(slots.ptr, 0, slot_bytes * grid, s) != cudaSuccess)
         return set_error(ctx, VB_ERR_CUDA, "vb_hs_plan_gradient: memset failed");
     if ((st = acb.allocate(ctx, sizeof(double) * (size_t)chunk * std::max(R, 1))) != VB_OK) return st;
@@ -1183,6 +1187,7 @@ extern "C" vb_status vb_hs_plan_gradient(vb_hs_plan* p, const double* S, const d
                 pbuf.release();
             }
             BackArgs c = b;
+            c.certificate2 = strings ? kOwnInverseCondition2 : kCertificate2;
             c.items = ditems.as<int2>();
             c.item_row = drows.as<long long>();
             c.Q = qbuf.as<double>();

@@ -132,7 +132,9 @@ vb_status vb_hs_plan_destroy(vb_hs_plan* plan);
 /* Evaluate H and S (n_structures^2 each, column-major, symmetric).  Inputs: active overlap
  * S_act (n x n), one-electron h (n x n), packed (ij|kl) of length P(P+1)/2 with
  * P = n(n+1)/2.  mem_space says where all five pointers live.  Stream-ordered; with
- * VB_MEM_HOST the call returns after the results are on the host. */
+ * VB_MEM_HOST the call returns after the results are on the host.  A determinant pair that is not
+ * finite reaches the structures that use it and, where the structure reduction works on dense groups
+ * (covalent + ionic lists), up to 47 others that share determinants with them. */
 vb_status vb_hs_plan_execute(vb_hs_plan* plan, const double* ovlp_act, const double* h1e_act,
                              const double* eri_packed, int mem_space, double* hamiltonian_out,
                              double* overlap_out);

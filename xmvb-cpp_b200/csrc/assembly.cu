@@ -239,7 +239,9 @@ __global__ void __launch_bounds__(kBandWarps * 32, 3)
 // The tensor cores' share is 3.2 ms (216 M products for 34,188 determinants); takes 8.1 ms there
 // (8.3 ms with a second barrier per tile before Z is written), one CTA of 12 warps per SM.  The tiled form above takes 36.7 ms on such a list, and
 // 10.1 ms with 64-row tiles gathered from each group's own rows: one shared-memory load per nonzero and
-// column and 25 instructions around it.
+// column and 25 instructions around it.  14 orbitals (171,600 determinants; 64 a structure, so that eight
+// structures fill a group): 542 ms, against 613 ms tiled in the first-structure order.  T's zeros are
+// multiplied: a determinant pair that is not finite reaches every structure of the groups that hold it.
 constexpr int kDenseWarps = 12;    // 6 structure tiles x 2 column halves
 constexpr int kDenseColumns = 16;
 constexpr int kDenseLd = 2 * kDenseColumns + 4;  // 4 mod 16: fragment loads without bank conflicts

@@ -19,10 +19,11 @@
 // evaluates the other side and combines them.  (Both records in the exact path, 14 orbitals of which two
 // are nearly dependent: 520,853 of them in 8.7 ms, against 291,373 and 6.2 ms for the records alone.)
 //
-// 14 orbitals, 2.9 M orbits: 1361 us (1428 us with a test per row tile in the product), against 1280 us for the records and 537 us for the pairs gathered
-// from them; 12-orbital triplet: 160 us, against 235 us.  Bound by instruction issue (50 %) and the FP64
-// tensor cores (45 %): one CTA of up to 16 warps per SM, the two blocks and the warps' adj B slots in
-// shared memory.
+// 14 orbitals, 2.9 M orbits: 1361 us (1428 us with a test per row tile in the product), against 1280 us for
+// the records and 537 us for the pairs gathered from them; 12-orbital triplet: 160 us, against 235 us.
+// Bound by latency: one CTA of up to 16 warps per SM (two blocks and the warps' adj B slots in shared
+// memory, 128 registers a thread) waits on fixed latencies and on the tensor pipe, and saturates neither the
+// issue slots (45 %) nor the FP64 tensor pipe (37 % active).
 #include <cuda_runtime.h>
 #include <stdint.h>
 

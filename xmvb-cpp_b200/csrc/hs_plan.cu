@@ -760,7 +760,9 @@ vb_status execute_impl(vb_hs_plan* p, const double* S, const double* h, const do
     vb_status st = prepare_frame_tables(p, S, h, eri, mem, &dS, &dh, &deri, &launches);
     if (st != VB_OK) return st;
     // Covalent lists go from the frame tables straight to the determinant pairs, unless a gradient that
-    // reads the records follows.
+    // reads the records follows.  One band only (up to 8191 determinants under a budget of 8 GB or more): a
+    // left string's pairs and their spin flips lie anywhere in the triangle, so that every band would walk
+    // all pairs again.
     const bool covalent = !keep_records && p->covalent.list.ptr && p->bands.size() == 2 &&
                           covalent_pairs_supported(p->n, p->ka, p->kb, p->R);
     if (!covalent && (st = evaluate_spin_records(p, dS, dh, deri, &launches)) != VB_OK) return st;

@@ -23,7 +23,7 @@
 // the records and 537 us for the pairs gathered from them; 12-orbital triplet: 160 us, against 235 us.
 // Bound by latency: one CTA of up to 16 warps per SM (two blocks and the warps' adj B slots in shared
 // memory, 128 registers a thread) waits on fixed latencies and on the tensor pipe, and saturates neither the
-// issue slots (45 %) nor the FP64 tensor pipe (37 % active).
+// issue slots (42 %) nor the FP64 tensor pipe (37 % active).
 #include <cuda_runtime.h>
 #include <stdint.h>
 
